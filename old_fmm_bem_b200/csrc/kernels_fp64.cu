@@ -1,4 +1,5 @@
-// FP64 evaluation kernels: the plain-FP64 form of every FMM phase, and the
+// FP64 evaluation kernels: the plain-FP64 form of every FMM phase but the near
+// field (p2p_f64.cu), and the
 // P2M/M2M/L2L/L2P phases of the mixed-precision form (they are a few percent
 // of the work, so they stay FP64 there too).
 //
@@ -36,107 +37,6 @@ __global__ void gather_charges(int n, int nrhs, const int* perm, const float* q,
   if (i >= n) return;
   const int o = perm[i];
   for (int r = 0; r < nrhs; r++) qs[(size_t)r * n + i] = q[(size_t)r * n + o];
-}
-
-// ---------------------------------------------------------------- P2P (FP64)
-// kernel/G_p2p.cxx:12-37, Gni_p2p.cxx:12-28, Gnj_p2p.cxx:12-28: one block per
-// work item (up to 128 targets of a target leaf), its 27 neighbour slots
-// staged through shared memory.
-constexpr int kP2PThreads = 128;
-
-template <int KER>
-__global__ void __launch_bounds__(kP2PThreads) p2p_f64(const int2* __restrict__ work, const int2* __restrict__ leaf_i,
-                                                       const int2* __restrict__ leaf_j,
-                                                       const int* __restrict__ list, const float4* __restrict__ tpos,
-                                                       const float4* __restrict__ tnrm, const float4* __restrict__ spos,
-                                                       const float4* __restrict__ snrm, const float* __restrict__ qs,
-                                                       Sem s, double* __restrict__ pot, double* __restrict__ grad,
-                                                       int ni) {
-  __shared__ float4 sp[kP2PThreads];
-  __shared__ float4 sn[kP2PThreads];
-  __shared__ float sq[kP2PThreads];
-  const int2 wk = work[blockIdx.x];
-  const int b = wk.x;
-  int2 li = leaf_i[b];
-  li.x += wk.y;
-  li.y = min(kP2PThreads, li.y - wk.y);
-  for (int t0 = 0; t0 < li.y; t0 += kP2PThreads) {
-    const int i = li.x + t0 + threadIdx.x;
-    const bool act = (t0 + threadIdx.x) < li.y;
-    float4 xi = act ? tpos[i] : make_float4(0, 0, 0, 0);
-    float4 ni4 = (KER == FMMB_LAPLACE_GNI && act) ? tnrm[i] : make_float4(0, 0, 0, 0);
-    double p = 0, fx = 0, fy = 0, fz = 0;
-    for (int slot = 0; slot < kP2PSlots; slot++) {
-      const int jl = list[(size_t)b * kP2PSlots + slot];
-      if (jl < 0) continue;
-      const int2 lj = leaf_j[jl];
-      for (int j0 = 0; j0 < lj.y; j0 += kP2PThreads) {
-        const int nld = min(kP2PThreads, lj.y - j0);
-        __syncthreads();
-        if (threadIdx.x < nld) {
-          const int j = lj.x + j0 + threadIdx.x;
-          sp[threadIdx.x] = spos[j];
-          sq[threadIdx.x] = qs[j];
-          if (KER == FMMB_LAPLACE_GNJ) sn[threadIdx.x] = snrm[j];
-        }
-        __syncthreads();
-        for (int jj = 0; jj < nld; jj++) {
-          const float4 xj = sp[jj];
-          double dx, dy, dz;
-          if (s.ref) {  // float differences, as the reference (kernel/G_p2p.cxx:21-23)
-            dx = (double)__fsub_rn(xi.x, xj.x);
-            dy = (double)__fsub_rn(xi.y, xj.y);
-            dz = (double)__fsub_rn(xi.z, xj.z);
-          } else {
-            dx = (double)xi.x - (double)xj.x;
-            dy = (double)xi.y - (double)xj.y;
-            dz = (double)xi.z - (double)xj.z;
-          }
-          if (s.excl_self && dx == 0.0 && dy == 0.0 && dz == 0.0) continue;
-          const double r2 = dx * dx + dy * dy + dz * dz + s.eps2;
-          const double rinv = 1.0 / sqrt(r2);
-          const double qr = s.coef * (double)sq[jj] * rinv;
-          if (KER == FMMB_LAPLACE_G) {
-            const double qr3 = qr * rinv * rinv;
-            p += qr;
-            fx -= dx * qr3;
-            fy -= dy * qr3;
-            fz -= dz * qr3;
-          } else {
-            // Gni: n = the target's normal; Gnj: the source's.  With a gradient
-            // (accurate semantics): d/dx_i of q (d.n) / r^3 = q n / r^3 - 3 q (d.n) d / r^5
-            double nx, ny, nz;
-            if (KER == FMMB_LAPLACE_GNI) {
-              nx = ni4.x;
-              ny = ni4.y;
-              nz = ni4.z;
-            } else {
-              const float4 nj = sn[jj];
-              nx = nj.x;
-              ny = nj.y;
-              nz = nj.z;
-            }
-            const double qr3 = qr * rinv * rinv, dot = dx * nx + dy * ny + dz * nz;
-            p += dot * qr * rinv * rinv;  // the potential's operation order as without the gradient
-            if (grad) {
-              const double c = -3.0 * dot * qr3 * rinv * rinv;
-              fx += qr3 * nx + c * dx;
-              fy += qr3 * ny + c * dy;
-              fz += qr3 * nz + c * dz;
-            }
-          }
-        }
-      }
-    }
-    if (act) {
-      pot[i] = p;
-      if (grad) {
-        grad[i] = fx;
-        grad[ni + i] = fy;
-        grad[2 * ni + i] = fz;
-      }
-    }
-  }
 }
 
 // ---------------------------------------------------------------- P2M
@@ -525,22 +425,6 @@ __global__ void __launch_bounds__(128) direct_f64(int i0, int i1, const int* __r
 // ---------------------------------------------------------------- launchers
 void launch_gather_charges(int n, int nrhs, const int* perm, const float* q, float* qs, cudaStream_t st) {
   gather_charges<<<nblk(n, 256), 256, 0, st>>>(n, nrhs, perm, q, qs);
-  FMMB_CHECK_LAUNCH();
-}
-
-void launch_p2p_f64(int kernel, int nwork, const int2* work, const int2* leaf_i, const int2* leaf_j, const int* list,
-                    const float4* tpos, const float4* tnrm, const float4* spos, const float4* snrm, const float* qs,
-                    const Sem& s, double* pot, double* grad, int ni, cudaStream_t st) {
-  if (nwork <= 0) return;
-  if (kernel == FMMB_LAPLACE_G)
-    p2p_f64<FMMB_LAPLACE_G><<<nwork, kP2PThreads, 0, st>>>(work, leaf_i, leaf_j, list, tpos, tnrm, spos, snrm, qs, s,
-                                                           pot, grad, ni);
-  else if (kernel == FMMB_LAPLACE_GNI)
-    p2p_f64<FMMB_LAPLACE_GNI><<<nwork, kP2PThreads, 0, st>>>(work, leaf_i, leaf_j, list, tpos, tnrm, spos, snrm, qs, s,
-                                                             pot, grad, ni);
-  else
-    p2p_f64<FMMB_LAPLACE_GNJ><<<nwork, kP2PThreads, 0, st>>>(work, leaf_i, leaf_j, list, tpos, tnrm, spos, snrm, qs, s,
-                                                             pot, grad, ni);
   FMMB_CHECK_LAUNCH();
 }
 

@@ -35,10 +35,9 @@
 // two shuffles, the warps of a team through shared memory.
 #include <cuda_runtime.h>
 
-#include <climits>
-
 #include "internal.h"
 #include "kernels.h"
+#include "p2p_list.cuh"
 
 namespace fmmb {
 namespace {
@@ -49,10 +48,7 @@ constexpr int kG = 8;          // targets of a group (lanes g = lane % 8)
 constexpr int kS = 32 / kG;    // source streams of a warp (s = lane / 8)
 constexpr int kMaxNT = 4;      // groups of a tile
 constexpr int kCap = 1024;     // staged sources per chunk (multiple of 32 * 4)
-constexpr int kSelfSlot = 13;  // offset (0, 0, 0) in the 27-slot list
 constexpr float kFar = 1e18f;  // padding sources: r^2 ~ 3e36 stays finite in FP32
-
-__device__ __forceinline__ int pad32(int n) { return (n + 31) & ~31; }
 
 // 1/sqrt(x) from the hardware approximation, subnormal inputs flushed to zero
 // (r^2 is either 0 -- coincident points, handled by the caller -- or far
@@ -97,8 +93,7 @@ struct Smem {
   float4 BQ[NP];                                      // (-z j, j+1, q j, j+1) or (-z j, j+1, qn_z j, j+1)
   float4 M[base(KER) == FMMB_LAPLACE_GNJ ? NP : 1];   // (qn_x j, j+1, qn_y j, j+1)
   double red[kWarps][kMaxNT][NC][kG];           // team partial sums
-  int2 seg[32];                                 // (first source, count), own leaf first
-  int vst[32];                                  // virtual start of each segment, then INT_MAX
+  SrcList src;                                  // the item's source list
 };
 
 struct Tgt {
@@ -172,17 +167,6 @@ __device__ __forceinline__ void run16(const Smem<KER>& S, int pb, const Tgt (&tg
 // packed pairs: each thread locates four sources (two pairs; binary search
 // over the segment starts), issues their loads, then stores them.
 template <int KER>
-__device__ __forceinline__ int locate(const Smem<KER>& S, int v, int c1) {
-  int sgi = 0;
-#pragma unroll
-  for (int st = 16; st > 0; st >>= 1)
-    if (S.vst[sgi + st] <= v) sgi += st;
-  const int2 sg = S.seg[sgi];
-  const int off = v - S.vst[sgi];
-  return (v < c1 && off < sg.y) ? sg.x + off : -1;
-}
-
-template <int KER>
 __device__ void stage(Smem<KER>& S, int c0, int c1, const float4* __restrict__ spos,
                       const float4* __restrict__ snrm, const float* __restrict__ qs) {
   __syncthreads();  // the previous chunk's readers are done
@@ -190,7 +174,7 @@ __device__ void stage(Smem<KER>& S, int c0, int c1, const float4* __restrict__ s
   for (int pb = threadIdx.x; pb < np; pb += 2 * kThreads) {
     int jj[4];
 #pragma unroll
-    for (int u = 0; u < 4; u++) jj[u] = locate(S, c0 + 2 * (pb + (u >> 1) * kThreads) + (u & 1), c1);
+    for (int u = 0; u < 4; u++) jj[u] = S.src.locate(c0 + 2 * (pb + (u >> 1) * kThreads) + (u & 1), c1);
     float4 x[4], n[4];
     float q[4];
 #pragma unroll
@@ -271,43 +255,10 @@ __global__ void __launch_bounds__(kThreads) p2p_mixed(const int2* __restrict__ w
   li.x += wk.y;
   li.y = min(kThreads, li.y - wk.y);
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, g = lane & (kG - 1), s = lane / kG;
-  // segment list: lane l of warp 0 reads neighbour slot l; the own leaf goes
-  // first, the non-empty others after it in slot order
-  if (warp == 0) {
-    int2 sg = make_int2(0, 0);
-    if (lane < kP2PSlots) {
-      const int jl = list[(size_t)b * kP2PSlots + lane];
-      if (jl >= 0) sg = leaf_j[jl];
-    }
-    const int self_end = pad32(__shfl_sync(0xffffffffu, sg.y, kSelfSlot));
-    const bool oth = lane != kSelfSlot && sg.y > 0;
-    const unsigned mask = __ballot_sync(0xffffffffu, oth);
-    const int pos = 1 + __popc(mask & ((1u << lane) - 1u));
-    const int cnt = oth ? sg.y : 0;
-    int incl = cnt;
-#pragma unroll
-    for (int o = 1; o < 32; o <<= 1) {
-      const int t = __shfl_up_sync(0xffffffffu, incl, o);
-      if (lane >= o) incl += t;
-    }
-    const int nseg = 1 + __popc(mask);
-    if (lane == kSelfSlot) {
-      S.seg[0] = sg;
-      S.vst[0] = 0;
-    }
-    if (oth) {
-      S.seg[pos] = sg;
-      S.vst[pos] = self_end + incl - cnt;
-    }
-    if (lane >= nseg) S.vst[lane] = INT_MAX;
-    const int n_other = __shfl_sync(0xffffffffu, incl, 31);
-    if (lane == 0) S.seg[31] = make_int2(0, n_other);  // slot 31 is never a segment: it holds n_other
-  }
+  if (warp == 0) S.src.build(b, list, leaf_j, lane);
   __syncthreads();
-  const int own = S.seg[0].y;
-  const int self_end = pad32(own);
-  const int n_other = S.seg[31].y;
-  const int vlen = self_end + pad32(n_other);
+  const int self_end = S.src.self_end();
+  const int vlen = S.src.length();
   const int nchunk = (vlen + kCap - 1) / kCap;
   // teams of m warps share a tile and split its runs
   const int ng = (li.y + kG - 1) / kG;
