@@ -106,7 +106,15 @@ void upload_static_ops(fmmb_plan* pl) {
   FMMB_CUDA(cudaMemcpyAsync(pl->d_slot_rel.get(), o.slot_rel.data(), o.slot_rel.size() * sizeof(int), cudaMemcpyHostToDevice, s));
   pl->d_rel_to_op.alloc(o.rel_to_op.size());
   FMMB_CUDA(cudaMemcpyAsync(pl->d_rel_to_op.get(), o.rel_to_op.data(), o.rel_to_op.size() * sizeof(int), cudaMemcpyHostToDevice, s));
-  FMMB_CUDA(cudaStreamSynchronize(s));
+  pl->d_rel_to_cls.alloc(o.rel_to_cls.size());
+  FMMB_CUDA(cudaMemcpyAsync(pl->d_rel_to_cls.get(), o.rel_to_cls.data(), o.rel_to_cls.size() * sizeof(int), cudaMemcpyHostToDevice, s));
+  upload(pl->d_phi, o.phi, s);
+}
+
+// FP64 M2L (m2l_parity.cu): the plain-FP64 form, the orders above the
+// tensor-core M2L's range, and the Helmholtz family
+bool parity_m2l(const fmmb_plan* pl) {
+  return pl->cfg.precision != FMMB_MIXED || pl->K > tc_max_k() || helm_family(pl->cfg.kernel);
 }
 
 // The tensor-core M2L's operator images (mixed form), rebuilt when the
@@ -206,9 +214,13 @@ int fmmb_plan_create(const fmmb_config* cfg, fmmb_plan** out) {
       build_static_operators(pl->ops, pl->p, pl->ref);
       upload_static_ops(pl);
       if (!pl->ref && !helm_family(cfg->kernel)) {  // geometry-independent M2L set
-        build_m2l_operators(pl->ops, 2, 1.0f);
-        upload(pl->d_m2l, pl->ops.m2l, pl->st.main);
-        m2l_images(pl);
+        if (parity_m2l(pl)) {
+          build_parity_operators(pl->ops, 2, 1.0f);
+          upload(pl->d_par, pl->ops.par, pl->st.main);
+        } else {
+          build_m2l_operators(pl->ops, 2, 1.0f);
+          m2l_images(pl);
+        }
       }
     } catch (...) {
       fmmb_plan_destroy(pl);
@@ -348,55 +360,18 @@ int geometry_impl(fmmb_plan* pl, int nprob, const int* toff, const int* soff, in
     }
     // reference semantics: the M2L distance carries an absolute eps, so the
     // operator set depends on the level sizes (rebuilt when they change)
-    if (pl->ref && (pl->ops.m2l_lmax != pl->lmax || pl->ops.m2l_rd != pl->bbox[3])) {
-      build_m2l_operators(pl->ops, pl->lmax, pl->bbox[3]);
-      upload(pl->d_m2l, pl->ops.m2l, s);
+    const bool par_m2l = parity_m2l(pl);
+    if (pl->ref && par_m2l && (pl->ops.par_lmax != pl->lmax || pl->ops.par_rd != pl->bbox[3])) {
+      build_parity_operators(pl->ops, pl->lmax, pl->bbox[3]);
+      upload(pl->d_par, pl->ops.par, s);
     }
-    // FP64 translation tiles (M2L, M2M, L2L) per level
-    std::vector<int> keys(pl->tot_i), keys_j(pl->tot_j), par_j(pl->tot_j), lst;
+    if (pl->ref && !par_m2l && (pl->ops.m2l_lmax != pl->lmax || pl->ops.m2l_rd != pl->bbox[3]))
+      build_m2l_operators(pl->ops, pl->lmax, pl->bbox[3]);
+    // M2M / L2L translation tiles per level
+    std::vector<int> keys(pl->tot_i), keys_j(pl->tot_j), par_j(pl->tot_j);
     FMMB_CUDA(cudaMemcpy(keys.data(), pl->key_i.get(), pl->tot_i * sizeof(int), cudaMemcpyDeviceToHost));
     FMMB_CUDA(cudaMemcpy(keys_j.data(), pl->key_j.get(), pl->tot_j * sizeof(int), cudaMemcpyDeviceToHost));
     FMMB_CUDA(cudaMemcpy(par_j.data(), pl->parent_j.get(), pl->tot_j * sizeof(int), cudaMemcpyDeviceToHost));
-    // the M2L lists on the host only for the work lists built there: the FP64
-    // M2L's box tiles and the TF32 form's tiles (the FP16 form's are built on
-    // the device, setup.cu)
-    const bool tc_m2l = pl->cfg.precision == FMMB_MIXED && pl->K <= tc_max_k();
-    const bool h16_m2l = pl->cfg.precision == FMMB_MIXED && pl->K <= h16_max_k();
-    if (!h16_m2l) {
-      lst.resize((size_t)pl->tot_i * kM2LSlots);
-      FMMB_CUDA(cudaMemcpy(lst.data(), pl->m2l_list.get(), lst.size() * sizeof(int), cudaMemcpyDeviceToHost));
-    }
-    const int XT = translate_tile_size();
-    auto make_tiles = [&](const std::vector<std::vector<int>>& groups, int nslots, auto op_of) {
-      std::unique_ptr<fmmb_plan::TileSet> ts(new fmmb_plan::TileSet());
-      std::vector<int> tb, to;
-      for (const auto& g : groups)
-        for (size_t k = 0; k < g.size(); k += XT) {
-          const size_t e = std::min(g.size(), k + XT);
-          std::vector<int> ops_row(nslots, -1);
-          bool any_slot = false;
-          for (int sl = 0; sl < nslots; sl++)
-            for (size_t t = k; t < e; t++) {
-              const int o = op_of(g[t], sl);
-              if (o >= 0) {
-                ops_row[sl] = o;
-                any_slot = true;
-                break;
-              }
-            }
-          if (!any_slot) continue;
-          for (int t = 0; t < XT; t++) tb.push_back(k + t < e ? g[k + t] : -1);
-          to.insert(to.end(), ops_row.begin(), ops_row.end());
-        }
-      ts->ntile = (int)tb.size() / XT;
-      ts->boxes.alloc(tb.size());
-      ts->ops.alloc(to.size());
-      if (!tb.empty()) {
-        FMMB_CUDA(cudaMemcpy(ts->boxes.get(), tb.data(), tb.size() * sizeof(int), cudaMemcpyHostToDevice));
-        FMMB_CUDA(cudaMemcpy(ts->ops.get(), to.data(), to.size() * sizeof(int), cudaMemcpyHostToDevice));
-      }
-      return ts;
-    };
     // M2M child lists: [parent][octant] -> child within the child level
     std::vector<int> m2m_list((size_t)pl->tot_j * 8, -1);
     for (int lev = pl->lmax; lev >= 3; lev--)
@@ -404,20 +379,6 @@ int geometry_impl(fmmb_plan* pl, int nprob, const int* toff, const int* soff, in
         const int par = par_j[pl->off_j[lev] + c];
         m2m_list[(size_t)(pl->off_j[lev - 1] + par) * 8 + (keys_j[pl->off_j[lev] + c] & 7)] = c;
       }
-    pl->m2m_list.alloc(m2m_list.size());
-    FMMB_CUDA(cudaMemcpy(pl->m2m_list.get(), m2m_list.data(), m2m_list.size() * sizeof(int), cudaMemcpyHostToDevice));
-    pl->m2l_tiles.clear();
-    // the FP64 M2L's box tiles (the tensor-core forms use the pair tiles below)
-    const bool fp64_m2l = !tc_m2l;
-    for (int lev = 0; lev <= pl->lmax; lev++) {
-      std::vector<std::vector<int>> by_oct(8);
-      if (lev >= 2 && fp64_m2l)
-        for (int b = 0; b < pl->nbox_i[lev]; b++) by_oct[keys[pl->off_i[lev] + b] & 7].push_back(pl->off_i[lev] + b);
-      pl->m2l_tiles.push_back(make_tiles(by_oct, kM2LSlots, [&](int box, int sl) {
-        if (lst[(size_t)box * kM2LSlots + sl] < 0) return -1;
-        return pl->ops.rel_to_op[pl->ops.slot_rel[(keys[box] & 7) * kM2LSlots + sl]];
-      }));
-    }
     int dev_sms = 148;
     cudaDeviceGetAttribute(&dev_sms, cudaDevAttrMultiProcessorCount, pl->device);
     pl->nsm = dev_sms;
@@ -486,6 +447,10 @@ int geometry_impl(fmmb_plan* pl, int nprob, const int* toff, const int* soff, in
     pl->use_tc = mixed && !pl->use_h16 && pl->K <= tc_max_k();
     init_fac32();
     prepare_translate_pairs_f64();
+    if (par_m2l) {
+      prepare_m2l_parity(0, pl->p);
+      build_parity_job(pl, s);
+    }
     if (pl->use_tc) prepare_translate_tc();
     if (pl->use_h16) prepare_translate_h16();
     if (pl->use_tc || pl->use_h16) {
@@ -553,10 +518,8 @@ int geometry_impl(fmmb_plan* pl, int nprob, const int* toff, const int* soff, in
       };
       // M2L, all levels in one job: operator = set(level)*316 + relative position
       if (!(pl->use_h16 && build_m2l_job_dev(pl, pl->tc_m2l, (K + 3) / 4 * 4, s))) {
-        if (lst.empty()) {
-          lst.resize((size_t)pl->tot_i * kM2LSlots);
-          FMMB_CUDA(cudaMemcpy(lst.data(), pl->m2l_list.get(), lst.size() * sizeof(int), cudaMemcpyDeviceToHost));
-        }
+        std::vector<int> lst((size_t)pl->tot_i * kM2LSlots);
+        FMMB_CUDA(cudaMemcpy(lst.data(), pl->m2l_list.get(), lst.size() * sizeof(int), cudaMemcpyDeviceToHost));
         std::vector<Pair> pairs;
         for (int lev = 2; lev <= pl->lmax; lev++) {
           const int set = pl->ops.m2l_sets > 1 ? lev - 2 : 0;
@@ -632,12 +595,6 @@ int fmmb_set_geometry_batch(fmmb_plan* pl, int nprob, const int* t_off, const fl
 
 namespace {
 
-// Slot split of a translation launch: enough blocks for ~8 per SM on 148 SMs.
-int split_for(int ntile, int nslots) {
-  if (ntile <= 0) return 1;
-  return std::max(1, std::min(std::min(nslots, 27), (8 * 148 + ntile - 1) / ntile));
-}
-
 // Brackets one launch with a pair of pool events (phase 0..5 as in
 // fmmb_get_timings); silently stops timing when the pool is exhausted.
 // Records a timing event; while the evaluate is being captured into a graph,
@@ -665,6 +622,26 @@ struct PhaseTimer {
     }
   }
 };
+
+// The FP64 M2L of all levels: M -> L (added to).
+void run_parity(fmmb_plan* pl, int mode, cudaStream_t m) {
+  const fmmb_plan::PairJob& job = pl->par_m2l;
+  if (job.ntile <= 0) return;
+  PhaseTimer tm(pl, 3, m);
+  ParityArgs a{};
+  a.ntile = job.ntile;
+  a.p = pl->p;
+  a.tile_cls = job.tile_op.get();
+  a.tile_src = job.tile_src.get();
+  a.tile_dst = job.tile_dst.get();
+  a.tile_phi = job.tile_phi.get();
+  a.img = pl->d_par.get();
+  a.img_stride = parity_img_stride(mode, pl->p);
+  a.phi = reinterpret_cast<const double2*>(pl->d_phi.get());
+  a.xin = pl->M.get();
+  a.out = pl->L.get();
+  launch_m2l_parity(mode, a, m);
+}
 
 // One right-hand side of the complex Helmholtz kernel: qs (sorted complex
 // charges) -> near / far sorted complex potentials.  P2P on the side stream;
@@ -721,7 +698,7 @@ void run_one_helm(fmmb_plan* pl, const float* qs) {
   for (int lev = lmax - 1; lev >= 2; lev--) pairs_run(*pl->m2m_pairs[lev], pl->M.get(), pl->M.get(), 1, 2);
   FMMB_CUDA(time_mark(pl, pl->ev[4], m));
   FMMB_CUDA(cudaMemsetAsync(pl->L.get(), 0, (size_t)pl->tot_i * 2 * K * sizeof(double), m));
-  pairs_run(*pl->h_m2l, pl->M.get(), pl->L.get(), 1, 3);
+  run_parity(pl, yuk ? 2 : 1, m);
   for (int lev = 3; lev <= lmax; lev++) pairs_run(*pl->l2l_pairs[lev], pl->L.get(), pl->L.get(), 1, 4);
   FMMB_CUDA(time_mark(pl, pl->ev[5], m));
   {
@@ -881,15 +858,7 @@ void run_one(fmmb_plan* pl, const float* qs, bool want_grad) {
                         pl->L.get(), m);
     pl->launches++;
   } else {
-    const size_t opsz = (size_t)316 * K * K;
-    for (int lev = 2; lev <= lmax; lev++) {
-      PhaseTimer tm(pl, 3, m);
-      const int set = pl->ops.m2l_sets > 1 ? lev - 2 : 0;
-      const auto& ts = *pl->m2l_tiles[lev];
-      launch_translate_f64(ts.ntile, split_for(ts.ntile, kM2LSlots), K, kM2LSlots, ts.boxes.get(), ts.ops.get(),
-                           pl->m2l_list.get(), pl->d_m2l.get() + set * opsz, pl->M.get() + (size_t)pl->off_j[lev] * K,
-                           pl->L.get(), m);
-    }
+    run_parity(pl, 0, m);
   }
   near_field(p2p_split, pl->p2p_nwork, true);
   for (int lev = 3; lev <= lmax; lev++)  // children at lev from their parent (one pair each, added by one atomic)

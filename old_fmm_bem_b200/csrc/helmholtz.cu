@@ -24,7 +24,8 @@
 // points) and projected on the target basis, conj(Y) and a division by the
 // target radial function at the sphere's radius.  The operators are stored in
 // the real 2K x 2K form acting on [re | im] (transposed, row stride 2K) and
-// applied by the FP64 pair kernel of kernels_fp64.cu.
+// applied by the FP64 pair kernel of kernels_fp64.cu; the M2L operators, only
+// those at azimuth 0, as the reflection blocks of m2l_parity.cu.
 //
 // The same code serves the Yukawa kernel (FMMB_YUKAWA, the reference's neq 10,
 // kernel/Helmholtz_G_p2p.cxx:18-23: (pi/2) e^{-lambda r} / (lambda r)) through
@@ -538,10 +539,27 @@ __global__ void __launch_bounds__(128) helm_direct(int i0, int i1, const int* __
 }
 
 // ---------------------------------------------------------------- operators
+// (n, m) of row r of the parity images: (n, m > 0) by degree, O of them, then (n, 0)
+__device__ __forceinline__ void parity_row(int r, int O, int& n, int& m) {
+  if (r >= O) {
+    n = r - O;
+    m = 0;
+    return;
+  }
+  n = 1;
+  while ((n + 1) * n / 2 <= r) n++;
+  m = r - n * (n - 1) / 2 + 1;
+}
+
 // One block per (operator, source coefficient).  f = source basis function
 // R_n(k|v|) Y_n^m(v^) at v = D + rad * s_q over the quadrature points s_q;
 // g[i][m'] = sum_j f[i][j] e^{-i m' phi_j} 2 pi / NP;
 // T[n'm'] = sum_i w_i g[i][m'] Ybar_n'^|m'|(x_i) / R'_n'(k rad).
+// PAR: the M2L operators at azimuth 0 as the images of m2l_parity.cu, T = A + iB
+// combined over +-m' (rows) for columns (n, m >= 0): even block T_{m'm} +
+// T_{-m'm}, odd block T_{m'm} - T_{-m'm}, halved for m' > 0 since the sum and
+// difference of the two blocks' results give orders m' and -m'.
+template <bool PAR>
 __global__ void __launch_bounds__(256) helm_build_ops(int p, int K, double k, int yuk, const HelmOp* __restrict__ ops,
                                                       int NQ, int NP, const double* __restrict__ gl_x,
                                                       const double* __restrict__ gl_w,
@@ -553,9 +571,14 @@ __global__ void __launch_bounds__(256) helm_build_ops(int p, int K, double k, in
   double2* rt = g + (size_t)NQ * (2 * p + 1);  // [p+1] target radial values at rad
   const int o = blockIdx.y, c = blockIdx.x;
   const HelmOp op = ops[o];
-  int n = 0;
-  while ((n + 1) * (n + 1) <= c) n++;
-  const int m = c - n * n - n;
+  const int E = (p + 1) * (p + 2) / 2, O = p * (p + 1) / 2;
+  int n = 0, m;
+  if (PAR) {
+    parity_row(c, O, n, m);
+  } else {
+    while ((n + 1) * (n + 1) <= c) n++;
+    m = c - n * n - n;
+  }
   const int am = m < 0 ? -m : m;
   double rad[kMaxP + 1], rad2[kMaxP + 1];
   // 1. samples of the source basis function
@@ -621,12 +644,7 @@ __global__ void __launch_bounds__(256) helm_build_ops(int p, int K, double k, in
   }
   __syncthreads();
   // 3. polar transform, division by the target radial function, real form
-  double* col_re = opT + (size_t)o * ostride + (size_t)c * (2 * K);        // input re[c]
-  double* col_im = opT + (size_t)o * ostride + (size_t)(K + c) * (2 * K);  // input im[c]
-  for (int t = threadIdx.x; t < K; t += blockDim.x) {
-    int n2 = 0;
-    while ((n2 + 1) * (n2 + 1) <= t) n2++;
-    const int m2 = t - n2 * n2 - n2;
+  auto target = [&](int n2, int m2) -> double2 {
     const int am2 = m2 < 0 ? -m2 : m2;
     double sr = 0, si = 0;
     for (int iq = 0; iq < NQ; iq++) {
@@ -637,7 +655,37 @@ __global__ void __launch_bounds__(256) helm_build_ops(int p, int K, double k, in
     }
     const double2 d = rt[n2];
     const double den = d.x * d.x + d.y * d.y;
-    const double tr = (sr * d.x + si * d.y) / den, ti = (si * d.x - sr * d.y) / den;
+    return make_double2((sr * d.x + si * d.y) / den, (si * d.x - sr * d.y) / den);
+  };
+  if (PAR) {
+    const int RE = (E + 7) / 8 * 8, RO = (O + 7) / 8 * 8, nprod = yuk ? 1 : 3;
+    const size_t se = (size_t)RE * (RE + 4), so = (size_t)RO * (RO + 4);
+    double* img = opT + (size_t)o * ostride;
+    for (int t = threadIdx.x; t < E; t += blockDim.x) {
+      int n2, m2;
+      parity_row(t, O, n2, m2);
+      double2 e = target(n2, m2), d = make_double2(0.0, 0.0);
+      if (m2 > 0) {
+        const double2 v = target(n2, -m2);
+        d = make_double2(0.5 * (e.x - v.x), 0.5 * (e.y - v.y));
+        e = make_double2(0.5 * (e.x + v.x), 0.5 * (e.y + v.y));
+      }
+      for (int pd = 0; pd < nprod; pd++) {  // A, -(A + B), B - A
+        img[pd * se + (size_t)c * (RE + 4) + t] = pd == 0 ? e.x : pd == 1 ? -(e.x + e.y) : e.y - e.x;
+        if (t < O && c < O)
+          img[nprod * se + pd * so + (size_t)c * (RO + 4) + t] = pd == 0 ? d.x : pd == 1 ? -(d.x + d.y) : d.y - d.x;
+      }
+    }
+    return;
+  }
+  double* col_re = opT + (size_t)o * ostride + (size_t)c * (2 * K);        // input re[c]
+  double* col_im = opT + (size_t)o * ostride + (size_t)(K + c) * (2 * K);  // input im[c]
+  for (int t = threadIdx.x; t < K; t += blockDim.x) {
+    int n2 = 0;
+    while ((n2 + 1) * (n2 + 1) <= t) n2++;
+    const int m2 = t - n2 * n2 - n2;
+    const double2 T = target(n2, m2);
+    const double tr = T.x, ti = T.y;
     col_re[t] = tr;
     col_re[K + t] = ti;
     col_im[t] = -ti;
@@ -776,19 +824,32 @@ size_t helm_build_smem(int p) {
   return ((size_t)NQ * NP + (size_t)NQ * (2 * p + 1) + (p + 1)) * sizeof(double2);
 }
 
-void launch_helm_build_ops(int p, double k, bool yuk, int nops, const HelmOp* ops, const double* gl_x,
-                           const double* gl_w, const double* ybar_q, double* opT, cudaStream_t st) {
+namespace {
+template <bool PAR>
+void build_ops(int p, double k, bool yuk, int nops, const HelmOp* ops, const double* gl_x, const double* gl_w,
+               const double* ybar_q, double* opT, size_t ostride, cudaStream_t st) {
   if (nops <= 0) return;
   const int K = (p + 1) * (p + 1), NQ = 2 * p + 8, NP = 2 * NQ;
   const size_t smem = helm_build_smem(p);
-  FMMB_CUDA(cudaFuncSetAttribute(helm_build_ops, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-  const size_t ostride = (size_t)4 * K * K;
+  FMMB_CUDA(cudaFuncSetAttribute(helm_build_ops<PAR>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
   for (int o0 = 0; o0 < nops; o0 += 65535) {
-    dim3 grid(K, std::min(65535, nops - o0));
-    helm_build_ops<<<grid, 256, smem, st>>>(p, K, k, yuk ? 1 : 0, ops + o0, NQ, NP, gl_x, gl_w, ybar_q,
-                                            opT + (size_t)o0 * ostride, ostride);
+    dim3 grid(PAR ? (p + 1) * (p + 2) / 2 : K, std::min(65535, nops - o0));
+    helm_build_ops<PAR><<<grid, 256, smem, st>>>(p, K, k, yuk ? 1 : 0, ops + o0, NQ, NP, gl_x, gl_w, ybar_q,
+                                                 opT + (size_t)o0 * ostride, ostride);
     FMMB_CHECK_LAUNCH();
   }
+}
+}  // namespace
+
+void launch_helm_build_ops(int p, double k, bool yuk, int nops, const HelmOp* ops, const double* gl_x,
+                           const double* gl_w, const double* ybar_q, double* opT, cudaStream_t st) {
+  const size_t K = (size_t)(p + 1) * (p + 1);
+  build_ops<false>(p, k, yuk, nops, ops, gl_x, gl_w, ybar_q, opT, 4 * K * K, st);
+}
+
+void launch_helm_build_parity(int p, double k, bool yuk, int nops, const HelmOp* ops, const double* gl_x,
+                              const double* gl_w, const double* ybar_q, double* img, size_t stride, cudaStream_t st) {
+  build_ops<true>(p, k, yuk, nops, ops, gl_x, gl_w, ybar_q, img, stride, st);
 }
 
 }  // namespace fmmb

@@ -116,8 +116,7 @@ void helm_setup(fmmb_plan* pl) {
   const double k = pl->cfg.wavenumber, rd = pl->bbox[3];
   cudaStream_t s = pl->st.main;
   auto width = [&](int l) { return rd / (double)(1 << l); };
-  // operators: M2M for child levels 3..lmax (8 octants each), L2L likewise,
-  // M2L for levels 2..lmax (316 relative positions each)
+  // operators: M2M for child levels 3..lmax (8 octants each), L2L likewise
   std::vector<HelmOp> ops;
   auto octant_offset = [&](int oct, double wc, double* o) {  // child centre - parent centre
     o[0] = (((oct >> 1) & 1) - 0.5) * wc;  // key bit 1: x
@@ -141,13 +140,12 @@ void helm_setup(fmmb_plan* pl) {
       octant_offset(oct, width(lc), o);
       ops.push_back({o[0], o[1], o[2], std::min(0.8660254037844386 * width(lc), rad_cap), 0, 0});
     }
-  pl->hop_m2l0 = (int)ops.size();
+  // M2L: levels 2..lmax x the 61 classes, at azimuth 0
+  std::vector<HelmOp> mops;
   for (int l = 2; l <= lmax; l++)
-    for (int slot = 0; slot < 316; slot++) {
-      const int code = pl->ops.op_rel[slot];
+    for (const auto& g : pl->ops.cls_geom) {
       const double w = width(l);
-      ops.push_back({(code / 49 - 3) * w, ((code / 7) % 7 - 3) * w, (code % 7 - 3) * w,
-                     std::min(0.8660254037844386 * w, rad_cap), 1, 0});
+      mops.push_back({std::sqrt((double)g[0]) * w, 0.0, g[1] * w, std::min(0.8660254037844386 * w, rad_cap), 1, 0});
     }
   const int nops = (int)ops.size();
   const size_t ostride = (size_t)4 * K * K;
@@ -159,22 +157,26 @@ void helm_setup(fmmb_plan* pl) {
     std::vector<double> yb((size_t)NQ * P);
     for (int i = 0; i < NQ; i++) ybar_table(p, gx[i], yb.data() + (size_t)i * P);
     DevBuf<double> d_gx, d_gw, d_yb;
-    DevBuf<HelmOp> d_ops;
+    DevBuf<HelmOp> d_ops, d_mops;
     upload_vec(d_gx, gx);
     upload_vec(d_gw, gw);
     upload_vec(d_yb, yb);
     upload_vec(d_ops, ops);
     launch_helm_build_ops(p, k, yuk, nops, d_ops.get(), d_gx.get(), d_gw.get(), d_yb.get(), pl->d_hops.get(), s);
+    const size_t pstride = parity_img_stride(yuk ? 2 : 1, p);
+    pl->d_par.alloc(mops.size() * pstride);
+    FMMB_CUDA(cudaMemsetAsync(pl->d_par.get(), 0, mops.size() * pstride * sizeof(double), s));  // the padding stays zero
+    upload_vec(d_mops, mops);
+    launch_helm_build_parity(p, k, yuk, (int)mops.size(), d_mops.get(), d_gx.get(), d_gw.get(), d_yb.get(),
+                             pl->d_par.get(), pstride, s);
     FMMB_CUDA(cudaStreamSynchronize(s));
   }
   // pair jobs (rows are indices into the all-level M / L arrays)
-  std::vector<int> par_i(pl->tot_i), par_j(pl->tot_j), key_i(pl->tot_i), key_j(pl->tot_j),
-      lst((size_t)pl->tot_i * kM2LSlots);
+  std::vector<int> par_i(pl->tot_i), par_j(pl->tot_j), key_i(pl->tot_i), key_j(pl->tot_j);
   FMMB_CUDA(cudaMemcpy(par_i.data(), pl->parent_i.get(), pl->tot_i * sizeof(int), cudaMemcpyDeviceToHost));
   FMMB_CUDA(cudaMemcpy(par_j.data(), pl->parent_j.get(), pl->tot_j * sizeof(int), cudaMemcpyDeviceToHost));
   FMMB_CUDA(cudaMemcpy(key_i.data(), pl->key_i.get(), pl->tot_i * sizeof(int), cudaMemcpyDeviceToHost));
   FMMB_CUDA(cudaMemcpy(key_j.data(), pl->key_j.get(), pl->tot_j * sizeof(int), cudaMemcpyDeviceToHost));
-  FMMB_CUDA(cudaMemcpy(lst.data(), pl->m2l_list.get(), lst.size() * sizeof(int), cudaMemcpyDeviceToHost));
   int nsm = 148;
   cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, pl->device);
   pl->nsm = nsm;
@@ -197,18 +199,8 @@ void helm_setup(fmmb_plan* pl) {
     pl->m2m_pairs.push_back(pair_job(up, 2 * K, nsm));
     pl->l2l_pairs.push_back(pair_job(down, 2 * K, nsm));
   }
-  std::vector<P3> m2l;
-  for (int lev = 2; lev <= lmax; lev++)
-    for (int b = 0; b < pl->nbox_i[lev]; b++) {
-      const int box = pl->off_i[lev] + b;
-      for (int sl = 0; sl < kM2LSlots; sl++) {
-        const int src = lst[(size_t)box * kM2LSlots + sl];
-        if (src < 0) continue;
-        const int slot = pl->ops.rel_to_op[pl->ops.slot_rel[(key_i[box] & 7) * kM2LSlots + sl]];
-        m2l.push_back({pl->hop_m2l0 + (lev - 2) * 316 + slot, pl->off_j[lev] + src, box});
-      }
-    }
-  pl->h_m2l = pair_job(m2l, 2 * K, nsm);
+  prepare_m2l_parity(yuk ? 2 : 1, p);
+  build_parity_job(pl, s);
   // P2P work items: every target leaf in pieces of 256 targets
   {
     const int nleaf = pl->nbox_i[lmax];

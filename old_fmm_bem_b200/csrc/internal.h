@@ -3,6 +3,7 @@
 
 #include <cuda_runtime.h>
 
+#include <array>
 #include <complex>
 #include <cstdint>
 #include <memory>
@@ -125,6 +126,14 @@ struct Operators {
   std::vector<int> rel_to_op;  // [343] -> operator slot (0..315) or -1
   std::vector<int> op_rel;     // [316] rel code of each operator slot
   std::vector<int> slot_rel;   // [8][189] rel code of each M2L slot per octant
+  // FP64 M2L (m2l_parity.cu): the relative positions of one (dx^2 + dy^2, dz)
+  // share an operator, taken at azimuth 0; azimuth index of a code: code / 7
+  std::vector<int> rel_to_cls;               // [343] -> class (0..60) or -1
+  std::vector<std::array<int, 2>> cls_geom;  // [61] (dx^2 + dy^2, dz)
+  std::vector<double> par;                   // [par_sets][61] operator images
+  int par_sets = 0, par_lmax = 0;
+  float par_rd = 0;
+  std::vector<double> phi;                   // [49][21][2] (cos m phi, sin m phi)
   // Wigner rotation tables per relative position (forward, inverse)
   std::vector<std::vector<std::vector<std::complex<double>>>> Wf, Wb;
 };
@@ -133,6 +142,9 @@ void build_static_operators(Operators& ops, int p, bool ref_semantics);
 // M2L sets: one in accurate semantics; one per level 2..lmax in reference
 // semantics, where the distance carries an absolute eps (needs the root size).
 void build_m2l_operators(Operators& ops, int lmax, float rd);
+// the FP64 M2L's operator images of the Laplace kernels: one set, or (reference
+// semantics) one per level 2..lmax
+void build_parity_operators(Operators& ops, int lmax, float rd);
 // TF32 hi/lo images of nmat K x K operators in the tensor-core operand layout
 void build_tc_images(const std::vector<double>& mats, int nmat, int K, int kpad, std::vector<float>& img);
 // FP16 hi/lo images (row-scaled) for the FP16x3 M2L, img_bytes each
@@ -204,7 +216,11 @@ struct fmmb_plan {
   fmmb::DevBuf<int> child_count_j;
 
   // operators on the device
-  fmmb::DevBuf<double> d_fac, d_m2l;
+  fmmb::DevBuf<double> d_fac;
+  // FP64 M2L: operator images (Laplace FP64 form; Helmholtz family: levels
+  // 2..lmax x 61), rotation table, class of a relative position
+  fmmb::DevBuf<double> d_par, d_phi;
+  fmmb::DevBuf<int> d_rel_to_cls;
   fmmb::DevBuf<double> d_m2m_t, d_l2l_t;    // [8][column][row] (transposed for the FP64 pair kernel)
   fmmb::DevBuf<int> d_slot_rel, d_rel_to_op;
   fmmb::DevBuf<float> d_img_m2l;             // [sets*316][4 K-blocks][2][128*32] TF32 images (mixed)
@@ -280,31 +296,22 @@ struct fmmb_plan {
   // at a level), index = level
   struct PairJob {
     int ntile = 0, tp = 0;
-    fmmb::DevBuf<int> tile_op, tile_src, tile_dst;
+    fmmb::DevBuf<int> tile_op, tile_src, tile_dst, tile_phi;
   };
+  PairJob par_m2l;  // FP64 M2L, all levels (tile_op: set * 61 + class)
   std::vector<std::unique_ptr<PairJob>> m2m_pairs, l2l_pairs;
   // complex Helmholtz: dense operators in the real 2K x 2K form (transposed),
-  // [M2M child levels 3..lmax x 8 | L2L likewise | M2L levels 2..lmax x 316],
-  // and the M2L pairs of all levels
+  // [M2M child levels 3..lmax x 8 | L2L likewise]
   fmmb::DevBuf<double> d_hops;
-  int hop_m2m0 = 0, hop_l2l0 = 0, hop_m2l0 = 0;
+  int hop_m2m0 = 0, hop_l2l0 = 0;
   fmmb::DevBuf<int2> h_p2p_work;  // P2P work items: (target leaf, first target), up to 256 targets each
   int h_p2p_nwork = 0;
-  std::unique_ptr<PairJob> h_m2l;
   fmmb::DevBuf<double> pot_s, grad_s;        // sorted outputs [ni], [3][ni]
   fmmb::DevBuf<float> stage_f;               // host<->device staging
   fmmb::DevBuf<double> stage_d;
   fmmb::DevBuf<int> inv_i;                   // caller index -> sorted target position
   fmmb::DevBuf<char> stage_out;              // device staging of host outputs
   bool timings_valid = false;
-  // FP64 translation tiles per level (kernels_fp64.cu translate_f64): output
-  // boxes [ntile][32] and per-tile operator index per slot [ntile][nslots]
-  struct TileSet {
-    int ntile = 0;
-    fmmb::DevBuf<int> boxes, ops;
-  };
-  std::vector<std::unique_ptr<TileSet>> m2l_tiles;  // index = level
-  fmmb::DevBuf<int> m2m_list;                                            // [tot_j][8] child (within level) or -1
 };
 
 namespace fmmb {
@@ -312,6 +319,8 @@ namespace fmmb {
 // tiles and reduction CSR (false: too large for the int enumeration, build on
 // the host), the near-field work items, the inverse target permutation
 bool build_m2l_job_dev(fmmb_plan* pl, fmmb_plan::TcJob& job, int ys, cudaStream_t s);
+// the FP64 M2L's pair tiles
+void build_parity_job(fmmb_plan* pl, cudaStream_t s);
 void build_p2p_work_dev(fmmb_plan* pl, cudaStream_t s);
 void build_p2m_work_dev(fmmb_plan* pl, cudaStream_t s);
 void build_inverse_perm_dev(fmmb_plan* pl, cudaStream_t s);

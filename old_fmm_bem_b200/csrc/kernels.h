@@ -67,10 +67,6 @@ bool launch_p2m_f32(int kernel, int nwork, const int2* work, int p, int K, const
 bool launch_l2p_f32(int kernel, int nwork, const int2* work, int p, int K, const int* keys, const int2* leaf,
                     const float4* tpos, const float4* tnrm, const double* fac, const float* bbox, double rb,
                     double coef, const double* L, double* pot, double* grad, int ni, cudaStream_t st);
-int translate_tile_size();
-// batched FP64 translation (M2L / M2M / L2L), see kernels_fp64.cu
-void launch_translate_f64(int ntile, int nsplit, int K, int nslots, const int* tile_boxes, const int* tile_ops,
-                          const int* list, const double* ops, const double* in, double* out, cudaStream_t st);
 void launch_l2p(int kernel, int nleaf, int p, int K, const int* keys, const int2* leaf, const float4* tpos, const float4* tnrm,
                 const double* fac, const Sem& s, const float* bbox, double rb, const double* L, double* pot, double* grad,
                 int ni, cudaStream_t st);
@@ -105,6 +101,20 @@ int pairs_f64_tile(int K, int npair, int nsm);
 // once per device, before any launch (and outside stream capture)
 void prepare_translate_pairs_f64();
 void launch_translate_pairs_f64(const PairArgs& a, cudaStream_t st);
+// FP64 M2L (m2l_parity.cu) over tiles of 32 pairs {operator, source row, target
+// row, azimuth} of one operator: mode 0 Laplace, 1 Helmholtz, 2 Yukawa
+struct ParityArgs {
+  int ntile, p;
+  const int *tile_cls, *tile_src, *tile_dst, *tile_phi;  // [ntile], [ntile][32] each (-1: no pair)
+  const double* img;                                     // operator images, img_stride doubles each
+  size_t img_stride;
+  const double2* phi;  // [49 azimuths][21 orders] (cos m phi, sin m phi)
+  const double* xin;   // source expansions
+  double* out;         // target expansions, added to
+};
+size_t parity_img_stride(int mode, int p);
+void prepare_m2l_parity(int mode, int p);  // once per device, outside stream capture
+void launch_m2l_parity(int mode, const ParityArgs& a, cudaStream_t st);
 // constant table of the FP32 P2M, once per device (outside stream capture)
 void init_fac32();
 void launch_split_tf32(int nbox, int K, int kpad, const double* M, float* Mtf, cudaStream_t st);
@@ -182,4 +192,7 @@ void launch_helm_finalize(int n, const int* perm, const double* near, const doub
 // operators in the real 2K x 2K form, transposed ([op][column][row], row stride 2K)
 void launch_helm_build_ops(int p, double k, bool yuk, int nops, const HelmOp* ops, const double* gl_x,
                            const double* gl_w, const double* ybar_q, double* opT, cudaStream_t st);
+// the M2L operators as images of m2l_parity.cu, `stride` doubles each (zeroed before)
+void launch_helm_build_parity(int p, double k, bool yuk, int nops, const HelmOp* ops, const double* gl_x,
+                              const double* gl_w, const double* ybar_q, double* img, size_t stride, cudaStream_t st);
 }  // namespace fmmb

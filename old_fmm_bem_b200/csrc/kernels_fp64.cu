@@ -154,93 +154,6 @@ __global__ void __launch_bounds__(128) p2m_f64(int p, int K, const int* __restri
   for (int k = threadIdx.x; k < K; k += blockDim.x) M[(size_t)b * K + k] = acc[k] + acc[K + k] + acc[2 * K + k] + acc[3 * K + k];
 }
 
-// ---------------------------------------------------------------- translations (FP64)
-// One kernel for the three box-to-box translations (M2L, M2M, L2L): a block
-// owns a tile of up to 32 output boxes and walks `nslots` slots; slot s of
-// output box b reads input box list[b*nslots + s] (an index into `in`, or
-// -1) through operator tile_ops[tile*nslots + s] (-1: no box of the tile uses
-// the slot).  Per slot the K x K operator is streamed through shared memory
-// in column panels and applied to the tile's gathered inputs -- a batched
-// K x K x 32 DGEMM whose operator is shared by the whole tile.  grid.y
-// splits the slots when there are few tiles; the shares are then added with
-// FP64 atomics.
-//   M2L: tiles of target boxes of one octant, 189 interaction slots
-//        (kernel/m2l.cxx:30-83);
-//   M2M: tiles of parent boxes, 8 child slots (kernel/m2m.cxx:28-62);
-//   L2L: tiles of child boxes of one octant, 1 parent slot (kernel/l2l.cxx:44-78).
-constexpr int kXTile = 32;    // output boxes per block
-constexpr int kXPanel = 16;   // operator columns per shared-memory panel
-constexpr int kXThreads = 256;
-
-__global__ void __launch_bounds__(kXThreads) translate_f64(int K, int nslots, const int* __restrict__ tile_boxes,
-                                                           const int* __restrict__ tile_ops, const int* __restrict__ list,
-                                                           const double* __restrict__ ops, const double* __restrict__ in,
-                                                           double* __restrict__ out) {
-  constexpr int RPT = 8;  // rows per thread: ty + 16*r covers 128 rows
-  __shared__ double sT[kXPanel][128 + 1];
-  __shared__ double sB[kXPanel][kXTile + 1];
-  __shared__ int sSrc[kXTile];
-  __shared__ int sBox[kXTile];
-  const int tile = blockIdx.x;
-  const int tx = threadIdx.x & 15, ty = threadIdx.x >> 4;  // 16 x 16 threads
-  if (threadIdx.x < kXTile) sBox[threadIdx.x] = tile_boxes[tile * kXTile + threadIdx.x];
-  __syncthreads();
-  const int s0 = (blockIdx.y * nslots) / gridDim.y, s1 = ((blockIdx.y + 1) * nslots) / gridDim.y;
-  for (int rb0 = 0; rb0 < K; rb0 += 128) {
-    double acc[RPT][2];
-#pragma unroll
-    for (int r = 0; r < RPT; r++) acc[r][0] = acc[r][1] = 0.0;
-    for (int slot = s0; slot < s1; slot++) {
-      const int op = tile_ops[(size_t)tile * nslots + slot];
-      if (op < 0) continue;
-      __syncthreads();
-      if (threadIdx.x < kXTile) {
-        const int box = sBox[threadIdx.x];
-        sSrc[threadIdx.x] = box >= 0 ? list[(size_t)box * nslots + slot] : -1;
-      }
-      const double* T = ops + (size_t)op * K * K;
-      for (int k0 = 0; k0 < K; k0 += kXPanel) {
-        __syncthreads();
-        for (int e = threadIdx.x; e < kXPanel * 128; e += kXThreads) {
-          const int row = e / kXPanel, kk = e % kXPanel;
-          const int gr = rb0 + row, gk = k0 + kk;
-          sT[kk][row] = (gr < K && gk < K) ? T[(size_t)gr * K + gk] : 0.0;
-        }
-        for (int e = threadIdx.x; e < kXPanel * kXTile; e += kXThreads) {
-          const int t = e / kXPanel, kk = e % kXPanel;
-          const int src = sSrc[t], gk = k0 + kk;
-          sB[kk][t] = (src >= 0 && gk < K) ? in[(size_t)src * K + gk] : 0.0;
-        }
-        __syncthreads();
-#pragma unroll 4
-        for (int kk = 0; kk < kXPanel; kk++) {
-          const double b0 = sB[kk][tx], b1 = sB[kk][tx + 16];
-#pragma unroll
-          for (int r = 0; r < RPT; r++) {
-            const double a = sT[kk][ty + 16 * r];
-            acc[r][0] += a * b0;
-            acc[r][1] += a * b1;
-          }
-        }
-      }
-    }
-#pragma unroll
-    for (int r = 0; r < RPT; r++) {
-      const int row = rb0 + ty + 16 * r;
-      if (row < K) {
-        const int b0 = sBox[tx], b1 = sBox[tx + 16];
-        if (gridDim.y > 1) {
-          if (b0 >= 0) atomicAdd(&out[(size_t)b0 * K + row], acc[r][0]);
-          if (b1 >= 0) atomicAdd(&out[(size_t)b1 * K + row], acc[r][1]);
-        } else {
-          if (b0 >= 0) out[(size_t)b0 * K + row] += acc[r][0];
-          if (b1 >= 0) out[(size_t)b1 * K + row] += acc[r][1];
-        }
-      }
-    }
-  }
-}
-
 // ---------------------------------------------------------------- L2P
 constexpr int kL2PThreads = 64;
 
@@ -436,15 +349,6 @@ void launch_p2m(int kernel, int nleaf, int p, int K, const int* keys, const int2
     p2m_f64<FMMB_LAPLACE_GNJ><<<nleaf, 128, sm, st>>>(p, K, keys, leaf, spos, snrm, qs, fac, s, bbox[0], bbox[1], bbox[2], rb, M);
   else
     p2m_f64<FMMB_LAPLACE_G><<<nleaf, 128, sm, st>>>(p, K, keys, leaf, spos, snrm, qs, fac, s, bbox[0], bbox[1], bbox[2], rb, M);
-  FMMB_CHECK_LAUNCH();
-}
-
-int translate_tile_size() { return kXTile; }
-
-void launch_translate_f64(int ntile, int nsplit, int K, int nslots, const int* tile_boxes, const int* tile_ops,
-                          const int* list, const double* ops, const double* in, double* out, cudaStream_t st) {
-  if (ntile <= 0) return;
-  translate_f64<<<dim3(ntile, std::max(1, nsplit)), kXThreads, 0, st>>>(K, nslots, tile_boxes, tile_ops, list, ops, in, out);
   FMMB_CHECK_LAUNCH();
 }
 

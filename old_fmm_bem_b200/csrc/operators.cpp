@@ -28,6 +28,7 @@
 #include <vector>
 
 #include "internal.h"
+#include "kernels.h"
 
 namespace fmmb {
 namespace {
@@ -280,10 +281,52 @@ void build_static_operators(Operators& ops, int p, bool ref) {
               }
   }
 
+  // classes of relative positions with one operator up to a rotation about z
+  ops.rel_to_cls.assign(kRelCodes, -1);
+  ops.cls_geom.clear();
+  for (int code : op_rel) {
+    const int dx = code / 49 - 3, dy = (code / 7) % 7 - 3, dz = code % 7 - 3;
+    const std::array<int, 2> g{dx * dx + dy * dy, dz};
+    size_t c = 0;
+    while (c < ops.cls_geom.size() && ops.cls_geom[c] != g) c++;
+    if (c == ops.cls_geom.size()) ops.cls_geom.push_back(g);
+    ops.rel_to_cls[code] = (int)c;
+  }
+  ops.phi.assign((size_t)49 * 21 * 2, 0.0);
+  for (int a = 0; a < 49; a++) {
+    const double be = azimuth(a / 7 - 3, a % 7 - 3, ref);
+    for (int m = 0; m <= 20; m++) {
+      ops.phi[(a * 21 + m) * 2] = std::cos(m * be);
+      ops.phi[(a * 21 + m) * 2 + 1] = std::sin(m * be);
+    }
+  }
+
   ops.m2l.clear();
   ops.m2l_sets = 0;
   ops.m2l_lmax = 0;
 }
+
+namespace {
+// Z(j, n, k) of the M2L (kernel/m2l.cxx:56-77) at distance rho box sides
+struct M2LZ {
+  const std::vector<double>& anm;
+  bool ref;
+  double rho;
+  double A(int n, int m) const { return anm[ifull(n, m)]; }
+  double operator()(int j, int n, int k) const {
+    if (n < k) return 0.0;
+    // sr of kernel/precalc.cxx:33-43
+    return to_ref_float(std::pow(-1.0, j + k) * A(n, k) * A(j, k) / A(j + n, 0), ref) / std::pow(rho, j + n + 1);
+  }
+};
+// distance of a relative position in box sides; reference semantics: (|d| rb + eps) / rb on level 2 + set
+double m2l_distance(int d2, int set, float rd, bool ref) {
+  const double rho = std::sqrt((double)d2);
+  if (!ref) return rho;
+  const double rb = (double)(rd / (float)(1 << (2 + set)));
+  return (rb * rho + kEpsF) / rb;
+}
+}  // namespace
 
 // M2L operators (kernel/m2l.cxx:43-78): one set, or one per level when the
 // distance carries the reference's absolute eps.
@@ -291,13 +334,7 @@ void build_m2l_operators(Operators& ops, int lmax, float rd) {
   const int p = ops.p, K = ops.K;
   const bool ref = ops.ref;
   const std::vector<double> anm = anm_table(p, ref);
-  auto A = [&](int n, int m) { return anm[ifull(n, m)]; };
-  // sr of kernel/precalc.cxx:33-43
-  auto SR = [&](int j, int k, int n) { return to_ref_float(std::pow(-1.0, j + k) * A(n, k) * A(j, k) / A(j + n, 0), ref); };
-  const double rho_eps = ref ? kEpsF : 0.0;
   const auto& op_rel = ops.op_rel;
-  const auto& Wf = ops.Wf;
-  const auto& Wb = ops.Wb;
   const int nops = (int)op_rel.size();  // 316
   ops.m2l_sets = ref ? (lmax - 1) : 1;
   ops.m2l_lmax = lmax;
@@ -309,17 +346,50 @@ void build_m2l_operators(Operators& ops, int lmax, float rd) {
     const int dx = code / 49 - 3, dy = (code / 7) % 7 - 3, dz = code % 7 - 3;
     int nc[3] = {dx + 3, dy + 3, dz + 3};
     const int je = encode3(nc, 3);
-    double rho = std::sqrt((double)(dx * dx + dy * dy + dz * dz));
-    if (ref) {
-      const int lev = 2 + set;
-      const double rb = (double)(rd / (float)(1 << lev));
-      rho = (rb * rho + rho_eps) / rb;  // (|d| rb + eps) in units of rb
+    const M2LZ Z{anm, ref, m2l_distance(dx * dx + dy * dy + dz * dz, set, rd, ref)};
+    compose(p, ops.Wf[je], ops.Wb[je], Z, nullptr, &ops.m2l[((size_t)set * nops + o) * K * K]);
+  });
+}
+
+// The FP64 M2L's images (m2l_parity.cu): the operator of each class composed at
+// azimuth 0, where the rotations are real and Re, Im of the coefficients do
+// not mix: the even block acts on the Re parts (rows and columns (n, m > 0) by
+// degree, then (n, 0)), the odd one on the Im parts.
+void build_parity_operators(Operators& ops, int lmax, float rd) {
+  const int p = ops.p, K = ops.K;
+  const bool ref = ops.ref;
+  const std::vector<double> anm = anm_table(p, ref);
+  const int ncls = (int)ops.cls_geom.size(), E = (p + 1) * (p + 2) / 2, O = p * (p + 1) / 2;
+  const int RE = (E + 7) / 8 * 8, RO = (O + 7) / 8 * 8;
+  const size_t stride = parity_img_stride(0, p);
+  ops.par_sets = ref ? lmax - 1 : 1;
+  ops.par_lmax = lmax;
+  ops.par_rd = rd;
+  ops.par.assign((size_t)ops.par_sets * ncls * stride, 0.0);
+  std::vector<int> re(E), im(O);  // real-packed index of each row
+  for (int n = 0; n <= p; n++) {
+    re[O + n] = n * n;
+    for (int m = 1; m <= n; m++) {
+      re[n * (n - 1) / 2 + m - 1] = n * n + 2 * m - 1;
+      im[n * (n - 1) / 2 + m - 1] = n * n + 2 * m;
     }
-    auto Z = [&](int j, int n, int k) -> double {
-      if (n < k) return 0.0;
-      return SR(j, k, n) / std::pow(rho, j + n + 1);
-    };
-    compose(p, Wf[je], Wb[je], Z, nullptr, &ops.m2l[((size_t)set * nops + o) * K * K]);
+  }
+  parallel_for(ops.par_sets * ncls, [&](int w) {
+    const int set = w / ncls;
+    const auto g = ops.cls_geom[w % ncls];
+    const double rh = std::sqrt((double)(g[0] + g[1] * g[1])) + (ref ? kEpsF : 0.0), al = std::acos(g[1] / rh);
+    std::vector<std::vector<cd>> Wf, Wb;
+    wigner(al, 0.0, p, Wf);
+    wigner(-al, 0.0, p, Wb);
+    std::vector<double> T((size_t)K * K);
+    const M2LZ Z{anm, ref, m2l_distance(g[0] + g[1] * g[1], set, rd, ref)};
+    compose(p, Wf, Wb, Z, nullptr, T.data());
+    double* e = &ops.par[(size_t)w * stride];
+    double* o = e + (size_t)RE * (RE + 4);
+    for (int c = 0; c < E; c++)
+      for (int r = 0; r < E; r++) e[(size_t)c * (RE + 4) + r] = T[(size_t)re[r] * K + re[c]];
+    for (int c = 0; c < O; c++)
+      for (int r = 0; r < O; r++) o[(size_t)c * (RO + 4) + r] = T[(size_t)im[r] * K + im[c]];
   });
 }
 

@@ -11,6 +11,8 @@
 // them) in the order the kernels want it.
 #include <cuda_runtime.h>
 
+#include <algorithm>
+#include <array>
 #include <vector>
 
 #include "internal.h"
@@ -55,11 +57,12 @@ __global__ void m2l_pair_flags(int V, LevTab T, const int* __restrict__ lst, int
   flag[v] = lst[(size_t)(T.boxoff[l] + b) * kM2LSlots + sl] >= 0 ? 1 : 0;
 }
 
-// pair k (in enumeration order) -> operator key, source row, target row
+// pair k (in enumeration order) -> operator key, source row, target row and,
+// when wanted, azimuth index of the relative position; `per` operators a set
 __global__ void m2l_pair_emit(int V, LevTab T, const int* __restrict__ lst, const int* __restrict__ key_i,
-                              const int* __restrict__ slot_rel, const int* __restrict__ rel_to_op,
+                              const int* __restrict__ slot_rel, const int* __restrict__ rel_to_op, int per,
                               const int* __restrict__ pos, int* __restrict__ opk, int* __restrict__ ord,
-                              int* __restrict__ src, int* __restrict__ dst) {
+                              int* __restrict__ src, int* __restrict__ dst, int* __restrict__ phi) {
   const int v = blockIdx.x * blockDim.x + threadIdx.x;
   if (v >= V) return;
   int l, b, sl;
@@ -68,7 +71,9 @@ __global__ void m2l_pair_emit(int V, LevTab T, const int* __restrict__ lst, cons
   const int s = lst[(size_t)box * kM2LSlots + sl];
   if (s < 0) return;
   const int k = pos[v];
-  opk[k] = T.set[l] * 316 + rel_to_op[slot_rel[(key_i[box] & 7) * kM2LSlots + sl]];
+  const int rel = slot_rel[(key_i[box] & 7) * kM2LSlots + sl];
+  opk[k] = T.set[l] * per + rel_to_op[rel];
+  if (phi) phi[k] = rel / 7;
   ord[k] = k;
   src[k] = T.srcoff[l] + s;
   dst[k] = box;
@@ -79,23 +84,25 @@ __global__ void count_keys(int n, const int* __restrict__ key, int* __restrict__
   if (j < n) atomicAdd(&cnt[key[j]], 1);
 }
 
-__global__ void tiles_per_key(int nk, const int* __restrict__ cnt, int* __restrict__ tiles) {
+__global__ void tiles_per_key(int nk, int tt, const int* __restrict__ cnt, int* __restrict__ tiles) {
   const int o = blockIdx.x * blockDim.x + threadIdx.x;
-  if (o < nk) tiles[o] = (cnt[o] + 127) / 128;
+  if (o < nk) tiles[o] = (cnt[o] + tt - 1) / tt;
 }
 
-// sorted pair j -> tile tile_base[op] + r / 128, column r % 128 (r = its rank
+// sorted pair j -> tile tile_base[op] + r / tt, column r % tt (r = its rank
 // among the pairs of its operator)
-__global__ void fill_tiles(int n, const int* __restrict__ opk, const int* __restrict__ ord,
-                           const int* __restrict__ src, const int* __restrict__ dst, const int* __restrict__ op_start,
-                           const int* __restrict__ tile_base, int* __restrict__ tile_op, int* __restrict__ tile_src,
-                           int* __restrict__ tdst) {
+__global__ void fill_tiles(int n, int tt, const int* __restrict__ opk, const int* __restrict__ ord,
+                           const int* __restrict__ src, const int* __restrict__ dst, const int* __restrict__ phi,
+                           const int* __restrict__ op_start, const int* __restrict__ tile_base,
+                           int* __restrict__ tile_op, int* __restrict__ tile_src, int* __restrict__ tdst,
+                           int* __restrict__ tile_phi) {
   const int j = blockIdx.x * blockDim.x + threadIdx.x;
   if (j >= n) return;
   const int op = opk[j], r = j - op_start[op];
-  const int t = tile_base[op] + r / 128, c = r % 128;
-  tile_src[(size_t)t * 128 + c] = src[ord[j]];
-  tdst[(size_t)t * 128 + c] = dst[ord[j]];
+  const int t = tile_base[op] + r / tt, c = r % tt;
+  tile_src[(size_t)t * tt + c] = src[ord[j]];
+  tdst[(size_t)t * tt + c] = dst[ord[j]];
+  if (phi) tile_phi[(size_t)t * tt + c] = phi[ord[j]];
   if (c == 0) tile_op[t] = op;
 }
 
@@ -203,7 +210,17 @@ int d2h_int(const int* p, cudaStream_t s) {
 
 }  // namespace
 
-bool build_m2l_job_dev(fmmb_plan* pl, fmmb_plan::TcJob& job, int ys, cudaStream_t s) {
+namespace {
+
+// The M2L pairs of levels 2..lmax sorted by operator, in tiles of tt pairs:
+// the operator of pair (level, relative position r) is set(level) * per +
+// rel_to_op[r].  phi (may be null): the azimuth index of each pair.  False when
+// the enumeration does not fit an int.
+struct M2LTiles {
+  int npair = 0, ntile = 0;
+};
+bool build_m2l_tiles(fmmb_plan* pl, bool sets, int per, const int* rel_to_op, int tt, DevBuf<int>& tile_op,
+                     DevBuf<int>& tile_src, DevBuf<int>* tile_phi, M2LTiles& out, TmpBuf<int>& tdst, cudaStream_t s) {
   const int lmax = pl->lmax;
   if (lmax - 1 > kMaxLev) return false;
   LevTab T{};
@@ -214,13 +231,13 @@ bool build_m2l_job_dev(fmmb_plan* pl, fmmb_plan::TcJob& job, int ys, cudaStream_
     T.vstart[l] = (int)V;
     T.boxoff[l] = pl->off_i[lev];
     T.srcoff[l] = pl->off_j[lev];
-    T.set[l] = pl->ops.m2l_sets > 1 ? lev - 2 : 0;
+    T.set[l] = sets ? lev - 2 : 0;
     V += (long long)pl->nbox_i[lev] * kM2LSlots;
+    if (V >= (1LL << 31) - 1) return false;  // the host loops take such sizes
   }
-  if (V >= (1LL << 31) - 1) return false;  // the host loops take such sizes
   T.vstart[T.nlev] = (int)V;
   const int nv = (int)V;
-  const int nops = pl->ops.m2l_sets * 316;
+  const int nops = (sets ? lmax - 1 : 1) * per;
   TmpBuf<int> pos(s);
   pos.alloc((size_t)nv + 1);
   m2l_pair_flags<<<nblk(nv, kT), kT, 0, s>>>(nv, T, pl->m2l_list.get(), pos.get());
@@ -228,17 +245,18 @@ bool build_m2l_job_dev(fmmb_plan* pl, fmmb_plan::TcJob& job, int ys, cudaStream_
   FMMB_CUDA(cudaMemsetAsync(pos.get() + nv, 0, sizeof(int), s));
   exclusive_scan(pos.get(), nv + 1, s);
   const int npair = d2h_int(pos.get() + nv, s);
-  TmpBuf<int> opk(s), ord(s), src(s), dst(s);
+  TmpBuf<int> opk(s), ord(s), src(s), dst(s), phi(s);
   opk.alloc(npair);
   ord.alloc(npair);
   src.alloc(npair);
   dst.alloc(npair);
+  if (tile_phi) phi.alloc(npair);
   m2l_pair_emit<<<nblk(nv, kT), kT, 0, s>>>(nv, T, pl->m2l_list.get(), pl->key_i.get(), pl->d_slot_rel.get(),
-                                           pl->d_rel_to_op.get(), pos.get(), opk.get(), ord.get(), src.get(),
-                                           dst.get());
+                                           rel_to_op, per, pos.get(), opk.get(), ord.get(), src.get(), dst.get(),
+                                           tile_phi ? phi.get() : nullptr);
   FMMB_CHECK_LAUNCH();
   radix_sort(opk.get(), ord.get(), npair, bits_for(nops), s);  // stable: enumeration order within an operator
-  // tiles of 128 pairs per operator
+  // tiles of tt pairs per operator
   TmpBuf<int> cnt(s), op_start(s), tile_base(s);
   cnt.alloc(nops + 1);
   op_start.alloc(nops + 1);
@@ -249,24 +267,92 @@ bool build_m2l_job_dev(fmmb_plan* pl, fmmb_plan::TcJob& job, int ys, cudaStream_
     FMMB_CHECK_LAUNCH();
   }
   FMMB_CUDA(cudaMemcpyAsync(op_start.get(), cnt.get(), (nops + 1) * sizeof(int), cudaMemcpyDeviceToDevice, s));
-  tiles_per_key<<<nblk(nops + 1, kT), kT, 0, s>>>(nops + 1, cnt.get(), tile_base.get());
+  tiles_per_key<<<nblk(nops + 1, kT), kT, 0, s>>>(nops + 1, tt, cnt.get(), tile_base.get());
   FMMB_CHECK_LAUNCH();
   exclusive_scan(op_start.get(), nops + 1, s);
   exclusive_scan(tile_base.get(), nops + 1, s);
   const int ntile = d2h_int(tile_base.get() + nops, s);
-  job.ntile = ntile;
-  job.tile_op.alloc(std::max(ntile, 1));
-  job.tile_src.alloc((size_t)std::max(ntile, 1) * 128);
-  job.tile_y.alloc((size_t)std::max(ntile, 1) * 2);
-  TmpBuf<int> tdst(s);
-  tdst.alloc((size_t)std::max(ntile, 1) * 128);
-  FMMB_CUDA(cudaMemsetAsync(job.tile_src.get(), 0xff, (size_t)ntile * 128 * sizeof(int), s));
-  FMMB_CUDA(cudaMemsetAsync(tdst.get(), 0xff, (size_t)ntile * 128 * sizeof(int), s));
+  const size_t ncol = (size_t)std::max(ntile, 1) * tt;
+  tile_op.alloc(std::max(ntile, 1));
+  tile_src.alloc(ncol);
+  tdst.alloc(ncol);
+  FMMB_CUDA(cudaMemsetAsync(tile_src.get(), 0xff, ncol * sizeof(int), s));
+  FMMB_CUDA(cudaMemsetAsync(tdst.get(), 0xff, ncol * sizeof(int), s));
+  if (tile_phi) {
+    tile_phi->alloc(ncol);
+    FMMB_CUDA(cudaMemsetAsync(tile_phi->get(), 0, ncol * sizeof(int), s));
+  }
   if (npair > 0) {
-    fill_tiles<<<nblk(npair, kT), kT, 0, s>>>(npair, opk.get(), ord.get(), src.get(), dst.get(), op_start.get(),
-                                             tile_base.get(), job.tile_op.get(), job.tile_src.get(), tdst.get());
+    fill_tiles<<<nblk(npair, kT), kT, 0, s>>>(npair, tt, opk.get(), ord.get(), src.get(), dst.get(),
+                                             tile_phi ? phi.get() : nullptr, op_start.get(), tile_base.get(),
+                                             tile_op.get(), tile_src.get(), tdst.get(),
+                                             tile_phi ? tile_phi->get() : nullptr);
     FMMB_CHECK_LAUNCH();
   }
+  out.npair = npair;
+  out.ntile = ntile;
+  return true;
+}
+
+}  // namespace
+
+void build_parity_job(fmmb_plan* pl, cudaStream_t s) {
+  const int ncls = (int)pl->ops.cls_geom.size();
+  const bool helm = helm_family(pl->cfg.kernel), sets = helm || pl->ref;
+  fmmb_plan::PairJob& job = pl->par_m2l;
+  M2LTiles t;
+  TmpBuf<int> tdst(s);
+  if (build_m2l_tiles(pl, sets, ncls, pl->d_rel_to_cls.get(), 32, job.tile_op, job.tile_src, &job.tile_phi, t, tdst, s)) {
+    job.tile_dst.alloc((size_t)std::max(t.ntile, 1) * 32);
+    FMMB_CUDA(cudaMemcpyAsync(job.tile_dst.get(), tdst.get(), (size_t)t.ntile * 32 * sizeof(int), cudaMemcpyDeviceToDevice, s));
+    FMMB_CUDA(cudaStreamSynchronize(s));
+    job.ntile = t.ntile;
+    job.tp = 32;
+    return;
+  }
+  // more box slots than an int enumerates: the same lists on the host
+  std::vector<int> key(pl->tot_i), lst((size_t)pl->tot_i * kM2LSlots);
+  FMMB_CUDA(cudaMemcpy(key.data(), pl->key_i.get(), key.size() * sizeof(int), cudaMemcpyDeviceToHost));
+  FMMB_CUDA(cudaMemcpy(lst.data(), pl->m2l_list.get(), lst.size() * sizeof(int), cudaMemcpyDeviceToHost));
+  std::vector<std::vector<std::array<int, 3>>> by((size_t)(sets ? pl->lmax - 1 : 1) * ncls);
+  for (int lev = 2; lev <= pl->lmax; lev++)
+    for (int b = 0; b < pl->nbox_i[lev]; b++) {
+      const int box = pl->off_i[lev] + b;
+      for (int sl = 0; sl < kM2LSlots; sl++) {
+        const int src = lst[(size_t)box * kM2LSlots + sl];
+        if (src < 0) continue;
+        const int rel = pl->ops.slot_rel[(key[box] & 7) * kM2LSlots + sl];
+        by[(size_t)(sets ? lev - 2 : 0) * ncls + pl->ops.rel_to_cls[rel]].push_back({pl->off_j[lev] + src, box, rel / 7});
+      }
+    }
+  std::vector<int> top, col[3];
+  for (size_t o = 0; o < by.size(); o++)
+    for (size_t k = 0; k < by[o].size(); k += 32) {
+      top.push_back((int)o);
+      for (size_t c = k; c < k + 32; c++)
+        for (int w = 0; w < 3; w++) col[w].push_back(c < by[o].size() ? by[o][c][w] : (w == 2 ? 0 : -1));
+    }
+  auto up = [](DevBuf<int>& d, const std::vector<int>& h) {
+    d.alloc(h.size());
+    if (!h.empty()) FMMB_CUDA(cudaMemcpy(d.get(), h.data(), h.size() * sizeof(int), cudaMemcpyHostToDevice));
+  };
+  up(job.tile_op, top);
+  up(job.tile_src, col[0]);
+  up(job.tile_dst, col[1]);
+  up(job.tile_phi, col[2]);
+  job.ntile = (int)top.size();
+  job.tp = 32;
+}
+
+bool build_m2l_job_dev(fmmb_plan* pl, fmmb_plan::TcJob& job, int ys, cudaStream_t s) {
+  M2LTiles t;
+  TmpBuf<int> tdst(s);
+  if (!build_m2l_tiles(pl, pl->ops.m2l_sets > 1, 316, pl->d_rel_to_op.get(), 128, job.tile_op, job.tile_src, nullptr, t,
+                       tdst, s))
+    return false;
+  const int npair = t.npair, ntile = t.ntile;
+  job.ntile = ntile;
+  job.tile_y.alloc((size_t)std::max(ntile, 1) * 2);
   if (ntile > 0) {
     fill_tile_y<<<nblk(ntile, kT), kT, 0, s>>>(ntile, job.tile_y.get());
     FMMB_CHECK_LAUNCH();

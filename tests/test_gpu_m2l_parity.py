@@ -1,0 +1,68 @@
+"""FP64 M2L by azimuth and reflection blocks: every block size (multiples of 8 and remainders, one and two tiles of
+rows per warp, the 16-pair form), all azimuths, several levels, part-filled tiles."""
+import numpy as np
+import pytest
+
+import old_fmm_bem_b200 as ob
+from oracle import pyoracle
+
+pytestmark = pytest.mark.gpu
+
+
+@pytest.mark.parametrize("ref", [False, True])
+@pytest.mark.parametrize("p", [1, 2, 3, 5, 6, 8, 11, 12, 14, 16, 20])
+def test_laplace_matches_oracle(p, ref):
+    # the local expansions and, in accurate semantics (the oracle sums in float in the other), the outputs; lists of a
+    # full 4^3 and 8^3 grid hold every relative position; the oracle applies the rotate / translate / rotate back steps
+    # one after another.  Bound: (p + 1)^2 roundings of 2^-53 per sum, growth of the recurrences below 100.
+    if ref and p == 20:
+        pytest.skip("the reference's float tables underflow at this order")
+    rng = np.random.default_rng(p)
+    n = 900
+    x = rng.random((3, n)).astype(np.float32)
+    q = rng.standard_normal(n).astype(np.float32)
+    with ob.Plan(kernel=ob.LAPLACE_G, p=p, lmax=3, precision=ob.FP64,
+                 semantics=ob.SEM_REFERENCE if ref else ob.SEM_ACCURATE, exclude_self=not ref) as pl:
+        pl.set_geometry(x, x, bbox=(0, 0, 0, 1))
+        pot, grad = pl.evaluate(q, f64=True)
+        loc = pl.expansions(1)
+    po, go = pyoracle.oracle_fmm(x, x, q, neq=0, p=p, lmax=3, ref_semantics=ref, exclude_self=not ref)[:2]
+    lo = pyoracle.oracle_expansions(1)
+    tol = 100 * (p + 1) ** 2 * 2.0 ** -53
+    assert np.linalg.norm(loc - lo) <= tol * np.linalg.norm(lo)
+    if not ref:
+        assert np.linalg.norm(pot - po) <= tol * np.linalg.norm(po)
+        assert np.linalg.norm(grad.reshape(3, -1) - go) <= tol * np.linalg.norm(go)
+
+
+@pytest.mark.parametrize("kernel", [ob.HELMHOLTZ_G, ob.YUKAWA])
+@pytest.mark.parametrize("p", [5, 8, 10, 13, 16, 17, 20])
+def test_helmholtz_axes_permuted(kernel, p):
+    # a cyclic permutation of the axes changes every azimuth and class but not the truncated expansions; the operators
+    # are projections on 2p + 8 by 4p + 16 nodes, whose aliased terms carry (radius / distance)^(2p + 16) <= 0.44^26 =
+    # 5e-10 (a wrong phase or block shows at the size of the far field itself)
+    rng = np.random.default_rng(100 + p)
+    n = 700
+    x = rng.random((3, n)).astype(np.float32)
+    q = rng.standard_normal(n) + (1j * rng.standard_normal(n) if kernel == ob.HELMHOLTZ_G else 0)
+    q = q.astype(np.complex64 if kernel == ob.HELMHOLTZ_G else np.float32)
+    res = []
+    for perm in ([0, 1, 2], [1, 2, 0]):
+        y = np.ascontiguousarray(x[perm])
+        with ob.Plan(kernel=kernel, p=p, lmax=3, precision=ob.FP64, semantics=ob.SEM_ACCURATE, exclude_self=True,
+                     wavenumber=3.0) as pl:
+            pl.set_geometry(y, y, bbox=(0, 0, 0, 1))
+            res.append(np.asarray(pl.evaluate(q, f64=True)[0]))
+    assert np.linalg.norm(res[0] - res[1]) <= 1e-9 * np.linalg.norm(res[0])
+
+
+def test_mixed_above_the_tensor_core_orders():
+    # p = 16 in the mixed form takes the FP64 M2L
+    rng = np.random.default_rng(3)
+    x = rng.random((3, 3000)).astype(np.float32)
+    q = rng.standard_normal(3000).astype(np.float32)
+    with ob.Plan(kernel=ob.LAPLACE_G, p=16, lmax=3, precision=ob.MIXED, semantics=ob.SEM_ACCURATE, exclude_self=True) as pl:
+        pl.set_geometry(x, x, bbox=(0, 0, 0, 1))
+        pot, _ = pl.evaluate(q, f64=True)
+        want, _ = pl.direct(q)
+    assert np.linalg.norm(pot - want) <= 1e-6 * np.linalg.norm(want)
