@@ -111,7 +111,7 @@ void upload_static_ops(fmmb_plan* pl) {
   upload(pl->d_phi, o.phi, s);
 }
 
-// FP64 M2L (m2l_parity.cu): the plain-FP64 form, the orders above the
+// FP64 M2L (m2l_parity.cuh): the plain-FP64 form, the orders above the
 // tensor-core M2L's range, and the Helmholtz family
 bool parity_m2l(const fmmb_plan* pl) {
   return pl->cfg.precision != FMMB_MIXED || pl->K > tc_max_k() || helm_family(pl->cfg.kernel);
@@ -640,6 +640,7 @@ void run_parity(fmmb_plan* pl, int mode, cudaStream_t m) {
   a.phi = reinterpret_cast<const double2*>(pl->d_phi.get());
   a.xin = pl->M.get();
   a.out = pl->L.get();
+  a.err = pl->d_err.get();
   launch_m2l_parity(mode, a, m);
 }
 
@@ -957,7 +958,7 @@ int evaluate_impl(fmmb_plan* pl, const float* q, T* pot, T* grad) {
       const int e = *pl->h_err;
       *pl->h_err = 0;
       FMMB_CUDA(cudaMemsetAsync(pl->d_err.get(), 0, sizeof(int), pl->st.main));
-      throw Error{FMMB_ERR_CUDA, "tensor-core M2L pipeline wait timed out (code " + std::to_string(e) + ")"};
+      throw Error{FMMB_ERR_CUDA, "M2L pipeline wait timed out (code " + std::to_string(e) + ")"};
     }
     pl->ev_used = 0;
     pl->ev_phase.clear();
@@ -1676,7 +1677,7 @@ int fmmb_get_timings(fmmb_plan* pl, float* ms) {
     FMMB_REQUIRE(pl->timings_valid, FMMB_ERR_STATE, "no evaluate yet");
     FMMB_CUDA(cudaStreamSynchronize(pl->st.main));
     FMMB_CUDA(cudaStreamSynchronize(pl->st.side));
-    FMMB_REQUIRE(*pl->h_err == 0, FMMB_ERR_CUDA, "tensor-core M2L pipeline wait timed out");
+    FMMB_REQUIRE(*pl->h_err == 0, FMMB_ERR_CUDA, "M2L pipeline wait timed out");
     for (int k = 0; k < 7; k++) ms[k] = 0.0f;
     for (auto& ph : pl->ev_phase) {
       float t = 0;

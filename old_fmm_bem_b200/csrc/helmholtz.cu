@@ -25,7 +25,7 @@
 // target radial function at the sphere's radius.  The operators are stored in
 // the real 2K x 2K form acting on [re | im] (transposed, row stride 2K) and
 // applied by the FP64 pair kernel of kernels_fp64.cu; the M2L operators, only
-// those at azimuth 0, as the reflection blocks of m2l_parity.cu.
+// those at azimuth 0, as the reflection blocks of m2l_parity.cuh.
 //
 // The same code serves the Yukawa kernel (FMMB_YUKAWA, the reference's neq 10,
 // kernel/Helmholtz_G_p2p.cxx:18-23: (pi/2) e^{-lambda r} / (lambda r)) through
@@ -540,7 +540,7 @@ __global__ void __launch_bounds__(128) helm_direct(int i0, int i1, const int* __
 
 // ---------------------------------------------------------------- operators
 // (n, m) of row r of the parity images: (n, m > 0) by degree, O of them, then (n, 0)
-__device__ __forceinline__ void parity_row(int r, int O, int& n, int& m) {
+__device__ __forceinline__ void row_order(int r, int O, int& n, int& m) {
   if (r >= O) {
     n = r - O;
     m = 0;
@@ -555,7 +555,7 @@ __device__ __forceinline__ void parity_row(int r, int O, int& n, int& m) {
 // R_n(k|v|) Y_n^m(v^) at v = D + rad * s_q over the quadrature points s_q;
 // g[i][m'] = sum_j f[i][j] e^{-i m' phi_j} 2 pi / NP;
 // T[n'm'] = sum_i w_i g[i][m'] Ybar_n'^|m'|(x_i) / R'_n'(k rad).
-// PAR: the M2L operators at azimuth 0 as the images of m2l_parity.cu, T = A + iB
+// PAR: the M2L operators at azimuth 0 as the images of m2l_parity.cuh, T = A + iB
 // combined over +-m' (rows) for columns (n, m >= 0): even block T_{m'm} +
 // T_{-m'm}, odd block T_{m'm} - T_{-m'm}, halved for m' > 0 since the sum and
 // difference of the two blocks' results give orders m' and -m'.
@@ -574,7 +574,7 @@ __global__ void __launch_bounds__(256) helm_build_ops(int p, int K, double k, in
   const int E = (p + 1) * (p + 2) / 2, O = p * (p + 1) / 2;
   int n = 0, m;
   if (PAR) {
-    parity_row(c, O, n, m);
+    row_order(c, O, n, m);
   } else {
     while ((n + 1) * (n + 1) <= c) n++;
     m = c - n * n - n;
@@ -658,12 +658,12 @@ __global__ void __launch_bounds__(256) helm_build_ops(int p, int K, double k, in
     return make_double2((sr * d.x + si * d.y) / den, (si * d.x - sr * d.y) / den);
   };
   if (PAR) {
-    const int RE = (E + 7) / 8 * 8, RO = (O + 7) / 8 * 8, nprod = yuk ? 1 : 3;
-    const size_t se = (size_t)RE * (RE + 4), so = (size_t)RO * (RO + 4);
+    const int te = parity_tiles(E), to = parity_tiles(O), nprod = yuk ? 1 : 3;
+    const size_t se = parity_block(te), so = parity_block(to);
     double* img = opT + (size_t)o * ostride;
     for (int t = threadIdx.x; t < E; t += blockDim.x) {
       int n2, m2;
-      parity_row(t, O, n2, m2);
+      row_order(t, O, n2, m2);
       double2 e = target(n2, m2), d = make_double2(0.0, 0.0);
       if (m2 > 0) {
         const double2 v = target(n2, -m2);
@@ -671,9 +671,9 @@ __global__ void __launch_bounds__(256) helm_build_ops(int p, int K, double k, in
         e = make_double2(0.5 * (e.x + v.x), 0.5 * (e.y + v.y));
       }
       for (int pd = 0; pd < nprod; pd++) {  // A, -(A + B), B - A
-        img[pd * se + (size_t)c * (RE + 4) + t] = pd == 0 ? e.x : pd == 1 ? -(e.x + e.y) : e.y - e.x;
+        img[pd * se + parity_at(te, c, t)] = pd == 0 ? e.x : pd == 1 ? -(e.x + e.y) : e.y - e.x;
         if (t < O && c < O)
-          img[nprod * se + pd * so + (size_t)c * (RO + 4) + t] = pd == 0 ? d.x : pd == 1 ? -(d.x + d.y) : d.y - d.x;
+          img[nprod * se + pd * so + parity_at(to, c, t)] = pd == 0 ? d.x : pd == 1 ? -(d.x + d.y) : d.y - d.x;
       }
     }
     return;

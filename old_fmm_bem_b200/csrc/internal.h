@@ -126,7 +126,7 @@ struct Operators {
   std::vector<int> rel_to_op;  // [343] -> operator slot (0..315) or -1
   std::vector<int> op_rel;     // [316] rel code of each operator slot
   std::vector<int> slot_rel;   // [8][189] rel code of each M2L slot per octant
-  // FP64 M2L (m2l_parity.cu): the relative positions of one (dx^2 + dy^2, dz)
+  // FP64 M2L (m2l_parity.cuh): the relative positions of one (dx^2 + dy^2, dz)
   // share an operator, taken at azimuth 0; azimuth index of a code: code / 7
   std::vector<int> rel_to_cls;               // [343] -> class (0..60) or -1
   std::vector<std::array<int, 2>> cls_geom;  // [61] (dx^2 + dy^2, dz)

@@ -101,7 +101,7 @@ int pairs_f64_tile(int K, int npair, int nsm);
 // once per device, before any launch (and outside stream capture)
 void prepare_translate_pairs_f64();
 void launch_translate_pairs_f64(const PairArgs& a, cudaStream_t st);
-// FP64 M2L (m2l_parity.cu) over tiles of 32 pairs {operator, source row, target
+// FP64 M2L (m2l_parity.cuh) over tiles of 32 pairs {operator, source row, target
 // row, azimuth} of one operator: mode 0 Laplace, 1 Helmholtz, 2 Yukawa
 struct ParityArgs {
   int ntile, p;
@@ -111,8 +111,18 @@ struct ParityArgs {
   const double2* phi;  // [49 azimuths][21 orders] (cos m phi, sin m phi)
   const double* xin;   // source expansions
   double* out;         // target expansions, added to
+  int* err;            // set to a nonzero code on timeout
 };
-size_t parity_img_stride(int mode, int p);
+// An operator image: the blocks of `rows` rows and columns in chunks of 8
+// columns [chunk][k % 4][row, padded][k / 4]; a complex operator's three
+// images of the even block come before those of the odd one.
+constexpr int parity_tiles(int rows) { return (rows + 7) / 8; }
+constexpr int parity_row(int tiles) { return 8 * tiles + 2; }
+constexpr size_t parity_block(int tiles) { return (size_t)8 * tiles * parity_row(tiles); }
+__host__ __device__ inline size_t parity_at(int tiles, int col, int row) {
+  return (size_t)(col / 8) * 8 * parity_row(tiles) + 2 * ((col % 4) * parity_row(tiles) + row) + (col % 8) / 4;
+}
+size_t parity_img_stride(int mode, int p);  // doubles of one operator
 void prepare_m2l_parity(int mode, int p);  // once per device, outside stream capture
 void launch_m2l_parity(int mode, const ParityArgs& a, cudaStream_t st);
 // constant table of the FP32 P2M, once per device (outside stream capture)

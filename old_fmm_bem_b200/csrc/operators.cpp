@@ -351,7 +351,7 @@ void build_m2l_operators(Operators& ops, int lmax, float rd) {
   });
 }
 
-// The FP64 M2L's images (m2l_parity.cu): the operator of each class composed at
+// The FP64 M2L's images (m2l_parity.cuh): the operator of each class composed at
 // azimuth 0, where the rotations are real and Re, Im of the coefficients do
 // not mix: the even block acts on the Re parts (rows and columns (n, m > 0) by
 // degree, then (n, 0)), the odd one on the Im parts.
@@ -360,7 +360,7 @@ void build_parity_operators(Operators& ops, int lmax, float rd) {
   const bool ref = ops.ref;
   const std::vector<double> anm = anm_table(p, ref);
   const int ncls = (int)ops.cls_geom.size(), E = (p + 1) * (p + 2) / 2, O = p * (p + 1) / 2;
-  const int RE = (E + 7) / 8 * 8, RO = (O + 7) / 8 * 8;
+  const int te = parity_tiles(E), to = parity_tiles(O);
   const size_t stride = parity_img_stride(0, p);
   ops.par_sets = ref ? lmax - 1 : 1;
   ops.par_lmax = lmax;
@@ -385,11 +385,11 @@ void build_parity_operators(Operators& ops, int lmax, float rd) {
     const M2LZ Z{anm, ref, m2l_distance(g[0] + g[1] * g[1], set, rd, ref)};
     compose(p, Wf, Wb, Z, nullptr, T.data());
     double* e = &ops.par[(size_t)w * stride];
-    double* o = e + (size_t)RE * (RE + 4);
+    double* o = e + parity_block(te);
     for (int c = 0; c < E; c++)
-      for (int r = 0; r < E; r++) e[(size_t)c * (RE + 4) + r] = T[(size_t)re[r] * K + re[c]];
+      for (int r = 0; r < E; r++) e[parity_at(te, c, r)] = T[(size_t)re[r] * K + re[c]];
     for (int c = 0; c < O; c++)
-      for (int r = 0; r < O; r++) o[(size_t)c * (RO + 4) + r] = T[(size_t)im[r] * K + im[c]];
+      for (int r = 0; r < O; r++) o[parity_at(to, c, r)] = T[(size_t)im[r] * K + im[c]];
   });
 }
 
