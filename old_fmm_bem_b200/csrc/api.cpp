@@ -655,7 +655,7 @@ void run_one_helm(fmmb_plan* pl, const float* qs) {
   cudaStream_t m = pl->st.main, side = pl->serial ? m : pl->st.side;
   double* pot_near = pl->pot_s.get();
   double* pot_far = pl->pot_s.get() + 2 * (size_t)pl->ni;
-  const int nleaf_i = pl->nbox_i[lmax], nleaf_j = pl->nbox_j[lmax];
+  const int nleaf_j = pl->nbox_j[lmax];
   const double wleaf = (double)pl->bbox[3] / (double)(1 << lmax);
   FMMB_CUDA(cudaEventRecord(pl->st.fork, m));
   FMMB_CUDA(cudaStreamWaitEvent(side, pl->st.fork, 0));
@@ -663,7 +663,7 @@ void run_one_helm(fmmb_plan* pl, const float* qs) {
   {
     PhaseTimer tm(pl, 0, side);
     launch_helm_p2p(pl->cfg.precision == FMMB_MIXED, yuk, (float)k, (float)pl->cfg.eps2, pl->cfg.exclude_self != 0,
-                    (float)wleaf, pl->h_p2p_nwork, pl->h_p2p_work.get(),
+                    (float)wleaf, pl->p2p_nwork, pl->p2p_work.get(),
                     pl->leaf_i.get(), pl->leaf_j.get(), pl->p2p_list.get(), pl->tpos.get(), pl->spos.get(), qs,
                     pot_near, side);
   }
@@ -672,8 +672,8 @@ void run_one_helm(fmmb_plan* pl, const float* qs) {
   FMMB_CUDA(time_mark(pl, pl->ev[2], m));
   {
     PhaseTimer tm(pl, 1, m);
-    launch_helm_p2m(nleaf_j, p, k, yuk, pl->leafkey_j.get(), pl->leaf_j.get(), pl->spos.get(), qs, pl->bbox, wleaf,
-                    pl->M.get() + (size_t)pl->off_j[lmax] * 2 * K, m);
+    launch_helm_p2m(nleaf_j, p, k, yuk, pl->leafkey_j.get(), pl->leaf_j.get(), pl->spos.get(), qs,
+                    pl->d_ylm.get(), pl->bbox, wleaf, pl->M.get() + (size_t)pl->off_j[lmax] * 2 * K, m);
   }
   FMMB_CUDA(time_mark(pl, pl->ev[3], m));
   auto pairs_run = [&](const fmmb_plan::PairJob& job, double* xin, double* out, int atomic, int phase) {
@@ -704,7 +704,8 @@ void run_one_helm(fmmb_plan* pl, const float* qs) {
   FMMB_CUDA(time_mark(pl, pl->ev[5], m));
   {
     PhaseTimer tm(pl, 5, m);
-    launch_helm_l2p(nleaf_i, p, k, yuk, pl->leafkey_i.get(), pl->leaf_i.get(), pl->tpos.get(), pl->bbox, wleaf,
+    launch_helm_l2p(pl->m_p2p_nwork, p, k, yuk, pl->m_p2p_work.get(), pl->leafkey_i.get(), pl->leaf_i.get(),
+                    pl->tpos.get(), pl->d_ylm.get(), pl->bbox, wleaf,
                     pl->L.get() + (size_t)pl->off_i[lmax] * 2 * K, pot_far, m);
   }
   FMMB_CUDA(time_mark(pl, pl->ev[6], m));

@@ -47,24 +47,25 @@ namespace {
 
 constexpr int kMaxP = 20;
 
-// j_n(x), n = 0..nmax, x >= 0
+// j_n(x), n = 0..nmax, x >= 0, at j[n ST]
+template <int ST = 1>
 __device__ void sph_j(int nmax, double x, double* j) {
   if (x < 1e-6) {  // x^n / (2n+1)!! (1 - x^2 / (2 (2n+3)))
     double t = 1.0;
     for (int n = 0; n <= nmax; n++) {
-      j[n] = t * (1.0 - x * x / (2.0 * (2 * n + 3)));
+      j[n * ST] = t * (1.0 - x * x / (2.0 * (2 * n + 3)));
       t *= x / (2 * n + 3);
     }
     return;
   }
   double s, c;
   sincos(x, &s, &c);
-  const double j0 = s / x, j1 = s / (x * x) - c / x;
+  const double xi = 1.0 / x, j0 = s * xi, j1 = (j0 - c) * xi;
   j[0] = j0;
   if (nmax == 0) return;
   if (x > (double)nmax) {  // upward recurrence is stable
-    j[1] = j1;
-    for (int n = 1; n < nmax; n++) j[n + 1] = (2 * n + 1) / x * j[n] - j[n - 1];
+    j[ST] = j1;
+    for (int n = 1; n < nmax; n++) j[(n + 1) * ST] = (2 * n + 1) * xi * j[n * ST] - j[(n - 1) * ST];
     return;
   }
   // Miller: backward from N with arbitrary start, rescaled on the way, then
@@ -72,18 +73,18 @@ __device__ void sph_j(int nmax, double x, double* j) {
   const int N = nmax + 24 + (int)x;
   double jp1 = 0.0, jn = 1e-250;
   for (int n = N; n >= 1; n--) {
-    const double jm1 = (2 * n + 1) / x * jn - jp1;
+    const double jm1 = (2 * n + 1) * xi * jn - jp1;
     jp1 = jn;
     jn = jm1;
-    if (n - 1 <= nmax) j[n - 1] = jm1;
+    if (n - 1 <= nmax) j[(n - 1) * ST] = jm1;
     if (fabs(jn) > 1e250) {
       jn *= 1e-250;
       jp1 *= 1e-250;
-      for (int k = max(n - 1, 0); k <= nmax; k++) j[k] *= 1e-250;
+      for (int k = max(n - 1, 0); k <= nmax; k++) j[k * ST] *= 1e-250;
     }
   }
-  const double sc = fabs(j0) >= fabs(j1) ? j0 / j[0] : j1 / j[1];
-  for (int n = 0; n <= nmax; n++) j[n] *= sc;
+  const double sc = fabs(j0) >= fabs(j1) ? j0 / j[0] : j1 / j[ST];
+  for (int n = 0; n <= nmax; n++) j[n * ST] *= sc;
 }
 
 // y_n(x), n = 0..nmax, x > 0 (upward recurrence)
@@ -97,30 +98,32 @@ __device__ void sph_y(int nmax, double x, double* y) {
 
 // i_n(x), n = 0..nmax, x >= 0: Miller's backward recurrence
 // i_{n-1} = i_{n+1} + (2n+1)/x i_n, normalised by i_0 = sinh(x)/x
+template <int ST = 1>
 __device__ void sph_i(int nmax, double x, double* v) {
   if (x < 1e-6) {  // x^n / (2n+1)!! (1 + x^2 / (2 (2n+3)))
     double t = 1.0;
     for (int n = 0; n <= nmax; n++) {
-      v[n] = t * (1.0 + x * x / (2.0 * (2 * n + 3)));
+      v[n * ST] = t * (1.0 + x * x / (2.0 * (2 * n + 3)));
       t *= x / (2 * n + 3);
     }
     return;
   }
   const int N = nmax + 24 + (int)x;
   double ip1 = 0.0, in = 1e-250;
+  const double xi = 1.0 / x;
   for (int n = N; n >= 1; n--) {
-    const double im1 = (2 * n + 1) / x * in + ip1;
+    const double im1 = (2 * n + 1) * xi * in + ip1;
     ip1 = in;
     in = im1;
-    if (n - 1 <= nmax) v[n - 1] = im1;
+    if (n - 1 <= nmax) v[(n - 1) * ST] = im1;
     if (fabs(in) > 1e250) {
       in *= 1e-250;
       ip1 *= 1e-250;
-      for (int q = max(n - 1, 0); q <= nmax; q++) v[q] *= 1e-250;
+      for (int q = max(n - 1, 0); q <= nmax; q++) v[q * ST] *= 1e-250;
     }
   }
   const double sc = (sinh(x) / x) / v[0];
-  for (int n = 0; n <= nmax; n++) v[n] *= sc;
+  for (int n = 0; n <= nmax; n++) v[n * ST] *= sc;
 }
 
 // k_n(x), n = 0..nmax, x > 0, normalised k_0 = (pi/2) e^{-x} / x (upward recurrence)
@@ -132,9 +135,10 @@ __device__ void sph_k(int nmax, double x, double* v) {
 }
 
 // regular radial functions: j_n (Helmholtz) or i_n (Yukawa)
+template <int ST>
 __device__ __forceinline__ void radial_reg(int yuk, int nmax, double x, double* v) {
-  if (yuk) sph_i(nmax, x, v);
-  else sph_j(nmax, x, v);
+  if (yuk) sph_i<ST>(nmax, x, v);
+  else sph_j<ST>(nmax, x, v);
 }
 
 // direction of v: cos(theta), and e^{i phi} (1 on the axis)
@@ -198,305 +202,218 @@ __device__ __forceinline__ void box_centre(int key, Corner bbox, double w, doubl
   z = bbox.z + (cz + 0.5) * w;
 }
 
-__device__ __forceinline__ double warp_sum(double v) {
-  for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
-  return v;
+constexpr int kPts = 128;  // points per block of P2M and L2P
+
+// What P2M and L2P need of a point relative to its box centre.
+struct PointGeo {
+  double ct, st, cp, sp;
+};
+// direction of v, and the radial functions of k|v| at jv[n kPts]
+__device__ __forceinline__ PointGeo point_geo(int yuk, int p, double k, double vx, double vy, double vz, double* jv) {
+  const double r = sqrt(vx * vx + vy * vy + vz * vz);
+  PointGeo g;
+  direction(vx, vy, vz, r, g.ct, g.st, g.cp, g.sp);
+  radial_reg<kPts>(yuk, p, k * r, jv);
+  return g;
 }
 
+__device__ __forceinline__ void dmma884(double (&c)[2], double a, double b) {
+  asm volatile("mma.sync.aligned.m8n8k4.row.col.f64.f64.f64.f64 {%0,%1}, {%2}, {%3}, {%0,%1};"
+               : "+d"(c[0]), "+d"(c[1])
+               : "d"(a), "d"(b));
+}
+
+// The recurrence coefficients of Ybar (ylm, [n (n+1) / 2 + m]): n = m: Ybar_m^m =
+// x st Ybar_{m-1}^{m-1}; n = m + 1: x ct Ybar_m^m; above: x ct Ybar_{n-1}^m - y Ybar_{n-2}^m.
+
 // ---------------------------------------------------------------- P2M
-// One block (4 warps) per source leaf; a warp takes 32 points at a time, each
-// lane streams its point's terms over (m, n), warp sums go to shared FP64
-// accumulators; M = ik * sum.
-__global__ void __launch_bounds__(128) helm_p2m(int p, int K, double k, int yuk, const int* __restrict__ keys,
-                                                const int2* __restrict__ leaf, const float4* __restrict__ spos,
-                                                const float2* __restrict__ q, Corner bbox, double w,
-                                                double* __restrict__ M) {
-  extern __shared__ double acc[];  // [2K]
-  const int b = blockIdx.x;
-  for (int c = threadIdx.x; c < 2 * K; c += blockDim.x) acc[c] = 0.0;
-  __syncthreads();
+// One block (4 warps) per source leaf, 128 points at a time.
+//   M_n^{+-m} = ik sum_j (j_n Ybar_n^m)(j) (q_j e^{-+i m phi_j})
+// is for each order m a product of a (p + 1 - m) x points matrix and a points x
+// 4 one (real and imaginary parts, both signs), done on the FP64 tensor
+// instruction: the thread of a point leaves its radial functions in shared
+// memory; then every warp takes orders of its own (dealt so that all have the
+// same number of terms), evaluates the column of Ybar for 32 points at a time,
+// one a lane, and multiplies.  (Before, a warp added each coefficient over its
+// lanes with shuffles and computed a square root and a division for every
+// term: 1,048,576 points at p = 16 took 2.3 ms; 0.74 now.)
+constexpr int kMaxRow = kMaxP + 1;
+constexpr int kPS = 36;  // row stride of a warp's staging: 32 points, conflict-free fragment reads
+
+__global__ void __launch_bounds__(kPts) helm_p2m(int p, int K, double k, int yuk, const int* __restrict__ keys,
+                                                 const int2* __restrict__ leaf, const float4* __restrict__ spos,
+                                                 const float2* __restrict__ q, const double2* __restrict__ ylm,
+                                                 Corner bbox, double w, double* __restrict__ M) {
+  extern __shared__ double sm[];
+  const int NT = (p + 1) * (p + 2) / 2;
+  double* jv = sm;                            // [p + 1][kPts]
+  double* geo = jv + (p + 1) * kPts;          // ct, st, cos phi, sin phi, Re q, Im q: [6][kPts]
+  double* sum = geo + 6 * kPts;               // [terms, by order][4]
+  double* mine = sum + 4 * NT + (threadIdx.x >> 5) * (kMaxRow + 3 + 4) * kPS;  // the warp's [24 rows][kPS], [4][kPS]
+  double* wq = mine + (kMaxRow + 3) * kPS;
+  const int b = blockIdx.x, lane = threadIdx.x & 31, warp = threadIdx.x >> 5, gq = lane >> 2, tq = lane & 3;
+  for (int c = threadIdx.x; c < 4 * NT; c += kPts) sum[c] = 0.0;
   double xc, yc, zc;
   box_centre(keys[b], bbox, w, xc, yc, zc);
   const int2 lf = leaf[b];
-  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-  double jv[kMaxP + 1];
-  for (int base = warp * 32; base < lf.y; base += 128) {
-    const int i = base + lane;
-    const bool on = i < lf.y;
-    double vx = 0, vy = 0, vz = 0, qr = 0, qi = 0;
-    if (on) {
-      const float4 s = spos[lf.x + i];
-      const float2 qq = q[lf.x + i];
-      vx = (double)s.x - xc;
-      vy = (double)s.y - yc;
-      vz = (double)s.z - zc;
-      qr = qq.x;
-      qi = qq.y;
-    }
-    const double r = sqrt(vx * vx + vy * vy + vz * vz);
-    double ct, st, cp, sp;
-    direction(vx, vy, vz, r, ct, st, cp, sp);
-    radial_reg(yuk, p, k * r, jv);
-    double ymm = 0.28209479177387814, er = 1.0, ei = 0.0;  // Ybar_m^m, e^{i m phi}
-    for (int m = 0; m <= p; m++) {
-      if (m > 0) {
-        ymm = ybar_mm_next(m, st, ymm);
-        const double t = er * cp - ei * sp;
-        ei = er * sp + ei * cp;
-        er = t;
+  for (int base = 0; base < lf.y; base += kPts) {
+    __syncthreads();  // the previous points are done with
+    {
+      const int i = base + threadIdx.x;
+      double v[3] = {0.0, 0.0, 0.0};
+      float2 qq = make_float2(0.f, 0.f);
+      if (i < lf.y) {
+        const float4 s = spos[lf.x + i];
+        qq = q[lf.x + i];
+        v[0] = (double)s.x - xc;
+        v[1] = (double)s.y - yc;
+        v[2] = (double)s.z - zc;
       }
-      double y2 = 0.0, y1 = ymm;
-      for (int n = m; n <= p; n++) {
-        double y;
-        if (n == m) y = ymm;
-        else if (n == m + 1) y = sqrt(2.0 * m + 3.0) * ct * ymm;
-        else y = ybar_next(n, m, ct, y1, y2);
-        if (n > m) {
+      const PointGeo g = point_geo(yuk, p, k, v[0], v[1], v[2], jv + threadIdx.x);
+      const double o[6] = {g.ct, g.st, g.cp, g.sp, qq.x, qq.y};
+#pragma unroll
+      for (int c = 0; c < 6; c++) geo[c * kPts + threadIdx.x] = o[c];
+    }
+    __syncthreads();
+    const int nch = min(kPts, lf.y - base + 31) / 32;  // groups of 32 points
+    double ymm[4], er[4], ei[4];                       // Ybar_m^m and e^{i m phi} of the lane's point of each group
+#pragma unroll
+    for (int ch = 0; ch < 4; ch++) {
+      ymm[ch] = 0.28209479177387814;  // 1 / sqrt(4 pi)
+      er[ch] = 1.0;
+      ei[ch] = 0.0;
+    }
+    int row0 = 0;
+    for (int m = 0; m <= p; row0 += p + 1 - m, m++) {
+      if (m > 0) {
+        const double xm = ylm[m * (m + 1) / 2 + m].x;
+#pragma unroll
+        for (int ch = 0; ch < 4; ch++) {
+          if (ch >= nch) break;
+          const int pt = 32 * ch + lane;
+          const double cp = geo[2 * kPts + pt], sp = geo[3 * kPts + pt];
+          ymm[ch] *= xm * geo[kPts + pt];
+          const double t = er[ch] * cp - ei[ch] * sp;
+          ei[ch] = er[ch] * sp + ei[ch] * cp;
+          er[ch] = t;
+        }
+      }
+      if (((m & 4) ? 3 - (m & 3) : (m & 3)) != warp) continue;  // another warp's order
+      double acc[3][2] = {};
+      const int nrow = p + 1 - m;
+#pragma unroll
+      for (int ch = 0; ch < 4; ch++) {
+        if (ch >= nch) break;
+        const int pt = 32 * ch + lane;
+        const double ct = geo[pt], qr = geo[4 * kPts + pt], qi = geo[5 * kPts + pt];
+        double y1 = ymm[ch], y2 = 0.0;
+        __syncwarp();  // the previous group's reads are done
+        mine[lane] = jv[m * kPts + pt] * y1;
+        for (int n = m + 1; n <= p; n++) {
+          const double2 c = ylm[n * (n + 1) / 2 + m];
+          const double y = fma(c.x * ct, y1, -c.y * y2);
           y2 = y1;
           y1 = y;
+          mine[(n - m) * kPS + lane] = jv[n * kPts + pt] * y;
         }
-        const double a = on ? jv[n] * y : 0.0;
-        // conj(Y_n^m) = Ybar e^{-i m phi}: q a (er - i ei)
-        double tr = warp_sum(a * (qr * er + qi * ei));
-        double ti = warp_sum(a * (qi * er - qr * ei));
-        if (lane == 0) {
-          atomicAdd(&acc[n * n + n + m], tr);
-          atomicAdd(&acc[K + n * n + n + m], ti);
+        wq[lane] = qr * er[ch] + qi * ei[ch];  // q e^{-i m phi}
+        wq[kPS + lane] = qi * er[ch] - qr * ei[ch];
+        wq[2 * kPS + lane] = qr * er[ch] - qi * ei[ch];  // q e^{+i m phi}
+        wq[3 * kPS + lane] = qi * er[ch] + qr * ei[ch];
+        __syncwarp();
+#pragma unroll
+        for (int k4 = 0; k4 < 32; k4 += 4) {
+          const double bf = gq < 4 ? wq[gq * kPS + k4 + tq] : 0.0;
+#pragma unroll
+          for (int rt = 0; rt < 3; rt++)
+            if (8 * rt < nrow) dmma884(acc[rt], mine[(8 * rt + gq) * kPS + k4 + tq], bf);
         }
-        if (m > 0) {  // conj(Y_n^{-m}) = Ybar e^{+i m phi}
-          tr = warp_sum(a * (qr * er - qi * ei));
-          ti = warp_sum(a * (qi * er + qr * ei));
-          if (lane == 0) {
-            atomicAdd(&acc[n * n + n - m], tr);
-            atomicAdd(&acc[K + n * n + n - m], ti);
+      }
+      if (tq < 2) {  // columns 2 tq, 2 tq + 1 of the four
+#pragma unroll
+        for (int rt = 0; rt < 3; rt++)
+          if (8 * rt + gq < nrow) {
+            sum[4 * (row0 + 8 * rt + gq) + 2 * tq] += acc[rt][0];
+            sum[4 * (row0 + 8 * rt + gq) + 2 * tq + 1] += acc[rt][1];
           }
-        }
       }
     }
   }
   __syncthreads();
   double* out = M + (size_t)b * 2 * K;
-  for (int c = threadIdx.x; c < K; c += blockDim.x) {
+  for (int c = threadIdx.x; c < K; c += kPts) {
+    int n = 0;
+    while ((n + 1) * (n + 1) <= c) n++;
+    const int m = c - n * n - n, am = abs(m);
+    const double* s = sum + 4 * (am * (p + 1) - am * (am - 1) / 2 + n - am) + (m < 0 ? 2 : 0);
     if (yuk) {  // (2 l / pi) (a + ib)
-      out[c] = 2.0 * k / M_PI * acc[c];
-      out[K + c] = 2.0 * k / M_PI * acc[K + c];
+      out[c] = 2.0 * k / M_PI * s[0];
+      out[K + c] = 2.0 * k / M_PI * s[1];
     } else {  // ik (a + ib) = -k b + i k a
-      out[c] = -k * acc[K + c];
-      out[K + c] = k * acc[c];
+      out[c] = -k * s[1];
+      out[K + c] = k * s[0];
     }
   }
 }
 
 // ---------------------------------------------------------------- L2P
-// One block per target leaf, one thread per target: phi = sum L j_n(kr) Y_n^m.
-__global__ void __launch_bounds__(128) helm_l2p(int p, int K, double k, int yuk, const int* __restrict__ keys,
-                                                const int2* __restrict__ leaf, const float4* __restrict__ tpos,
-                                                Corner bbox, double w, const double* __restrict__ L,
-                                                double2* __restrict__ pot) {
-  extern __shared__ double Ls[];  // [2K]
-  const int b = blockIdx.x;
-  for (int c = threadIdx.x; c < 2 * K; c += blockDim.x) Ls[c] = L[(size_t)b * 2 * K + c];
+// One block per work item of up to 128 targets of a leaf, one thread per
+// target: phi = sum L j_n(kr) Y_n^m, the recurrences' coefficients from the
+// table (computed per term, a square root and a division each, the 1,048,576
+// targets at p = 16 took 1.07 ms; 0.33 now).
+__global__ void __launch_bounds__(kPts) helm_l2p(int p, int K, double k, int yuk, const int2* __restrict__ work,
+                                                 const int* __restrict__ keys, const int2* __restrict__ leaf,
+                                                 const float4* __restrict__ tpos, const double2* __restrict__ ylm,
+                                                 Corner bbox, double w, const double* __restrict__ L,
+                                                 double2* __restrict__ pot) {
+  extern __shared__ double sm[];
+  double* Ls = sm;               // [2K]
+  double* jv = sm + 2 * K;       // [p + 1][kPts]
+  const int2 wk = work[blockIdx.x];
+  const int b = wk.x;
+  for (int c = threadIdx.x; c < 2 * K; c += kPts) Ls[c] = L[(size_t)b * 2 * K + c];
   __syncthreads();
   double xc, yc, zc;
   box_centre(keys[b], bbox, w, xc, yc, zc);
   const int2 lf = leaf[b];
-  double jv[kMaxP + 1];
-  for (int i = threadIdx.x; i < lf.y; i += blockDim.x) {
-    const float4 t = tpos[lf.x + i];
-    const double vx = (double)t.x - xc, vy = (double)t.y - yc, vz = (double)t.z - zc;
-    const double r = sqrt(vx * vx + vy * vy + vz * vz);
-    double ct, st, cp, sp;
-    direction(vx, vy, vz, r, ct, st, cp, sp);
-    radial_reg(yuk, p, k * r, jv);
-    double pr = 0, pi = 0;
-    double ymm = 0.28209479177387814, er = 1.0, ei = 0.0;
-    for (int m = 0; m <= p; m++) {
-      if (m > 0) {
-        ymm = ybar_mm_next(m, st, ymm);
-        const double tt = er * cp - ei * sp;
-        ei = er * sp + ei * cp;
-        er = tt;
+  const int i = wk.y + threadIdx.x;
+  if (i >= lf.y) return;
+  const float4 t = tpos[lf.x + i];
+  jv += threadIdx.x;
+  const PointGeo g = point_geo(yuk, p, k, (double)t.x - xc, (double)t.y - yc, (double)t.z - zc, jv);
+  double pr = 0, pi = 0;
+  double ymm = 0.28209479177387814, er = 1.0, ei = 0.0;
+  for (int m = 0; m <= p; m++) {
+    if (m > 0) {
+      ymm *= ylm[m * (m + 1) / 2 + m].x * g.st;
+      const double tt = er * g.cp - ei * g.sp;
+      ei = er * g.sp + ei * g.cp;
+      er = tt;
+    }
+    double y2 = 0.0, y1 = ymm;
+    double ar = 0, ai = 0, br = 0, bi = 0;  // sums over n of L_n^m and L_n^-m
+    for (int n = m; n <= p; n++) {
+      if (n > m) {
+        const double2 c = ylm[n * (n + 1) / 2 + m];
+        const double y = fma(c.x * g.ct, y1, -c.y * y2);
+        y2 = y1;
+        y1 = y;
       }
-      double y2 = 0.0, y1 = ymm;
-      for (int n = m; n <= p; n++) {
-        double y;
-        if (n == m) y = ymm;
-        else if (n == m + 1) y = sqrt(2.0 * m + 3.0) * ct * ymm;
-        else y = ybar_next(n, m, ct, y1, y2);
-        if (n > m) {
-          y2 = y1;
-          y1 = y;
-        }
-        const double a = jv[n] * y;
-        const int c = n * n + n + m;
-        // L_n^m e^{i m phi}
-        pr += a * (Ls[c] * er - Ls[K + c] * ei);
-        pi += a * (Ls[c] * ei + Ls[K + c] * er);
-        if (m > 0) {  // L_n^{-m} e^{-i m phi}
-          const int c2 = n * n + n - m;
-          pr += a * (Ls[c2] * er + Ls[K + c2] * ei);
-          pi += a * (Ls[K + c2] * er - Ls[c2] * ei);
-        }
-      }
+      const double a = jv[n * kPts] * y1;
+      const double* l = Ls + n * n + n;
+      ar = fma(a, l[m], ar);
+      ai = fma(a, l[K + m], ai);
+      br = fma(a, l[-m], br);
+      bi = fma(a, l[K - m], bi);
     }
-    pot[lf.x + i] = make_double2(pr, pi);
-  }
-}
-
-// ---------------------------------------------------------------- P2P
-// Pairs at zero distance are skipped when the plan excludes them; eps2 (the
-// plan's softening) is added to r^2.
-// One block (128 threads) per work item = up to 256 targets of one leaf, two
-// per thread (one shared-memory read of a source serves both); the sources of
-// the leaf's 27 neighbour slots are staged through shared memory in chunks of
-// 128.  Work items split large leaves, so the launch is not bound by the
-// densest leaf.  Mixed form: FP32 terms (hardware sine / cosine of the
-// phase reduced to [-pi, pi]), summed over 32 sources, then added in FP64;
-// FP64 form: everything in FP64.  Zero-distance pairs
-// contribute nothing (their inverse distance is taken as 0).
-template <bool YUK, bool REDUCE>
-__device__ __forceinline__ void helm_pair(float k, float eps2, bool excl, const float4 x, const float4 s,
-                                          const float2 q, float& fr, float& fi) {
-  const float dx = x.x - s.x, dy = x.y - s.y, dz = x.z - s.z;
-  const float d2 = dx * dx + dy * dy + dz * dz, r2 = d2 + eps2;
-  const float rinv = (excl && d2 == 0.f) || r2 == 0.f ? 0.f : rsqrtf(r2);
-  if (YUK) {  // real kernel e^{-l r} / r
-    const float e = __expf(-k * (r2 * rinv)) * rinv;
-    fr = fmaf(q.x, e, fr);
-    fi = fmaf(q.y, e, fi);
-    return;
-  }
-  // phase k r reduced to [-pi, pi] (the identity for k r < pi, the usual
-  // near-field range), then the hardware sine / cosine (absolute error ~4e-7
-  // there)
-  const float ph = k * (r2 * rinv);
-  const float red = REDUCE ? fmaf(-6.28318530717958647f, rintf(ph * 0.159154943091895336f), ph) : ph;
-  float sn, cs;
-  __sincosf(red, &sn, &cs);
-  fr += (q.x * cs - q.y * sn) * rinv;
-  fi += (q.x * sn + q.y * cs) * rinv;
-}
-template <bool YUK>
-__device__ __forceinline__ void helm_pair64(double k, double eps2, bool excl, const float4 x, const float4 s,
-                                            const float2 q, double& ar, double& ai) {
-  const double dx = (double)x.x - s.x, dy = (double)x.y - s.y, dz = (double)x.z - s.z;
-  const double d2 = dx * dx + dy * dy + dz * dz, r2 = d2 + eps2;
-  if ((excl && d2 == 0.0) || r2 == 0.0) return;
-  const double r = sqrt(r2);
-  if (YUK) {
-    const double e = exp(-k * r) / r;
-    ar += q.x * e;
-    ai += q.y * e;
-    return;
-  }
-  double sn, cs;
-  sincos(k * r, &sn, &cs);
-  ar += (q.x * cs - q.y * sn) / r;
-  ai += (q.x * sn + q.y * cs) / r;
-}
-
-// Near field.  A block of 128 threads takes a work item of up to 256 targets
-// of one leaf (2 per thread).  The sources of its (up to 27) neighbour leaves
-// are staged into shared memory as one list in chunks of kHC (warp 0 lays the
-// leaves end to end with one lane per neighbour slot: ballot + scan), so a
-// chunk costs two barriers whatever the leaf sizes -- the former per-leaf
-// staging paid two barriers per 128 sources of every leaf.  Each thread sums
-// runs of 32 sources in FP32 (mixed form) and promotes each run's partial sum
-// to FP64.  REDUCE: reduce the phase k r to [-pi, pi] before the hardware sine
-// and cosine; the launcher leaves it out when every near-field distance is
-// below pi / k (then the reduction is the identity: same values).
-constexpr int kHC = 1024;
-
-template <bool F32, bool YUK, bool REDUCE>
-__global__ void __launch_bounds__(128) helm_p2p(float k, float eps2, int excl, const int2* __restrict__ work,
-                                                const int2* __restrict__ leaf_i,
-                                                const int2* __restrict__ leaf_j, const int* __restrict__ list,
-                                                const float4* __restrict__ tpos, const float4* __restrict__ spos,
-                                                const float2* __restrict__ q, double2* __restrict__ pot) {
-  __shared__ float4 sp[kHC];
-  __shared__ float2 sq[kHC];
-  __shared__ int2 seg[32];  // (first source, count) of each non-empty neighbour leaf
-  __shared__ int vst[33];   // start of each leaf in the staged list, then the total
-  __shared__ int nseg_s;
-  const int2 wk = work[blockIdx.x];
-  const int b = wk.x;
-  const int2 li = leaf_i[b];
-  const int i0 = wk.y + threadIdx.x, i1 = i0 + 128;
-  const bool on0 = i0 < li.y, on1 = i1 < li.y;
-  const float4 x0 = on0 ? tpos[li.x + i0] : make_float4(0.f, 0.f, 0.f, 0.f);
-  const float4 x1 = on1 ? tpos[li.x + i1] : make_float4(0.f, 0.f, 0.f, 0.f);
-  if (threadIdx.x < 32) {
-    const int lane = threadIdx.x;
-    int2 sg = make_int2(0, 0);
-    if (lane < kP2PSlots) {
-      const int jl = list[(size_t)b * kP2PSlots + lane];
-      if (jl >= 0) sg = leaf_j[jl];
-    }
-    const bool has = sg.y > 0;
-    const unsigned mask = __ballot_sync(0xffffffffu, has);
-    const int pos = __popc(mask & ((1u << lane) - 1u));
-    int incl = has ? sg.y : 0;
-#pragma unroll
-    for (int o = 1; o < 32; o <<= 1) {
-      const int t = __shfl_up_sync(0xffffffffu, incl, o);
-      if (lane >= o) incl += t;
-    }
-    if (has) {
-      seg[pos] = sg;
-      vst[pos] = incl - sg.y;
-    }
-    if (lane == 31) {
-      vst[__popc(mask)] = incl;  // the total
-      nseg_s = __popc(mask);
+    pr += ar * er - ai * ei;  // e^{i m phi}
+    pi += ar * ei + ai * er;
+    if (m > 0) {  // e^{-i m phi}
+      pr += br * er + bi * ei;
+      pi += bi * er - br * ei;
     }
   }
-  __syncthreads();
-  const int nseg = nseg_s, ntot = vst[nseg];
-  double ar0 = 0, ai0 = 0, ar1 = 0, ai1 = 0;
-  for (int c0 = 0; c0 < ntot; c0 += kHC) {
-    const int nc = min(kHC, ntot - c0);
-    __syncthreads();  // the previous chunk's readers are done
-    for (int u = threadIdx.x; u < nc; u += 128) {
-      const int v = c0 + u;
-      int sgi = 0;
-      while (sgi + 1 < nseg && vst[sgi + 1] <= v) sgi++;
-      const int j = seg[sgi].x + (v - vst[sgi]);
-      sp[u] = spos[j];
-      sq[u] = q[j];
-    }
-    __syncthreads();
-    if (!on0) continue;
-    for (int r0 = 0; r0 < nc; r0 += 32) {
-      const int re = min(nc, r0 + 32);
-      if (F32) {
-        float fr0 = 0.f, fi0 = 0.f, fr1 = 0.f, fi1 = 0.f;
-        if (on1) {
-          for (int jj = r0; jj < re; jj++) {
-            const float4 sv = sp[jj];
-            const float2 qq = sq[jj];
-            helm_pair<YUK, REDUCE>(k, eps2, excl, x0, sv, qq, fr0, fi0);
-            helm_pair<YUK, REDUCE>(k, eps2, excl, x1, sv, qq, fr1, fi1);
-          }
-        } else {
-          for (int jj = r0; jj < re; jj++) helm_pair<YUK, REDUCE>(k, eps2, excl, x0, sp[jj], sq[jj], fr0, fi0);
-        }
-        ar0 += fr0;
-        ai0 += fi0;
-        ar1 += fr1;
-        ai1 += fi1;
-      } else {
-        for (int jj = r0; jj < re; jj++) {
-          const float4 sv = sp[jj];
-          const float2 qq = sq[jj];
-          helm_pair64<YUK>((double)k, (double)eps2, excl, x0, sv, qq, ar0, ai0);
-          if (on1) helm_pair64<YUK>((double)k, (double)eps2, excl, x1, sv, qq, ar1, ai1);
-        }
-      }
-    }
-  }
-  const double coef = 0.25 / M_PI;
-  if (on0) pot[li.x + i0] = make_double2(coef * ar0, coef * ai0);
-  if (on1) pot[li.x + i1] = make_double2(coef * ar1, coef * ai1);
+  pot[lf.x + i] = make_double2(pr, pi);
 }
 
 // ---------------------------------------------------------------- direct
@@ -732,35 +649,16 @@ __global__ void helm_finalize(int n, const int* __restrict__ perm, const double2
 
 unsigned nb(size_t n, int t) { return (unsigned)((n + t - 1) / t); }
 
+size_t helm_p2m_smem(int p) {
+  return ((size_t)(p + 1 + 6) * kPts + 2 * (size_t)(p + 1) * (p + 2) + (kPts / 32) * (size_t)(kMaxRow + 3 + 4) * kPS) *
+         sizeof(double);
+}
+
 }  // namespace
 
 void launch_helm_gather(int n, int nrhs, const int* perm, const float* q, float* qs, cudaStream_t st) {
   if (n <= 0) return;
   helm_gather<<<nb((size_t)n * nrhs, 256), 256, 0, st>>>(n, nrhs, perm, (const float2*)q, (float2*)qs);
-  FMMB_CHECK_LAUNCH();
-}
-
-void launch_helm_p2p(bool f32, bool yuk, float k, float eps2, bool excl, float leaf_side, int nwork,
-                     const int2* work, const int2* leaf_i, const int2* leaf_j, const int* list, const float4* tpos,
-                     const float4* spos, const float* qs, double* pot, cudaStream_t st) {
-  if (nwork <= 0) return;
-  const float2* q2 = (const float2*)qs;
-  double2* p2 = (double2*)pot;
-  const int ex = excl ? 1 : 0;
-  // points of neighbouring leaves lie at most 2 sqrt(3) leaf sides apart:
-  // below pi / k (with a margin for the float phase) no reduction is needed
-  const double rmax = std::sqrt(12.0 * (double)leaf_side * leaf_side + (double)eps2);
-  const bool reduce = !((double)k * rmax < 0.999 * M_PI);
-  if (f32 && !yuk && reduce)
-    helm_p2p<true, false, true><<<nwork, 128, 0, st>>>(k, eps2, ex, work, leaf_i, leaf_j, list, tpos, spos, q2, p2);
-  else if (f32 && !yuk)
-    helm_p2p<true, false, false><<<nwork, 128, 0, st>>>(k, eps2, ex, work, leaf_i, leaf_j, list, tpos, spos, q2, p2);
-  else if (f32)
-    helm_p2p<true, true, false><<<nwork, 128, 0, st>>>(k, eps2, ex, work, leaf_i, leaf_j, list, tpos, spos, q2, p2);
-  else if (!yuk)
-    helm_p2p<false, false, false><<<nwork, 128, 0, st>>>(k, eps2, ex, work, leaf_i, leaf_j, list, tpos, spos, q2, p2);
-  else
-    helm_p2p<false, true, false><<<nwork, 128, 0, st>>>(k, eps2, ex, work, leaf_i, leaf_j, list, tpos, spos, q2, p2);
   FMMB_CHECK_LAUNCH();
 }
 
@@ -783,23 +681,28 @@ template void launch_helm_finalize_real<double>(int, const int*, const double*, 
                                                 cudaStream_t);
 
 void launch_helm_p2m(int nleaf, int p, double k, bool yuk, const int* keys, const int2* leaf, const float4* spos,
-                     const float* qs, const float* bbox, double w, double* M, cudaStream_t st) {
+                     const float* qs, const double* ylm, const float* bbox, double w, double* M, cudaStream_t st) {
   if (nleaf <= 0) return;
   const int K = (p + 1) * (p + 1);
   const Corner c{bbox[0], bbox[1], bbox[2]};  // host array
-  helm_p2m<<<nleaf, 128, 2 * K * sizeof(double), st>>>(p, K, k, yuk ? 1 : 0, keys, leaf, spos, (const float2*)qs, c,
-                                                        w, M);
+  helm_p2m<<<nleaf, kPts, helm_p2m_smem(p), st>>>(p, K, k, yuk ? 1 : 0, keys, leaf, spos, (const float2*)qs,
+                                                  (const double2*)ylm, c, w, M);
   FMMB_CHECK_LAUNCH();
 }
 
-void launch_helm_l2p(int nleaf, int p, double k, bool yuk, const int* keys, const int2* leaf, const float4* tpos,
-                     const float* bbox, double w, const double* L, double* pot, cudaStream_t st) {
-  if (nleaf <= 0) return;
+void launch_helm_l2p(int nwork, int p, double k, bool yuk, const int2* work, const int* keys, const int2* leaf,
+                     const float4* tpos, const double* ylm, const float* bbox, double w, const double* L, double* pot,
+                     cudaStream_t st) {
+  if (nwork <= 0) return;
   const int K = (p + 1) * (p + 1);
   const Corner c{bbox[0], bbox[1], bbox[2]};  // host array
-  helm_l2p<<<nleaf, 128, 2 * K * sizeof(double), st>>>(p, K, k, yuk ? 1 : 0, keys, leaf, tpos, c, w, L,
-                                                        (double2*)pot);
+  helm_l2p<<<nwork, kPts, (2 * (size_t)K + (p + 1) * kPts) * sizeof(double), st>>>(
+      p, K, k, yuk ? 1 : 0, work, keys, leaf, tpos, (const double2*)ylm, c, w, L, (double2*)pot);
   FMMB_CHECK_LAUNCH();
+}
+
+void prepare_helm(int p) {
+  FMMB_CUDA(cudaFuncSetAttribute(helm_p2m, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)helm_p2m_smem(p)));
 }
 
 void launch_helm_direct(int i0, int i1, const int* inv_i, const float4* tpos, int nj, const float4* spos,

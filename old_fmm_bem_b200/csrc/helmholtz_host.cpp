@@ -201,23 +201,26 @@ void helm_setup(fmmb_plan* pl) {
   }
   prepare_m2l_parity(yuk ? 2 : 1, p);
   build_parity_job(pl, s);
-  // P2P work items: every target leaf in pieces of 256 targets
-  {
-    const int nleaf = pl->nbox_i[lmax];
-    std::vector<int2> leaf(nleaf), work;
-    FMMB_CUDA(cudaMemcpy(leaf.data(), pl->leaf_i.get(), nleaf * sizeof(int2), cudaMemcpyDeviceToHost));
-    for (int b = 0; b < nleaf; b++)
-      for (int t = 0; t < leaf[b].y; t += 256) work.push_back(make_int2(b, t));
-    upload_vec(pl->h_p2p_work, work);
-    pl->h_p2p_nwork = (int)work.size();
-  }
-  // inverse target permutation (caller -> sorted) for the direct sum
-  {
-    std::vector<int> perm(pl->ni), inv(pl->ni);
-    FMMB_CUDA(cudaMemcpy(perm.data(), pl->perm_i.get(), pl->ni * sizeof(int), cudaMemcpyDeviceToHost));
-    for (int i = 0; i < pl->ni; i++) inv[perm[i]] = i;
-    upload_vec(pl->inv_i, inv);
-  }
+  // near-field work items and the inverse target permutation of the direct sum
+  build_p2p_work_dev(pl, s);
+  build_inverse_perm_dev(pl, s);
+  // recurrence coefficients of Ybar
+  std::vector<double> ylm((size_t)(p + 1) * (p + 2), 0.0);
+  for (int n = 0; n <= p; n++)
+    for (int m = 0; m <= n; m++) {
+      double* c = &ylm[(size_t)(n * (n + 1) / 2 + m) * 2];
+      if (n == m) {
+        c[0] = m ? std::sqrt((2.0 * m + 1.0) / (2.0 * m)) : 1.0;
+      } else if (n == m + 1) {
+        c[0] = std::sqrt(2.0 * m + 3.0);
+      } else {
+        const double a = std::sqrt((4.0 * n * n - 1.0) / ((double)n * n - (double)m * m));
+        c[0] = a;
+        c[1] = a * std::sqrt((((double)n - 1) * (n - 1) - (double)m * m) / (4.0 * (n - 1) * (n - 1) - 1.0));
+      }
+    }
+  upload_vec(pl->d_ylm, ylm);
+  prepare_helm(p);
   const int nr = pl->cfg.nrhs;
   pl->qs.alloc((size_t)2 * pl->nj * nr);
   pl->M.alloc((size_t)pl->tot_j * 2 * K);

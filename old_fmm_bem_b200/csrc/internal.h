@@ -304,8 +304,7 @@ struct fmmb_plan {
   // [M2M child levels 3..lmax x 8 | L2L likewise]
   fmmb::DevBuf<double> d_hops;
   int hop_m2m0 = 0, hop_l2l0 = 0;
-  fmmb::DevBuf<int2> h_p2p_work;  // P2P work items: (target leaf, first target), up to 256 targets each
-  int h_p2p_nwork = 0;
+  fmmb::DevBuf<double> d_ylm;  // [n (n+1) / 2 + m][2] recurrence coefficients of Ybar (helmholtz.cu)
   fmmb::DevBuf<double> pot_s, grad_s;        // sorted outputs [ni], [3][ni]
   fmmb::DevBuf<float> stage_f;               // host<->device staging
   fmmb::DevBuf<double> stage_d;

@@ -192,9 +192,11 @@ void launch_helm_finalize_real(int n, const int* perm, const double* near, const
                                cudaStream_t st);
 // bbox: the plan's host copy {xmin, ymin, zmin, rd}
 void launch_helm_p2m(int nleaf, int p, double k, bool yuk, const int* keys, const int2* leaf, const float4* spos,
-                     const float* qs, const float* bbox, double w, double* M, cudaStream_t st);
-void launch_helm_l2p(int nleaf, int p, double k, bool yuk, const int* keys, const int2* leaf, const float4* tpos,
-                     const float* bbox, double w, const double* L, double* pot, cudaStream_t st);
+                     const float* qs, const double* ylm, const float* bbox, double w, double* M, cudaStream_t st);
+void launch_helm_l2p(int nwork, int p, double k, bool yuk, const int2* work, const int* keys, const int2* leaf,
+                     const float4* tpos, const double* ylm, const float* bbox, double w, const double* L, double* pot,
+                     cudaStream_t st);
+void prepare_helm(int p);  // shared-memory limits, outside stream capture
 void launch_helm_direct(int i0, int i1, const int* inv_i, const float4* tpos, int nj, const float4* spos,
                         const float* qs, double k, bool yuk, double eps2, bool excl, double* out, cudaStream_t st);
 template <typename T>
