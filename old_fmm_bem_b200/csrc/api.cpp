@@ -778,8 +778,8 @@ void run_one(fmmb_plan* pl, const float* qs, bool want_grad) {
                               pl->spos.get(), pl->snrm.get(), qs, pl->bbox, rb_leaf, Mleaf, m);
       }
       if (!done)
-        launch_p2m_cart(ker, nleaf_j, p, K, pl->leafkey_j.get(), pl->leaf_j.get(), pl->spos.get(), pl->snrm.get(), qs,
-                        pl->d_fac.get(), pl->bbox, rb_leaf, Mleaf, m);
+        launch_p2m_dmma(ker, nleaf_j, p, K, pl->leafkey_j.get(), pl->leaf_j.get(), pl->spos.get(), pl->snrm.get(), qs,
+                        pl->d_fac.get(), s, pl->bbox, rb_leaf, Mleaf, m);
     }
   }
   FMMB_CUDA(time_mark(pl, pl->ev[3], m));
@@ -875,9 +875,10 @@ void run_one(fmmb_plan* pl, const float* qs, bool want_grad) {
                launch_l2p_f32(ker, pl->m_p2p_nwork, pl->m_p2p_work.get(), p, K, pl->leafkey_i.get(), pl->leaf_i.get(), pl->tpos.get(),
                               pl->tnrm.get(), pl->d_fac.get(), pl->bbox, rb_leaf, s.coef,
                               pl->L.get() + (size_t)pl->off_i[lmax] * K, pot_far, g_far, pl->ni, m)))
-      launch_l2p_cart(ker, nleaf_i, p, K, pl->leafkey_i.get(), pl->leaf_i.get(), pl->tpos.get(),
-                      pl->tnrm.get(), pl->d_fac.get(), pl->bbox, rb_leaf, s.coef, pl->L.get() + (size_t)pl->off_i[lmax] * K,
-                      pot_far, ker == FMMB_LAPLACE_GNI ? nullptr : g_far, pl->ni, m);
+      launch_l2p_cart(ker, pl->m_p2p_nwork, pl->m_p2p_work.get(), p, K, pl->leafkey_i.get(), pl->leaf_i.get(),
+                      pl->tpos.get(), pl->tnrm.get(), pl->d_fac.get(), pl->bbox, rb_leaf, s.coef,
+                      pl->L.get() + (size_t)pl->off_i[lmax] * K, pot_far, ker == FMMB_LAPLACE_GNI ? nullptr : g_far,
+                      pl->ni, m);
     if (want_grad && ker == FMMB_LAPLACE_GNI && !pl->ref)  // its gradient needs the Hessian of the local expansion
       launch_l2p_hess_gni(nleaf_i, p, K, pl->leafkey_i.get(), pl->leaf_i.get(), pl->tpos.get(), pl->tnrm.get(),
                           pl->d_fac.get(), pl->bbox, rb_leaf, s.coef, pl->L.get() + (size_t)pl->off_i[lmax] * K, g_far,

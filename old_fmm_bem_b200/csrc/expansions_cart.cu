@@ -40,6 +40,20 @@ __constant__ double c_inv[41] = {0.0,      1.0 / 1,  1.0 / 2,  1.0 / 3,  1.0 / 4
                                  1.0 / 24, 1.0 / 25, 1.0 / 26, 1.0 / 27, 1.0 / 28, 1.0 / 29, 1.0 / 30, 1.0 / 31,
                                  1.0 / 32, 1.0 / 33, 1.0 / 34, 1.0 / 35, 1.0 / 36, 1.0 / 37, 1.0 / 38, 1.0 / 39,
                                  1.0 / 40};
+// Recurrence of A_n^m (below): A_n = alpha z A_{n-1} - beta r^2 A_{n-2}, alpha =
+// (2n-1)/(n-m), beta = (n+m-1)/(n-m), at n (n+1) / 2 + m
+struct RecTab {
+  double2 d[231];
+  constexpr RecTab() : d() {
+    for (int n = 0; n <= 20; n++)
+      for (int m = 0; m < n; m++) {
+        d[n * (n + 1) / 2 + m].x = (2.0 * n - 1.0) / (n - m);
+        d[n * (n + 1) / 2 + m].y = (n + m - 1.0) / (n - m);
+      }
+  }
+  __device__ const double2& operator[](int i) const { return d[i]; }
+};
+__constant__ RecTab c_rec = RecTab();
 __device__ __forceinline__ cplx cmul(cplx a, cplx b) { return {a.re * b.re - a.im * b.im, a.re * b.im + a.im * b.re}; }
 __device__ __forceinline__ cplx cscale(cplx a, double s) { return {a.re * s, a.im * s}; }
 
@@ -57,109 +71,182 @@ __device__ __forceinline__ void box_center(int key, float xmin, float ymin, floa
 }
 
 // ------------------------------------------------------------------ P2M
-// One block (128 threads) per source leaf.  Lanes are grouped in segments of
-// SEG; lane m of a segment owns order m (column m of S) of one point, so a
-// block processes 128/SEG points at a time.  The dipole needs the neighbouring
-// columns m-1 and m+1 of the previous degree, which come from the adjacent
-// lanes by shuffles.  Each segment accumulates into its own shared-memory
-// copy of the multipole; the copies are summed at the end.
-template <int KER, int SEG>
-__global__ void __launch_bounds__(128) p2m_cart(int p, int K, const int* __restrict__ keys, const int2* __restrict__ leaf,
+// One block (4 warps) per source leaf, 128 points at a time.  With
+//   S_n^m = A_n^m s_m,  s_m = -(2m-1) (x + i y) s_{m-1},  A_m^m = 1 and A real,
+//   (n-m) A_n^m = (2n-1) z A_{n-1}^m - (n+m-1) r^2 A_{n-2}^m,
+// the sums over the points are, for each order m, a product of the real
+// (p + 1 - m) x points matrix A with a points x NCOL one (w s_m, real and
+// imaginary parts), done on the FP64 tensor instruction: every warp takes orders
+// of its own (dealt so that all have about the same number of terms), evaluates
+// the column of A for 32 points at a time, one a lane, and multiplies.  Charges
+// take one complex w = q; dipoles three, ((n_x - i n_y) / 2, (n_x + i n_y) / 2,
+// n_z) q, whose sums U_1..U_3 give by the ladder identities
+//   n . grad S_n^m: U_1[n-1, m+1] - (n+m)(n+m-1) U_2[n-1, m-1] + (n+m) U_3[n-1, m].
+// Reference semantics take the same sums with the reference's angles and
+// eps-shifted radius (kernel/G_p2m.cxx:28-55) in place of the coordinates.
+// Bound: the FP64 pipe (a quarter of the tensor instruction's columns hold a
+// charge's sums).  One lane per order and a shared-memory sum per term before:
+// 262,144 clustered points, p = 12: 0.93 ms; 0.19 now.
+constexpr int kPts = 128;
+constexpr int kPS = 36;     // row stride of a warp's staging: 32 points, conflict-free fragment reads
+constexpr int kRows = 24;   // orders' columns: up to 21 rows in tiles of 8
+
+__device__ __forceinline__ void dmma884(double (&c)[2], double a, double b) {
+  asm volatile("mma.sync.aligned.m8n8k4.row.col.f64.f64.f64.f64 {%0,%1}, {%2}, {%3}, {%0,%1};"
+               : "+d"(c[0]), "+d"(c[1])
+               : "d"(a), "d"(b));
+}
+
+// the reference's azimuth (kernel/G_p2m.cxx:33-41), coordinates relative to the box centre
+__device__ __forceinline__ double ref_azimuth(double x, double y, const Sem& s) {
+  if (fabs(x) + fabs(y) < s.ang_eps) return 0.0;
+  if (fabs(x) < s.ang_eps) return y / fabs(y) * s.pi_ang * 0.5;
+  if (x > 0) return atan(y / x);
+  return atan(y / x) + s.pi_ang;
+}
+
+template <int KER, bool REF>
+__global__ void __launch_bounds__(kPts) p2m_dmma(int p, int K, const int* __restrict__ keys, const int2* __restrict__ leaf,
                                                 const float4* __restrict__ spos, const float4* __restrict__ snrm,
-                                                const float* __restrict__ qs, const double* __restrict__ fac, float xmin,
-                                                float ymin, float zmin, double rb, double* __restrict__ M) {
-  constexpr int G = 128 / SEG;
-  extern __shared__ double acc[];  // [G][K]
-  const int g = threadIdx.x / SEG, m = threadIdx.x % SEG;
-  for (int k = threadIdx.x; k < G * K; k += blockDim.x) acc[k] = 0.0;
+                                                const float* __restrict__ qs, const double* __restrict__ fac, Sem sem,
+                                                float xmin, float ymin, float zmin, double rb, double* __restrict__ M) {
+  constexpr bool DIP = KER == FMMB_LAPLACE_GNJ;
+  constexpr int NCOL = DIP ? 6 : 2;
+  extern __shared__ double sm[];
+  const int NT = (p + 1) * (p + 2) / 2, lane = threadIdx.x & 31, warp = threadIdx.x >> 5, gq = lane >> 2, tq = lane & 3;
+  double* sum = sm;                                              // [terms, by order][NCOL]
+  double* mine = sum + NCOL * NT + warp * (kRows + NCOL) * kPS;  // the warp's columns of A and w s_m
+  double* wq = mine + kRows * kPS;
+  for (int c = threadIdx.x; c < NCOL * NT; c += kPts) sum[c] = 0.0;
   __syncthreads();
   const int b = blockIdx.x;
   double xc, yc, zc;
   box_center(keys[b], xmin, ymin, zmin, rb, xc, yc, zc);
   const int2 lf = leaf[b];
-  double* my = acc + g * K;
   const double inv_rb = 1.0 / rb;
-  const unsigned segmask = 0xffffffffu;  // every lane of the warp runs the same loop trip counts
-  const int rounds = (lf.y + G - 1) / G;
-  for (int it = 0; it < rounds; it++) {
-    const int jj = it * G + g;
-    const bool act = jj < lf.y;
-    const int j = lf.x + (act ? jj : 0);
-    const float4 xs = spos[j];
-    const double q = act ? (double)qs[j] : 0.0;
-    const double x = ((double)xs.x - xc) * inv_rb, y = ((double)xs.y - yc) * inv_rb, z = ((double)xs.z - zc) * inv_rb;
-    const double r2 = x * x + y * y + z * z;
-    // S_m^m = prod_{k<m} -(2k+1) (x + i y)
-    cplx smm = {1.0, 0.0};
-    for (int k = 0; k < m; k++) smm = cscale(cmul(smm, cplx{x, y}), -(2.0 * k + 1.0));
-    cplx s1 = {0.0, 0.0}, s2 = {0.0, 0.0};  // S_{n-1}^m, S_{n-2}^m
-    double qnx = 0, qny = 0, qnz = 0;
-    if (KER == FMMB_LAPLACE_GNJ) {
-      const float4 nv = snrm[j];
-      const float qf = act ? qs[j] : 0.f;
-      qnx = (double)(qf * nv.x) * inv_rb;
-      qny = (double)(qf * nv.y) * inv_rb;
-      qnz = (double)(qf * nv.z) * inv_rb;
-    }
-    for (int n = 0; n <= p; n++) {
-      cplx sn;
-      if (n < m) sn = {0.0, 0.0};
-      else if (n == m) sn = smm;
-      else if (n == m + 1) sn = cscale(s1, (2.0 * m + 1.0) * z);
-      else {
-        const double inv = c_inv[n - m];
-        const double a = (2.0 * n - 1.0) * z * inv, c = (n + m - 1.0) * r2 * inv;
-        sn = {a * s1.re - c * s2.re, a * s1.im - c * s2.im};
-      }
-      if (KER != FMMB_LAPLACE_GNJ) {
-        if (n >= m && m <= p) {
-          const double f = q * fac[ifull_d(n, m)];
-          if (m == 0) my[n * n] += f * sn.re;
-          else {
-            my[n * n + 2 * m - 1] += f * sn.re;
-            my[n * n + 2 * m] -= f * sn.im;
-          }
-        }
+  for (int base = 0; base < lf.y; base += kPts) {
+    const int nch = min(kPts, lf.y - base + 31) / 32;  // groups of 32 points, one point of each a lane
+    double x[4], y[4], z[4], r2[4], sr[4], si[4], w[4][DIP ? 3 : 1];
+#pragma unroll
+    for (int ch = 0; ch < 4; ch++) {
+      const int i = base + 32 * ch + lane;
+      const bool on = i < lf.y;
+      const int j = lf.x + (on ? i : 0);
+      const float4 v = spos[j];
+      const float q = on ? qs[j] : 0.f;
+      const double dx = (double)v.x - xc, dy = (double)v.y - yc, dz = (double)v.z - zc;
+      if (REF) {
+        const double rh = sqrt(dx * dx + dy * dy + dz * dz) + sem.rho_eps;
+        const double al = rh == 0.0 ? 0.0 : acos(dz / rh);
+        double sb, cb;
+        sincos(ref_azimuth(dx, dy, sem), &sb, &cb);
+        const double rs = rh / rb, xx = cos(al), s2 = sqrt((1 - xx) * (1 + xx));
+        x[ch] = rs * s2 * cb;
+        y[ch] = rs * s2 * sb;
+        z[ch] = rs * xx;
+        r2[ch] = rs * rs;
       } else {
-        // n . grad S_n^m from degree n-1 (s1): columns m+1 (lane above) and
-        // m-1 (lane below; for m = 0 the conjugate of column 1)
-        cplx up, dn;
-        up.re = __shfl_down_sync(segmask, s1.re, 1, SEG);
-        up.im = __shfl_down_sync(segmask, s1.im, 1, SEG);
-        dn.re = __shfl_up_sync(segmask, s1.re, 1, SEG);
-        dn.im = __shfl_up_sync(segmask, s1.im, 1, SEG);
-        if (m == SEG - 1) up = {0.0, 0.0};
-        double cm;
-        if (m == 0) {
-          dn = {up.re, -up.im};
-          cm = 1.0;
-        } else {
-          cm = -(double)(n + m) * (double)(n + m - 1);
-        }
-        if (n >= 1 && n >= m && m <= p) {
-          // D = 1/2 (nx - i ny) up + 1/2 (nx + i ny) cm dn + nz (n+m) s1
-          const cplx a = cmul(cplx{0.5 * qnx, -0.5 * qny}, up);
-          const cplx c = cmul(cplx{0.5 * qnx * cm, 0.5 * qny * cm}, dn);
-          const double d = qnz * (n + m);
-          const double Dre = a.re + c.re + d * s1.re, Dim = a.im + c.im + d * s1.im;
-          const double f = fac[ifull_d(n, m)];
-          if (m == 0) my[n * n] += f * Dre;
-          else {
-            my[n * n + 2 * m - 1] += f * Dre;
-            my[n * n + 2 * m] -= f * Dim;
-          }
+        x[ch] = dx * inv_rb;
+        y[ch] = dy * inv_rb;
+        z[ch] = dz * inv_rb;
+        r2[ch] = x[ch] * x[ch] + y[ch] * y[ch] + z[ch] * z[ch];
+      }
+      if (DIP) {
+        const float4 n = snrm[j];
+        w[ch][0] = 0.5 * ((double)(q * n.x) * inv_rb);
+        w[ch][DIP ? 1 : 0] = 0.5 * ((double)(q * n.y) * inv_rb);
+        w[ch][DIP ? 2 : 0] = (double)(q * n.z) * inv_rb;
+      } else {
+        w[ch][0] = (double)q;
+      }
+      sr[ch] = 1.0;
+      si[ch] = 0.0;
+    }
+    int row0 = 0;
+    for (int m = 0; m <= p; row0 += p + 1 - m, m++) {
+      if (m > 0) {
+        const double f = -(2.0 * m - 1.0);
+#pragma unroll
+        for (int ch = 0; ch < 4; ch++) {
+          const double t = f * (sr[ch] * x[ch] - si[ch] * y[ch]);
+          si[ch] = f * (sr[ch] * y[ch] + si[ch] * x[ch]);
+          sr[ch] = t;
         }
       }
-      s2 = s1;
-      s1 = sn;
+      if (((m & 4) ? 3 - (m & 3) : (m & 3)) != warp) continue;  // another warp's order
+      double acc[3][2] = {};
+      const int nrow = p + 1 - m;
+#pragma unroll
+      for (int ch = 0; ch < 4; ch++) {
+        if (ch >= nch) break;
+        __syncwarp();  // the previous group's reads are done
+        double a1 = 1.0, a2 = 0.0;
+        mine[lane] = 1.0;
+        for (int n = m + 1; n <= p; n++) {
+          const double2 ab = c_rec[n * (n + 1) / 2 + m];
+          const double a = fma(ab.x * z[ch], a1, -(ab.y * r2[ch]) * a2);
+          a2 = a1;
+          a1 = a;
+          mine[(n - m) * kPS + lane] = a;
+        }
+        if (DIP) {
+          const double cx = w[ch][0], cy = w[ch][DIP ? 1 : 0], cz = w[ch][DIP ? 2 : 0];
+          wq[lane] = cx * sr[ch] + cy * si[ch];  // (n_x - i n_y) / 2
+          wq[kPS + lane] = cx * si[ch] - cy * sr[ch];
+          wq[2 * kPS + lane] = cx * sr[ch] - cy * si[ch];  // (n_x + i n_y) / 2
+          wq[3 * kPS + lane] = cx * si[ch] + cy * sr[ch];
+          wq[4 * kPS + lane] = cz * sr[ch];
+          wq[5 * kPS + lane] = cz * si[ch];
+        } else {
+          wq[lane] = w[ch][0] * sr[ch];
+          wq[kPS + lane] = w[ch][0] * si[ch];
+        }
+        __syncwarp();
+#pragma unroll
+        for (int k4 = 0; k4 < 32; k4 += 4) {
+          const double bf = gq < NCOL ? wq[gq * kPS + k4 + tq] : 0.0;
+#pragma unroll
+          for (int rt = 0; rt < 3; rt++)
+            if (8 * rt < nrow) dmma884(acc[rt], mine[(8 * rt + gq) * kPS + k4 + tq], bf);
+        }
+      }
+      if (2 * tq < NCOL) {
+#pragma unroll
+        for (int rt = 0; rt < 3; rt++)
+          if (8 * rt + gq < nrow) {
+            sum[NCOL * (row0 + 8 * rt + gq) + 2 * tq] += acc[rt][0];
+            sum[NCOL * (row0 + 8 * rt + gq) + 2 * tq + 1] += acc[rt][1];
+          }
+      }
     }
   }
   __syncthreads();
-  for (int k = threadIdx.x; k < K; k += blockDim.x) {
-    double t = 0.0;
-#pragma unroll
-    for (int gg = 0; gg < G; gg++) t += acc[gg * K + k];
-    M[(size_t)b * K + k] = t;
+  auto U = [&](int n, int m, int u) -> cplx {
+    if (m < 0 || m > n) return {0.0, 0.0};
+    const double* s = sum + NCOL * (m * (p + 1) - m * (m - 1) / 2 + n - m) + 2 * u;
+    return {s[0], s[1]};
+  };
+  for (int idx = threadIdx.x; idx < NT; idx += kPts) {
+    int n = 0;
+    while ((n + 1) * (n + 2) / 2 <= idx) n++;
+    const int m = idx - n * (n + 1) / 2;
+    const double f = fac[ifull_d(n, m)];
+    cplx v = {0.0, 0.0};
+    if (!DIP) {
+      v = U(n, m, 0);
+    } else if (n > 0) {
+      const cplx up = U(n - 1, m + 1, 0), md = U(n - 1, m, DIP ? 2 : 0);
+      const cplx dn = m == 0 ? cplx{up.re, -up.im} : U(n - 1, m - 1, DIP ? 1 : 0);
+      const double cm = m == 0 ? 1.0 : -(double)(n + m) * (double)(n + m - 1);
+      v = {up.re + cm * dn.re + (n + m) * md.re, up.im + cm * dn.im + (n + m) * md.im};
+    }
+    double* o = M + (size_t)b * K + n * n;
+    if (m == 0) {
+      o[0] = f * v.re;
+    } else {
+      o[2 * m - 1] = f * v.re;
+      o[2 * m] = -f * v.im;
+    }
   }
 }
 
@@ -314,101 +401,140 @@ __global__ void __launch_bounds__(kP2MThreads) p2m_f32(int p, int K, const int2*
 }
 
 // ------------------------------------------------------------------ L2P
-// One block (64 threads) per target leaf.  The leaf's local expansion is
-// turned once into the coefficients of the potential and of the three
-// derivative expansions (ladder identities above), then each thread walks
-// the S_n^m of its point column by column.
+// One block (64 threads) per work item of up to 128 targets of a leaf, two
+// targets a thread.  The leaf's local expansion is turned once into the
+// coefficients of the potential (C_F) and of its three derivatives by the
+// ladder identities above (C_z; the x and y derivatives as the real part of
+// C_X S and the imaginary part of C_Y S); with S_n^m = A_n^m s_m, A real, a thread
+// sums the coefficients of an order over its degrees as reals times A and
+// multiplies by the complex s_m once per order.
+// Bound: the FP64 pipe and the recurrence's latency.  (One block per leaf and
+// complex sums per term: 262,144 clustered points, p = 12: 0.37 ms; 0.07 now.
+// The same loops in FP32, two targets side by side, ran the mixed form's L2P of
+// 1,048,576 points in 0.25 ms against 0.20 of the unrolled l2p_f32.)
 constexpr int kL2PThreads = 64;
 
-template <int KER>
-__global__ void __launch_bounds__(kL2PThreads) l2p_cart(int p, int K, const int* __restrict__ keys,
-                                                        const int2* __restrict__ leaf, const float4* __restrict__ tpos,
-                                                        const float4* __restrict__ tnrm, const double* __restrict__ fac,
-                                                        float xmin, float ymin, float zmin, double rb, double coef,
-                                                        const double* __restrict__ L, double* __restrict__ pot,
-                                                        double* __restrict__ grad, int ni) {
-  extern __shared__ double sm[];
-  const int P = (p + 1) * (p + 2) / 2;
-  cplx* Cphi = reinterpret_cast<cplx*>(sm);
-  cplx* Cz = Cphi + P;
-  cplx* Cp = Cz + P;
-  cplx* Cm = Cp + P;
-  double* Cs = reinterpret_cast<double*>(Cm + P);  // [p+1]
-  const int b = blockIdx.x;
+// POT / DER: the potential, its derivatives
+template <int KER, bool POT, bool DER>
+__global__ void __launch_bounds__(kL2PThreads) l2p_cart(int p, int K, const int2* __restrict__ work,
+                                                   const int* __restrict__ keys, const int2* __restrict__ leaf,
+                                                   const float4* __restrict__ tpos, const float4* __restrict__ tnrm,
+                                                   const double* __restrict__ fac, float xmin, float ymin, float zmin,
+                                                   double rb, double coef, const double* __restrict__ L,
+                                                   double* __restrict__ pot, double* __restrict__ grad, int ni) {
+  constexpr int NS = (POT ? 1 : 0) + (DER ? 3 : 0);  // complex sums per order
+  extern __shared__ double2 C[];                     // their coefficients [terms, by order][NS]
+  const int NT = (p + 1) * (p + 2) / 2;
+  const int2 wk = work[blockIdx.x];
+  const int b = wk.x;
   const double* Lb = L + (size_t)b * K;
   auto Lnm = [&](int n, int m) -> cplx {
     if (m == 0) return {Lb[n * n], 0.0};
     return {Lb[n * n + 2 * m - 1], Lb[n * n + 2 * m]};
   };
-  for (int idx = threadIdx.x; idx < P; idx += blockDim.x) {
+  for (int idx = threadIdx.x; idx < NT; idx += kL2PThreads) {
     int n = 0;
     while ((n + 1) * (n + 2) / 2 <= idx) n++;
     const int m = idx - n * (n + 1) / 2;
     const double wm = m ? 2.0 : 1.0;
-    Cphi[idx] = cscale(Lnm(n, m), wm * fac[ifull_d(n, m)]);
-    if (n < p) {
-      Cz[idx] = cscale(Lnm(n + 1, m), wm * fac[ifull_d(n + 1, m)] * (n + 1 + m));
-      Cp[idx] = (m >= 1) ? cscale(Lnm(n + 1, m - 1), (m - 1 ? 2.0 : 1.0) * fac[ifull_d(n + 1, m - 1)]) : cplx{0.0, 0.0};
-      Cm[idx] = cscale(Lnm(n + 1, m + 1), -2.0 * fac[ifull_d(n + 1, m + 1)] * (double)(n + m + 2) * (double)(n + m + 1));
-    } else {
-      Cz[idx] = Cp[idx] = Cm[idx] = cplx{0.0, 0.0};
+    double2* c = C + NS * (m * (p + 1) - m * (m - 1) / 2 + n - m);
+    auto put = [&](int k, cplx v) { c[k] = make_double2(v.re, v.im); };
+    if (POT) put(0, cscale(Lnm(n, m), wm * fac[ifull_d(n, m)]));
+    if (DER) {
+      cplx cz = {0.0, 0.0}, cx = cz, cy = cz;
+      if (n < p) {
+        cz = cscale(Lnm(n + 1, m), wm * fac[ifull_d(n + 1, m)] * (n + 1 + m));
+        const cplx cp = m >= 1 ? cscale(Lnm(n + 1, m - 1), (m - 1 ? 2.0 : 1.0) * fac[ifull_d(n + 1, m - 1)]) : cplx{0.0, 0.0};
+        const cplx cm = cscale(Lnm(n + 1, m + 1), -2.0 * fac[ifull_d(n + 1, m + 1)] * (double)(n + m + 2) * (double)(n + m + 1));
+        const double cs = m == 1 ? fac[ifull_d(n + 1, 0)] * Lb[(n + 1) * (n + 1)] : 0.0;  // of conj(S_n^1)
+        cx = {cp.re + cm.re + cs, cp.im + cm.im};
+        cy = {cp.re - cm.re + cs, cp.im - cm.im};
+      }
+      put(NS - 3, cz);
+      put(NS - 2, cx);
+      put(NS - 1, cy);
     }
   }
-  for (int n = threadIdx.x; n <= p; n += blockDim.x) Cs[n] = (n < p) ? fac[ifull_d(n + 1, 0)] * Lb[(n + 1) * (n + 1)] : 0.0;
   __syncthreads();
   double xc, yc, zc;
   box_center(keys[b], xmin, ymin, zmin, rb, xc, yc, zc);
   const int2 lf = leaf[b];
   const double inv_rb = 1.0 / rb;
-  for (int ii = threadIdx.x; ii < lf.y; ii += blockDim.x) {
-    const int i = lf.x + ii;
-    const float4 xt = tpos[i];
-    const double x = ((double)xt.x - xc) * inv_rb, y = ((double)xt.y - yc) * inv_rb, z = ((double)xt.z - zc) * inv_rb;
-    const double r2 = x * x + y * y + z * z;
-    double F = 0, dzr = 0, dpr = 0, dpi = 0, dmr = 0, dmi = 0;
-    cplx smm = {1.0, 0.0};
-    for (int m = 0; m <= p; m++) {
-      if (m > 0) smm = cscale(cmul(smm, cplx{x, y}), -(2.0 * m - 1.0));
-      cplx s1 = {0.0, 0.0}, s2 = {0.0, 0.0};
-      for (int n = m; n <= p; n++) {
-        cplx sn;
-        if (n == m) sn = smm;
-        else if (n == m + 1) sn = cscale(s1, (2.0 * m + 1.0) * z);
-        else {
-          const double inv = c_inv[n - m];
-        const double a = (2.0 * n - 1.0) * z * inv, c = (n + m - 1.0) * r2 * inv;
-          sn = {a * s1.re - c * s2.re, a * s1.im - c * s2.im};
+  const int i0 = wk.y + threadIdx.x, end = min(lf.y, wk.y + 2 * kL2PThreads);
+  if (i0 >= end) return;
+  const int it[2] = {lf.x + i0, lf.x + (i0 + kL2PThreads < end ? i0 + kL2PThreads : i0)};
+  double x[2], y[2], z[2], r2[2], sr[2], si[2];
+  double F[2] = {0, 0}, gx[2] = {0, 0}, gy[2] = {0, 0}, gz[2] = {0, 0};
+#pragma unroll
+  for (int t = 0; t < 2; t++) {
+    const float4 v = tpos[it[t]];
+    x[t] = ((double)v.x - xc) * inv_rb;
+    y[t] = ((double)v.y - yc) * inv_rb;
+    z[t] = ((double)v.z - zc) * inv_rb;
+    r2[t] = x[t] * x[t] + y[t] * y[t] + z[t] * z[t];
+    sr[t] = 1.0;
+    si[t] = 0.0;
+  }
+  const double2* c = C;
+  for (int m = 0; m <= p; m++) {
+    double ur[2][NS], ui[2][NS], a1[2], a2[2];  // sums; A_n^m, A_{n-1}^m
+#pragma unroll
+    for (int t = 0; t < 2; t++) {
+      if (m > 0) {  // s_m = -(2m-1) (x + i y) s_{m-1}
+        const double f = -(2.0 * m - 1.0), tr = f * (sr[t] * x[t] - si[t] * y[t]);
+        si[t] = f * (sr[t] * y[t] + si[t] * x[t]);
+        sr[t] = tr;
+      }
+      a1[t] = 1.0;
+      a2[t] = 0.0;
+#pragma unroll
+      for (int k = 0; k < NS; k++) ur[t][k] = ui[t][k] = 0.0;
+    }
+    for (int n = m;; n++) {
+#pragma unroll
+      for (int k = 0; k < NS; k++) {
+        const double2 ck = c[k];
+#pragma unroll
+        for (int t = 0; t < 2; t++) {
+          ur[t][k] = fma(ck.x, a1[t], ur[t][k]);
+          ui[t][k] = fma(ck.y, a1[t], ui[t][k]);
         }
-        const int idx = n * (n + 1) / 2 + m;
-        const cplx cf = Cphi[idx];
-        F += cf.re * sn.re - cf.im * sn.im;  // Re(C S)
-        if (n < p) {
-          const cplx cz = Cz[idx], cp = Cp[idx], cmm = Cm[idx];
-          dzr += cz.re * sn.re - cz.im * sn.im;
-          dpr += cp.re * sn.re - cp.im * sn.im;
-          dpi += cp.re * sn.im + cp.im * sn.re;
-          dmr += cmm.re * sn.re - cmm.im * sn.im;
-          dmi += cmm.re * sn.im + cmm.im * sn.re;
-          if (m == 1) {  // Cs[n] * conj(S_n^1)
-            dmr += Cs[n] * sn.re;
-            dmi -= Cs[n] * sn.im;
-          }
-        }
-        s2 = s1;
-        s1 = sn;
+      }
+      c += NS;
+      if (n == p) break;
+      const double2 ab = c_rec[(n + 1) * (n + 2) / 2 + m];
+#pragma unroll
+      for (int t = 0; t < 2; t++) {
+        const double an = fma(ab.x * z[t], a1[t], -(ab.y * r2[t]) * a2[t]);
+        a2[t] = a1[t];
+        a1[t] = an;
       }
     }
-    const double gx = 0.5 * (dpr + dmr), gy = 0.5 * (dpi - dmi), gz = dzr;
-    const double c1 = coef * inv_rb, c2 = coef * inv_rb * inv_rb;
+    // times s_m: the potential and d/dz the real parts, d/dx the real part of X s, d/dy the imaginary part of Y s
+#pragma unroll
+    for (int t = 0; t < 2; t++) {
+      if (POT) F[t] += ur[t][0] * sr[t] - ui[t][0] * si[t];
+      if (DER) {
+        gz[t] += ur[t][NS - 3] * sr[t] - ui[t][NS - 3] * si[t];
+        gx[t] += ur[t][NS - 2] * sr[t] - ui[t][NS - 2] * si[t];
+        gy[t] += ur[t][NS - 1] * si[t] + ui[t][NS - 1] * sr[t];
+      }
+    }
+  }
+  const double c1 = coef * inv_rb, c2 = coef * inv_rb * inv_rb;
+#pragma unroll
+  for (int t = 0; t < 2; t++) {
+    if (t == 1 && i0 + kL2PThreads >= end) break;
+    const int i = it[t];
     if (KER == FMMB_LAPLACE_GNI) {
       const float4 nv = tnrm[i];
-      pot[i] = -c2 * ((double)nv.x * gx + (double)nv.y * gy + (double)nv.z * gz);
+      pot[i] = -c2 * ((double)nv.x * (0.5 * gx[t]) + (double)nv.y * (0.5 * gy[t]) + (double)nv.z * gz[t]);
     } else {
-      pot[i] = c1 * F;
-      if (grad) {  // G and Gnj: the local expansion is the potential itself
-        grad[i] = c2 * gx;
-        grad[ni + i] = c2 * gy;
-        grad[2 * ni + i] = c2 * gz;
+      pot[i] = c1 * F[t];
+      if (DER) {  // G and Gnj: the local expansion is the potential itself
+        grad[i] = c2 * (0.5 * gx[t]);
+        grad[ni + (size_t)i] = c2 * (0.5 * gy[t]);
+        grad[2 * (size_t)ni + i] = c2 * gz[t];
       }
     }
   }
@@ -733,23 +859,19 @@ void l2p_f32_launch(int kernel, int nwork, const int2* work, int p, int K, const
 
 }  // namespace
 
-void launch_p2m_cart(int kernel, int nleaf, int p, int K, const int* keys, const int2* leaf, const float4* spos,
-                     const float4* snrm, const float* qs, const double* fac, const float* bbox, double rb, double* M,
-                     cudaStream_t st) {
+void launch_p2m_dmma(int kernel, int nleaf, int p, int K, const int* keys, const int2* leaf, const float4* spos,
+                    const float4* snrm, const float* qs, const double* fac, const Sem& s, const float* bbox, double rb,
+                    double* M, cudaStream_t st) {
   if (nleaf <= 0) return;
-  if (p <= 14) {
-    const size_t sm = (size_t)(128 / 16) * K * sizeof(double);
-    if (kernel == FMMB_LAPLACE_GNJ)
-      p2m_cart<FMMB_LAPLACE_GNJ, 16><<<nleaf, 128, sm, st>>>(p, K, keys, leaf, spos, snrm, qs, fac, bbox[0], bbox[1], bbox[2], rb, M);
-    else
-      p2m_cart<FMMB_LAPLACE_G, 16><<<nleaf, 128, sm, st>>>(p, K, keys, leaf, spos, snrm, qs, fac, bbox[0], bbox[1], bbox[2], rb, M);
-  } else {
-    const size_t sm = (size_t)(128 / 32) * K * sizeof(double);
-    if (kernel == FMMB_LAPLACE_GNJ)
-      p2m_cart<FMMB_LAPLACE_GNJ, 32><<<nleaf, 128, sm, st>>>(p, K, keys, leaf, spos, snrm, qs, fac, bbox[0], bbox[1], bbox[2], rb, M);
-    else
-      p2m_cart<FMMB_LAPLACE_G, 32><<<nleaf, 128, sm, st>>>(p, K, keys, leaf, spos, snrm, qs, fac, bbox[0], bbox[1], bbox[2], rb, M);
-  }
+  const bool dip = kernel == FMMB_LAPLACE_GNJ;
+  const int ncol = dip ? 6 : 2;
+  const size_t sm = ((size_t)ncol * (p + 1) * (p + 2) / 2 + (kPts / 32) * (size_t)(kRows + ncol) * kPS) * sizeof(double);
+  auto go = [&](auto k) {
+    k<<<nleaf, kPts, sm, st>>>(p, K, keys, leaf, spos, snrm, qs, fac, s, bbox[0], bbox[1], bbox[2], rb, M);
+  };
+  if (dip) go(p2m_dmma<FMMB_LAPLACE_GNJ, false>);
+  else if (s.ref) go(p2m_dmma<FMMB_LAPLACE_G, true>);
+  else go(p2m_dmma<FMMB_LAPLACE_G, false>);
   FMMB_CHECK_LAUNCH();
 }
 
@@ -796,18 +918,18 @@ bool launch_p2m_f32(int kernel, int nwork, const int2* work, int p, int K, const
   return true;
 }
 
-void launch_l2p_cart(int kernel, int nleaf, int p, int K, const int* keys, const int2* leaf, const float4* tpos,
-                     const float4* tnrm, const double* fac, const float* bbox, double rb, double coef, const double* L,
-                     double* pot, double* grad, int ni, cudaStream_t st) {
-  if (nleaf <= 0) return;
-  const int P = (p + 1) * (p + 2) / 2;
-  const size_t sm = (size_t)4 * P * 2 * sizeof(double) + (p + 1) * sizeof(double);
-  if (kernel == FMMB_LAPLACE_G)
-    l2p_cart<FMMB_LAPLACE_G><<<nleaf, kL2PThreads, sm, st>>>(p, K, keys, leaf, tpos, tnrm, fac, bbox[0], bbox[1], bbox[2], rb, coef, L, pot, grad, ni);
-  else if (kernel == FMMB_LAPLACE_GNI)
-    l2p_cart<FMMB_LAPLACE_GNI><<<nleaf, kL2PThreads, sm, st>>>(p, K, keys, leaf, tpos, tnrm, fac, bbox[0], bbox[1], bbox[2], rb, coef, L, pot, grad, ni);
-  else
-    l2p_cart<FMMB_LAPLACE_GNJ><<<nleaf, kL2PThreads, sm, st>>>(p, K, keys, leaf, tpos, tnrm, fac, bbox[0], bbox[1], bbox[2], rb, coef, L, pot, grad, ni);
+void launch_l2p_cart(int kernel, int nwork, const int2* work, int p, int K, const int* keys, const int2* leaf,
+                     const float4* tpos, const float4* tnrm, const double* fac, const float* bbox, double rb, double coef,
+                     const double* L, double* pot, double* grad, int ni, cudaStream_t st) {
+  if (nwork <= 0) return;
+  const size_t terms = (size_t)(p + 1) * (p + 2) / 2;
+  auto go = [&](auto k, int ns) {
+    k<<<nwork, kL2PThreads, terms * ns * sizeof(double2), st>>>(p, K, work, keys, leaf, tpos, tnrm, fac, bbox[0], bbox[1],
+                                                                bbox[2], rb, coef, L, pot, grad, ni);
+  };
+  if (kernel == FMMB_LAPLACE_GNI) go(l2p_cart<FMMB_LAPLACE_GNI, false, true>, 3);
+  else if (grad) go(l2p_cart<FMMB_LAPLACE_G, true, true>, 4);
+  else go(l2p_cart<FMMB_LAPLACE_G, true, false>, 1);
   FMMB_CHECK_LAUNCH();
 }
 

@@ -34,13 +34,15 @@ void launch_p2p_mixed(int kernel, int nwork, const int2* work, const int2* leaf_
                       const Sem& s, double* pot, double* grad, int ni, cudaStream_t st);
 void launch_p2m(int kernel, int nleaf, int p, int K, const int* keys, const int2* leaf, const float4* spos, const float4* snrm,
                 const float* qs, const double* fac, const Sem& s, const float* bbox, double rb, double* M, cudaStream_t st);
-// trig-free Cartesian P2M / L2P (accurate semantics), expansions_cart.cu
-void launch_p2m_cart(int kernel, int nleaf, int p, int K, const int* keys, const int2* leaf, const float4* spos,
-                     const float4* snrm, const float* qs, const double* fac, const float* bbox, double rb, double* M,
-                     cudaStream_t st);
-void launch_l2p_cart(int kernel, int nleaf, int p, int K, const int* keys, const int2* leaf, const float4* tpos,
-                     const float4* tnrm, const double* fac, const float* bbox, double rb, double coef, const double* L,
-                     double* pot, double* grad, int ni, cudaStream_t st);
+// Cartesian P2M (reference semantics too, not its dipoles) and L2P (accurate
+// semantics), expansions_cart.cu
+void launch_p2m_dmma(int kernel, int nleaf, int p, int K, const int* keys, const int2* leaf, const float4* spos,
+                     const float4* snrm, const float* qs, const double* fac, const Sem& s, const float* bbox, double rb,
+                     double* M, cudaStream_t st);
+// (work: (target leaf, first target) items of up to 128 targets)
+void launch_l2p_cart(int kernel, int nwork, const int2* work, int p, int K, const int* keys, const int2* leaf,
+                     const float4* tpos, const float4* tnrm, const double* fac, const float* bbox, double rb, double coef,
+                     const double* L, double* pot, double* grad, int ni, cudaStream_t st);
 // far-field gradient of the Gni potential w.r.t. the target position
 // (normal fixed), -(1/4pi) H n from the local expansions (accurate semantics)
 void launch_l2p_hess_gni(int nleaf, int p, int K, const int* keys, const int2* leaf, const float4* tpos,
@@ -204,7 +206,7 @@ void launch_helm_finalize(int n, const int* perm, const double* near, const doub
 // operators in the real 2K x 2K form, transposed ([op][column][row], row stride 2K)
 void launch_helm_build_ops(int p, double k, bool yuk, int nops, const HelmOp* ops, const double* gl_x,
                            const double* gl_w, const double* ybar_q, double* opT, cudaStream_t st);
-// the M2L operators as images of m2l_parity.cu, `stride` doubles each (zeroed before)
+// the M2L operators as images of m2l_parity.cuh, `stride` doubles each (zeroed before)
 void launch_helm_build_parity(int p, double k, bool yuk, int nops, const HelmOp* ops, const double* gl_x,
                               const double* gl_w, const double* ybar_q, double* img, size_t stride, cudaStream_t st);
 }  // namespace fmmb

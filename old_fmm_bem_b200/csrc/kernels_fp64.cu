@@ -40,10 +40,10 @@ __global__ void gather_charges(int n, int nrhs, const int* perm, const float* q,
 }
 
 // ---------------------------------------------------------------- P2M
-// One block per source leaf: 4 groups of 32 lanes, lane m owns the order-m
-// coefficients; groups take every 4th point and are summed at the end.
-template <int KER>
-__global__ void __launch_bounds__(128) p2m_f64(int p, int K, const int* __restrict__ keys, const int2* __restrict__ leaf,
+// Dipoles in reference semantics.  One block per source leaf: 4 groups of 32
+// lanes, lane m owns the order-m coefficients; groups take every 4th point and
+// are summed at the end.
+__global__ void __launch_bounds__(128) p2m_dipole_f64(int p, int K, const int* __restrict__ keys, const int2* __restrict__ leaf,
                                                const float4* __restrict__ spos, const float4* __restrict__ snrm,
                                                const float* __restrict__ qs, const double* __restrict__ fac, Sem s,
                                                float xmin, float ymin, float zmin, double rb, double* __restrict__ M) {
@@ -82,28 +82,7 @@ __global__ void __launch_bounds__(128) p2m_f64(int p, int K, const int* __restri
       double rm1 = 1.0;  // rs^(m-1) for m >= 1
       for (int i = 1; i < m; i++) rm1 *= rs;
       const double rm = (m == 0) ? 1.0 : rm1 * rs;
-      if (KER != FMMB_LAPLACE_GNJ) {
-        // M^_n^m += q r^n fac P_n^m(cos al) e^{-i m be}
-        const double q = (double)qs[j];
-        double pv = pmm, p1 = pmm, p2 = 0.0;
-        double rn = rm;
-        for (int n = m; n <= p; n++) {
-          if (n > m) {
-            const double pn = (n == m + 1) ? xx * (2 * m + 1) * p1 : (xx * (2 * n - 1) * p1 - (n - 1 + m) * p2) / (n - m);
-            p2 = p1;
-            p1 = pn;
-            pv = pn;
-          }
-          const double bnm = rn * fac[ifull_d(n, m)] * pv;
-          if (m == 0) {
-            my[n * n] += q * bnm;
-          } else {
-            my[n * n + 2 * m - 1] += q * bnm * cb;
-            my[n * n + 2 * m] -= q * bnm * sb;
-          }
-          rn *= rs;
-        }
-      } else {
+      {
         // dipole: sum (q n) . grad R(x - c), in scaled form (1/rb) x the
         // reference's expression with the scaled radius (kernel/Gn_p2m.cxx:42-57)
         const float4 nv = snrm[j];
@@ -344,11 +323,12 @@ void launch_gather_charges(int n, int nrhs, const int* perm, const float* q, flo
 void launch_p2m(int kernel, int nleaf, int p, int K, const int* keys, const int2* leaf, const float4* spos, const float4* snrm,
                 const float* qs, const double* fac, const Sem& s, const float* bbox, double rb, double* M, cudaStream_t st) {
   if (nleaf <= 0) return;
+  if (kernel != FMMB_LAPLACE_GNJ) {  // charges: the sums of expansions_cart.cu at the reference's angles and radius
+    launch_p2m_dmma(FMMB_LAPLACE_G, nleaf, p, K, keys, leaf, spos, snrm, qs, fac, s, bbox, rb, M, st);
+    return;
+  }
   const size_t sm = 4 * (size_t)K * sizeof(double);
-  if (kernel == FMMB_LAPLACE_GNJ)
-    p2m_f64<FMMB_LAPLACE_GNJ><<<nleaf, 128, sm, st>>>(p, K, keys, leaf, spos, snrm, qs, fac, s, bbox[0], bbox[1], bbox[2], rb, M);
-  else
-    p2m_f64<FMMB_LAPLACE_G><<<nleaf, 128, sm, st>>>(p, K, keys, leaf, spos, snrm, qs, fac, s, bbox[0], bbox[1], bbox[2], rb, M);
+  p2m_dipole_f64<<<nleaf, 128, sm, st>>>(p, K, keys, leaf, spos, snrm, qs, fac, s, bbox[0], bbox[1], bbox[2], rb, M);
   FMMB_CHECK_LAUNCH();
 }
 
