@@ -301,6 +301,7 @@ int geometry_impl(fmmb_plan* pl, int nprob, const int* toff, const int* soff, in
                    "problem offsets must run from 0 to the point counts");
     }
     for (int w = 0; w < 4; w++) {  // captured evaluates refer to the old buffers
+      pl->gused[w] = false;
       if (pl->gexec[w]) {
         FMMB_CUDA(cudaStreamSynchronize(pl->st.main));
         cudaGraphExecDestroy(pl->gexec[w]);
@@ -328,11 +329,22 @@ int geometry_impl(fmmb_plan* pl, int nprob, const int* toff, const int* soff, in
     cudaStream_t s = pl->st.main;
     pl->have_geometry = false;
     pl->have_expansions = false;
-    DevBuf<float> st[12];
-    const float* d[12] = {to_device(tx, ni, st[0], s),  to_device(ty, ni, st[1], s),  to_device(tz, ni, st[2], s),
-                          to_device(tnx, ni, st[3], s), to_device(tny, ni, st[4], s), to_device(tnz, ni, st[5], s),
-                          to_device(sx, nj, st[6], s),  to_device(sy, nj, st[7], s),  to_device(sz, nj, st[8], s),
-                          to_device(snx, nj, st[9], s), to_device(sny, nj, st[10], s), to_device(snz, nj, st[11], s)};
+    pl->same_tree = ni == nj && tx == sx && ty == sy && tz == sz && to == so;
+    std::vector<TmpBuf<float>> st;
+    for (int k = 0; k < 12; k++) st.emplace_back(s);
+    const float* src[12] = {tx, ty, tz, tnx, tny, tnz, sx, sy, sz, snx, sny, snz};
+    const float* d[12];
+    for (int k = 0; k < 12; k++) {
+      const size_t n = k < 6 ? ni : nj;
+      d[k] = src[k];
+      if (k >= 6 && pl->same_tree && src[k] == src[k - 6]) {
+        d[k] = d[k - 6];
+      } else if (src[k] && !is_device_ptr(src[k])) {
+        st[k].alloc(n);
+        FMMB_CUDA(cudaMemcpyAsync(st[k].get(), src[k], n * sizeof(float), cudaMemcpyHostToDevice, s));
+        d[k] = st[k].get();
+      }
+    }
     pl->nprob = nprob;
     pl->prob_toff = to;
     pl->prob_soff = so;
@@ -367,76 +379,10 @@ int geometry_impl(fmmb_plan* pl, int nprob, const int* toff, const int* soff, in
     }
     if (pl->ref && !par_m2l && (pl->ops.m2l_lmax != pl->lmax || pl->ops.m2l_rd != pl->bbox[3]))
       build_m2l_operators(pl->ops, pl->lmax, pl->bbox[3]);
-    // M2M / L2L translation tiles per level
-    std::vector<int> keys(pl->tot_i), keys_j(pl->tot_j), par_j(pl->tot_j);
-    FMMB_CUDA(cudaMemcpy(keys.data(), pl->key_i.get(), pl->tot_i * sizeof(int), cudaMemcpyDeviceToHost));
-    FMMB_CUDA(cudaMemcpy(keys_j.data(), pl->key_j.get(), pl->tot_j * sizeof(int), cudaMemcpyDeviceToHost));
-    FMMB_CUDA(cudaMemcpy(par_j.data(), pl->parent_j.get(), pl->tot_j * sizeof(int), cudaMemcpyDeviceToHost));
-    // M2M child lists: [parent][octant] -> child within the child level
-    std::vector<int> m2m_list((size_t)pl->tot_j * 8, -1);
-    for (int lev = pl->lmax; lev >= 3; lev--)
-      for (int c = 0; c < pl->nbox_j[lev]; c++) {
-        const int par = par_j[pl->off_j[lev] + c];
-        m2m_list[(size_t)(pl->off_j[lev - 1] + par) * 8 + (keys_j[pl->off_j[lev] + c] & 7)] = c;
-      }
     int dev_sms = 148;
     cudaDeviceGetAttribute(&dev_sms, cudaDevAttrMultiProcessorCount, pl->device);
     pl->nsm = dev_sms;
-    // M2M / L2L pair tiles: {operator = child octant, input row, output row},
-    // grouped by operator, tiles of tp pairs
-    {
-      using P3 = std::array<int, 3>;
-      auto pair_job = [&](std::vector<P3>& pairs) {
-        std::unique_ptr<fmmb_plan::PairJob> job(new fmmb_plan::PairJob());
-        std::stable_sort(pairs.begin(), pairs.end(), [](const P3& x, const P3& y) { return x[0] < y[0]; });
-        const int tp = pairs_f64_tile(pl->K, (int)pairs.size(), dev_sms);
-        std::vector<int> top, tsrc, tdst;
-        for (size_t i = 0; i < pairs.size();) {
-          size_t j = i;
-          while (j < pairs.size() && pairs[j][0] == pairs[i][0]) j++;
-          for (size_t k = i; k < j; k += tp) {
-            top.push_back(pairs[i][0]);
-            for (int c = 0; c < tp; c++) {
-              tsrc.push_back(k + c < j ? pairs[k + c][1] : -1);
-              tdst.push_back(k + c < j ? pairs[k + c][2] : -1);
-            }
-          }
-          i = j;
-        }
-        job->ntile = (int)top.size();
-        job->tp = tp;
-        auto up = [&](DevBuf<int>& d, const std::vector<int>& h) {
-          d.alloc(h.size());
-          if (!h.empty()) FMMB_CUDA(cudaMemcpy(d.get(), h.data(), h.size() * sizeof(int), cudaMemcpyHostToDevice));
-        };
-        up(job->tile_op, top);
-        up(job->tile_src, tsrc);
-        up(job->tile_dst, tdst);
-        return job;
-      };
-      std::vector<int> par_i(pl->tot_i);
-      FMMB_CUDA(cudaMemcpy(par_i.data(), pl->parent_i.get(), pl->tot_i * sizeof(int), cudaMemcpyDeviceToHost));
-      pl->m2m_pairs.clear();
-      pl->l2l_pairs.clear();
-      for (int lev = 0; lev <= pl->lmax; lev++) {
-        std::vector<P3> up_pairs, down_pairs;
-        if (lev >= 2 && lev < pl->lmax)
-          for (int b = 0; b < pl->nbox_j[lev]; b++) {
-            const int box = pl->off_j[lev] + b;
-            for (int sl = 0; sl < 8; sl++) {
-              const int c = m2m_list[(size_t)box * 8 + sl];
-              if (c >= 0) up_pairs.push_back({sl, pl->off_j[lev + 1] + c, box});
-            }
-          }
-        if (lev >= 3)
-          for (int b = 0; b < pl->nbox_i[lev]; b++) {
-            const int box = pl->off_i[lev] + b;
-            down_pairs.push_back({keys[box] & 7, pl->off_i[lev - 1] + par_i[box], box});
-          }
-        pl->m2m_pairs.push_back(pair_job(up_pairs));
-        pl->l2l_pairs.push_back(pair_job(down_pairs));
-      }
-    }
+    build_pair_jobs(pl, 0, 0, 0, s);  // M2M / L2L: operator = child octant
     // tensor-core M2L (mixed precision, K <= tc_max_k()): operator images (one
     // per operator and block of 128 output rows), the TF32 split of M, and
     // the work items over the pair tiles of all levels
@@ -518,7 +464,8 @@ int geometry_impl(fmmb_plan* pl, int nprob, const int* toff, const int* soff, in
       };
       // M2L, all levels in one job: operator = set(level)*316 + relative position
       if (!(pl->use_h16 && build_m2l_job_dev(pl, pl->tc_m2l, (K + 3) / 4 * 4, s))) {
-        std::vector<int> lst((size_t)pl->tot_i * kM2LSlots);
+        std::vector<int> keys(pl->tot_i), lst((size_t)pl->tot_i * kM2LSlots);
+        FMMB_CUDA(cudaMemcpy(keys.data(), pl->key_i.get(), pl->tot_i * sizeof(int), cudaMemcpyDeviceToHost));
         FMMB_CUDA(cudaMemcpy(lst.data(), pl->m2l_list.get(), lst.size() * sizeof(int), cudaMemcpyDeviceToHost));
         std::vector<Pair> pairs;
         for (int lev = 2; lev <= pl->lmax; lev++) {
@@ -623,6 +570,16 @@ struct PhaseTimer {
   }
 };
 
+// The pair kernel's tiles of child level lev.
+void tiles_of(const fmmb_plan::PairTiles& job, int lev, PairArgs& a) {
+  const size_t t0 = job.first[lev];
+  a.ntile = job.ntile[lev];
+  a.tp = pairs_f64_tile();
+  a.tile_op = job.op.get() + t0;
+  a.tile_src = job.src.get() + t0 * a.tp;
+  a.tile_dst = job.dst.get() + t0 * a.tp;
+}
+
 // The FP64 M2L of all levels: M -> L (added to).
 void run_parity(fmmb_plan* pl, int mode, cudaStream_t m) {
   const fmmb_plan::PairJob& job = pl->par_m2l;
@@ -676,17 +633,13 @@ void run_one_helm(fmmb_plan* pl, const float* qs) {
                     pl->d_ylm.get(), pl->bbox, wleaf, pl->M.get() + (size_t)pl->off_j[lmax] * 2 * K, m);
   }
   FMMB_CUDA(time_mark(pl, pl->ev[3], m));
-  auto pairs_run = [&](const fmmb_plan::PairJob& job, double* xin, double* out, int atomic, int phase) {
-    if (job.ntile <= 0) return;
+  auto pairs_run = [&](const fmmb_plan::PairTiles& job, int lev, double* xin, double* out, int atomic, int phase) {
+    if (job.ntile[lev] <= 0) return;
     PhaseTimer tm(pl, phase, m);
     PairArgs a{};
-    a.ntile = job.ntile;
-    a.tp = job.tp;
     a.K = 2 * K;
     a.atomic = atomic;
-    a.tile_op = job.tile_op.get();
-    a.tile_src = job.tile_src.get();
-    a.tile_dst = job.tile_dst.get();
+    tiles_of(job, lev, a);
     a.opT = pl->d_hops.get();
     a.ostride = (size_t)4 * K * K;
     a.xin = xin;
@@ -696,11 +649,11 @@ void run_one_helm(fmmb_plan* pl, const float* qs) {
   // parents are accumulated from their children, level by level
   const size_t above = (size_t)(pl->tot_j - pl->nbox_j[lmax]) * 2 * K;
   if (above) FMMB_CUDA(cudaMemsetAsync(pl->M.get() + (size_t)pl->off_j[lmax - 1] * 2 * K, 0, above * sizeof(double), m));
-  for (int lev = lmax - 1; lev >= 2; lev--) pairs_run(*pl->m2m_pairs[lev], pl->M.get(), pl->M.get(), 1, 2);
+  for (int lev = lmax - 1; lev >= 2; lev--) pairs_run(pl->m2m_tiles, lev + 1, pl->M.get(), pl->M.get(), 1, 2);
   FMMB_CUDA(time_mark(pl, pl->ev[4], m));
   FMMB_CUDA(cudaMemsetAsync(pl->L.get(), 0, (size_t)pl->tot_i * 2 * K * sizeof(double), m));
   run_parity(pl, yuk ? 2 : 1, m);
-  for (int lev = 3; lev <= lmax; lev++) pairs_run(*pl->l2l_pairs[lev], pl->L.get(), pl->L.get(), 1, 4);
+  for (int lev = 3; lev <= lmax; lev++) pairs_run(pl->l2l_tiles, lev, pl->L.get(), pl->L.get(), 1, 4);
   FMMB_CUDA(time_mark(pl, pl->ev[5], m));
   {
     PhaseTimer tm(pl, 5, m);
@@ -809,18 +762,14 @@ void run_one(fmmb_plan* pl, const float* qs, bool want_grad) {
     PhaseTimer tm(pl, phase, m);
     launch_split_tf32(n, K, tc_kpad(K), X + (size_t)off * K, Xtf + (size_t)off * 2 * tc_kpad(K), m);
   };
-  auto pairs_run = [&](const fmmb_plan::PairJob& job, const double* opT, const double* xin, double* out, int atomic,
-                       int phase) {
-    if (job.ntile <= 0) return;
+  auto pairs_run = [&](const fmmb_plan::PairTiles& job, int lev, const double* opT, const double* xin, double* out,
+                       int atomic, int phase) {
+    if (job.ntile[lev] <= 0) return;
     PhaseTimer tm(pl, phase, m);
     PairArgs a{};
-    a.ntile = job.ntile;
-    a.tp = job.tp;
     a.K = K;
     a.atomic = atomic;
-    a.tile_op = job.tile_op.get();
-    a.tile_src = job.tile_src.get();
-    a.tile_dst = job.tile_dst.get();
+    tiles_of(job, lev, a);
     a.opT = opT;
     a.ostride = pair_op_stride(K);
     a.xin = xin;
@@ -828,7 +777,7 @@ void run_one(fmmb_plan* pl, const float* qs, bool want_grad) {
     launch_translate_pairs_f64(a, m);
   };
   for (int lev = lmax - 1; lev >= 2; lev--)  // parents at lev from their children (several per parent)
-    pairs_run(*pl->m2m_pairs[lev], pl->d_m2m_t.get(), pl->M.get(), pl->M.get(), 1, 2);
+    pairs_run(pl->m2m_tiles, lev + 1, pl->d_m2m_t.get(), pl->M.get(), pl->M.get(), 1, 2);
   if (pl->use_tc) split(pl->M.get(), pl->Mtf.get(), 0, pl->tot_j, 2);  // every level, for the M2L
   if (pl->use_h16) {
     PhaseTimer tm(pl, 2, m);
@@ -864,7 +813,7 @@ void run_one(fmmb_plan* pl, const float* qs, bool want_grad) {
   }
   near_field(p2p_split, pl->p2p_nwork, true);
   for (int lev = 3; lev <= lmax; lev++)  // children at lev from their parent (one pair each, added by one atomic)
-    pairs_run(*pl->l2l_pairs[lev], pl->d_l2l_t.get(), pl->L.get(), pl->L.get(), 1, 4);
+    pairs_run(pl->l2l_tiles, lev, pl->d_l2l_t.get(), pl->L.get(), pl->L.get(), 1, 4);
   FMMB_CUDA(time_mark(pl, pl->ev[5], m));
   {
     PhaseTimer tm(pl, 5, m);
@@ -888,17 +837,32 @@ void run_one(fmmb_plan* pl, const float* qs, bool want_grad) {
   FMMB_CUDA(cudaStreamWaitEvent(m, pl->st.join, 0));
 }
 
-// One right-hand side through its captured graph: captured on first use
-// after each fmmb_set_geometry (run_one with the plan's private capture stream
-// standing in for the main stream, in thread-local capture mode, the side
-// stream joining through the fork/join events), then replayed with one launch
-// on the main stream (which may be a legacy default stream, where capture is
-// not possible).  A graph that fails to instantiate turns graphs off for the
-// plan and runs the evaluate directly.
+// One right-hand side: the first after each fmmb_set_geometry launched directly
+// (capturing and instantiating its graph costs the host several times the
+// launches, more than a caller whose points move every step gets back), the
+// next ones through its captured graph: captured on the second use (run_one with
+// the plan's private capture stream standing in for the main stream, in
+// thread-local capture mode, the side stream joining through the fork/join
+// events), then replayed with one launch on the main stream (which may be a
+// legacy default stream, where capture is not possible).  A graph that fails to
+// instantiate turns graphs off for the plan and runs the evaluate directly.
 void run_graph(fmmb_plan* pl, bool want_grad, bool far_only = false) {
   const int w = (want_grad ? 1 : 0) + (far_only ? 2 : 0);
   const float* qin = far_only ? pl->qs_far.get() : pl->qs.get();
   cudaStream_t m = pl->st.main;
+  if (!pl->gexec[w] && !pl->gused[w]) {
+    pl->gused[w] = true;
+    pl->gbase[w] = pl->launches;
+    pl->far_only = far_only;
+    try {
+      run_one(pl, qin, want_grad);
+    } catch (...) {
+      pl->far_only = false;
+      throw;
+    }
+    pl->far_only = false;
+    return;
+  }
   if (!pl->gexec[w]) {
     cudaStream_t c = pl->st.cap;
     FMMB_CUDA(cudaStreamBeginCapture(c, cudaStreamCaptureModeThreadLocal));
@@ -906,6 +870,9 @@ void run_graph(fmmb_plan* pl, bool want_grad, bool far_only = false) {
     pl->st.main = c;
     pl->capturing = true;
     pl->far_only = far_only;
+    pl->ev_used = 0;  // the graph's own timing events, and its launches counted as in the direct run
+    pl->ev_phase.clear();
+    pl->launches = pl->gbase[w];
     try {
       run_one(pl, qin, want_grad);
     } catch (...) {

@@ -458,9 +458,7 @@ extern "C" int fmmb_gpu_m2l(const int* nvecd, const double* rb, float* arex, flo
     // tiles of same-operator pairs for the pair kernel
     std::stable_sort(pairs.begin(), pairs.end(),
                      [](const std::array<int, 3>& a, const std::array<int, 3>& b) { return a[0] < b[0]; });
-    int nsm = 148;
-    cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, 0);
-    const int tp = pairs_f64_tile(K, (int)pairs.size(), nsm);
+    const int tp = pairs_f64_tile();
     std::vector<int> top, tsrc, tdst;
     for (size_t i = 0; i < pairs.size();) {
       size_t j = i;

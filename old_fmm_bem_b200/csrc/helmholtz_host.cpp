@@ -82,33 +82,6 @@ void upload_vec(DevBuf<T>& d, const std::vector<T>& h) {
   if (!h.empty()) FMMB_CUDA(cudaMemcpy(d.get(), h.data(), h.size() * sizeof(T), cudaMemcpyHostToDevice));
 }
 
-// {operator, input row, output row} -> tiles of tp pairs of one operator
-std::unique_ptr<fmmb_plan::PairJob> pair_job(std::vector<std::array<int, 3>>& pairs, int Kreal, int nsm) {
-  std::unique_ptr<fmmb_plan::PairJob> job(new fmmb_plan::PairJob());
-  std::stable_sort(pairs.begin(), pairs.end(),
-                   [](const std::array<int, 3>& a, const std::array<int, 3>& b) { return a[0] < b[0]; });
-  const int tp = pairs_f64_tile(Kreal, (int)pairs.size(), nsm);
-  std::vector<int> top, tsrc, tdst;
-  for (size_t i = 0; i < pairs.size();) {
-    size_t j = i;
-    while (j < pairs.size() && pairs[j][0] == pairs[i][0]) j++;
-    for (size_t k = i; k < j; k += tp) {
-      top.push_back(pairs[i][0]);
-      for (int c = 0; c < tp; c++) {
-        tsrc.push_back(k + c < j ? pairs[k + c][1] : -1);
-        tdst.push_back(k + c < j ? pairs[k + c][2] : -1);
-      }
-    }
-    i = j;
-  }
-  job->ntile = (int)top.size();
-  job->tp = tp;
-  upload_vec(job->tile_op, top);
-  upload_vec(job->tile_src, tsrc);
-  upload_vec(job->tile_dst, tdst);
-  return job;
-}
-
 }  // namespace
 
 void helm_setup(fmmb_plan* pl) {
@@ -171,34 +144,11 @@ void helm_setup(fmmb_plan* pl) {
                              pl->d_par.get(), pstride, s);
     FMMB_CUDA(cudaStreamSynchronize(s));
   }
-  // pair jobs (rows are indices into the all-level M / L arrays)
-  std::vector<int> par_i(pl->tot_i), par_j(pl->tot_j), key_i(pl->tot_i), key_j(pl->tot_j);
-  FMMB_CUDA(cudaMemcpy(par_i.data(), pl->parent_i.get(), pl->tot_i * sizeof(int), cudaMemcpyDeviceToHost));
-  FMMB_CUDA(cudaMemcpy(par_j.data(), pl->parent_j.get(), pl->tot_j * sizeof(int), cudaMemcpyDeviceToHost));
-  FMMB_CUDA(cudaMemcpy(key_i.data(), pl->key_i.get(), pl->tot_i * sizeof(int), cudaMemcpyDeviceToHost));
-  FMMB_CUDA(cudaMemcpy(key_j.data(), pl->key_j.get(), pl->tot_j * sizeof(int), cudaMemcpyDeviceToHost));
   int nsm = 148;
   cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, pl->device);
   pl->nsm = nsm;
   prepare_translate_pairs_f64();
-  using P3 = std::array<int, 3>;
-  pl->m2m_pairs.clear();
-  pl->l2l_pairs.clear();
-  for (int lev = 0; lev <= lmax; lev++) {
-    std::vector<P3> up, down;
-    if (lev >= 2 && lev < lmax)  // children at lev + 1 into their parents at lev
-      for (int c = 0; c < pl->nbox_j[lev + 1]; c++) {
-        const int box = pl->off_j[lev + 1] + c;
-        up.push_back({pl->hop_m2m0 + (lev + 1 - 3) * 8 + (key_j[box] & 7), box, pl->off_j[lev] + par_j[box]});
-      }
-    if (lev >= 3)  // parents at lev - 1 into their children at lev
-      for (int b = 0; b < pl->nbox_i[lev]; b++) {
-        const int box = pl->off_i[lev] + b;
-        down.push_back({pl->hop_l2l0 + (lev - 3) * 8 + (key_i[box] & 7), pl->off_i[lev - 1] + par_i[box], box});
-      }
-    pl->m2m_pairs.push_back(pair_job(up, 2 * K, nsm));
-    pl->l2l_pairs.push_back(pair_job(down, 2 * K, nsm));
-  }
+  build_pair_jobs(pl, pl->hop_m2m0, pl->hop_l2l0, 8, s);
   prepare_m2l_parity(yuk ? 2 : 1, p);
   build_parity_job(pl, s);
   // near-field work items and the inverse target permutation of the direct sum

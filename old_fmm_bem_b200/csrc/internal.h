@@ -212,8 +212,6 @@ struct fmmb_plan {
   int nprob = 1;
   std::vector<int> prob_toff, prob_soff;
   fmmb::DevBuf<int> d_prob_off;
-  fmmb::DevBuf<int> child_start_j;           // for M2M: per source box at level l (<lmax): first child index, count
-  fmmb::DevBuf<int> child_count_j;
 
   // operators on the device
   fmmb::DevBuf<double> d_fac;
@@ -248,12 +246,16 @@ struct fmmb_plan {
   fmmb::DevBuf<float> geo;
   bool geo_tn = false, geo_sn = false;
   bool same_sets = false;  // targets and sources given as the same arrays (one problem)
+  bool same_tree = false;  // the same arrays and the same problems: one tree serves both sides
   fmmb_plan* tplan = nullptr;  // == this plan for a symmetric kernel on one point set
   fmmb::DevBuf<double> pg_tmp;                 // position-gradient work space
   fmmb::DevBuf<double> adj_tmp;                // fmmb_adjoint_f64 work space
   fmmb::DevBuf<float> adj_qs, adj_ws;          // its staged charges and weights
   // graphs [without / with gradient] x [whole evaluate / far field only]
   cudaGraphExec_t gexec[4] = {nullptr, nullptr, nullptr, nullptr};
+  // run once since the last geometry (captured on the second use), and the launches of the evaluate before it
+  bool gused[4] = {false, false, false, false};
+  int gbase[4] = {0, 0, 0, 0};
   std::vector<std::pair<int, int>> gphase[4];
   int glaunches[4] = {0, 0, 0, 0};
   // many right-hand sides (mixed form): the near field of all of them in one
@@ -292,14 +294,18 @@ struct fmmb_plan {
   fmmb::DevBuf<float> tc_y;                                  // pair rows of the M2L launch
   TcJob tc_m2l;                                              // all levels
   int nsm = 148;                                             // SMs of the plan's device
-  // FP64 pair tiles of M2M (into parents at a level) and L2L (into children
-  // at a level), index = level
+  // FP64 pair tiles of M2M and L2L, of all child levels 3..lmax (build_pair_jobs):
+  // per child level its first tile and the number of tiles
+  struct PairTiles {
+    fmmb::DevBuf<int> op, src, dst;
+    std::vector<int> first, ntile;
+  };
+  PairTiles m2m_tiles, l2l_tiles;
   struct PairJob {
-    int ntile = 0, tp = 0;
+    int ntile = 0;
     fmmb::DevBuf<int> tile_op, tile_src, tile_dst, tile_phi;
   };
   PairJob par_m2l;  // FP64 M2L, all levels (tile_op: set * 61 + class)
-  std::vector<std::unique_ptr<PairJob>> m2m_pairs, l2l_pairs;
   // complex Helmholtz: dense operators in the real 2K x 2K form (transposed),
   // [M2M child levels 3..lmax x 8 | L2L likewise]
   fmmb::DevBuf<double> d_hops;
@@ -318,6 +324,8 @@ namespace fmmb {
 // tiles and reduction CSR (false: too large for the int enumeration, build on
 // the host), the near-field work items, the inverse target permutation
 bool build_m2l_job_dev(fmmb_plan* pl, fmmb_plan::TcJob& job, int ys, cudaStream_t s);
+// the M2M and L2L tiles: operators m2m0 / l2l0 + ops_per_level (child level - 3) + octant
+void build_pair_jobs(fmmb_plan* pl, int m2m0, int l2l0, int ops_per_level, cudaStream_t s);
 // the FP64 M2L's pair tiles
 void build_parity_job(fmmb_plan* pl, cudaStream_t s);
 void build_p2p_work_dev(fmmb_plan* pl, cudaStream_t s);

@@ -92,14 +92,13 @@ void launch_weight_field(int n, const float* w, const double* field, double* out
 // FP64 box-pair translations (M2M, L2L): tiles of tp pairs of one operator
 struct PairArgs {
   int ntile, tp, K, atomic;
-  const int *tile_op, *tile_src, *tile_dst;  // [ntile], [ntile][tp], [ntile][tp]
+  const int *tile_op, *tile_src, *tile_dst;  // [ntile] (-1: no tile), [ntile][tp], [ntile][tp]
   const double* opT;                         // operators transposed, [op][column][row], row stride K rounded up to even
   size_t ostride;                            // doubles per operator: K * (K rounded up to even)
   const double* xin;                         // input expansions [rows][K]
   double* out;                               // output expansions [rows][K]
 };
-// pairs per tile (the FP64 tensor-core kernel's 32)
-int pairs_f64_tile(int K, int npair, int nsm);
+constexpr int pairs_f64_tile() { return 32; }  // pairs per tile
 // once per device, before any launch (and outside stream capture)
 void prepare_translate_pairs_f64();
 void launch_translate_pairs_f64(const PairArgs& a, cudaStream_t st);

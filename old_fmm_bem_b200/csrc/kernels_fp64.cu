@@ -367,7 +367,7 @@ namespace {
 // also for L2L, although each of its output rows receives one pair: the
 // single atomic addition gives the value of a read-modify-write without the
 // warp waiting for the read.
-constexpr int kGN = 32;  // pairs per tile (at most)
+constexpr int kGN = pairs_f64_tile();  // pairs per tile (at most)
 
 __device__ __forceinline__ uint32_t smem_addr(const void* p) {
   return static_cast<uint32_t>(__cvta_generic_to_shared(p));
@@ -406,6 +406,7 @@ __global__ void __launch_bounds__(kDT) pairs_dmma_f64(PairArgs P) {
   double* Xs = dsm2 + kDS * kDK * kDAs;  // [kDS][kDK][kDXs]: inputs x_p[c] at [c][p]
   __shared__ int ssrc[kDN], sdst[kDN];
   const int g = blockIdx.x, r0 = blockIdx.y * kDM, K = P.K, KP = (K + 1) & ~1, tp = P.tp;
+  if (P.tile_op[g] < 0) return;  // placed by an upper bound, not there
   const double* T = P.opT + (size_t)P.tile_op[g] * P.ostride;
   if (threadIdx.x < kDN) {
     const bool on = (int)threadIdx.x < tp;
@@ -497,10 +498,6 @@ __global__ void __launch_bounds__(kDT) pairs_dmma_f64(PairArgs P) {
     }
 }
 }  // namespace
-
-// One operator's tiles of up to 32 pairs (the tensor-core kernel's block
-// width); a tile of fewer pairs leaves the rest of the block's columns idle.
-int pairs_f64_tile(int, int, int) { return kGN; }
 
 void prepare_translate_pairs_f64() {
   FMMB_CUDA(cudaFuncSetAttribute(pairs_dmma_f64, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kDSmem));

@@ -1,10 +1,17 @@
 // Device-side construction of the evaluation work lists of a geometry
-// (fmmb_set_geometry): the tensor-core M2L's pair tiles and the CSR of its
-// per-box reduction, the near-field work items, the inverse target
-// permutation.  Scans and stable radix sorts (tree.cu) over the device lists
-// the tree build produced, so that none of it is copied to the host; the
-// results are the ones the former host loops gave (same orders, ties kept in
-// input order).
+// (fmmb_set_geometry): the M2L pair tiles (tensor-core and FP64 forms) and the CSR
+// of the tensor-core form's per-box reduction, the M2M / L2L tiles, the near-field
+// work items, the inverse target permutation.  Scans and stable radix sorts
+// (tree.cu) over the device lists the tree build produced, so that none of it is
+// copied to the host.
+//
+// Bound: launches and the few read-backs (pair, tile and item counts) that
+// allocations wait for; the lists themselves are a few passes over the box slots.
+// Measured on one B200 against M2M / L2L tiles and tree checks on the host, a
+// second sort for the CSR, one atomic per pair or box and a second tree build for
+// a set that is both targets and sources, fmmb_set_geometry: 131,071 clustered
+// points 2.34 -> 1.00 ms, 1,048,576 13.3 -> 8.8 ms, 100,000 points in reference
+// semantics from host arrays 2.68 -> 0.86 ms.
 //
 // The lists restate the work of the reference's fmm() driver
 // (fmm/fmm.cxx:29-152: ijbox's lists per level, kernel/m2l.cxx:13-93 over
@@ -79,29 +86,39 @@ __global__ void m2l_pair_emit(int V, LevTab T, const int* __restrict__ lst, cons
   dst[k] = box;
 }
 
-__global__ void count_keys(int n, const int* __restrict__ key, int* __restrict__ cnt) {
-  const int j = blockIdx.x * blockDim.x + threadIdx.x;
-  if (j < n) atomicAdd(&cnt[key[j]], 1);
+// first position of each key in the sorted list, for keys 0..nk (start[nk] = n)
+__global__ void key_starts(int nk, int n, const int* __restrict__ key, int* __restrict__ start) {
+  const int o = blockIdx.x * blockDim.x + threadIdx.x;
+  if (o > nk) return;
+  int lo = 0, hi = n;
+  while (lo < hi) {
+    const int mid = (lo + hi) >> 1;
+    if (key[mid] < o) lo = mid + 1;
+    else hi = mid;
+  }
+  start[o] = lo;
 }
 
-__global__ void tiles_per_key(int nk, int tt, const int* __restrict__ cnt, int* __restrict__ tiles) {
+__global__ void tiles_per_key(int nk, int tt, const int* __restrict__ start, int* __restrict__ tiles) {
   const int o = blockIdx.x * blockDim.x + threadIdx.x;
-  if (o < nk) tiles[o] = (cnt[o] + tt - 1) / tt;
+  if (o <= nk) tiles[o] = o < nk ? (start[o + 1] - start[o] + tt - 1) / tt : 0;
 }
 
 // sorted pair j -> tile tile_base[op] + r / tt, column r % tt (r = its rank
-// among the pairs of its operator)
+// among the pairs of its operator); col (may be null): the column of each pair
+// in enumeration order, tile * tt + column
 __global__ void fill_tiles(int n, int tt, const int* __restrict__ opk, const int* __restrict__ ord,
                            const int* __restrict__ src, const int* __restrict__ dst, const int* __restrict__ phi,
                            const int* __restrict__ op_start, const int* __restrict__ tile_base,
                            int* __restrict__ tile_op, int* __restrict__ tile_src, int* __restrict__ tdst,
-                           int* __restrict__ tile_phi) {
+                           int* __restrict__ tile_phi, int* __restrict__ col) {
   const int j = blockIdx.x * blockDim.x + threadIdx.x;
   if (j >= n) return;
   const int op = opk[j], r = j - op_start[op];
   const int t = tile_base[op] + r / tt, c = r % tt;
   tile_src[(size_t)t * tt + c] = src[ord[j]];
-  tdst[(size_t)t * tt + c] = dst[ord[j]];
+  if (tdst) tdst[(size_t)t * tt + c] = dst[ord[j]];
+  if (col) col[ord[j]] = t * tt + c;
   if (phi) tile_phi[(size_t)t * tt + c] = phi[ord[j]];
   if (c == 0) tile_op[t] = op;
 }
@@ -113,35 +130,70 @@ __global__ void fill_tile_y(int ntile, int* __restrict__ ty) {
   ty[2 * t + 1] = 0;
 }
 
-__global__ void nonneg_flags(int n, const int* __restrict__ a, int* __restrict__ flag) {
-  const int k = blockIdx.x * blockDim.x + threadIdx.x;
-  if (k < n) flag[k] = a[k] >= 0 ? 1 : 0;
-}
-
-// column k of the tiles with a target -> (target row, k), in k order
-__global__ void compact_cols(int n, const int* __restrict__ tdst, const int* __restrict__ pos,
-                             int* __restrict__ rowk, int* __restrict__ colk) {
-  const int k = blockIdx.x * blockDim.x + threadIdx.x;
-  if (k >= n || tdst[k] < 0) return;
-  rowk[pos[k]] = tdst[k];
-  colk[pos[k]] = k;
-}
-
-__global__ void run_starts(int n, const int* __restrict__ key, int* __restrict__ flag) {
-  const int m = blockIdx.x * blockDim.x + threadIdx.x;
-  if (m < n) flag[m] = (m == 0 || key[m] != key[m - 1]) ? 1 : 0;
-}
-
-__global__ void emit_runs(int n, const int* __restrict__ key, const int* __restrict__ pos, int* __restrict__ rows,
-                          int* __restrict__ ptr) {
-  const int m = blockIdx.x * blockDim.x + threadIdx.x;
-  if (m >= n) return;
-  const bool st = m == 0 || key[m] != key[m - 1];  // pos[m]: the runs started before m
-  if (st) {
-    rows[pos[m]] = key[m];
-    ptr[pos[m]] = m;
+// row (target box) -> its pairs: the enumeration visits the boxes in order, so
+// they are consecutive; ptr[row] from the scanned slot flags
+__global__ void row_ptrs(int nrow, LevTab T, const int* __restrict__ pos, int npair, int* __restrict__ rows,
+                         int* __restrict__ ptr) {
+  const int r = blockIdx.x * blockDim.x + threadIdx.x;
+  if (r > nrow) return;
+  if (r == nrow) {
+    ptr[r] = npair;
+    return;
   }
-  if (m == n - 1) ptr[pos[m] + (st ? 1 : 0)] = n;
+  // rows in enumeration order: level l's boxes are vstart[l] / 189 + ...
+  int l = 0;
+  while (l + 1 < T.nlev && T.vstart[l + 1] / kM2LSlots <= r) l++;
+  rows[r] = T.boxoff[l] + r - T.vstart[l] / kM2LSlots;
+  ptr[r] = pos[r * kM2LSlots];
+}
+
+// ---- M2M / L2L pair tiles: {operator, input row, output row} of every box of
+// levels 3..lmax and its parent, grouped by level and child octant ----
+struct PairTab {
+  int lmax;
+  int off[kMaxLev], tile0[kMaxLev];  // per level: first box in the all-level arrays (lmax first), first tile
+  int op0[kMaxLev];                  // operator of octant 0 of the level's pairs
+};
+__device__ __forceinline__ int level_of(const PairTab& T, int c) {
+  int lev = T.lmax;
+  while (lev > 3 && c >= T.off[lev - 1]) lev--;
+  return lev;
+}
+// rank of box c among the boxes of its (level, octant): one atomic per warp and group
+__device__ __forceinline__ int group_rank(int g, int* cnt) {
+  const unsigned peers = __match_any_sync(__activemask(), g);
+  const int lane = threadIdx.x & 31, lead = __ffs(peers) - 1;
+  int base = 0;
+  if (lane == lead) base = atomicAdd(&cnt[g], __popc(peers));
+  return __shfl_sync(peers, base, lead) + __popc(peers & ((1u << lane) - 1u));
+}
+__global__ void pair_counts(int n, PairTab T, const int* __restrict__ key, int* __restrict__ cnt) {
+  const int c = blockIdx.x * blockDim.x + threadIdx.x;
+  if (c < n) group_rank(8 * level_of(T, c) + (key[c] & 7), cnt);
+}
+// one block: first tile of each (level, octant), and the tiles' operators
+__global__ void pair_bases(PairTab T, int tt, const int* __restrict__ cnt, int* __restrict__ base, int* __restrict__ tile_op) {
+  for (int lev = 3; lev <= T.lmax; lev++) {
+    int t = T.tile0[lev];
+    for (int o = 0; o < 8; o++) {
+      const int nt = (cnt[8 * lev + o] + tt - 1) / tt;
+      if (threadIdx.x == 0) base[8 * lev + o] = t;
+      for (int k = threadIdx.x; k < nt; k += blockDim.x) tile_op[t + k] = T.op0[lev] + o;
+      t += nt;
+    }
+  }
+}
+// up: the parent is the output (M2M), else the input (L2L)
+__global__ void pair_fill(int n, PairTab T, int tt, bool up, const int* __restrict__ key, const int* __restrict__ parent,
+                          const int* __restrict__ base, int* __restrict__ cursor, int* __restrict__ tile_src,
+                          int* __restrict__ tile_dst) {
+  const int c = blockIdx.x * blockDim.x + threadIdx.x;
+  if (c >= n) return;
+  const int lev = level_of(T, c), g = 8 * lev + (key[c] & 7);
+  const size_t at = (size_t)base[g] * tt + group_rank(g, cursor);
+  const int par = T.off[lev - 1] + parent[c];
+  tile_src[at] = up ? c : par;
+  tile_dst[at] = up ? par : c;
 }
 
 // ---- near-field work items ----
@@ -214,13 +266,16 @@ namespace {
 
 // The M2L pairs of levels 2..lmax sorted by operator, in tiles of tt pairs:
 // the operator of pair (level, relative position r) is set(level) * per +
-// rel_to_op[r].  phi (may be null): the azimuth index of each pair.  False when
-// the enumeration does not fit an int.
+// rel_to_op[r].  tile_dst / tile_phi (may be null): the target row and the azimuth
+// index of each pair; csr (may be null): per target box its pairs' columns
+// (tile * tt + column), in slot order.  False when the enumeration does not fit
+// an int.
 struct M2LTiles {
   int npair = 0, ntile = 0;
 };
 bool build_m2l_tiles(fmmb_plan* pl, bool sets, int per, const int* rel_to_op, int tt, DevBuf<int>& tile_op,
-                     DevBuf<int>& tile_src, DevBuf<int>* tile_phi, M2LTiles& out, TmpBuf<int>& tdst, cudaStream_t s) {
+                     DevBuf<int>& tile_src, DevBuf<int>* tile_dst, DevBuf<int>* tile_phi, fmmb_plan::TcJob* csr,
+                     M2LTiles& out, cudaStream_t s) {
   const int lmax = pl->lmax;
   if (lmax - 1 > kMaxLev) return false;
   LevTab T{};
@@ -245,6 +300,15 @@ bool build_m2l_tiles(fmmb_plan* pl, bool sets, int per, const int* rel_to_op, in
   FMMB_CUDA(cudaMemsetAsync(pos.get() + nv, 0, sizeof(int), s));
   exclusive_scan(pos.get(), nv + 1, s);
   const int npair = d2h_int(pos.get() + nv, s);
+  if (csr) {
+    const int nrow = nv / kM2LSlots;
+    csr->nred = npair > 0 ? nrow : 0;
+    csr->red_rows.alloc(std::max(nrow, 1));
+    csr->red_ptr.alloc((size_t)nrow + 1);
+    csr->red_idx.alloc(std::max(npair, 1));
+    row_ptrs<<<nblk(nrow + 1, kT), kT, 0, s>>>(nrow, T, pos.get(), npair, csr->red_rows.get(), csr->red_ptr.get());
+    FMMB_CHECK_LAUNCH();
+  }
   TmpBuf<int> opk(s), ord(s), src(s), dst(s), phi(s);
   opk.alloc(npair);
   ord.alloc(npair);
@@ -257,27 +321,23 @@ bool build_m2l_tiles(fmmb_plan* pl, bool sets, int per, const int* rel_to_op, in
   FMMB_CHECK_LAUNCH();
   radix_sort(opk.get(), ord.get(), npair, bits_for(nops), s);  // stable: enumeration order within an operator
   // tiles of tt pairs per operator
-  TmpBuf<int> cnt(s), op_start(s), tile_base(s);
-  cnt.alloc(nops + 1);
+  TmpBuf<int> op_start(s), tile_base(s);
   op_start.alloc(nops + 1);
   tile_base.alloc(nops + 1);
-  FMMB_CUDA(cudaMemsetAsync(cnt.get(), 0, (nops + 1) * sizeof(int), s));
-  if (npair > 0) {
-    count_keys<<<nblk(npair, kT), kT, 0, s>>>(npair, opk.get(), cnt.get());
-    FMMB_CHECK_LAUNCH();
-  }
-  FMMB_CUDA(cudaMemcpyAsync(op_start.get(), cnt.get(), (nops + 1) * sizeof(int), cudaMemcpyDeviceToDevice, s));
-  tiles_per_key<<<nblk(nops + 1, kT), kT, 0, s>>>(nops + 1, tt, cnt.get(), tile_base.get());
+  key_starts<<<nblk(nops + 1, kT), kT, 0, s>>>(nops, npair, opk.get(), op_start.get());
   FMMB_CHECK_LAUNCH();
-  exclusive_scan(op_start.get(), nops + 1, s);
+  tiles_per_key<<<nblk(nops + 1, kT), kT, 0, s>>>(nops, tt, op_start.get(), tile_base.get());
+  FMMB_CHECK_LAUNCH();
   exclusive_scan(tile_base.get(), nops + 1, s);
   const int ntile = d2h_int(tile_base.get() + nops, s);
   const size_t ncol = (size_t)std::max(ntile, 1) * tt;
   tile_op.alloc(std::max(ntile, 1));
   tile_src.alloc(ncol);
-  tdst.alloc(ncol);
   FMMB_CUDA(cudaMemsetAsync(tile_src.get(), 0xff, ncol * sizeof(int), s));
-  FMMB_CUDA(cudaMemsetAsync(tdst.get(), 0xff, ncol * sizeof(int), s));
+  if (tile_dst) {
+    tile_dst->alloc(ncol);
+    FMMB_CUDA(cudaMemsetAsync(tile_dst->get(), 0xff, ncol * sizeof(int), s));
+  }
   if (tile_phi) {
     tile_phi->alloc(ncol);
     FMMB_CUDA(cudaMemsetAsync(tile_phi->get(), 0, ncol * sizeof(int), s));
@@ -285,8 +345,8 @@ bool build_m2l_tiles(fmmb_plan* pl, bool sets, int per, const int* rel_to_op, in
   if (npair > 0) {
     fill_tiles<<<nblk(npair, kT), kT, 0, s>>>(npair, tt, opk.get(), ord.get(), src.get(), dst.get(),
                                              tile_phi ? phi.get() : nullptr, op_start.get(), tile_base.get(),
-                                             tile_op.get(), tile_src.get(), tdst.get(),
-                                             tile_phi ? tile_phi->get() : nullptr);
+                                             tile_op.get(), tile_src.get(), tile_dst ? tile_dst->get() : nullptr,
+                                             tile_phi ? tile_phi->get() : nullptr, csr ? csr->red_idx.get() : nullptr);
     FMMB_CHECK_LAUNCH();
   }
   out.npair = npair;
@@ -301,13 +361,9 @@ void build_parity_job(fmmb_plan* pl, cudaStream_t s) {
   const bool helm = helm_family(pl->cfg.kernel), sets = helm || pl->ref;
   fmmb_plan::PairJob& job = pl->par_m2l;
   M2LTiles t;
-  TmpBuf<int> tdst(s);
-  if (build_m2l_tiles(pl, sets, ncls, pl->d_rel_to_cls.get(), 32, job.tile_op, job.tile_src, &job.tile_phi, t, tdst, s)) {
-    job.tile_dst.alloc((size_t)std::max(t.ntile, 1) * 32);
-    FMMB_CUDA(cudaMemcpyAsync(job.tile_dst.get(), tdst.get(), (size_t)t.ntile * 32 * sizeof(int), cudaMemcpyDeviceToDevice, s));
-    FMMB_CUDA(cudaStreamSynchronize(s));
+  if (build_m2l_tiles(pl, sets, ncls, pl->d_rel_to_cls.get(), 32, job.tile_op, job.tile_src, &job.tile_dst, &job.tile_phi,
+                      nullptr, t, s)) {
     job.ntile = t.ntile;
-    job.tp = 32;
     return;
   }
   // more box slots than an int enumerates: the same lists on the host
@@ -341,64 +397,70 @@ void build_parity_job(fmmb_plan* pl, cudaStream_t s) {
   up(job.tile_dst, col[1]);
   up(job.tile_phi, col[2]);
   job.ntile = (int)top.size();
-  job.tp = 32;
+}
+
+// The tiles are placed by an upper bound of their number (a level's boxes / 32 +
+// 8), so that nothing is read back: the few left over have operator -1 and no
+// work.
+void build_pair_jobs(fmmb_plan* pl, int m2m0, int l2l0, int ops_per_level, cudaStream_t s) {
+  const int lmax = pl->lmax, tt = pairs_f64_tile();
+  for (int up = 0; up < 2; up++) {
+    const std::vector<int>& nbox = up ? pl->nbox_j : pl->nbox_i;
+    const std::vector<int>& off = up ? pl->off_j : pl->off_i;
+    fmmb_plan::PairTiles& job = up ? pl->m2m_tiles : pl->l2l_tiles;
+    PairTab T{};
+    T.lmax = lmax;
+    job.first.assign(lmax + 1, 0);
+    job.ntile.assign(lmax + 1, 0);
+    int nt = 0;
+    for (int lev = lmax; lev >= 2; lev--) {
+      T.off[lev] = off[lev];
+      T.tile0[lev] = nt;
+      T.op0[lev] = (up ? m2m0 : l2l0) + (lev - 3) * ops_per_level;
+      if (lev < 3) continue;
+      job.first[lev] = nt;
+      job.ntile[lev] = nbox[lev] / tt + 8;
+      nt += job.ntile[lev];
+    }
+    const int n = lmax >= 3 ? off[2] : 0;  // boxes of levels 3..lmax
+    const size_t ncol = (size_t)std::max(nt, 1) * tt;
+    job.op.alloc(std::max(nt, 1));
+    job.src.alloc(ncol);
+    job.dst.alloc(ncol);
+    if (n == 0) continue;
+    FMMB_CUDA(cudaMemsetAsync(job.op.get(), 0xff, nt * sizeof(int), s));
+    FMMB_CUDA(cudaMemsetAsync(job.src.get(), 0xff, ncol * sizeof(int), s));
+    FMMB_CUDA(cudaMemsetAsync(job.dst.get(), 0xff, ncol * sizeof(int), s));
+    TmpBuf<int> tab(s);  // counts, cursors, first tiles of each (level, octant)
+    const int ng = 8 * (lmax + 1);
+    tab.alloc(3 * ng);
+    FMMB_CUDA(cudaMemsetAsync(tab.get(), 0, 3 * ng * sizeof(int), s));
+    const int* key = (up ? pl->key_j : pl->key_i).get();
+    const int* parent = (up ? pl->parent_j : pl->parent_i).get();
+    pair_counts<<<nblk(n, kT), kT, 0, s>>>(n, T, key, tab.get());
+    FMMB_CHECK_LAUNCH();
+    pair_bases<<<1, kT, 0, s>>>(T, tt, tab.get(), tab.get() + 2 * ng, job.op.get());
+    FMMB_CHECK_LAUNCH();
+    pair_fill<<<nblk(n, kT), kT, 0, s>>>(n, T, tt, up == 1, key, parent, tab.get() + 2 * ng, tab.get() + ng,
+                                         job.src.get(), job.dst.get());
+    FMMB_CHECK_LAUNCH();
+  }
 }
 
 bool build_m2l_job_dev(fmmb_plan* pl, fmmb_plan::TcJob& job, int ys, cudaStream_t s) {
   M2LTiles t;
-  TmpBuf<int> tdst(s);
-  if (!build_m2l_tiles(pl, pl->ops.m2l_sets > 1, 316, pl->d_rel_to_op.get(), 128, job.tile_op, job.tile_src, nullptr, t,
-                       tdst, s))
+  if (!build_m2l_tiles(pl, pl->ops.m2l_sets > 1, 316, pl->d_rel_to_op.get(), 128, job.tile_op, job.tile_src, nullptr,
+                       nullptr, &job, t, s))
     return false;
-  const int npair = t.npair, ntile = t.ntile;
+  const int ntile = t.ntile;
   job.ntile = ntile;
   job.tile_y.alloc((size_t)std::max(ntile, 1) * 2);
   if (ntile > 0) {
     fill_tile_y<<<nblk(ntile, kT), kT, 0, s>>>(ntile, job.tile_y.get());
     FMMB_CHECK_LAUNCH();
   }
-  // per output box, its pair rows (tile * 128 + column) in increasing order
-  const int ncol = ntile * 128;
-  TmpBuf<int> cpos(s);
-  cpos.alloc((size_t)ncol + 1);
-  if (ncol > 0) {
-    nonneg_flags<<<nblk(ncol, kT), kT, 0, s>>>(ncol, tdst.get(), cpos.get());
-    FMMB_CHECK_LAUNCH();
-  }
-  FMMB_CUDA(cudaMemsetAsync(cpos.get() + ncol, 0, sizeof(int), s));
-  exclusive_scan(cpos.get(), ncol + 1, s);
-  TmpBuf<int> rowk(s), colk(s);
-  rowk.alloc(std::max(npair, 1));
-  colk.alloc(std::max(npair, 1));
-  if (ncol > 0) {
-    compact_cols<<<nblk(ncol, kT), kT, 0, s>>>(ncol, tdst.get(), cpos.get(), rowk.get(), colk.get());
-    FMMB_CHECK_LAUNCH();
-  }
-  radix_sort(rowk.get(), colk.get(), npair, bits_for(pl->tot_i), s);
-  TmpBuf<int> rpos(s);
-  rpos.alloc((size_t)npair + 1);
-  if (npair > 0) {
-    run_starts<<<nblk(npair, kT), kT, 0, s>>>(npair, rowk.get(), rpos.get());
-    FMMB_CHECK_LAUNCH();
-  }
-  FMMB_CUDA(cudaMemsetAsync(rpos.get() + npair, 0, sizeof(int), s));
-  exclusive_scan(rpos.get(), npair + 1, s);
-  const int nred = d2h_int(rpos.get() + npair, s);
-  job.nred = nred;
-  job.red_rows.alloc(std::max(nred, 1));
-  job.red_ptr.alloc((size_t)nred + 1);
-  if (npair > 0) {
-    emit_runs<<<nblk(npair, kT), kT, 0, s>>>(npair, rowk.get(), rpos.get(), job.red_rows.get(), job.red_ptr.get());
-    FMMB_CHECK_LAUNCH();
-  } else {
-    FMMB_CUDA(cudaMemsetAsync(job.red_ptr.get(), 0, sizeof(int), s));
-  }
-  job.red_idx.alloc(std::max(npair, 1));
-  if (npair > 0)
-    FMMB_CUDA(cudaMemcpyAsync(job.red_idx.get(), colk.get(), (size_t)npair * sizeof(int), cudaMemcpyDeviceToDevice, s));
   job.ys = ys;
   pl->tc_y.alloc((size_t)std::max(ntile, 1) * 128 * ys);
-  FMMB_CUDA(cudaStreamSynchronize(s));
   return true;
 }
 

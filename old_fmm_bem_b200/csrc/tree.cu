@@ -34,63 +34,114 @@ namespace fmmb {
 namespace {
 
 constexpr int kScanThreads = 256;
-constexpr int kScanItems = 4;
+constexpr int kScanItems = 16;
 constexpr int kScanTile = kScanThreads * kScanItems;
 
-// Exclusive scan of each tile; tile sums to `sums`.
-__global__ void scan_tiles(int* data, int n, int* sums) {
-  __shared__ int s[kScanThreads];
-  const int base = blockIdx.x * kScanTile + threadIdx.x * kScanItems;
-  int v[kScanItems];
+// exclusive prefix of v over the block's threads; total: the block's sum
+__device__ __forceinline__ int block_prefix(int v, int& total) {
+  __shared__ int ws[kScanThreads / 32];
+  const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
+  int incl = v;
+#pragma unroll
+  for (int o = 1; o < 32; o <<= 1) {
+    const int t = __shfl_up_sync(0xffffffffu, incl, o);
+    if (lane >= o) incl += t;
+  }
+  __syncthreads();  // the previous use of ws is over
+  if (lane == 31) ws[w] = incl;
+  __syncthreads();
+  int before = 0;
+  total = 0;
+#pragma unroll
+  for (int k = 0; k < kScanThreads / 32; k++) {
+    if (k < w) before += ws[k];
+    total += ws[k];
+  }
+  return before + incl - v;
+}
+
+// sum of each tile
+__global__ void __launch_bounds__(kScanThreads) scan_sums(const int* __restrict__ data, int n, int* __restrict__ sums) {
+  const int base = blockIdx.x * kScanTile;
   int t = 0;
 #pragma unroll
   for (int i = 0; i < kScanItems; i++) {
-    v[i] = (base + i < n) ? data[base + i] : 0;
-    t += v[i];
+    const int j = base + i * kScanThreads + threadIdx.x;
+    t += j < n ? data[j] : 0;
   }
-  s[threadIdx.x] = t;
-  __syncthreads();
-  for (int off = 1; off < kScanThreads; off <<= 1) {
-    int x = (threadIdx.x >= off) ? s[threadIdx.x - off] : 0;
-    __syncthreads();
-    s[threadIdx.x] += x;
-    __syncthreads();
-  }
-  int run = s[threadIdx.x] - t;
-#pragma unroll
-  for (int i = 0; i < kScanItems; i++) {
-    if (base + i < n) data[base + i] = run;
-    run += v[i];
-  }
-  if (threadIdx.x == kScanThreads - 1 && sums) sums[blockIdx.x] = s[threadIdx.x];
+  int total;
+  block_prefix(t, total);
+  if (threadIdx.x == 0) sums[blockIdx.x] = total;
 }
 
-__global__ void scan_add(int* data, int n, const int* offs) {
-  const int i = blockIdx.x * kScanTile + threadIdx.x;
-  const int b = blockIdx.x;
-  for (int k = 0; k < kScanItems; k++) {
-    int j = i + k * kScanThreads;
-    if (j < n) data[j] += offs[b];
+// exclusive scan of each tile, from the sum of the tiles before it (`sums`:
+// their sums, or, PREFIX, already their exclusive scan; null: one tile)
+template <bool PREFIX>
+__global__ void __launch_bounds__(kScanThreads) scan_tiles(int* __restrict__ data, int n, const int* __restrict__ sums) {
+  int off = 0;
+  if (sums) {
+    if (PREFIX) {
+      off = sums[blockIdx.x];
+    } else {
+      int t = 0;
+      for (int k = threadIdx.x; k < (int)blockIdx.x; k += kScanThreads) t += sums[k];
+      block_prefix(t, off);
+    }
+  }
+  // a warp's items are consecutive: 16 rows of 32
+  const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
+  const int base = blockIdx.x * kScanTile + w * 32 * kScanItems;
+  int v[kScanItems], t = 0;
+#pragma unroll
+  for (int i = 0; i < kScanItems; i++) {
+    const int j = base + i * 32 + lane;
+    v[i] = j < n ? data[j] : 0;
+    t += v[i];
+  }
+  int wsum = t;
+#pragma unroll
+  for (int o = 16; o; o >>= 1) wsum += __shfl_xor_sync(0xffffffffu, wsum, o);
+  int total;
+  const int before = block_prefix(lane == 0 ? wsum : 0, total);
+  int run = off + __shfl_sync(0xffffffffu, before, 0);
+#pragma unroll
+  for (int i = 0; i < kScanItems; i++) {
+    const int j = base + i * 32 + lane;
+    int incl = v[i];
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+      const int x = __shfl_up_sync(0xffffffffu, incl, o);
+      if (lane >= o) incl += x;
+    }
+    if (j < n) data[j] = run + incl - v[i];
+    run += __shfl_sync(0xffffffffu, incl, 31);
   }
 }
 
 }  // namespace
 
-// In-place exclusive scan (multi-level).
+// In-place exclusive scan: the tiles' sums, then every tile on top of the sums
+// before it, which its block adds up itself (two launches; three tile-local
+// passes before).  Above 4,096 tiles (16.8 M items) the sums are scanned first:
+// adding them up per block would read more than the data.
 void exclusive_scan(int* data, int n, cudaStream_t s) {
   if (n <= 0) return;
-  int nb = (n + kScanTile - 1) / kScanTile;
+  const int nb = (n + kScanTile - 1) / kScanTile;
   if (nb == 1) {
-    scan_tiles<<<1, kScanThreads, 0, s>>>(data, n, nullptr);
+    scan_tiles<false><<<1, kScanThreads, 0, s>>>(data, n, nullptr);
     FMMB_CHECK_LAUNCH();
     return;
   }
   TmpBuf<int> sums(s);  // freed in stream order
   sums.alloc(nb);
-  scan_tiles<<<nb, kScanThreads, 0, s>>>(data, n, sums.get());
+  scan_sums<<<nb, kScanThreads, 0, s>>>(data, n, sums.get());
   FMMB_CHECK_LAUNCH();
-  exclusive_scan(sums.get(), nb, s);
-  scan_add<<<nb, kScanThreads, 0, s>>>(data, n, sums.get());
+  if (nb <= 4096) {
+    scan_tiles<false><<<nb, kScanThreads, 0, s>>>(data, n, sums.get());
+  } else {
+    exclusive_scan(sums.get(), nb, s);
+    scan_tiles<true><<<nb, kScanThreads, 0, s>>>(data, n, sums.get());
+  }
   FMMB_CHECK_LAUNCH();
 }
 
@@ -311,19 +362,16 @@ __global__ void leaf_ranges(int nleaf, int n, const int* first, int2* leaf) {
   leaf[b] = make_int2(f, e - f);
 }
 
-// child ranges of each parent (children of one parent are contiguous and
-// every parent has at least one child): first the starts, then (next launch)
-// the counts from consecutive starts.
-__global__ void child_starts(int nchild, const int* parent, int* start) {
+// A broken tree must not reach the expansion kernels: the parents of a level's
+// boxes start at 0, grow by 0 or 1, end at nparent - 1 and none has more than 8
+// children.
+__global__ void check_parents(int nchild, const int* __restrict__ parent, int nparent, int* __restrict__ bad) {
   const int c = blockIdx.x * blockDim.x + threadIdx.x;
   if (c >= nchild) return;
-  const int p = parent[c];
-  if (c == 0 || parent[c - 1] != p) start[p] = c;
-}
-__global__ void child_counts(int nparent, int nchild, const int* start, int* count) {
-  const int p = blockIdx.x * blockDim.x + threadIdx.x;
-  if (p >= nparent) return;
-  count[p] = ((p + 1 < nparent) ? start[p + 1] : nchild) - start[p];
+  const int p = parent[c], before = c ? parent[c - 1] : -1;
+  const bool ok = p >= 0 && p < nparent && (c == 0 ? p == 0 : (p == before || p == before + 1)) &&
+                  (c < nchild - 1 || p == nparent - 1) && (c < 8 || parent[c - 8] != p);
+  if (!ok) *bad = 1;
 }
 
 __device__ __forceinline__ int find_key(const int* keys, int n, int k) {
@@ -337,23 +385,20 @@ __device__ __forceinline__ int find_key(const int* keys, int n, int k) {
 }
 
 // Near-field slots (fmm/ijbox.cxx:30-53): jx, jy, jz ascending over the 3x3x3
-// neighbourhood, self included.
+// neighbourhood, self included; one thread per slot.
 __global__ void p2p_lists(int nleaf_i, const int* key_i, int nleaf_j, const int* key_j, int lev, int* list) {
-  const int b = blockIdx.x * blockDim.x + threadIdx.x;
-  if (b >= nleaf_i) return;
+  const long long t = blockIdx.x * (long long)blockDim.x + threadIdx.x;
+  if (t >= (long long)nleaf_i * kP2PSlots) return;
+  const int b = (int)(t / kP2PSlots), s = (int)(t % kP2PSlots);
   int ix, iy, iz;
   const int smask = (1 << (3 * lev)) - 1, prob = key_i[b] & ~smask;
   demorton(key_i[b] & smask, ix, iy, iz);
   const int kl = 1 << lev;
-  int s = 0;
-  for (int jx = ix - 1; jx <= ix + 1; jx++)
-    for (int jy = iy - 1; jy <= iy + 1; jy++)
-      for (int jz = iz - 1; jz <= iz + 1; jz++) {
-        int v = -1;
-        if (jx >= 0 && jx < kl && jy >= 0 && jy < kl && jz >= 0 && jz < kl)
-          v = find_key(key_j, nleaf_j, prob | morton(jx, jy, jz, lev));
-        list[(size_t)b * kP2PSlots + s++] = v;
-      }
+  const int jx = ix + s / 9 - 1, jy = iy + (s / 3) % 3 - 1, jz = iz + s % 3 - 1;
+  int v = -1;
+  if (jx >= 0 && jx < kl && jy >= 0 && jy < kl && jz >= 0 && jz < kl)
+    v = find_key(key_j, nleaf_j, prob | morton(jx, jy, jz, lev));
+  list[t] = v;
 }
 
 // Interaction-list slots (fmm/ijbox.cxx:74-109), relative offsets per octant
@@ -376,23 +421,34 @@ __global__ void m2l_lists(int nbox_i, const int* key_i, int nbox_j, const int* k
   list[t] = v;
 }
 
+// adds v over the block's threads to *out with one atomic
+__device__ __forceinline__ void block_add(unsigned long long v, unsigned long long* out) {
+  __shared__ unsigned long long ws[32];
+  for (int o = 16; o; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
+  if ((threadIdx.x & 31) == 0) ws[threadIdx.x >> 5] = v;
+  __syncthreads();
+  if (threadIdx.x == 0) {
+    for (int k = 1; k < (int)blockDim.x / 32; k++) v += ws[k];
+    if (v) atomicAdd(out, v);
+  }
+}
+
 __global__ void count_p2p_pairs(int nleaf_i, const int2* leaf_i, const int2* leaf_j, const int* list,
                                 unsigned long long* out) {
-  const int b = blockIdx.x * blockDim.x + threadIdx.x;
-  if (b >= nleaf_i) return;
   unsigned long long acc = 0;
-  for (int s = 0; s < kP2PSlots; s++) {
-    const int j = list[(size_t)b * kP2PSlots + s];
-    if (j >= 0) acc += (unsigned long long)leaf_i[b].y * (unsigned long long)leaf_j[j].y;
+  const size_t n = (size_t)nleaf_i * kP2PSlots;
+  for (size_t t = blockIdx.x * (size_t)blockDim.x + threadIdx.x; t < n; t += (size_t)gridDim.x * blockDim.x) {
+    const int j = list[t];
+    if (j >= 0) acc += (unsigned long long)leaf_i[t / kP2PSlots].y * (unsigned long long)leaf_j[j].y;
   }
-  atomicAdd(out, acc);
+  block_add(acc, out);
 }
 
 __global__ void count_nonneg(size_t n, const int* list, unsigned long long* out) {
-  size_t i = blockIdx.x * (size_t)blockDim.x + threadIdx.x;
   unsigned long long acc = 0;
-  for (; i < n; i += (size_t)gridDim.x * blockDim.x) acc += list[i] >= 0;
-  atomicAdd(out, acc);
+  for (size_t i = blockIdx.x * (size_t)blockDim.x + threadIdx.x; i < n; i += (size_t)gridDim.x * blockDim.x)
+    acc += list[i] >= 0;
+  block_add(acc, out);
 }
 
 __global__ void minmax_kernel(int n, const float* x, float* out /*[2] min,max*/) {
@@ -435,7 +491,8 @@ int prob_bits(int nprob) {
 }
 
 // Builds keys, order, sorted points and all levels of one point set.
-void build_side(fmmb_plan* pl, const Side& sd, bool is_target, cudaStream_t s) {
+// bad: device flag, set when the levels do not fit together.
+void build_side(fmmb_plan* pl, const Side& sd, bool is_target, int* bad, cudaStream_t s) {
   const int n = sd.n, lmax = pl->lmax;
   TmpBuf<int> key(s), idx(s), flag(s), flag2(s), nbd(s);
   key.alloc(n);
@@ -528,42 +585,33 @@ void build_side(fmmb_plan* pl, const Side& sd, bool is_target, cudaStream_t s) {
   mask_keys<<<blocks(nbox[lmax], 256), 256, 0, s>>>(nbox[lmax], keys_all.get() + off[lmax], (1 << (3 * lmax)) - 1,
                                                     lk.get());
   FMMB_CHECK_LAUNCH();
-  if (!is_target) {
-    pl->child_start_j.alloc(tot);
-    pl->child_count_j.alloc(tot);
-    FMMB_CUDA(cudaMemsetAsync(pl->child_count_j.get(), 0, tot * sizeof(int), s));
-    for (int lev = lmax; lev >= 3; lev--) {
-      // children at lev, parents at lev-1 (indices within the level)
-      child_starts<<<blocks(nbox[lev], 256), 256, 0, s>>>(nbox[lev], parent_all.get() + off[lev],
-                                                         pl->child_start_j.get() + off[lev - 1]);
-      FMMB_CHECK_LAUNCH();
-      child_counts<<<blocks(nbox[lev - 1], 256), 256, 0, s>>>(nbox[lev - 1], nbox[lev], pl->child_start_j.get() + off[lev - 1],
-                                                             pl->child_count_j.get() + off[lev - 1]);
-      FMMB_CHECK_LAUNCH();
-    }
+  for (int lev = lmax; lev >= 3; lev--) {
+    check_parents<<<blocks(nbox[lev], 256), 256, 0, s>>>(nbox[lev], parent_all.get() + off[lev], nbox[lev - 1], bad);
+    FMMB_CHECK_LAUNCH();
   }
-  {
-    // cheap host checks that keep a broken tree from reaching the expansion
-    // kernels: every parent owns 1..8 children, every parent index is in range
-    std::vector<int> pa(tot), cc;
-    FMMB_CUDA(cudaMemcpyAsync(pa.data(), parent_all.get(), tot * sizeof(int), cudaMemcpyDeviceToHost, s));
-    if (!is_target) {
-      cc.resize(tot);
-      FMMB_CUDA(cudaMemcpyAsync(cc.data(), pl->child_count_j.get(), tot * sizeof(int), cudaMemcpyDeviceToHost, s));
-    }
-    FMMB_CUDA(cudaStreamSynchronize(s));
-    if (!is_target)
-      for (int lev = lmax - 1; lev >= 2; lev--)
-        for (int b = 0; b < nbox[lev]; b++) {
-          const int c = cc[off[lev] + b];
-          FMMB_REQUIRE(c >= 1 && c <= 8, FMMB_ERR_STATE, "tree build: inconsistent child count");
-        }
-    for (int lev = lmax; lev >= 3; lev--)
-      for (int b = 0; b < nbox[lev]; b++) {
-        const int q = pa[off[lev] + b];
-        FMMB_REQUIRE(q >= 0 && q < nbox[lev - 1], FMMB_ERR_STATE, "tree build: parent index out of range");
-      }
-  }
+}
+
+// The sources' tree where they are the targets' points, given as the same
+// arrays: a copy of the targets' (the normals may differ).
+void copy_side(fmmb_plan* pl, const Side& sd, cudaStream_t s) {
+  const int n = sd.n, lmax = pl->lmax;
+  pl->nbox_j = pl->nbox_i;
+  pl->off_j = pl->off_i;
+  pl->tot_j = pl->tot_i;
+  auto copy = [&](auto& to, const auto& from, size_t cnt) {
+    to.alloc(cnt);
+    FMMB_CUDA(cudaMemcpyAsync(to.get(), from.get(), cnt * sizeof(*to.get()), cudaMemcpyDeviceToDevice, s));
+  };
+  copy(pl->perm_j, pl->perm_i, n);
+  copy(pl->key_j, pl->key_i, pl->tot_i);
+  copy(pl->parent_j, pl->parent_i, pl->tot_i);
+  copy(pl->leaf_j, pl->leaf_i, pl->nbox_i[lmax]);
+  copy(pl->leafkey_j, pl->leafkey_i, pl->nbox_i[lmax]);
+  pl->spos.alloc(n);
+  pl->snrm.alloc(n);
+  gather_points<<<blocks(n, 256), 256, 0, s>>>(n, pl->perm_j.get(), sd.x, sd.y, sd.z, sd.nx, sd.ny, sd.nz,
+                                               pl->spos.get(), pl->snrm.get());
+  FMMB_CHECK_LAUNCH();
 }
 
 }  // namespace
@@ -626,13 +674,19 @@ void build_tree(fmmb_plan* pl, int ni, const float* tx, const float* ty, const f
     pl->bbox[3] = rd;
   }
   FMMB_REQUIRE(pl->bbox[3] > 0, FMMB_ERR_ARG, "root box side must be positive");
-  build_side(pl, Side{tx, ty, tz, tnx, tny, tnz, ni, pl->d_prob_off.get()}, true, s);
-  build_side(pl, Side{sx, sy, sz, snx, sny, snz, nj, pl->d_prob_off.get() + pl->nprob + 1}, false, s);
+  TmpBuf<unsigned long long> cnt(s);  // near-field pairs, M2L pairs, the tree check's flag
+  cnt.alloc(3);
+  FMMB_CUDA(cudaMemsetAsync(cnt.get(), 0, 3 * sizeof(unsigned long long), s));
+  int* bad = reinterpret_cast<int*>(cnt.get() + 2);
+  build_side(pl, Side{tx, ty, tz, tnx, tny, tnz, ni, pl->d_prob_off.get()}, true, bad, s);
+  const Side src{sx, sy, sz, snx, sny, snz, nj, pl->d_prob_off.get() + pl->nprob + 1};
+  if (pl->same_tree) copy_side(pl, src, s);
+  else build_side(pl, src, false, bad, s);
 
   const int lmax = pl->lmax;
   const int nleaf_i = pl->nbox_i[lmax], nleaf_j = pl->nbox_j[lmax];
   pl->p2p_list.alloc((size_t)nleaf_i * kP2PSlots);
-  p2p_lists<<<blocks(nleaf_i, 128), 128, 0, s>>>(nleaf_i, pl->key_i.get() + pl->off_i[lmax], nleaf_j,
+  p2p_lists<<<blocks((size_t)nleaf_i * kP2PSlots, 256), 256, 0, s>>>(nleaf_i, pl->key_i.get() + pl->off_i[lmax], nleaf_j,
                                                  pl->key_j.get() + pl->off_j[lmax], lmax, pl->p2p_list.get());
   FMMB_CHECK_LAUNCH();
   pl->m2l_list.alloc((size_t)pl->tot_i * kM2LSlots);
@@ -643,17 +697,15 @@ void build_tree(fmmb_plan* pl, int ni, const float* tx, const float* ty, const f
         pl->d_slot_rel.get(), pl->m2l_list.get() + (size_t)pl->off_i[lev] * kM2LSlots);
     FMMB_CHECK_LAUNCH();
   }
-  TmpBuf<unsigned long long> cnt(s);
-  cnt.alloc(2);
-  FMMB_CUDA(cudaMemsetAsync(cnt.get(), 0, 2 * sizeof(unsigned long long), s));
-  count_p2p_pairs<<<blocks(nleaf_i, 128), 128, 0, s>>>(nleaf_i, pl->leaf_i.get(), pl->leaf_j.get(), pl->p2p_list.get(),
+  count_p2p_pairs<<<std::min(blocks((size_t)nleaf_i * kP2PSlots, 256), 1184), 256, 0, s>>>(nleaf_i, pl->leaf_i.get(), pl->leaf_j.get(), pl->p2p_list.get(),
                                                        cnt.get());
   FMMB_CHECK_LAUNCH();
-  count_nonneg<<<256, 256, 0, s>>>((size_t)pl->tot_i * kM2LSlots, pl->m2l_list.get(), cnt.get() + 1);
+  count_nonneg<<<std::min(blocks((size_t)pl->tot_i * kM2LSlots, 1024), 1184), 256, 0, s>>>((size_t)pl->tot_i * kM2LSlots, pl->m2l_list.get(), cnt.get() + 1);
   FMMB_CHECK_LAUNCH();
-  unsigned long long h[2];
+  unsigned long long h[3];
   FMMB_CUDA(cudaMemcpyAsync(h, cnt.get(), sizeof(h), cudaMemcpyDeviceToHost, s));
   FMMB_CUDA(cudaStreamSynchronize(s));
+  FMMB_REQUIRE(h[2] == 0, FMMB_ERR_STATE, "tree build: inconsistent levels");
   pl->p2p_pairs = (long long)h[0];
   pl->m2l_pairs = (long long)h[1];
 }
