@@ -728,7 +728,7 @@ void run_one(fmmb_plan* pl, const float* qs, bool want_grad) {
         if (pl->p2m_nwork > nleaf_j)  // some leaf is summed by several items: its rows start at zero
           FMMB_CUDA(cudaMemsetAsync(Mleaf, 0, (size_t)nleaf_j * K * sizeof(double), m));
         done = launch_p2m_f32(ker, pl->p2m_nwork, pl->p2m_work.get(), p, K, pl->leafkey_j.get(), pl->leaf_j.get(),
-                              pl->spos.get(), pl->snrm.get(), qs, pl->bbox, rb_leaf, Mleaf, m);
+                              pl->spos.get(), pl->snrm.get(), qs, pl->d_fac.get(), pl->bbox, rb_leaf, Mleaf, m);
       }
       if (!done)
         launch_p2m_dmma(ker, nleaf_j, p, K, pl->leafkey_j.get(), pl->leaf_j.get(), pl->spos.get(), pl->snrm.get(), qs,

@@ -54,6 +54,29 @@ struct RecTab {
   __device__ const double2& operator[](int i) const { return d[i]; }
 };
 __constant__ RecTab c_rec = RecTab();
+// The FP32 kernels write S_n^m = g_n^m B_n^m t^m, t = x + i y, with the monic recurrence
+//   B_m = 1,  B_n = z B_{n-1} - c_n r^2 B_{n-2},  c_n = (n+m-1)(n-m-1) / ((2n-1)(2n-3)):
+// three operations a term, the factors g taken up by the coefficients.
+// g_n^m = (-1)^m (2m-1)!! prod_{k=m+1..n} (2k-1)/(k-m), at n (n+1) / 2 + m
+struct MonicTab {
+  double g[231];
+  constexpr MonicTab() : g() {
+    double f = 1.0;  // (-1)^m (2m-1)!!
+    for (int m = 0; m <= 20; m++) {
+      if (m > 0) f *= -(2.0 * m - 1.0);
+      double v = f;
+      for (int n = m; n <= 20; n++) {
+        if (n > m) v *= (2.0 * n - 1.0) / (n - m);
+        g[n * (n + 1) / 2 + m] = v;
+      }
+    }
+  }
+};
+__constant__ MonicTab c_monic = MonicTab();
+
+__device__ constexpr float monic_c(int n, int m) {  // c_n, n > m
+  return n > m + 1 ? (float)((double)((n + m - 1) * (n - m - 1)) / (double)((2 * n - 1) * (2 * n - 3))) : 0.f;
+}
 __device__ __forceinline__ cplx cmul(cplx a, cplx b) { return {a.re * b.re - a.im * b.im, a.re * b.im + a.im * b.re}; }
 __device__ __forceinline__ cplx cscale(cplx a, double s) { return {a.re * s, a.im * s}; }
 
@@ -250,8 +273,119 @@ __global__ void __launch_bounds__(kPts) p2m_dmma(int p, int K, const int* __rest
   }
 }
 
+// ------------------------------------------------------------------ P2M (FP32), charges
+// The mixed form's P2M of charges: the sums of p2m_dmma in FP32 and the monic form
+// (c_monic), one warp per work item of up to kP2MItem = 64 sources of a leaf.  A
+// lane evaluates two points side by side in the two-lane FP32 instructions and
+// leaves the columns of consecutive orders in shared memory until they fill 16
+// rows; then lane (row, re / im) adds its row over the points.  FP32 terms and
+// sums over one item's points; a leaf of several items (the dense leaves of
+// clustered points) is summed in FP64 by atomics into zeroed rows.
+// Bound: issue slots, the rows' sums (64 shared-memory reads and as many FMAs per
+// 16 rows) above the recurrences; 7 KB of shared memory a warp.  (One thread per
+// point with all (p+1)^2 terms staged, 43 KB per 64 points: 1,048,576 clustered
+// points, p = 12: 0.150 ms; 0.087 now.)
+constexpr int kFP = kP2MItem + 4;  // row stride of the staging (floats)
+constexpr int kFRows = 16, kFOrders = 5;  // staged rows; orders they span at most (1 + ... + 5 = 15)
+constexpr int kFWarps = 4;
+
+template <int P>
+__global__ void __launch_bounds__(32 * kFWarps) p2m_f32_charges(int p, int K, int nwork, const int2* __restrict__ work,
+                                                                const int* __restrict__ keys, const int2* __restrict__ leaf,
+                                                                const float4* __restrict__ spos,
+                                                                const float* __restrict__ qs,
+                                                                const double* __restrict__ fac, float xmin, float ymin,
+                                                                float zmin, double rb, double* __restrict__ M) {
+  __shared__ __align__(16) float sA[kFWarps][kFRows][kFP], sW[kFWarps][2 * kFOrders][kFP];
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  const int item = blockIdx.x * kFWarps + warp;
+  if (item >= nwork) return;
+  const int2 wk = work[item];
+  const int b = wk.x;
+  double xc, yc, zc;
+  box_center(keys[b], xmin, ymin, zmin, rb, xc, yc, zc);
+  const int2 lb = leaf[b];
+  const bool shared_leaf = lb.y > kP2MItem;  // summed by several items
+  const int first = lb.x + wk.y, cnt = min(kP2MItem, lb.y - wk.y);
+  const double inv_rb = 1.0 / rb;
+  float px[2], py[2], pz[2], pq[2];
+#pragma unroll
+  for (int h = 0; h < 2; h++) {  // the lane's points 2 lane, 2 lane + 1
+    const bool on = 2 * lane + h < cnt;
+    const int j = first + (on ? 2 * lane + h : 0);
+    const float4 v = spos[j];
+    pq[h] = on ? qs[j] : 0.f;
+    px[h] = (float)(((double)v.x - xc) * inv_rb);
+    py[h] = (float)(((double)v.y - yc) * inv_rb);
+    pz[h] = (float)(((double)v.z - zc) * inv_rb);
+  }
+  const float2 x = make_float2(px[0], px[1]), y = make_float2(py[0], py[1]), z = make_float2(pz[0], pz[1]);
+  const float2 nx = make_float2(-px[0], -px[1]), ny = make_float2(-py[0], -py[1]);
+  const float2 mr2 = __ffma2_rn(nx, x, __ffma2_rn(ny, y, __fmul2_rn(make_float2(-pz[0], -pz[1]), z)));  // -r^2
+  float2 tr = make_float2(pq[0], pq[1]), ti = make_float2(0.f, 0.f);  // q t^m
+  int rows = 0, m0 = 0;  // staged rows: the columns n = m..P of orders m0, m0 + 1, ... (constants once unrolled)
+  auto flush = [&](int nrow, int ma) {  // lane (row, component) adds its row over the points
+    __syncwarp();
+    const int r = lane >> 1, c = lane & 1;
+    if (r < nrow) {
+      int mm = ma, k0 = r;
+      while (k0 > P - mm) {
+        k0 -= P + 1 - mm;
+        mm++;
+      }
+      const int nn = mm + k0;
+      const float4* ar = reinterpret_cast<const float4*>(sA[warp][r]);
+      const float4* wr = reinterpret_cast<const float4*>(sW[warp][2 * (mm - ma) + c]);
+      float2 a0 = make_float2(0.f, 0.f), a1 = a0;
+      const int quads = (cnt + 3) / 4;
+#pragma unroll 4
+      for (int k = 0; k < quads; k++) {
+        const float4 a = ar[k], w = wr[k];
+        a0 = __ffma2_rn(make_float2(a.x, a.y), make_float2(w.x, w.y), a0);
+        a1 = __ffma2_rn(make_float2(a.z, a.w), make_float2(w.z, w.w), a1);
+      }
+      if (nn <= p && (mm > 0 || c == 0)) {
+        const double f = fac[ifull_d(nn, mm)] * c_monic.g[nn * (nn + 1) / 2 + mm];
+        const double v = (c ? -f : f) * (double)((a0.x + a0.y) + (a1.x + a1.y));
+        double* o = M + (size_t)b * K + nn * nn + (mm ? 2 * mm - 1 + c : 0);
+        if (shared_leaf) atomicAdd(o, v);
+        else *o = v;
+      }
+    }
+    __syncwarp();
+  };
+#pragma unroll
+  for (int m = 0; m <= P; m++) {
+    if (m > 0) {
+      const float2 t = __ffma2_rn(tr, x, __fmul2_rn(ti, ny));
+      ti = __ffma2_rn(tr, y, __fmul2_rn(ti, x));
+      tr = t;
+    }
+    if (rows + P + 1 - m > kFRows) {
+      flush(rows, m0);
+      rows = 0;
+    }
+    if (rows == 0) m0 = m;
+    reinterpret_cast<float2*>(sW[warp][2 * (m - m0)])[lane] = tr;
+    reinterpret_cast<float2*>(sW[warp][2 * (m - m0) + 1])[lane] = ti;
+    float2 b1 = make_float2(1.f, 1.f), b2 = make_float2(0.f, 0.f);
+#pragma unroll
+    for (int n = m; n <= P; n++, rows++) {
+      reinterpret_cast<float2*>(sA[warp][rows])[lane] = b1;
+      if (n < P) {
+        const float c = monic_c(n + 1, m);
+        const float2 bn = n == m ? __fmul2_rn(z, b1)
+                                 : __ffma2_rn(z, b1, __fmul2_rn(__fmul2_rn(make_float2(c, c), mr2), b2));
+        b2 = b1;
+        b1 = bn;
+      }
+    }
+  }
+  flush(rows, m0);
+}
+
 // ------------------------------------------------------------------ P2M (FP32)
-// Mixed-precision P2M: one thread per source point evaluates every S_n^m of
+// Mixed-precision P2M of dipoles: one thread per source point evaluates every S_n^m of
 // its point in FP32 with the degree rows held in registers (order P fixed at
 // compile time, runtime order p <= P), writes its contributions to shared
 // memory, and the block reduces the columns in FP64.  The multipole of a leaf
@@ -264,7 +398,7 @@ __constant__ float c_fac32[21 * 21 + 21];  // fac(n, m) at n*n+n+m, n <= 20
 
 constexpr int kP2MThreads = kP2MItem;
 
-template <int KER, int P>
+template <int P>
 __global__ void __launch_bounds__(kP2MThreads) p2m_f32(int p, int K, const int2* __restrict__ work,
                                                        const int* __restrict__ keys,
                                                        const int2* __restrict__ leaf, const float4* __restrict__ spos,
@@ -280,12 +414,9 @@ __global__ void __launch_bounds__(kP2MThreads) p2m_f32(int p, int K, const int2*
   const bool shared_leaf = leaf_b.y > kP2MThreads;  // summed by several items
   const int2 lf = make_int2(leaf_b.x + wk.y, min(kP2MThreads, leaf_b.y - wk.y));
   const double inv_rb = 1.0 / rb;
-  double acc0 = 0.0, acc1 = 0.0;  // columns threadIdx.x and threadIdx.x + 64 (K <= 128 per pass)
   double acc[(P + 1) * (P + 1) / kP2MThreads + 1];
 #pragma unroll
   for (int i = 0; i < (P + 1) * (P + 1) / kP2MThreads + 1; i++) acc[i] = 0.0;
-  (void)acc0;
-  (void)acc1;
   float* my = contrib + threadIdx.x * K;
   for (int j0 = 0; j0 < lf.y; j0 += kP2MThreads) {
     const int jj = j0 + threadIdx.x;
@@ -296,14 +427,8 @@ __global__ void __launch_bounds__(kP2MThreads) p2m_f32(int p, int K, const int2*
     const float x = (float)(((double)xs.x - xc) * inv_rb), y = (float)(((double)xs.y - yc) * inv_rb),
                 z = (float)(((double)xs.z - zc) * inv_rb);
     const float r2 = x * x + y * y + z * z;
-    float qnx = 0.f, qny = 0.f, qnz = 0.f;
-    if (KER == FMMB_LAPLACE_GNJ) {
-      const float4 nv = snrm[j];
-      const float s = q * (float)inv_rb;
-      qnx = s * nv.x;
-      qny = s * nv.y;
-      qnz = s * nv.z;
-    }
+    const float4 nv = snrm[j];
+    const float s = q * (float)inv_rb, qnx = s * nv.x, qny = s * nv.y, qnz = s * nv.z;
     float r1re[P + 1], r1im[P + 1], r2re[P + 1], r2im[P + 1];
 #pragma unroll
     for (int m = 0; m <= P; m++) r1re[m] = r1im[m] = r2re[m] = r2im[m] = 0.f;
@@ -332,35 +457,29 @@ __global__ void __launch_bounds__(kP2MThreads) p2m_f32(int p, int K, const int2*
         }
         if (n > p) continue;
         float vre, vim;
-        if (KER != FMMB_LAPLACE_GNJ) {
-          const float f = q * c_fac32[n * n + n + m];
-          vre = f * cre[m];
-          vim = -f * cim[m];
+        if (n == 0) {
+          vre = vim = 0.f;
         } else {
-          if (n == 0) {
-            vre = vim = 0.f;
+          // n . grad S_n^m from degree n-1
+          const float upr = (m + 1 <= n - 1) ? r1re[m + 1 <= P ? m + 1 : P] : 0.f;
+          const float upi = (m + 1 <= n - 1) ? r1im[m + 1 <= P ? m + 1 : P] : 0.f;
+          float dnr, dni, cm;
+          if (m == 0) {  // conj(S_{n-1}^1)
+            dnr = (n - 1 >= 1) ? r1re[1 <= P ? 1 : P] : 0.f;
+            dni = (n - 1 >= 1) ? -r1im[1 <= P ? 1 : P] : 0.f;
+            cm = 1.f;
           } else {
-            // n . grad S_n^m from degree n-1
-            const float upr = (m + 1 <= n - 1) ? r1re[m + 1 <= P ? m + 1 : P] : 0.f;
-            const float upi = (m + 1 <= n - 1) ? r1im[m + 1 <= P ? m + 1 : P] : 0.f;
-            float dnr, dni, cm;
-            if (m == 0) {  // conj(S_{n-1}^1)
-              dnr = (n - 1 >= 1) ? r1re[1 <= P ? 1 : P] : 0.f;
-              dni = (n - 1 >= 1) ? -r1im[1 <= P ? 1 : P] : 0.f;
-              cm = 1.f;
-            } else {
-              dnr = r1re[m - 1 >= 0 ? m - 1 : 0];
-              dni = r1im[m - 1 >= 0 ? m - 1 : 0];
-              cm = -(float)(n + m) * (float)(n + m - 1);
-            }
-            const float s1r = (m <= n - 1) ? r1re[m] : 0.f, s1i = (m <= n - 1) ? r1im[m] : 0.f;
-            // D = 1/2 (nx - i ny) up + 1/2 cm (nx + i ny) dn + nz (n+m) s1
-            const float Dre = 0.5f * (qnx * upr + qny * upi) + 0.5f * cm * (qnx * dnr - qny * dni) + qnz * (n + m) * s1r;
-            const float Dim = 0.5f * (qnx * upi - qny * upr) + 0.5f * cm * (qnx * dni + qny * dnr) + qnz * (n + m) * s1i;
-            const float f = c_fac32[n * n + n + m];
-            vre = f * Dre;
-            vim = -f * Dim;
+            dnr = r1re[m - 1 >= 0 ? m - 1 : 0];
+            dni = r1im[m - 1 >= 0 ? m - 1 : 0];
+            cm = -(float)(n + m) * (float)(n + m - 1);
           }
+          const float s1r = (m <= n - 1) ? r1re[m] : 0.f, s1i = (m <= n - 1) ? r1im[m] : 0.f;
+          // D = 1/2 (nx - i ny) up + 1/2 cm (nx + i ny) dn + nz (n+m) s1
+          const float Dre = 0.5f * (qnx * upr + qny * upi) + 0.5f * cm * (qnx * dnr - qny * dni) + qnz * (n + m) * s1r;
+          const float Dim = 0.5f * (qnx * upi - qny * upr) + 0.5f * cm * (qnx * dni + qny * dnr) + qnz * (n + m) * s1i;
+          const float f = c_fac32[n * n + n + m];
+          vre = f * Dre;
+          vim = -f * Dim;
         }
         if (m == 0) my[n * n] = vre;
         else {
@@ -687,19 +806,20 @@ __global__ void __launch_bounds__(kL2PHThreads) l2p_hess_gni(int p, int K, const
   }
 }
 
-// FP32 L2P for the mixed form: the same coefficient arrays as l2p_cart
-// (computed in FP64, stored as FP32 pairs), the solid harmonics S_n^m of a
-// point by the P2M recurrence in FP32 registers (fully unrolled to order P),
-// each degree's partial sums in FP32 and promoted to FP64 accumulators.
-constexpr int kL2PF32Threads = 128;  // one work item of up to 128 targets per block
+// FP32 L2P for the mixed form, one thread per target, one block per work item of
+// up to 128 targets of a leaf.  As l2p_cart, S_n^m = A_n^m s_m: the coefficients of
+// an order are summed over its degrees as reals times A and multiplied by the
+// complex s_m once per order; here in the monic form (c_monic, above), fully
+// unrolled to order P (runtime order p <= P).  Coefficients are formed in
+// FP64 and rounded; B, the powers of t and the sums of one order are FP32, the
+// sums over the orders FP64.
+// Bound: the FP32 pipe: 3 + 8 lane operations a term and two 16-byte
+// shared-memory reads.  (Complex recurrences and derivative sums per term, 16
+// operations and three reads: 1,048,576 targets at p = 12: 0.20 ms; 0.11 now.)
+constexpr int kL2PF32Threads = 128;
 
-// Shared-memory coefficient reads.  A thread evaluates one point (a block is
-// one work item of up to 128 targets), so the compiler is free to schedule
-// these loads ahead of their use in the unrolled degree / order loops.
-__device__ __forceinline__ float2 lds2(const float2* p) { return *p; }
-__device__ __forceinline__ float lds1(const float* p) { return *p; }
-
-template <int KER, int P>
+// POT / DER: the potential, its derivatives
+template <int KER, bool POT, bool DER, int P>
 __global__ void __launch_bounds__(kL2PF32Threads) l2p_f32(int p, int K, const int2* __restrict__ work,
                                                           const int* __restrict__ keys,
                                                           const int2* __restrict__ leaf, const float4* __restrict__ tpos,
@@ -708,15 +828,8 @@ __global__ void __launch_bounds__(kL2PF32Threads) l2p_f32(int p, int K, const in
                                                           const double* __restrict__ L, double* __restrict__ pot,
                                                           double* __restrict__ grad, int ni) {
   constexpr int NT = (P + 1) * (P + 2) / 2;
-  constexpr bool DER = KER != FMMB_LAPLACE_GNJ;  // derivative sums needed
-  __shared__ float2 Cphi[NT], Cz[DER ? NT : 1], Cp[DER ? NT : 1], Cm[DER ? NT : 1];
-  __shared__ float Cs[P + 1];
-  // the derivative sums in pairs for the two-lane FP32 FMAs: (fn, zn) from
-  // CA = (Cphi.re, Cz.re, -Cphi.im, -Cz.im), (pr, mr) and (pi, mi) from
-  // CB = (Cp.re, Cm.re, -Cp.im, -Cm.im) and CC = (Cp.im, Cm.im); the same
-  // per-lane operations, in the same order, as the scalar sums
-  __shared__ float4 CA[DER ? NT : 1], CB[DER ? NT : 1];
-  __shared__ float2 CC[DER ? NT : 1];
+  __shared__ float4 CA[DER ? NT : 1], CB[DER ? NT : 1];  // (d/dx, d/dy), (d/dz, potential), by order
+  __shared__ float2 CF[DER ? 1 : NT];                    // the potential alone
   const int2 wk = work[blockIdx.x];
   const int b = wk.x;
   const double* Lb = L + (size_t)b * K;
@@ -725,122 +838,90 @@ __global__ void __launch_bounds__(kL2PF32Threads) l2p_f32(int p, int K, const in
     return {Lb[n * n + 2 * m - 1], Lb[n * n + 2 * m]};
   };
   auto f2 = [](cplx c) { return make_float2((float)c.re, (float)c.im); };
-  for (int idx = threadIdx.x; idx < NT; idx += blockDim.x) {
+  for (int idx = threadIdx.x; idx < NT; idx += kL2PF32Threads) {
     int n = 0;
     while ((n + 1) * (n + 2) / 2 <= idx) n++;
     const int m = idx - n * (n + 1) / 2;
-    const double wm = m ? 2.0 : 1.0;
-    Cphi[idx] = n <= p ? f2(cscale(Lnm(n, m), wm * fac[ifull_d(n, m)])) : make_float2(0.f, 0.f);
-    if (DER) {
-      if (n < p) {
-        Cz[idx] = f2(cscale(Lnm(n + 1, m), wm * fac[ifull_d(n + 1, m)] * (n + 1 + m)));
-        Cp[idx] = (m >= 1) ? f2(cscale(Lnm(n + 1, m - 1), (m - 1 ? 2.0 : 1.0) * fac[ifull_d(n + 1, m - 1)]))
-                           : make_float2(0.f, 0.f);
-        Cm[idx] = f2(cscale(Lnm(n + 1, m + 1), -2.0 * fac[ifull_d(n + 1, m + 1)] * (double)(n + m + 2) * (double)(n + m + 1)));
-      } else {
-        Cz[idx] = Cp[idx] = Cm[idx] = make_float2(0.f, 0.f);
-      }
+    const int at = m * (P + 1) - m * (m - 1) / 2 + n - m;
+    const double g = c_monic.g[idx], wm = m ? 2.0 : 1.0;
+    float2 cf = make_float2(0.f, 0.f), cx = cf, cy = cf, cz = cf;
+    if (n <= p && POT) cf = f2(cscale(Lnm(n, m), g * wm * fac[ifull_d(n, m)]));
+    if (DER && n < p) {  // as l2p_cart
+      cz = f2(cscale(Lnm(n + 1, m), g * wm * fac[ifull_d(n + 1, m)] * (n + 1 + m)));
+      const cplx cp = m >= 1 ? cscale(Lnm(n + 1, m - 1), (m - 1 ? 2.0 : 1.0) * fac[ifull_d(n + 1, m - 1)]) : cplx{0.0, 0.0};
+      const cplx cm = cscale(Lnm(n + 1, m + 1), -2.0 * fac[ifull_d(n + 1, m + 1)] * (double)(n + m + 2) * (double)(n + m + 1));
+      const double cs = m == 1 ? fac[ifull_d(n + 1, 0)] * Lb[(n + 1) * (n + 1)] : 0.0;
+      cx = f2({g * (cp.re + cm.re + cs), g * (cp.im + cm.im)});
+      cy = f2({g * (cp.re - cm.re + cs), g * (cp.im - cm.im)});
     }
-  }
-  for (int n = threadIdx.x; n <= P; n += blockDim.x) Cs[n] = (n < p) ? (float)(fac[ifull_d(n + 1, 0)] * Lb[(n + 1) * (n + 1)]) : 0.f;
-  if (DER) {
-    __syncthreads();
-    for (int idx = threadIdx.x; idx < NT; idx += blockDim.x) {
-      const float2 f = Cphi[idx], zz = Cz[idx], pp = Cp[idx], mm = Cm[idx];
-      CA[idx] = make_float4(f.x, zz.x, -f.y, -zz.y);
-      CB[idx] = make_float4(pp.x, mm.x, -pp.y, -mm.y);
-      CC[idx] = make_float2(pp.y, mm.y);
+    if (DER) {
+      CA[at] = make_float4(cx.x, cx.y, cy.x, cy.y);
+      CB[at] = make_float4(cz.x, cz.y, cf.x, cf.y);
+    } else {
+      CF[at] = cf;
     }
   }
   __syncthreads();
   double xc, yc, zc;
   box_center(keys[b], xmin, ymin, zmin, rb, xc, yc, zc);
-  const int2 leaf_b = leaf[b];
-  const int2 lf = make_int2(leaf_b.x + wk.y, min(kL2PF32Threads, leaf_b.y - wk.y));  // this item's targets
+  const int2 lf = leaf[b];
   const double inv_rb = 1.0 / rb;
-  if ((int)threadIdx.x < lf.y) {  // one target per thread
-    const int i = lf.x + threadIdx.x;
-    const float4 xt = tpos[i];
-    const float x = (float)(((double)xt.x - xc) * inv_rb), y = (float)(((double)xt.y - yc) * inv_rb),
-                z = (float)(((double)xt.z - zc) * inv_rb);
-    const float r2 = x * x + y * y + z * z;
-    double F = 0, dzr = 0, dpr = 0, dpi = 0, dmr = 0, dmi = 0;
-    float r1re[P + 1], r1im[P + 1], r2re[P + 1], r2im[P + 1];
+  const int it = wk.y + threadIdx.x;
+  if (it >= lf.y) return;
+  const int i = lf.x + it;
+  const float4 xt = tpos[i];
+  const float x = (float)(((double)xt.x - xc) * inv_rb), y = (float)(((double)xt.y - yc) * inv_rb),
+              z = (float)(((double)xt.z - zc) * inv_rb);
+  const float mr2 = -(x * x + y * y + z * z);
+  double F = 0, gx = 0, gy = 0, gz = 0;
+  float tr = 1.f, ti = 0.f;  // t^m
 #pragma unroll
-    for (int m = 0; m <= P; m++) r1re[m] = r1im[m] = r2re[m] = r2im[m] = 0.f;
+  for (int m = 0; m <= P; m++) {
+    if (m > 0) {
+      const float t = tr * x - ti * y;
+      ti = tr * y + ti * x;
+      tr = t;
+    }
+    const float2 zero = make_float2(0.f, 0.f);
+    float2 uf = zero, ux = zero, uy = zero, uz = zero;
+    float b1 = 1.f, b2 = 0.f;
 #pragma unroll
-    for (int n = 0; n <= P; n++) {
-      float cre[P + 1], cim[P + 1];
-      float fn = 0.f;
-      float2 fz = make_float2(0.f, 0.f), pmr = fz, pmi = fz;  // (fn, zn), (pr, mr), (pi, mi)
-#pragma unroll
-      for (int m = 0; m <= P; m++) {
-        cre[m] = cim[m] = 0.f;
-        if (m > n) continue;
-        if (n == 0) {
-          cre[0] = 1.f;
-        } else if (m == n) {  // S_n^n = -(2n-1) (x + i y) S_{n-1}^{n-1}
-          const float a = -(2.f * n - 1.f);
-          cre[m] = a * (x * r1re[n - 1] - y * r1im[n - 1]);
-          cim[m] = a * (x * r1im[n - 1] + y * r1re[n - 1]);
-        } else if (m == n - 1) {
-          const float a = (2.f * n - 1.f) * z;
-          cre[m] = a * r1re[m];
-          cim[m] = a * r1im[m];
-        } else {
-          const float inv = 1.f / (float)(n - m);
-          const float a = (2.f * n - 1.f) * z * inv, c = (float)(n + m - 1) * r2 * inv;
-          cre[m] = a * r1re[m] - c * r2re[m];
-          cim[m] = a * r1im[m] - c * r2im[m];
-        }
-        const int idx = n * (n + 1) / 2 + m;
-        if (DER) {
-          const float4 a = CA[idx], bq = CB[idx];
-          const float2 cc = CC[idx];
-          const float2 re2 = make_float2(cre[m], cre[m]), im2 = make_float2(cim[m], cim[m]);
-          fz = __ffma2_rn(make_float2(a.x, a.y), re2, __ffma2_rn(make_float2(a.z, a.w), im2, fz));
-          pmr = __ffma2_rn(make_float2(bq.x, bq.y), re2, __ffma2_rn(make_float2(bq.z, bq.w), im2, pmr));
-          pmi = __ffma2_rn(make_float2(bq.x, bq.y), im2, __ffma2_rn(cc, re2, pmi));
-          if (m == 1) {  // Cs[n] * conj(S_n^1)
-            const float cs = lds1(Cs + n);
-            pmr.y = fmaf(cs, cre[m], pmr.y);
-            pmi.y = fmaf(-cs, cim[m], pmi.y);
-          }
-        } else {
-          const float2 cf = lds2(Cphi + idx);
-          fn = fmaf(cf.x, cre[m], fmaf(-cf.y, cim[m], fn));
-        }
-      }
+    for (int n = m; n <= P; n++) {
+      const int at = m * (P + 1) - m * (m - 1) / 2 + n - m;
+      const float2 bb = make_float2(b1, b1);
       if (DER) {
-        F += (double)fz.x;
-        dzr += (double)fz.y;
-        dpr += (double)pmr.x;
-        dpi += (double)pmi.x;
-        dmr += (double)pmr.y;
-        dmi += (double)pmi.y;
+        const float4 ca = CA[at], cb = CB[at];
+        ux = __ffma2_rn(make_float2(ca.x, ca.y), bb, ux);
+        uy = __ffma2_rn(make_float2(ca.z, ca.w), bb, uy);
+        uz = __ffma2_rn(make_float2(cb.x, cb.y), bb, uz);
+        if (POT) uf = __ffma2_rn(make_float2(cb.z, cb.w), bb, uf);
       } else {
-        F += (double)fn;
+        uf = __ffma2_rn(CF[at], bb, uf);
       }
-#pragma unroll
-      for (int m = 0; m <= P; m++) {
-        r2re[m] = r1re[m];
-        r2im[m] = r1im[m];
-        r1re[m] = cre[m];
-        r1im[m] = cim[m];
+      if (n < P) {
+        const float bn = n == m ? z * b1 : fmaf(z, b1, (monic_c(n + 1, m) * mr2) * b2);
+        b2 = b1;
+        b1 = bn;
       }
     }
-    const double gx = 0.5 * (dpr + dmr), gy = 0.5 * (dpi - dmi), gz = dzr;
-    const double c1 = coef * inv_rb, c2 = coef * inv_rb * inv_rb;
-    if (KER == FMMB_LAPLACE_GNI) {
-      const float4 nv = tnrm[i];
-      pot[i] = -c2 * ((double)nv.x * gx + (double)nv.y * gy + (double)nv.z * gz);
-    } else {
-      pot[i] = c1 * F;
-      if (KER == FMMB_LAPLACE_G && grad) {
-        grad[i] = c2 * gx;
-        grad[ni + i] = c2 * gy;
-        grad[2 * ni + i] = c2 * gz;
-      }
+    // times t^m: potential and d/dz the real parts, d/dx the real part of X s, d/dy the imaginary part of Y s
+    if (POT) F += (double)(uf.x * tr - uf.y * ti);
+    if (DER) {
+      gx += (double)(ux.x * tr - ux.y * ti);
+      gy += (double)(uy.x * ti + uy.y * tr);
+      gz += (double)(uz.x * tr - uz.y * ti);
+    }
+  }
+  const double c1 = coef * inv_rb, c2 = coef * inv_rb * inv_rb;
+  if (KER == FMMB_LAPLACE_GNI) {
+    const float4 nv = tnrm[i];
+    pot[i] = -c2 * ((double)nv.x * (0.5 * gx) + (double)nv.y * (0.5 * gy) + (double)nv.z * gz);
+  } else {
+    pot[i] = c1 * F;
+    if (DER) {
+      grad[i] = c2 * (0.5 * gx);
+      grad[ni + (size_t)i] = c2 * (0.5 * gy);
+      grad[2 * (size_t)ni + i] = c2 * gz;
     }
   }
 }
@@ -849,12 +930,13 @@ template <int P>
 void l2p_f32_launch(int kernel, int nwork, const int2* work, int p, int K, const int* keys, const int2* leaf,
                     const float4* tpos, const float4* tnrm, const double* fac, const float* bbox, double rb,
                     double coef, const double* L, double* pot, double* grad, int ni, cudaStream_t st) {
-  if (kernel == FMMB_LAPLACE_G)
-    l2p_f32<FMMB_LAPLACE_G, P><<<nwork, kL2PF32Threads, 0, st>>>(p, K, work, keys, leaf, tpos, tnrm, fac, bbox[0], bbox[1], bbox[2], rb, coef, L, pot, grad, ni);
-  else if (kernel == FMMB_LAPLACE_GNI)
-    l2p_f32<FMMB_LAPLACE_GNI, P><<<nwork, kL2PF32Threads, 0, st>>>(p, K, work, keys, leaf, tpos, tnrm, fac, bbox[0], bbox[1], bbox[2], rb, coef, L, pot, grad, ni);
-  else
-    l2p_f32<FMMB_LAPLACE_GNJ, P><<<nwork, kL2PF32Threads, 0, st>>>(p, K, work, keys, leaf, tpos, tnrm, fac, bbox[0], bbox[1], bbox[2], rb, coef, L, pot, grad, ni);
+  auto go = [&](auto k) {
+    k<<<nwork, kL2PF32Threads, 0, st>>>(p, K, work, keys, leaf, tpos, tnrm, fac, bbox[0], bbox[1], bbox[2], rb, coef, L,
+                                        pot, grad, ni);
+  };
+  if (kernel == FMMB_LAPLACE_GNI) go(l2p_f32<FMMB_LAPLACE_GNI, false, true, P>);
+  else if (kernel == FMMB_LAPLACE_G && grad) go(l2p_f32<FMMB_LAPLACE_G, true, true, P>);
+  else go(l2p_f32<FMMB_LAPLACE_G, true, false, P>);
 }
 
 }  // namespace
@@ -878,13 +960,14 @@ void launch_p2m_dmma(int kernel, int nleaf, int p, int K, const int* keys, const
 namespace {
 template <int P>
 void p2m_f32_launch(int kernel, int nwork, const int2* work, int p, int K, const int* keys, const int2* leaf,
-                    const float4* spos, const float4* snrm, const float* qs, const float* bbox, double rb, double* M,
-                    cudaStream_t st) {
+                    const float4* spos, const float4* snrm, const float* qs, const double* fac, const float* bbox, double rb,
+                    double* M, cudaStream_t st) {
   const size_t sm = (size_t)kP2MThreads * K * sizeof(float);
   if (kernel == FMMB_LAPLACE_GNJ)
-    p2m_f32<FMMB_LAPLACE_GNJ, P><<<nwork, kP2MThreads, sm, st>>>(p, K, work, keys, leaf, spos, snrm, qs, bbox[0], bbox[1], bbox[2], rb, M);
+    p2m_f32<P><<<nwork, kP2MThreads, sm, st>>>(p, K, work, keys, leaf, spos, snrm, qs, bbox[0], bbox[1], bbox[2], rb, M);
   else
-    p2m_f32<FMMB_LAPLACE_G, P><<<nwork, kP2MThreads, sm, st>>>(p, K, work, keys, leaf, spos, snrm, qs, bbox[0], bbox[1], bbox[2], rb, M);
+    p2m_f32_charges<P><<<(nwork + kFWarps - 1) / kFWarps, 32 * kFWarps, 0, st>>>(
+        p, K, nwork, work, keys, leaf, spos, qs, fac, bbox[0], bbox[1], bbox[2], rb, M);
 }
 }  // namespace
 
@@ -905,15 +988,13 @@ void init_fac32() {
 }
 
 bool launch_p2m_f32(int kernel, int nwork, const int2* work, int p, int K, const int* keys, const int2* leaf,
-                    const float4* spos, const float4* snrm, const float* qs, const float* bbox, double rb, double* M,
-                    cudaStream_t st) {
-  if ((size_t)kP2MThreads * K * sizeof(float) > 48 * 1024) return false;  // per-point rows staged in shared memory
-  if (p > 16) return false;
+                    const float4* spos, const float4* snrm, const float* qs, const double* fac, const float* bbox,
+                    double rb, double* M, cudaStream_t st) {
+  if (p > 12) return false;  // FP64 above
   if (nwork <= 0) return true;
-  if (p <= 8) p2m_f32_launch<8>(kernel, nwork, work, p, K, keys, leaf, spos, snrm, qs, bbox, rb, M, st);
-  else if (p <= 10) p2m_f32_launch<10>(kernel, nwork, work, p, K, keys, leaf, spos, snrm, qs, bbox, rb, M, st);
-  else if (p <= 12) p2m_f32_launch<12>(kernel, nwork, work, p, K, keys, leaf, spos, snrm, qs, bbox, rb, M, st);
-  else p2m_f32_launch<16>(kernel, nwork, work, p, K, keys, leaf, spos, snrm, qs, bbox, rb, M, st);
+  if (p <= 8) p2m_f32_launch<8>(kernel, nwork, work, p, K, keys, leaf, spos, snrm, qs, fac, bbox, rb, M, st);
+  else if (p <= 10) p2m_f32_launch<10>(kernel, nwork, work, p, K, keys, leaf, spos, snrm, qs, fac, bbox, rb, M, st);
+  else p2m_f32_launch<12>(kernel, nwork, work, p, K, keys, leaf, spos, snrm, qs, fac, bbox, rb, M, st);
   FMMB_CHECK_LAUNCH();
   return true;
 }

@@ -1,0 +1,73 @@
+"""Mixed form at the edges of its tiles: the many-right-hand-side near field (tiles of 16 targets, teams of 8 warps, groups
+of 8 / 4 / 2 / 1 right-hand sides) and the FP32 P2M and L2P (items of 64 sources and 128 targets, 16 staged rows)."""
+import numpy as np
+import pytest
+
+import old_fmm_bem_b200 as ob
+
+pytestmark = pytest.mark.gpu
+
+
+def _unit(rng, n):
+    v = rng.standard_normal((3, n))
+    return (v / np.linalg.norm(v, axis=0)).astype(np.float32)
+
+
+@pytest.mark.parametrize("kernel", [ob.LAPLACE_G, ob.LAPLACE_GNI, ob.LAPLACE_GNJ])
+@pytest.mark.parametrize("nrhs", [2, 5, 8, 15])
+@pytest.mark.parametrize("ni,nj", [(1, 1), (9, 33), (17, 513), (33, 100), (65, 65), (129, 1100), (700, 31)])
+def test_many_rhs_near_field_equals_direct(kernel, nrhs, ni, nj):
+    # eight mutually neighbouring leaves: no far field.  Bound: at most 67 roundings of an FP32 sum and 13 of a term,
+    # 2^-24 each, of the sum of the terms' magnitudes
+    rng = np.random.default_rng(ni * 10007 + nj)
+    xt = (rng.random((3, ni)) * np.where(rng.random(ni) < 0.7, 0.24, 0.49)).astype(np.float32)
+    xs = (rng.random((3, nj)) * np.where(rng.random(nj) < 0.7, 0.24, 0.49)).astype(np.float32)
+    m = min(ni, nj) // 2
+    xs[:, :m] = xt[:, :m]  # coincident pairs
+    tn, sn = _unit(rng, ni), _unit(rng, nj)
+    q = rng.standard_normal((nrhs, nj)).astype(np.float32)
+    with ob.Plan(kernel=kernel, p=4, lmax=2, precision=ob.MIXED, semantics=ob.SEM_ACCURATE, exclude_self=True,
+                 nrhs=nrhs) as pl:
+        pl.set_geometry(xt, xs, tn if kernel == ob.LAPLACE_GNI else None, sn if kernel == ob.LAPLACE_GNJ else None,
+                        bbox=(0, 0, 0, 1))
+        pot, grad = pl.evaluate(q.reshape(-1), f64=True)
+    d = xt.astype(np.float64)[:, :, None] - xs.astype(np.float64)[:, None, :]
+    r2 = (d ** 2).sum(0)
+    ri = np.where(r2 > 0, 1.0 / np.sqrt(np.where(r2 > 0, r2, 1.0)), 0.0)
+    qd, c, tol = q.astype(np.float64).T, 0.25 / np.pi, 80 * 2.0 ** -24
+    if kernel == ob.LAPLACE_G:
+        t = [ri] + [-d[k] * ri ** 3 for k in range(3)]
+        mag = [abs(v) for v in t]
+    else:
+        n = (tn[:, :, None] if kernel == ob.LAPLACE_GNI else sn[:, None, :]).astype(np.float64)
+        t, mag = [(d * n).sum(0) * ri ** 3], [abs(d * n).sum(0) * ri ** 3]
+    assert np.all(abs(pot.reshape(nrhs, ni).T - c * t[0] @ qd) <= tol * c * (mag[0] @ abs(qd)))
+    if grad is not None:
+        g = grad.reshape(nrhs, 3, ni)
+        for k in range(3):
+            assert np.all(abs(g[:, k].T - c * t[1 + k] @ qd) <= tol * c * (mag[1 + k] @ abs(qd)))
+
+
+@pytest.mark.parametrize("kernel", [ob.LAPLACE_G, ob.LAPLACE_GNI, ob.LAPLACE_GNJ])
+@pytest.mark.parametrize("p", [1, 4, 5, 8, 9, 10, 11, 12, 14, 16])
+@pytest.mark.parametrize("ni,nj", [(1, 1), (31, 33), (64, 63), (65, 129), (300, 257)])
+def test_mixed_expansions_match_fp64(kernel, p, ni, nj):
+    # sources in one corner leaf, targets in the opposite one: P2M, one M2L, L2P.  2e-6 of the sum of magnitudes: FP32
+    # terms and sums of up to 64 points, 22-bit operators, FP32 sums of up to p + 1 terms
+    rng = np.random.default_rng(p * 977 + ni + 7 * nj)
+    xs = (rng.random((3, nj)) * 0.249).astype(np.float32)
+    xt = (0.751 + rng.random((3, ni)) * 0.248).astype(np.float32)
+    tn, sn = _unit(rng, ni), _unit(rng, nj)
+    q = (rng.random(nj) + 0.1).astype(np.float32)
+    out = []
+    for prec in (ob.MIXED, ob.FP64):
+        with ob.Plan(kernel=kernel, p=p, lmax=2, precision=prec, semantics=ob.SEM_ACCURATE, exclude_self=True) as pl:
+            pl.set_geometry(xt, xs, tn if kernel == ob.LAPLACE_GNI else None, sn if kernel == ob.LAPLACE_GNJ else None,
+                            bbox=(0, 0, 0, 1))
+            out.append(pl.evaluate(q, f64=True))
+    r = np.linalg.norm(xt.astype(np.float64)[:, :, None] - xs[:, None, :], axis=0)
+    mag = (q / (4 * np.pi * (r if kernel == ob.LAPLACE_G else r ** 2))).sum(1)
+    assert np.all(abs(out[0][0] - out[1][0]) <= 2e-6 * mag)
+    if kernel == ob.LAPLACE_G:
+        gm = (q / (4 * np.pi * r ** 2)).sum(1)
+        assert np.all(abs(out[0][1] - out[1][1]).reshape(3, -1) <= 2e-6 * gm)
