@@ -469,8 +469,8 @@ def run_ours(args, rank, world, secondary=False):
     phase /= args.steps
     launches = plan.stats()["launches"]
     # each kernel's own duration: the same steps with the near field run
-    # after the far field instead of beside it (phase timers, CUDA events on
-    # the launching stream, L2 flushed between steps)
+    # after the far field instead of beside it (phase timers: CUDA events on the
+    # launching stream around each phase of the step's launches run once more)
     plan.set_overlap(False)
     phase_alone = np.zeros(7)
     with torch.cuda.stream(stream):

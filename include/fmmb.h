@@ -347,9 +347,12 @@ FMMB_API int fmmb_get_tree(fmmb_plan* plan, int kind, int* out);
 FMMB_API long fmmb_get_expansion_size(fmmb_plan* plan, int which);
 FMMB_API int fmmb_get_expansions(fmmb_plan* plan, int which, double* out);
 
-/* Device time in ms of the phases of the last evaluate, summed over the
- * launches of each phase (all right-hand sides): [0] P2P, [1] P2M, [2] M2M,
- * [3] M2L, [4] L2L, [5] L2P, [6] whole evaluate (P2P overlaps the far field). */
+/* Device time in ms of the phases of the last evaluate (its last right-hand
+ * side), summed over the launches of each phase: [0] P2P, [1] P2M, [2] M2M,
+ * [3] M2L, [4] L2L, [5] L2P, [6] whole evaluate (P2P overlaps the far field).
+ * The phases are measured here, by running that evaluate's launches once more
+ * inside the plan (no output changes), so that the evaluates themselves carry no
+ * timing events; they read 0 when fmmb_set_geometry came since. */
 FMMB_API int fmmb_get_timings(fmmb_plan* plan, float* ms7);
 
 /* Overlap of the near field with the far field (default on).  With on = 0

@@ -300,6 +300,8 @@ int geometry_impl(fmmb_plan* pl, int nprob, const int* toff, const int* soff, in
       FMMB_REQUIRE(to[0] == 0 && so[0] == 0 && to[nprob] == ni && so[nprob] == nj, FMMB_ERR_ARG,
                    "problem offsets must run from 0 to the point counts");
     }
+    if (pl->phases.state == fmmb_plan::Phases::kPending)  // its charges and work lists go
+      pl->phases.state = fmmb_plan::Phases::kNone;
     for (int w = 0; w < 4; w++) {  // captured evaluates refer to the old buffers
       pl->gused[w] = false;
       if (pl->gexec[w]) {
@@ -542,29 +544,24 @@ int fmmb_set_geometry_batch(fmmb_plan* pl, int nprob, const int* t_off, const fl
 
 namespace {
 
-// Brackets one launch with a pair of pool events (phase 0..5 as in
-// fmmb_get_timings); silently stops timing when the pool is exhausted.
-// Records a timing event; while the evaluate is being captured into a graph,
-// as an event-record node (a plain record would only become a dependency).
-cudaError_t time_mark(const fmmb_plan* pl, cudaEvent_t e, cudaStream_t s) {
-  return cudaEventRecordWithFlags(e, s, pl->capturing ? cudaEventRecordExternal : cudaEventRecordDefault);
-}
-
+// Counts a phase's launch and, while the phases are being measured
+// (measure_phases), brackets it with a pair of pool events (phase 0..5 as in
+// fmmb_get_timings; silently untimed when the pool is exhausted).
 struct PhaseTimer {
   fmmb_plan* pl;
   int phase, idx;
   cudaStream_t s;
   PhaseTimer(fmmb_plan* p, int ph, cudaStream_t st) : pl(p), phase(ph), idx(-1), s(st) {
-    if (pl->ev_used + 2 <= fmmb_plan::kEvPool) {
+    if (pl->timing && pl->ev_used + 2 <= fmmb_plan::kEvPool) {
       idx = pl->ev_used;
       pl->ev_used += 2;
-      FMMB_CUDA(time_mark(pl, pl->evp[idx], s));
+      FMMB_CUDA(cudaEventRecord(pl->evp[idx], s));
     }
     pl->launches++;
   }
   ~PhaseTimer() {
     if (idx >= 0) {
-      time_mark(pl, pl->evp[idx + 1], s);
+      cudaEventRecord(pl->evp[idx + 1], s);
       pl->ev_phase.push_back({phase, idx});
     }
   }
@@ -616,7 +613,6 @@ void run_one_helm(fmmb_plan* pl, const float* qs) {
   const double wleaf = (double)pl->bbox[3] / (double)(1 << lmax);
   FMMB_CUDA(cudaEventRecord(pl->st.fork, m));
   FMMB_CUDA(cudaStreamWaitEvent(side, pl->st.fork, 0));
-  FMMB_CUDA(time_mark(pl, pl->ev[0], side));
   {
     PhaseTimer tm(pl, 0, side);
     launch_helm_p2p(pl->cfg.precision == FMMB_MIXED, yuk, (float)k, (float)pl->cfg.eps2, pl->cfg.exclude_self != 0,
@@ -624,15 +620,12 @@ void run_one_helm(fmmb_plan* pl, const float* qs) {
                     pl->leaf_i.get(), pl->leaf_j.get(), pl->p2p_list.get(), pl->tpos.get(), pl->spos.get(), qs,
                     pot_near, side);
   }
-  FMMB_CUDA(time_mark(pl, pl->ev[1], side));
   FMMB_CUDA(cudaEventRecord(pl->st.join, side));
-  FMMB_CUDA(time_mark(pl, pl->ev[2], m));
   {
     PhaseTimer tm(pl, 1, m);
     launch_helm_p2m(nleaf_j, p, k, yuk, pl->leafkey_j.get(), pl->leaf_j.get(), pl->spos.get(), qs,
                     pl->d_ylm.get(), pl->bbox, wleaf, pl->M.get() + (size_t)pl->off_j[lmax] * 2 * K, m);
   }
-  FMMB_CUDA(time_mark(pl, pl->ev[3], m));
   auto pairs_run = [&](const fmmb_plan::PairTiles& job, int lev, double* xin, double* out, int atomic, int phase) {
     if (job.ntile[lev] <= 0) return;
     PhaseTimer tm(pl, phase, m);
@@ -650,18 +643,15 @@ void run_one_helm(fmmb_plan* pl, const float* qs) {
   const size_t above = (size_t)(pl->tot_j - pl->nbox_j[lmax]) * 2 * K;
   if (above) FMMB_CUDA(cudaMemsetAsync(pl->M.get() + (size_t)pl->off_j[lmax - 1] * 2 * K, 0, above * sizeof(double), m));
   for (int lev = lmax - 1; lev >= 2; lev--) pairs_run(pl->m2m_tiles, lev + 1, pl->M.get(), pl->M.get(), 1, 2);
-  FMMB_CUDA(time_mark(pl, pl->ev[4], m));
   FMMB_CUDA(cudaMemsetAsync(pl->L.get(), 0, (size_t)pl->tot_i * 2 * K * sizeof(double), m));
   run_parity(pl, yuk ? 2 : 1, m);
   for (int lev = 3; lev <= lmax; lev++) pairs_run(pl->l2l_tiles, lev, pl->L.get(), pl->L.get(), 1, 4);
-  FMMB_CUDA(time_mark(pl, pl->ev[5], m));
   {
     PhaseTimer tm(pl, 5, m);
     launch_helm_l2p(pl->m_p2p_nwork, p, k, yuk, pl->m_p2p_work.get(), pl->leafkey_i.get(), pl->leaf_i.get(),
                     pl->tpos.get(), pl->d_ylm.get(), pl->bbox, wleaf,
                     pl->L.get() + (size_t)pl->off_i[lmax] * 2 * K, pot_far, m);
   }
-  FMMB_CUDA(time_mark(pl, pl->ev[6], m));
   FMMB_CUDA(cudaStreamWaitEvent(m, pl->st.join, 0));
 }
 
@@ -694,7 +684,6 @@ void run_one(fmmb_plan* pl, const float* qs, bool want_grad) {
     }
     FMMB_CUDA(cudaEventRecord(pl->st.fork, m));
     FMMB_CUDA(cudaStreamWaitEvent(side, pl->st.fork, 0));
-    if (l0 == 0) FMMB_CUDA(time_mark(pl, pl->ev[0], side));
     {
       PhaseTimer tm(pl, 0, side);
       const int2* wk = pl->p2p_work.get() + l0;
@@ -706,7 +695,6 @@ void run_one(fmmb_plan* pl, const float* qs, bool want_grad) {
                        pl->tnrm.get(), pl->spos.get(), pl->snrm.get(), qs, s, pot_near, g_near, pl->ni, side);
     }
     if (last) {
-      FMMB_CUDA(time_mark(pl, pl->ev[1], side));
       FMMB_CUDA(cudaEventRecord(pl->st.join, side));
     }
   };
@@ -714,7 +702,6 @@ void run_one(fmmb_plan* pl, const float* qs, bool want_grad) {
   near_field(0, p2p_split, false);
 
   // far field on the main stream
-  FMMB_CUDA(time_mark(pl, pl->ev[2], m));
   const double rb_leaf = (double)(pl->bbox[3] / (float)(1 << lmax));
   {
     PhaseTimer tm(pl, 1, m);
@@ -735,7 +722,6 @@ void run_one(fmmb_plan* pl, const float* qs, bool want_grad) {
                         pl->d_fac.get(), s, pl->bbox, rb_leaf, Mleaf, m);
     }
   }
-  FMMB_CUDA(time_mark(pl, pl->ev[3], m));
   // upward pass: parents accumulate their children (levels below lmax start at zero)
   if (lmax > 2)
     FMMB_CUDA(cudaMemsetAsync(pl->M.get() + (size_t)pl->off_j[lmax - 1] * K, 0,
@@ -783,7 +769,6 @@ void run_one(fmmb_plan* pl, const float* qs, bool want_grad) {
     PhaseTimer tm(pl, 2, m);
     launch_split_h16(pl->tot_j, K, pl->M.get(), pl->Xh.get(), pl->xexp.get(), m);
   }
-  FMMB_CUDA(time_mark(pl, pl->ev[4], m));
   // downward pass: M2L of every level into zeroed locals, then each level
   // adds its parent's translated local (L2L), top down
   FMMB_CUDA(cudaMemsetAsync(pl->L.get(), 0, (size_t)pl->tot_i * K * sizeof(double), m));
@@ -814,7 +799,6 @@ void run_one(fmmb_plan* pl, const float* qs, bool want_grad) {
   near_field(p2p_split, pl->p2p_nwork, true);
   for (int lev = 3; lev <= lmax; lev++)  // children at lev from their parent (one pair each, added by one atomic)
     pairs_run(pl->l2l_tiles, lev, pl->d_l2l_t.get(), pl->L.get(), pl->L.get(), 1, 4);
-  FMMB_CUDA(time_mark(pl, pl->ev[5], m));
   {
     PhaseTimer tm(pl, 5, m);
     if (pl->ref)
@@ -833,7 +817,6 @@ void run_one(fmmb_plan* pl, const float* qs, bool want_grad) {
                           pl->d_fac.get(), pl->bbox, rb_leaf, s.coef, pl->L.get() + (size_t)pl->off_i[lmax] * K, g_far,
                           pl->ni, m);
   }
-  FMMB_CUDA(time_mark(pl, pl->ev[6], m));
   FMMB_CUDA(cudaStreamWaitEvent(m, pl->st.join, 0));
 }
 
@@ -868,16 +851,12 @@ void run_graph(fmmb_plan* pl, bool want_grad, bool far_only = false) {
     FMMB_CUDA(cudaStreamBeginCapture(c, cudaStreamCaptureModeThreadLocal));
     cudaGraph_t graph = nullptr;
     pl->st.main = c;
-    pl->capturing = true;
     pl->far_only = far_only;
-    pl->ev_used = 0;  // the graph's own timing events, and its launches counted as in the direct run
-    pl->ev_phase.clear();
-    pl->launches = pl->gbase[w];
+    pl->launches = pl->gbase[w];  // counted as in the direct run
     try {
       run_one(pl, qin, want_grad);
     } catch (...) {
       pl->st.main = m;
-      pl->capturing = false;
       pl->far_only = false;
       cudaStreamEndCapture(c, &graph);
       if (graph) cudaGraphDestroy(graph);
@@ -885,7 +864,6 @@ void run_graph(fmmb_plan* pl, bool want_grad, bool far_only = false) {
       throw;
     }
     pl->st.main = m;
-    pl->capturing = false;
     pl->far_only = false;
     FMMB_CUDA(cudaStreamEndCapture(c, &graph));
     cudaGraphExec_t exec = nullptr;
@@ -894,20 +872,49 @@ void run_graph(fmmb_plan* pl, bool want_grad, bool far_only = false) {
     if (e != cudaSuccess) {
       cudaGetLastError();
       pl->use_graph = false;
-      pl->ev_used = 0;
-      pl->ev_phase.clear();
       pl->far_only = far_only;
       run_one(pl, qin, want_grad);
       pl->far_only = false;
       return;
     }
     pl->gexec[w] = exec;
-    pl->gphase[w] = pl->ev_phase;
     pl->glaunches[w] = pl->launches;
   }
-  pl->ev_phase = pl->gphase[w];
   pl->launches = pl->glaunches[w];
   FMMB_CUDA(cudaGraphLaunch(pl->gexec[w], m));
+}
+
+// The phase times of the last evaluate (its last right-hand side): its launches
+// run once more on the plan's own buffers, which hold its charges, with events
+// between the phases.  The evaluates themselves carry none: 26 event records took
+// 40 to 130 us of each (2,000 points, mixed: 117 us against 71 without).
+void measure_phases(fmmb_plan* pl) {
+  fmmb_plan::Phases& ph = pl->phases;
+  if (ph.state != fmmb_plan::Phases::kPending) return;
+  const int launches = pl->launches;
+  FMMB_CUDA(cudaEventSynchronize(pl->ev[1]));  // the stream may have been changed since
+  pl->timing = true;
+  pl->ev_used = 0;
+  pl->ev_phase.clear();
+  pl->far_only = ph.far_only;
+  try {
+    run_one(pl, (ph.far_only ? pl->qs_far.get() : pl->qs.get()) + ph.charges, ph.want_grad);
+  } catch (...) {
+    pl->timing = pl->far_only = false;
+    pl->launches = launches;
+    throw;
+  }
+  pl->timing = pl->far_only = false;
+  pl->launches = launches;
+  FMMB_CUDA(cudaStreamSynchronize(pl->st.main));
+  FMMB_CUDA(cudaStreamSynchronize(pl->st.side));
+  for (float& t : ph.ms) t = 0.f;
+  for (const auto& e : pl->ev_phase) {
+    float t = 0;
+    FMMB_CUDA(cudaEventElapsedTime(&t, pl->evp[e.second], pl->evp[e.second + 1]));
+    ph.ms[e.first] += t;
+  }
+  ph.state = fmmb_plan::Phases::kMeasured;
 }
 
 template <typename T>
@@ -929,10 +936,8 @@ int evaluate_impl(fmmb_plan* pl, const float* q, T* pot, T* grad) {
       FMMB_CUDA(cudaMemsetAsync(pl->d_err.get(), 0, sizeof(int), pl->st.main));
       throw Error{FMMB_ERR_CUDA, "M2L pipeline wait timed out (code " + std::to_string(e) + ")"};
     }
-    pl->ev_used = 0;
-    pl->ev_phase.clear();
     pl->launches = 0;
-    FMMB_CUDA(cudaEventRecord(pl->ev[7], m));
+    FMMB_CUDA(cudaEventRecord(pl->ev[0], m));
     if (helm_family(pl->cfg.kernel)) {
       // Helmholtz: complex charges and potentials, interleaved; Yukawa: real
       // ones, run through the same complex pipeline with zero imaginary parts
@@ -957,6 +962,7 @@ int evaluate_impl(fmmb_plan* pl, const float* q, T* pot, T* grad) {
         } else {
           run_one(pl, pl->qs.get() + (size_t)2 * r * nj, false);
         }
+        pl->phases = {fmmb_plan::Phases::kPending, false, false, pl->use_graph ? 0 : (size_t)2 * r * nj, {}};
         if (yuk)  // (pi/2) e^{-l r}/(l r) = (2 pi^2 / l) e^{-l r}/(4 pi r)
           launch_helm_finalize_real<T>(ni, pl->perm_i.get(), pl->pot_s.get(), pl->pot_s.get() + 2 * (size_t)ni,
                                        2.0 * M_PI * M_PI / pl->cfg.wavenumber, pd + (size_t)r * ni, m);
@@ -965,7 +971,7 @@ int evaluate_impl(fmmb_plan* pl, const float* q, T* pot, T* grad) {
                                   pd + (size_t)2 * r * ni, m);
         pl->launches++;
       }
-      FMMB_CUDA(cudaEventRecord(pl->ev[6], m));
+      FMMB_CUDA(cudaEventRecord(pl->ev[1], m));
       FMMB_CUDA(cudaMemcpyAsync(pl->h_err, pl->d_err.get(), sizeof(int), cudaMemcpyDeviceToHost, m));
       if (!pot_dev) FMMB_CUDA(cudaMemcpyAsync(pot, pd, cw * ni * nr * sizeof(T), cudaMemcpyDeviceToHost, m));
       if (!pot_dev || !is_device_ptr(q)) FMMB_CUDA(cudaStreamSynchronize(m));
@@ -1026,6 +1032,7 @@ int evaluate_impl(fmmb_plan* pl, const float* q, T* pot, T* grad) {
       } else {
         run_one(pl, pl->qs.get() + (size_t)r * nj, want_grad);
       }
+      pl->phases = {fmmb_plan::Phases::kPending, want_grad, multi, multi || pl->use_graph ? 0 : (size_t)r * nj, {}};
       // near and far parts of right-hand side r
       const double* pnear = multi ? pl->near_all.get() + (size_t)r * ni : pl->pot_s.get();
       const double* gnear = multi ? pl->near_all.get() + (size_t)nr * ni + (size_t)3 * r * ni : pl->grad_s.get();
@@ -1039,7 +1046,7 @@ int evaluate_impl(fmmb_plan* pl, const float* q, T* pot, T* grad) {
                             (double*)(pd + (size_t)r * ni), want_grad ? (double*)(gd + (size_t)3 * r * ni) : nullptr, m);
       pl->launches++;
     }
-    FMMB_CUDA(cudaEventRecord(pl->ev[6], m));
+    FMMB_CUDA(cudaEventRecord(pl->ev[1], m));
     FMMB_CUDA(cudaMemcpyAsync(pl->h_err, pl->d_err.get(), sizeof(int), cudaMemcpyDeviceToHost, m));
     if (!pot_dev) FMMB_CUDA(cudaMemcpyAsync(pot, pd, (size_t)ni * nr * sizeof(T), cudaMemcpyDeviceToHost, m));
     if (want_grad && !grad_dev) FMMB_CUDA(cudaMemcpyAsync(grad, gd, (size_t)3 * ni * nr * sizeof(T), cudaMemcpyDeviceToHost, m));
@@ -1647,14 +1654,10 @@ int fmmb_get_timings(fmmb_plan* pl, float* ms) {
     FMMB_CUDA(cudaStreamSynchronize(pl->st.main));
     FMMB_CUDA(cudaStreamSynchronize(pl->st.side));
     FMMB_REQUIRE(*pl->h_err == 0, FMMB_ERR_CUDA, "M2L pipeline wait timed out");
-    for (int k = 0; k < 7; k++) ms[k] = 0.0f;
-    for (auto& ph : pl->ev_phase) {
-      float t = 0;
-      FMMB_CUDA(cudaEventElapsedTime(&t, pl->evp[ph.second], pl->evp[ph.second + 1]));
-      ms[ph.first] += t;
-    }
     float tot = 0;
-    FMMB_CUDA(cudaEventElapsedTime(&tot, pl->ev[7], pl->ev[6]));
+    FMMB_CUDA(cudaEventElapsedTime(&tot, pl->ev[0], pl->ev[1]));
+    measure_phases(pl);
+    for (int k = 0; k < 6; k++) ms[k] = pl->phases.ms[k];
     ms[6] = tot;
   });
 }
@@ -1663,6 +1666,7 @@ int fmmb_set_overlap(fmmb_plan* pl, int on) {
   return guarded([&] {
     FMMB_REQUIRE(pl, FMMB_ERR_ARG, "null plan");
     if (pl->serial == (on == 0)) return;
+    measure_phases(pl);  // of the last evaluate, in the layout it ran in
     for (int w = 0; w < 4; w++) {  // captured with the other stream layout
       if (pl->gexec[w]) {
         FMMB_CUDA(cudaStreamSynchronize(pl->st.main));

@@ -170,9 +170,15 @@ struct fmmb_plan {
   int device = 0;
   fmmb::Stream2 st;
   bool own_stream = true;
-  cudaEvent_t ev[8] = {};
-  // per-launch timing: event pairs recorded around each phase launch and
-  // summed per phase when fmmb_get_timings is called
+  cudaEvent_t ev[2] = {};  // start and end of the last evaluate
+  // phase times (measure_phases): event pairs recorded around each phase's launches
+  bool timing = false;
+  struct Phases {
+    enum State { kNone, kPending, kMeasured } state = kNone;
+    bool want_grad = false, far_only = false;
+    size_t charges = 0;  // where the measured right-hand side's charges start
+    float ms[6] = {};
+  } phases;
   static constexpr int kEvPool = 96;
   cudaEvent_t evp[kEvPool] = {};
   int ev_used = 0;
@@ -236,10 +242,8 @@ struct fmmb_plan {
   fmmb::DevBuf<int> xexp;                    // [tot_j] its exponents
   // The plan-internal part of a one-right-hand-side evaluate (sorted charges ->
   // sorted outputs, plan-owned buffers only) captured once per geometry as a
-  // CUDA graph, without / with gradient, with the phase-timer records and the
-  // launch count of the capturing call.
+  // CUDA graph, without / with gradient, with its launch count.
   bool use_graph = true;
-  bool capturing = false;
   // transposed FMM (fmmb_evaluate_transpose, fmmb_position_grad): caller-order
   // copies of the geometry [tx ty tz tnx tny tnz | sx sy sz snx sny snz] and the
   // plan with targets and sources swapped, built on first use
@@ -256,7 +260,6 @@ struct fmmb_plan {
   // run once since the last geometry (captured on the second use), and the launches of the evaluate before it
   bool gused[4] = {false, false, false, false};
   int gbase[4] = {0, 0, 0, 0};
-  std::vector<std::pair<int, int>> gphase[4];
   int glaunches[4] = {0, 0, 0, 0};
   // many right-hand sides (mixed form): the near field of all of them in one
   // pass (p2p_multi.cu) into near_all ([nrhs][ni] potentials, then
