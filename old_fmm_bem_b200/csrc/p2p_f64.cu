@@ -25,7 +25,9 @@
 // Measured against one thread per target with a square root and a division per
 // pair (one B200, whole FP64 evaluate with gradient): 262,144 clustered points at
 // p = 12, depth 5 (1.54 G pairs) 13.15 -> 8.87 ms; 32,768 uniform points at p = 8,
-// depth 3 (43.5 M pairs) 1.08 -> 0.59 ms.
+// depth 3 (43.5 M pairs) 1.08 -> 0.59 ms.  The test for r = 0 and subnormal r^2
+// only where a pair can coincide, the targets' own leaf: this kernel with the
+// present far field beside it, 2.84 -> 2.62 and 0.281 -> 0.257 ms.
 #include <cuda_runtime.h>
 
 #include "internal.h"
@@ -42,21 +44,21 @@ constexpr int kS = 32 / kG;  // source streams of a warp (s = lane / 8)
 constexpr int kMaxNT = 4;    // groups of a tile
 constexpr int kCap = 512;    // staged sources per chunk (multiple of 32 * 4)
 
-// 1/sqrt(a) for a >= 0: the hardware's estimate y (relative error below 2^-19)
-// and the first three terms of (1 - e)^(-1/2) = 1 + e/2 + 3 e^2/8 + ...,
-// e = 1 - a y^2: what is left out, 5 e^3 / 16, is below 2^-54.  Subnormal a,
-// which the estimate flushes, is scaled by 2^200 first; a = 0 (a coincident pair
-// that is not excluded) gives infinity.
-__device__ __forceinline__ double inv_sqrt_normal(double a) {
+// 1/sqrt(a) for normal a > 0: the hardware's estimate y (relative error below
+// 2^-19) and the first three terms of (1 - e)^(-1/2) = 1 + e/2 + 3 e^2/8 + ...,
+// e = 1 - a y^2: what is left out, 5 e^3 / 16, is below 2^-54.  (Squared
+// differences of floats, at least 2^-298, are normal.)
+__device__ __forceinline__ double inv_sqrt(double a) {
   double y;
   asm("rsqrt.approx.ftz.f64 %0, %1;" : "=d"(y) : "d"(a));
   const double e = fma(-(a * y), y, 1.0);
   return fma(y * e, fma(0.375, e, 0.5), y);
 }
-__device__ __forceinline__ double inv_sqrt(double a) {
-  double y = inv_sqrt_normal(a);
-  if (__double2hiint(a) < 0x00100000) y = a > 0.0 ? inv_sqrt_normal(a * 0x1p200) * 0x1p100 : __longlong_as_double(0x7ff0000000000000ll);
-  return y;
+// a >= 0 of a pair that may coincide: subnormal a (a tiny softening), which the
+// estimate flushes, is scaled by 2^200 first; a = 0 gives infinity
+__device__ __forceinline__ double inv_sqrt_any(double a) {
+  if (__double2hiint(a) >= 0x00100000) return inv_sqrt(a);
+  return a > 0.0 ? inv_sqrt(a * 0x1p200) * 0x1p100 : __longlong_as_double(0x7ff0000000000000ll);
 }
 
 template <int KER, bool REF>
@@ -81,7 +83,9 @@ struct Tgt<true> {
 };
 
 // One run of 32 sources: the lane's 8 sources (j0 + s, + 4, ...) against its NT targets.
-template <int KER, bool GRAD, bool REF, bool EXCL, int NT>
+// OWN: a run of the targets' own leaf, where a pair may coincide (in reference
+// semantics its softening keeps r away from 0).
+template <int KER, bool GRAD, bool REF, bool EXCL, bool OWN, int NT>
 __device__ __forceinline__ void run32(const Smem<KER, REF>& S, int j0, double eps2, const Tgt<REF> (&tg)[kMaxNT],
                                       const double (&tn)[kMaxNT][3], double (&P)[kMaxNT][4]) {
 #pragma unroll 2
@@ -114,9 +118,10 @@ __device__ __forceinline__ void run32(const Smem<KER, REF>& S, int j0, double ep
         dy = tg[t].y - sy;
         dz = tg[t].z - sz;
       }
-      const double rinv = inv_sqrt(fma(dx, dx, fma(dy, dy, fma(dz, dz, eps2))));
+      const double r2 = fma(dx, dx, fma(dy, dy, fma(dz, dz, eps2)));
+      const double rinv = OWN && !REF ? inv_sqrt_any(r2) : inv_sqrt(r2);
       double qr = q * rinv;
-      if (EXCL) {
+      if (OWN && EXCL) {
         if (dx == 0.0 && dy == 0.0 && dz == 0.0) continue;
       }
       if (KER == FMMB_LAPLACE_G) {
@@ -182,10 +187,10 @@ __device__ __forceinline__ void tile_runs(const Smem<KER, REF>& S, int c0, int c
                                           double (&P)[kMaxNT][4]) {
   for (int r = (c0 >> 5) + k; r < (c1 >> 5); r += m) {  // c0 / 32 is a multiple of m
     const int j0 = r * 32 - c0 + s;
-    if (EXCL && r * 32 < self_end)
-      run32<KER, GRAD, REF, true, NT>(S, j0, eps2, tg, tn, P);
+    if (r * 32 < self_end)
+      run32<KER, GRAD, REF, EXCL, true, NT>(S, j0, eps2, tg, tn, P);
     else
-      run32<KER, GRAD, REF, false, NT>(S, j0, eps2, tg, tn, P);
+      run32<KER, GRAD, REF, EXCL, false, NT>(S, j0, eps2, tg, tn, P);
   }
 }
 
