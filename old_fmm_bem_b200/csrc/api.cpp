@@ -117,6 +117,31 @@ bool parity_m2l(const fmmb_plan* pl) {
   return pl->cfg.precision != FMMB_MIXED || pl->K > tc_max_k() || helm_family(pl->cfg.kernel);
 }
 
+// Few box pairs in the mixed form's FP16x3 range: the FP64 M2L, which is more
+// precise and, below some number of pairs, faster -- it needs no split of the
+// multipoles and no reduction of pair rows, and its 61 operators leave fewer
+// part-filled tiles than 316.  Its time grows as the pairs times K^2, the other's
+// starts from 35-50 us.  Measured with the split and the reduction (uniform points,
+// one B200): p = 6, 323,020 pairs 137 against 160 us, 640,584 pairs 244 / 238;
+// p = 8, 56,448: 53 / 85, 145,986: 117 / 112; p = 10, 27,748: 56 / 65, 52,494: 92 /
+// 73; p = 12, 26,964: 70 / 100, 50,828: 117 / 98.  The line lies below the crossing
+// at every order: 291,000 pairs at p = 6, 107,000, 48,000 and 24,500 at 8, 10, 12.
+bool few_pairs(const fmmb_plan* pl) {
+  return pl->cfg.precision == FMMB_MIXED && pl->K <= h16_max_k() &&
+         (double)pl->m2l_pairs * pl->K * pl->K <= 7e8;
+}
+
+// The FP64 M2L's images of the Laplace kernels on the device, (re)built where they
+// are missing or, in reference semantics, belong to other levels.
+void upload_parity(fmmb_plan* pl, int lmax, float rd) {
+  Operators& o = pl->ops;
+  if (o.par_sets == 0 || (pl->ref && (o.par_lmax != lmax || o.par_rd != rd))) build_parity_operators(o, lmax, rd);
+  if (pl->d_par.get() && pl->par_up_lmax == o.par_lmax && pl->par_up_rd == o.par_rd) return;
+  upload(pl->d_par, o.par, pl->st.main);
+  pl->par_up_lmax = o.par_lmax;
+  pl->par_up_rd = o.par_rd;
+}
+
 // The tensor-core M2L's operator images (mixed form), rebuilt when the
 // operator set changed: FP16 (hi, lo) for K <= h16_max_k(), TF32 above.
 void m2l_images(fmmb_plan* pl) {
@@ -214,10 +239,8 @@ int fmmb_plan_create(const fmmb_config* cfg, fmmb_plan** out) {
       build_static_operators(pl->ops, pl->p, pl->ref);
       upload_static_ops(pl);
       if (!pl->ref && !helm_family(cfg->kernel)) {  // geometry-independent M2L set
-        if (parity_m2l(pl)) {
-          build_parity_operators(pl->ops, 2, 1.0f);
-          upload(pl->d_par, pl->ops.par, pl->st.main);
-        } else {
+        if (parity_m2l(pl) || pl->K <= h16_max_k()) upload_parity(pl, 2, 1.0f);  // the latter for geometries of few_pairs
+        if (!parity_m2l(pl)) {
           build_m2l_operators(pl->ops, 2, 1.0f);
           m2l_images(pl);
         }
@@ -374,11 +397,8 @@ int geometry_impl(fmmb_plan* pl, int nprob, const int* toff, const int* soff, in
     }
     // reference semantics: the M2L distance carries an absolute eps, so the
     // operator set depends on the level sizes (rebuilt when they change)
-    const bool par_m2l = parity_m2l(pl);
-    if (pl->ref && par_m2l && (pl->ops.par_lmax != pl->lmax || pl->ops.par_rd != pl->bbox[3])) {
-      build_parity_operators(pl->ops, pl->lmax, pl->bbox[3]);
-      upload(pl->d_par, pl->ops.par, s);
-    }
+    const bool par_m2l = parity_m2l(pl) || few_pairs(pl);
+    if (par_m2l) upload_parity(pl, pl->lmax, pl->bbox[3]);
     if (pl->ref && !par_m2l && (pl->ops.m2l_lmax != pl->lmax || pl->ops.m2l_rd != pl->bbox[3]))
       build_m2l_operators(pl->ops, pl->lmax, pl->bbox[3]);
     int dev_sms = 148;
@@ -391,8 +411,8 @@ int geometry_impl(fmmb_plan* pl, int nprob, const int* toff, const int* soff, in
     // M2L on the tensor cores in the mixed form: FP16x3 for K <= h16_max_k()
     // (p <= 12), TF32x3 above
     const bool mixed = pl->cfg.precision == FMMB_MIXED;
-    pl->use_h16 = mixed && pl->K <= h16_max_k();
-    pl->use_tc = mixed && !pl->use_h16 && pl->K <= tc_max_k();
+    pl->use_h16 = !par_m2l && mixed && pl->K <= h16_max_k();
+    pl->use_tc = !par_m2l && mixed && !pl->use_h16 && pl->K <= tc_max_k();
     init_fac32();
     prepare_translate_pairs_f64();
     if (par_m2l) {

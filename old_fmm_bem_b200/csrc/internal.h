@@ -134,8 +134,6 @@ struct Operators {
   int par_sets = 0, par_lmax = 0;
   float par_rd = 0;
   std::vector<double> phi;                   // [49][21][2] (cos m phi, sin m phi)
-  // Wigner rotation tables per relative position (forward, inverse)
-  std::vector<std::vector<std::vector<std::complex<double>>>> Wf, Wb;
 };
 // fac, M2M, L2L, slot maps and rotation tables (independent of the geometry)
 void build_static_operators(Operators& ops, int p, bool ref_semantics);
@@ -224,6 +222,8 @@ struct fmmb_plan {
   // FP64 M2L: operator images (Laplace FP64 form; Helmholtz family: levels
   // 2..lmax x 61), rotation table, class of a relative position
   fmmb::DevBuf<double> d_par, d_phi;
+  int par_up_lmax = 0;  // the Laplace images on the device: as ops.par_lmax, ops.par_rd
+  float par_up_rd = 0;
   fmmb::DevBuf<int> d_rel_to_cls;
   fmmb::DevBuf<double> d_m2m_t, d_l2l_t;    // [8][column][row] (transposed for the FP64 pair kernel)
   fmmb::DevBuf<int> d_slot_rel, d_rel_to_op;

@@ -205,18 +205,6 @@ void build_static_operators(Operators& ops, int p, bool ref) {
   auto A = [&](int n, int m) { return anm[ifull(n, m)]; };
 
   const double rho_eps = ref ? kEpsF : 0.0;
-  // Rotation tables for the 512 relative positions and their inverses.
-  auto& Wf = ops.Wf;
-  auto& Wb = ops.Wb;
-  Wf.assign(512, {});
-  Wb.assign(512, {});
-  parallel_for(512, [&](int pos) {
-    double al, be;
-    direction(pos, rho_eps, ref, al, be);
-    wigner(al, be, p, Wf[pos]);
-    wigner(-al, -be, p, Wb[pos]);
-  });
-
   // M2M: child octant c -> parent, rho = sqrt(3)/4 in parent units
   // (kernel/m2m.cxx:28-61); input degree n' scaled by 2^-n'.
   std::vector<double> scale_m2m(mp), scale_l2l(mp);
@@ -226,29 +214,36 @@ void build_static_operators(Operators& ops, int p, bool ref) {
   }
   ops.m2m.assign((size_t)8 * K * K, 0.0);
   ops.l2l.assign((size_t)8 * K * K, 0.0);
-  for (int oct = 0; oct < 8; oct++) {
+  parallel_for(8, [&](int oct) {
     int c[3];
     decode3(oct, c);
     int nc[3] = {4 - 2 * c[0], 4 - 2 * c[1], 4 - 2 * c[2]};
-    int je = encode3(nc, 3);
+    std::vector<std::vector<cd>> Wf, Wb;  // rotation tables of a relative position and its inverse
+    auto rotations = [&](int pos) {
+      double al, be;
+      direction(pos, rho_eps, ref, al, be);
+      wigner(al, be, p, Wf);
+      wigner(-al, -be, p, Wb);
+    };
+    rotations(encode3(nc, 3));
     const double rh = std::sqrt(3.0) / 4;
     auto Zm = [&](int j, int n0, int k) -> double {  // from degree n0 = j - n
       int n = j - n0;
       if (n < 0 || n0 < k) return 0.0;
       return std::pow(-1.0, n) * A(n, 0) * A(j - n, k) / A(j, k) * std::pow(rh, n);
     };
-    compose(p, Wf[je], Wb[je], Zm, scale_m2m.data(), &ops.m2m[(size_t)oct * K * K]);
+    compose(p, Wf, Wb, Zm, scale_m2m.data(), &ops.m2m[(size_t)oct * K * K]);
     // L2L: parent -> child octant c, rho = sqrt(3)/2 in child units
     // (kernel/l2l.cxx:44-77); input degree n scaled by 2^-(n+1).
     int nl[3] = {2 * c[0] + 2, 2 * c[1] + 2, 2 * c[2] + 2};
-    int jl = encode3(nl, 3);
+    rotations(encode3(nl, 3));
     const double rl = std::sqrt(3.0) / 2;
     auto Zl = [&](int j, int n, int k) -> double {
       if (n < j || n < k) return 0.0;
       return A(n - j, 0) * A(j, k) / A(n, k) * std::pow(rl, n - j);
     };
-    compose(p, Wf[jl], Wb[jl], Zl, scale_l2l.data(), &ops.l2l[(size_t)oct * K * K]);
-  }
+    compose(p, Wf, Wb, Zl, scale_l2l.data(), &ops.l2l[(size_t)oct * K * K]);
+  });
 
   // M2L slot structure: for a target box in octant c, the reference's
   // interaction-list loop (fmm/ijbox.cxx:85-104) visits parent-neighbour
@@ -328,29 +323,6 @@ double m2l_distance(int d2, int set, float rd, bool ref) {
 }
 }  // namespace
 
-// M2L operators (kernel/m2l.cxx:43-78): one set, or one per level when the
-// distance carries the reference's absolute eps.
-void build_m2l_operators(Operators& ops, int lmax, float rd) {
-  const int p = ops.p, K = ops.K;
-  const bool ref = ops.ref;
-  const std::vector<double> anm = anm_table(p, ref);
-  const auto& op_rel = ops.op_rel;
-  const int nops = (int)op_rel.size();  // 316
-  ops.m2l_sets = ref ? (lmax - 1) : 1;
-  ops.m2l_lmax = lmax;
-  ops.m2l_rd = rd;
-  ops.m2l.assign((size_t)ops.m2l_sets * nops * K * K, 0.0);
-  parallel_for(ops.m2l_sets * nops, [&](int w) {
-    const int set = w / nops, o = w % nops;
-    const int code = op_rel[o];
-    const int dx = code / 49 - 3, dy = (code / 7) % 7 - 3, dz = code % 7 - 3;
-    int nc[3] = {dx + 3, dy + 3, dz + 3};
-    const int je = encode3(nc, 3);
-    const M2LZ Z{anm, ref, m2l_distance(dx * dx + dy * dy + dz * dz, set, rd, ref)};
-    compose(p, ops.Wf[je], ops.Wb[je], Z, nullptr, &ops.m2l[((size_t)set * nops + o) * K * K]);
-  });
-}
-
 // The FP64 M2L's images (m2l_parity.cuh): the operator of each class composed at
 // azimuth 0, where the rotations are real and Re, Im of the coefficients do
 // not mix: the even block acts on the Re parts (rows and columns (n, m > 0) by
@@ -390,6 +362,50 @@ void build_parity_operators(Operators& ops, int lmax, float rd) {
       for (int r = 0; r < E; r++) e[parity_at(te, c, r)] = T[(size_t)re[r] * K + re[c]];
     for (int c = 0; c < O; c++)
       for (int r = 0; r < O; r++) o[parity_at(to, c, r)] = T[(size_t)im[r] * K + im[c]];
+  });
+}
+
+// M2L operators (kernel/m2l.cxx:43-78) of all 316 relative positions: one set, or
+// one per level when the distance carries the reference's absolute eps.  Each is
+// its class's operator between a rotation by the azimuth and its inverse (the
+// order-m coefficients times e^{i m phi}), which is a few operations per entry of
+// the two blocks (composed one by one the 316 took 94 ms at p = 12 on 8 cores).
+void build_m2l_operators(Operators& ops, int lmax, float rd) {
+  const int p = ops.p, K = ops.K, E = (p + 1) * (p + 2) / 2, O = p * (p + 1) / 2;
+  if (ops.par_sets == 0 || (ops.ref && (ops.par_lmax != lmax || ops.par_rd != rd))) build_parity_operators(ops, lmax, rd);
+  const int te = parity_tiles(E), to = parity_tiles(O), nops = (int)ops.op_rel.size(), ncls = (int)ops.cls_geom.size();
+  const size_t stride = parity_img_stride(0, p);
+  ops.m2l_sets = ops.par_sets;
+  ops.m2l_lmax = lmax;
+  ops.m2l_rd = rd;
+  ops.m2l.resize((size_t)ops.m2l_sets * nops * K * K);
+  std::vector<int> at(E), ord(E);  // real-packed index of a row's real part (the imaginary part follows), its order
+  for (int n = 0; n <= p; n++) {
+    at[O + n] = n * n;
+    ord[O + n] = 0;
+    for (int m = 1; m <= n; m++) {
+      at[n * (n - 1) / 2 + m - 1] = n * n + 2 * m - 1;
+      ord[n * (n - 1) / 2 + m - 1] = m;
+    }
+  }
+  parallel_for(ops.m2l_sets * nops, [&](int w) {
+    const int set = w / nops, code = ops.op_rel[w % nops];
+    const double* e = &ops.par[((size_t)set * ncls + ops.rel_to_cls[code]) * stride];
+    const double* o = e + parity_block(te);
+    const double* phi = &ops.phi[(size_t)(code / 7) * 21 * 2];
+    double* T = &ops.m2l[(size_t)w * K * K];
+    for (int r = 0; r < E; r++) {
+      const double cr = phi[2 * ord[r]], sr = phi[2 * ord[r] + 1];
+      double* Tr = T + (size_t)at[r] * K;
+      for (int c = 0; c < E; c++) {
+        const double cc = phi[2 * ord[c]], sc = phi[2 * ord[c] + 1];
+        const double ev = e[parity_at(te, c, r)], ov = r < O && c < O ? o[parity_at(to, c, r)] : 0.0;
+        Tr[at[c]] = cr * ev * cc + sr * ov * sc;
+        if (c < O) Tr[at[c] + 1] = sr * ov * cc - cr * ev * sc;
+        if (r < O) Tr[K + at[c]] = cr * ov * sc - sr * ev * cc;
+        if (r < O && c < O) Tr[K + at[c] + 1] = cr * ov * cc + sr * ev * sc;
+      }
+    }
   });
 }
 

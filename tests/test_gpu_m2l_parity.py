@@ -66,3 +66,29 @@ def test_mixed_above_the_tensor_core_orders():
         pot, _ = pl.evaluate(q, f64=True)
         want, _ = pl.direct(q)
     assert np.linalg.norm(pot - want) <= 1e-6 * np.linalg.norm(want)
+
+
+@pytest.mark.parametrize("ref", [False, True])
+@pytest.mark.parametrize("p", [6, 12])
+def test_mixed_form_on_both_sides_of_the_pair_limit(p, ref):
+    # few box pairs (a corner, a thin layer) take the FP64 M2L, many (full grids) FP16x3; one plan goes to and fro, the
+    # box changes with it.  Against the FP64 form: inputs of FP32 expansions, (p + 1)^2 roundings of 2^-24 at random.
+    rng = np.random.default_rng(p)
+    lmax = 4 if p == 6 else 3
+    n = 6000
+    q = rng.standard_normal(n).astype(np.float32)
+    kw = dict(kernel=ob.LAPLACE_G, p=p, lmax=lmax, semantics=ob.SEM_REFERENCE if ref else ob.SEM_ACCURATE)
+    few = []
+    with ob.Plan(precision=ob.MIXED, **kw) as pm, ob.Plan(precision=ob.FP64, **kw) as pf:
+        for scale, box in (((1, 1, 1), 1.0), ((1, 1, 0.2), 1.0), ((0.4, 0.4, 0.4), 1.0), ((2, 2, 2), 2.0),
+                           ((2, 2, 0.3), 2.0), ((1, 1, 1), 1.0)):
+            x = (rng.random((3, n)) * np.array(scale)[:, None]).astype(np.float32)
+            loc = []
+            for pl in (pm, pf):
+                pl.set_geometry(x, x, bbox=(0, 0, 0, box))
+                for _ in range(3):  # launched, captured, replayed
+                    pot, _ = pl.evaluate(q, f64=True)
+                loc.append(pl.expansions(1))
+            few.append(pm.stats()["m2l_pairs"] * (p + 1) ** 4 <= 7e8)
+            assert np.linalg.norm(loc[0] - loc[1]) <= (p + 1) * 2.0 ** -23 * np.linalg.norm(loc[1])
+    assert True in few and False in few
