@@ -20,10 +20,13 @@
 // Kernel, one instance per order: a block per tile of 32 pairs of one operator
 // (16 pairs where 32 do not fit).  It gathers the tile's inputs, rotates and
 // combines them into shared memory once, then streams the operator through a
-// 4-slot ring of bulk copies in chunks of 8 columns (the warps wait for a chunk
-// and free its slot through mbarriers, without block barriers between chunks); a warp owns 8 pairs and every
-// second (fourth, eighth) 8-row tile of both blocks, with mma.sync m8n8k4 .f64
-// (256 FMA per warp instruction, the FP64 pipe's full rate).  Columns k, k + 4
+// 4-slot ring of bulk copies in chunks of 8 columns: the warps wait for a chunk
+// and free its slot through mbarriers, without block barriers between chunks, and
+// take turns at waiting for a free slot and sending for the next chunk (the same
+// warp each time fell behind and held the others up; a warp of its own for it
+// left 96 registers a thread and spilled).  A warp owns 8 pairs and every second
+// (fourth, eighth) 8-row tile of both blocks, with mma.sync m8n8k4 .f64 (256 FMA
+// per warp instruction, the FP64 pipe's full rate).  Columns k, k + 4
 // of a chunk lie side by side, operator and inputs alike, so that one 16-byte
 // read feeds two MMAs.  Rows of the two blocks are numbered alike, so the even
 // and odd results of an order meet in one thread; they are rotated back,
@@ -33,10 +36,11 @@
 //
 // Bound: the FP64 pipe.  Measured on one B200, M2L phase alone, against dense
 // K x K operators of all 316 positions: Laplace FP64 (box tiles, plain FMAs)
-// 262,144 clustered points, p = 12, depth 5 (206,548 box pairs) 5.68 -> 0.34 ms;
+// 262,144 clustered points, p = 12, depth 5 (206,548 box pairs) 5.68 -> 0.31 ms;
 // 100,000 uniform points, p = 8, depth 4 (640,584 pairs) 1.71 -> 0.37 ms;
 // Helmholtz (2K x 2K real form on the same tensor instruction) 1,048,576 sphere
-// points, p = 16, depth 5 (291,998 pairs) 7.84 -> 4.14 ms
+// points, p = 16, depth 5 (291,998 pairs) 7.84 -> 3.68 ms (4.13
+// with one warp sending for every chunk)
 // (8 instead of 16 warps where one block fills an SM: 5.22 ms, too few per
 // scheduler to hide the tensor instruction's and the shared-memory reads'
 // latency).
@@ -165,11 +169,13 @@ __global__ void __launch_bounds__(Cfg<MODE, P>::NW * 32) m2l_parity(ParityArgs A
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
   const double* img = A.img + (size_t)A.tile_cls[tile] * A.img_stride;
   constexpr int nE = C::NPROD * RTE, nch = nE + C::NPROD * RTO;  // chunks of the two blocks
-  // thread 0 copies chunk c into its slot once every warp is done with chunk c - kStages
+  int sent = -1;  // the last chunk this thread sent for
+  // copies chunk c into its slot once every warp is done with chunk c - kStages
   auto issue = [&](int c) {
     if (c >= nch) return true;
     if (c >= kStages && !mbar_wait(&empty[c % kStages], (c / kStages - 1) & 1)) return false;
     const double* src = img + (c < nE ? (size_t)c * kKC * RSE : (size_t)nE * kKC * RSE + (size_t)(c - nE) * kKC * RSO);
+    sent = c;
     bulk_g2s(ring + (size_t)(c % kStages) * kKC * RSE, src, (c < nE ? RSE : RSO) * kKC * 8, &full[c % kStages]);
     return true;
   };
@@ -265,7 +271,7 @@ __global__ void __launch_bounds__(Cfg<MODE, P>::NW * 32) m2l_parity(ParityArgs A
       }
     }
     for (int kc = 0; kc < RT && ok; kc++, c++, x += 4 * S) {
-      if (tid == 0) ok = issue(c + kLead);
+      if (warp == c % C::NW && lane == 0) ok = issue(c + kLead);  // the warps take turns
       ok = mbar_wait(&full[c % kStages], (c / kStages) & 1) && ok;
       if (!__all_sync(0xffffffffu, ok)) {
         ok = false;
@@ -295,8 +301,9 @@ __global__ void __launch_bounds__(Cfg<MODE, P>::NW * 32) m2l_parity(ParityArgs A
   }
   __syncthreads();  // the inputs are consumed: their memory takes the results, [pair][CX K]
   if (s_fail) {  // a wait timed out: let the copies in flight land, report, leave
+    if (sent >= 0) mbar_wait(&full[sent % kStages], (sent / kStages) & 1);
     if (tid == 0) {
-      for (int i = max(0, c - 1); i < min(nch, c + kLead + 1); i++) mbar_wait(&full[i % kStages], (i / kStages) & 1);
+      for (int i = 0; i < kLead; i++) mbar_wait(&full[i], 0);
       atomicExch(A.err, 100);
     }
     return;
