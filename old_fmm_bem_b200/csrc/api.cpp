@@ -513,8 +513,7 @@ int geometry_impl(fmmb_plan* pl, int nprob, const int* toff, const int* soff, in
     // evaluate, so that each launch starts with its longest blocks), on the
     // device (setup.cu)
     build_inverse_perm_dev(pl, s);
-    build_p2p_work_dev(pl, s);
-    build_p2m_work_dev(pl, s);
+    build_work_dev(pl, s);
     // evaluation buffers
     const int nr = pl->cfg.nrhs;
     pl->qs.alloc((size_t)nj * nr);

@@ -331,8 +331,7 @@ bool build_m2l_job_dev(fmmb_plan* pl, fmmb_plan::TcJob& job, int ys, cudaStream_
 void build_pair_jobs(fmmb_plan* pl, int m2m0, int l2l0, int ops_per_level, cudaStream_t s);
 // the FP64 M2L's pair tiles
 void build_parity_job(fmmb_plan* pl, cudaStream_t s);
-void build_p2p_work_dev(fmmb_plan* pl, cudaStream_t s);
-void build_p2m_work_dev(fmmb_plan* pl, cudaStream_t s);
+void build_work_dev(fmmb_plan* pl, cudaStream_t s);  // near-field and P2M work items
 void build_inverse_perm_dev(fmmb_plan* pl, cudaStream_t s);
 // complex Helmholtz and Yukawa operators, pair jobs and buffers (helmholtz_host.cpp)
 void helm_setup(fmmb_plan* pl);

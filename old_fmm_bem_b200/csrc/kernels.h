@@ -57,7 +57,7 @@ int launch_p2p_multi(int kernel, int nrhs, int nwork, const int2* work, const in
                      const float* qs, int nj, const Sem& s, double* pot, double* grad, int ni, cudaStream_t st);
 // FP32 P2M for the mixed form (accurate semantics, p <= 12); returns false
 // outside that range.  work: (source leaf, first source) items of up to
-// kP2MItem sources (build_p2m_work_dev); a leaf of more sources is summed by
+// kP2MItem sources (build_work_dev); a leaf of more sources is summed by
 // several items with FP64 atomics, so its rows of M must be zero beforehand.
 constexpr int kP2MItem = 64;
 bool launch_p2m_f32(int kernel, int nwork, const int2* work, int p, int K, const int* keys, const int2* leaf,

@@ -299,7 +299,7 @@ bool build_m2l_tiles(fmmb_plan* pl, bool sets, int per, const int* rel_to_op, in
   FMMB_CHECK_LAUNCH();
   FMMB_CUDA(cudaMemsetAsync(pos.get() + nv, 0, sizeof(int), s));
   exclusive_scan(pos.get(), nv + 1, s);
-  const int npair = d2h_int(pos.get() + nv, s);
+  const int npair = (int)pl->m2l_pairs;  // counted, and read back, with the tree
   if (csr) {
     const int nrow = nv / kM2LSlots;
     csr->nred = npair > 0 ? nrow : 0;
@@ -464,20 +464,31 @@ bool build_m2l_job_dev(fmmb_plan* pl, fmmb_plan::TcJob& job, int ys, cudaStream_
   return true;
 }
 
-void build_p2p_work_dev(fmmb_plan* pl, cudaStream_t s) {
-  const int nleaf = pl->nbox_i[pl->lmax];
-  TmpBuf<int> cnt(s);
+void build_work_dev(fmmb_plan* pl, cudaStream_t s) {
+  const int nleaf = pl->nbox_i[pl->lmax], nleaf_j = pl->nbox_j[pl->lmax], per = kP2MItem;
+  TmpBuf<int> cnt(s), cnt_j(s);
   TmpBuf<long long> nsrc(s);
   cnt.alloc((size_t)nleaf + 1);
+  cnt_j.alloc((size_t)nleaf_j + 1);
   nsrc.alloc(std::max(nleaf, 1));
   FMMB_CUDA(cudaMemsetAsync(cnt.get() + nleaf, 0, sizeof(int), s));
+  FMMB_CUDA(cudaMemsetAsync(cnt_j.get() + nleaf_j, 0, sizeof(int), s));
   if (nleaf > 0) {
     leaf_item_counts<<<nblk(nleaf, kT), kT, 0, s>>>(nleaf, pl->leaf_i.get(), pl->leaf_j.get(), pl->p2p_list.get(),
                                                    cnt.get(), nsrc.get());
     FMMB_CHECK_LAUNCH();
   }
+  if (nleaf_j > 0) {
+    src_item_counts<<<nblk(nleaf_j, kT), kT, 0, s>>>(nleaf_j, per, pl->leaf_j.get(), cnt_j.get());
+    FMMB_CHECK_LAUNCH();
+  }
   exclusive_scan(cnt.get(), nleaf + 1, s);
-  const int n = d2h_int(cnt.get() + nleaf, s);
+  exclusive_scan(cnt_j.get(), nleaf_j + 1, s);
+  int tot[2];
+  FMMB_CUDA(cudaMemcpyAsync(&tot[0], cnt.get() + nleaf, sizeof(int), cudaMemcpyDeviceToHost, s));
+  FMMB_CUDA(cudaMemcpyAsync(&tot[1], cnt_j.get() + nleaf_j, sizeof(int), cudaMemcpyDeviceToHost, s));
+  FMMB_CUDA(cudaStreamSynchronize(s));
+  const int n = tot[0];
   pl->m_p2p_work.alloc(std::max(n, 1));
   pl->m_p2p_nwork = n;
   TmpBuf<int> skey(s), sval(s);
@@ -497,27 +508,12 @@ void build_p2p_work_dev(fmmb_plan* pl, cudaStream_t s) {
   }
   pl->p2p_nwork = n;
   pl->p2p_nwork0 = n0;
-  FMMB_CUDA(cudaStreamSynchronize(s));
-}
-
-void build_p2m_work_dev(fmmb_plan* pl, cudaStream_t s) {
-  const int nleaf = pl->nbox_j[pl->lmax], per = kP2MItem;
-  TmpBuf<int> cnt(s);
-  cnt.alloc((size_t)nleaf + 1);
-  FMMB_CUDA(cudaMemsetAsync(cnt.get() + nleaf, 0, sizeof(int), s));
-  if (nleaf > 0) {
-    src_item_counts<<<nblk(nleaf, kT), kT, 0, s>>>(nleaf, per, pl->leaf_j.get(), cnt.get());
+  pl->p2m_work.alloc(std::max(tot[1], 1));
+  pl->p2m_nwork = tot[1];
+  if (nleaf_j > 0) {
+    src_items<<<nblk(nleaf_j, kT), kT, 0, s>>>(nleaf_j, per, pl->leaf_j.get(), cnt_j.get(), pl->p2m_work.get());
     FMMB_CHECK_LAUNCH();
   }
-  exclusive_scan(cnt.get(), nleaf + 1, s);
-  const int n = d2h_int(cnt.get() + nleaf, s);
-  pl->p2m_work.alloc(std::max(n, 1));
-  pl->p2m_nwork = n;
-  if (nleaf > 0) {
-    src_items<<<nblk(nleaf, kT), kT, 0, s>>>(nleaf, per, pl->leaf_j.get(), cnt.get(), pl->p2m_work.get());
-    FMMB_CHECK_LAUNCH();
-  }
-  FMMB_CUDA(cudaStreamSynchronize(s));
 }
 
 void build_inverse_perm_dev(fmmb_plan* pl, cudaStream_t s) {
