@@ -1132,7 +1132,8 @@ int autotune_impl(const fmmb_config* cfg, int ni, int nj, int lmin, int lmax_hi,
       float ms = -1.f;
       if (rc == FMMB_OK) {
         float* g = cfg->kernel == FMMB_LAPLACE_G ? dgrad.get() : nullptr;
-        rc = fmmb_evaluate(pl, dq.get(), dpot.get(), g);  // warm-up (captures the graph)
+        for (int r = 0; r < 2 && rc == FMMB_OK; r++)  // warm-up: launched directly, then captured
+          rc = fmmb_evaluate(pl, dq.get(), dpot.get(), g);
         if (rc == FMMB_OK) {
           FMMB_CUDA(cudaEventRecord(e0, pl->st.main));
           for (int r = 0; r < reps && rc == FMMB_OK; r++) rc = fmmb_evaluate(pl, dq.get(), dpot.get(), g);
