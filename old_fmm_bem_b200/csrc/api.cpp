@@ -509,11 +509,11 @@ int geometry_impl(fmmb_plan* pl, int nprob, const int* toff, const int* soff, in
     // near-field work items: pieces of up to 128 targets of a leaf (the
     // many-right-hand-side pass takes them in leaf order; the one-right-hand-
     // side kernels heaviest first -- targets x sources of the 27 neighbour
-    // leaves -- dealt alternately to the two near-field launches of an
-    // evaluate, so that each launch starts with its longest blocks), on the
+    // leaves -- and, where an evaluate has two near-field launches, dealt
+    // alternately to them, so that each starts with its longest blocks), on the
     // device (setup.cu)
     build_inverse_perm_dev(pl, s);
-    build_work_dev(pl, s);
+    build_work_dev(pl, !par_m2l, s);
     // evaluation buffers
     const int nr = pl->cfg.nrhs;
     pl->qs.alloc((size_t)nj * nr);
@@ -688,10 +688,11 @@ void run_one(fmmb_plan* pl, const float* qs, bool want_grad) {
   double* g_near = want_grad ? pl->grad_s.get() : nullptr;
   double* g_far = want_grad ? pl->grad_s.get() + 3 * (size_t)pl->ni : nullptr;
   const int nleaf_i = pl->nbox_i[lmax], nleaf_j = pl->nbox_j[lmax];
-  // Near field on the low-priority side stream, in two halves of the work
-  // items: the first overlaps the upward pass (P2M / M2M, short dependent
-  // launches that leave SMs idle), the second the downward tail (L2L / L2P);
-  // the tensor-core M2L, which needs whole SMs, runs between them.
+  // Near field on the low-priority side stream: one launch from the start or,
+  // where a tensor-core M2L, which needs whole SMs, meets many work items
+  // (build_work_dev in setup.cu), two halves of them: the first overlaps the
+  // upward pass (P2M / M2M, short dependent launches that leave SMs idle), the
+  // second the downward tail (L2L / L2P), and the M2L runs between them.
   auto near_field = [&](int l0, int l1, bool last) {
     if (pl->far_only) {  // the near field of this evaluate runs elsewhere
       if (last) FMMB_CUDA(cudaEventRecord(pl->st.join, m));

@@ -152,7 +152,7 @@ void helm_setup(fmmb_plan* pl) {
   prepare_m2l_parity(yuk ? 2 : 1, p);
   build_parity_job(pl, s);
   // near-field work items and the inverse target permutation of the direct sum
-  build_work_dev(pl, s);
+  build_work_dev(pl, false, s);
   build_inverse_perm_dev(pl, s);
   // recurrence coefficients of Ybar
   std::vector<double> ylm((size_t)(p + 1) * (p + 2), 0.0);

@@ -280,7 +280,7 @@ struct fmmb_plan {
   fmmb::DevBuf<int2> p2m_work;
   int p2m_nwork = 0;
   // the same items for the one-right-hand-side near field, heaviest first in
-  // each of its two launches: [0, p2p_nwork0) and [p2p_nwork0, p2p_nwork)
+  // each of its launches: [0, p2p_nwork0) and, if any are left, [p2p_nwork0, p2p_nwork)
   fmmb::DevBuf<int2> p2p_work;
   int p2p_nwork = 0, p2p_nwork0 = 0;
   int opimg_sets = 0;
@@ -331,7 +331,8 @@ bool build_m2l_job_dev(fmmb_plan* pl, fmmb_plan::TcJob& job, int ys, cudaStream_
 void build_pair_jobs(fmmb_plan* pl, int m2m0, int l2l0, int ops_per_level, cudaStream_t s);
 // the FP64 M2L's pair tiles
 void build_parity_job(fmmb_plan* pl, cudaStream_t s);
-void build_work_dev(fmmb_plan* pl, cudaStream_t s);  // near-field and P2M work items
+// near-field and P2M work items; tc_m2l: the tensor-core M2L runs beside the near field
+void build_work_dev(fmmb_plan* pl, bool tc_m2l, cudaStream_t s);
 void build_inverse_perm_dev(fmmb_plan* pl, cudaStream_t s);
 // complex Helmholtz and Yukawa operators, pair jobs and buffers (helmholtz_host.cpp)
 void helm_setup(fmmb_plan* pl);

@@ -240,12 +240,13 @@ __global__ void src_items(int nleaf, int per, const int2* __restrict__ leaf_j, c
   for (int t = 0, k = base[b]; t < n; t += per, k++) work[k] = make_int2(b, t);
 }
 
-// sorted item j -> launch (j & 1), position j >> 1 within it
+// one launch (n0 = n): in order; two: sorted item j -> launch (j & 1), position j >> 1 within it
 __global__ void deal_items(int n, int n0, const int* __restrict__ sorted, const int2* __restrict__ work,
                            int2* __restrict__ out) {
   const int j = blockIdx.x * blockDim.x + threadIdx.x;
   if (j >= n) return;
-  out[(j & 1) ? n0 + (j >> 1) : (j >> 1)] = work[sorted[j]];
+  const int o = n0 == n ? j : (j & 1) ? n0 + (j >> 1) : j >> 1;
+  out[o] = work[sorted[j]];
 }
 
 __global__ void invert_perm(int n, const int* __restrict__ perm, int* __restrict__ inv) {
@@ -464,7 +465,7 @@ bool build_m2l_job_dev(fmmb_plan* pl, fmmb_plan::TcJob& job, int ys, cudaStream_
   return true;
 }
 
-void build_work_dev(fmmb_plan* pl, cudaStream_t s) {
+void build_work_dev(fmmb_plan* pl, bool tc_m2l, cudaStream_t s) {
   const int nleaf = pl->nbox_i[pl->lmax], nleaf_j = pl->nbox_j[pl->lmax], per = kP2MItem;
   TmpBuf<int> cnt(s), cnt_j(s);
   TmpBuf<long long> nsrc(s);
@@ -500,7 +501,14 @@ void build_work_dev(fmmb_plan* pl, cudaStream_t s) {
     FMMB_CHECK_LAUNCH();
   }
   radix_sort(skey.get(), sval.get(), n, 30, s);  // stable: leaf order among equal costs
-  const int n0 = (n + 1) / 2;
+  // One launch of the near field, beside the far field from its start on; two
+  // halves, before and after the M2L, only where the tensor-core M2L, which takes
+  // whole SMs, would have to wait for a long first one.  One instead of two: 32,768
+  // points FP64 (512 items) 257 -> 173 us, 2,000 mixed 49 -> 42, 262,144 clustered
+  // FP64 2.60 -> 2.43 ms, 131,071 mixed (2,989 items) moved and evaluated 1.06 ->
+  // 1.04, 245,760 on a surface mixed (4,626) 0.348 / 0.347, but 1,048,576 clustered
+  // mixed (21,892), forward and backward, 9.70 -> 9.74.
+  const int n0 = tc_m2l && n > (1 << 13) ? (n + 1) / 2 : n;
   pl->p2p_work.alloc(std::max(n, 1));
   if (n > 0) {
     deal_items<<<nblk(n, kT), kT, 0, s>>>(n, n0, sval.get(), pl->m_p2p_work.get(), pl->p2p_work.get());

@@ -78,3 +78,25 @@ def test_sort_is_stable_at_tile_edges(n):
     c = np.floor(x * np.float32(16)).astype(np.int64)  # exact: a power of two
     key = sum((((c[1] >> b) & 1) | ((c[0] >> b) & 1) << 1 | ((c[2] >> b) & 1) << 2) << 3 * b for b in range(4))
     assert np.array_equal(perm, np.argsort(key, kind="stable"))
+
+
+@pytest.mark.parametrize("kernel,precision,n", [(ob.LAPLACE_G, ob.FP64, 592), (ob.LAPLACE_G, ob.FP64, 593),
+                                                (ob.HELMHOLTZ_G, ob.FP64, 592), (ob.HELMHOLTZ_G, ob.FP64, 593),
+                                                (ob.LAPLACE_G, ob.MIXED, 8192), (ob.LAPLACE_G, ob.MIXED, 8193),
+                                                (ob.LAPLACE_G, ob.FP64, 8193)])
+def test_near_field_launches_take_every_item_once(kernel, precision, n):
+    # one point a leaf, so n work items: blocks of 8 or 4 warps, one launch or two.  Equal charges: the neighbours' share
+    # of a potential is some per cent and more, the truncation at p = 8 below 1e-4
+    lmax = 4 if n < 4096 else 5
+    cells = np.random.default_rng(n).permutation(8 ** lmax)[:n]
+    c = np.array(np.unravel_index(cells, (2 ** lmax,) * 3))
+    x = ((c + 0.5 + 0.4 * (np.random.default_rng(1).random((3, n)) - 0.5)) / 2 ** lmax).astype(np.float32)
+    helm = kernel == ob.HELMHOLTZ_G
+    q = np.ones(n, np.complex64 if helm else np.float32)
+    with ob.Plan(kernel=kernel, p=8, lmax=lmax, precision=precision, semantics=ob.SEM_ACCURATE, exclude_self=True,
+                 **(dict(wavenumber=1.0) if helm else {})) as pl:
+        pl.set_geometry(x, x, bbox=(0, 0, 0, 1))
+        want = np.asarray(pl.direct(q)[0])
+        for _ in range(3):
+            got = np.asarray(pl.evaluate(q, f64=True)[0])
+            assert np.all(abs(got - want) <= 1e-3 * abs(want))
