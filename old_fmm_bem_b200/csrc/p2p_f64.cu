@@ -37,8 +37,13 @@
 namespace fmmb {
 namespace {
 
-constexpr int kThreads = 128;
-constexpr int kWarps = kThreads / 32;
+constexpr int kItem = 128;   // targets of a work item
+constexpr int kMaxWarps = 8;
+// Warps of a block: 4; 8 where all items are resident at once with 4 (4 blocks fit
+// an SM by their registers) and leave the FP64 pipe short of warps.  512 items
+// (32,768 points, depth 3): this kernel 0.115 ms with 4, 0.086 with 8; 262,144
+// clustered points (4,219 items): 2.52 ms a pass with 8, 2.43 with 4.
+constexpr int kFewItems = 4 * 148;
 constexpr int kG = 8;        // targets of a group (lanes g = lane % 8)
 constexpr int kS = 32 / kG;  // source streams of a warp (s = lane / 8)
 constexpr int kMaxNT = 4;    // groups of a tile
@@ -69,7 +74,7 @@ struct Smem {
   double Q[REF ? kCap : 1];
   double2 N[KER == FMMB_LAPLACE_GNJ ? kCap : 1];  // source normal (x, y), z
   double NZ[KER == FMMB_LAPLACE_GNJ ? kCap : 1];
-  double red[kWarps - 1][kMaxNT][4][kG];  // team partial sums
+  double red[kMaxWarps - 1][kMaxNT][4][kG];  // team partial sums
   SrcList src;
 };
 
@@ -154,7 +159,7 @@ template <int KER, bool REF>
 __device__ void stage(Smem<KER, REF>& S, int c0, int c1, const float4* __restrict__ spos,
                       const float4* __restrict__ snrm, const float* __restrict__ qs, double coef) {
   __syncthreads();  // the previous chunk's readers are done
-  for (int u = threadIdx.x; u < c1 - c0; u += kThreads) {
+  for (int u = threadIdx.x; u < c1 - c0; u += blockDim.x) {
     const int j = S.src.locate(c0 + u, c1);
     float4 x = make_float4(1e18f, 1e18f, 1e18f, 0.f), n = make_float4(0.f, 0.f, 0.f, 0.f);  // padding: far, no charge
     float q = 0.f;
@@ -195,7 +200,7 @@ __device__ __forceinline__ void tile_runs(const Smem<KER, REF>& S, int c0, int c
 }
 
 template <int KER, bool GRAD, bool REF, bool EXCL>
-__global__ void __launch_bounds__(kThreads) p2p_f64(const int2* __restrict__ work, const int2* __restrict__ leaf_i,
+__global__ void __launch_bounds__(32 * kMaxWarps) p2p_f64(const int2* __restrict__ work, const int2* __restrict__ leaf_i,
                                                     const int2* __restrict__ leaf_j, const int* __restrict__ list,
                                                     const float4* __restrict__ tpos, const float4* __restrict__ tnrm,
                                                     const float4* __restrict__ spos, const float4* __restrict__ snrm,
@@ -207,7 +212,7 @@ __global__ void __launch_bounds__(kThreads) p2p_f64(const int2* __restrict__ wor
   const int b = wk.x;
   int2 li = leaf_i[b];
   li.x += wk.y;
-  li.y = min(kThreads, li.y - wk.y);
+  li.y = min(kItem, li.y - wk.y);
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, g = lane & (kG - 1), s = lane / kG;
   if (warp == 0) S.src.build(b, list, leaf_j, lane);
   __syncthreads();
@@ -215,8 +220,9 @@ __global__ void __launch_bounds__(kThreads) p2p_f64(const int2* __restrict__ wor
   const int nchunk = (vlen + kCap - 1) / kCap;
   // teams of m warps share a tile of up to 4 groups of targets and split its runs
   const int ng = (li.y + kG - 1) / kG;
-  const int m = ng <= kMaxNT ? 4 : ng <= 2 * kMaxNT ? 2 : 1;  // block-uniform
-  const int nteam = kWarps / m, team = warp / m, k = warp % m;
+  const int nw = blockDim.x >> 5;  // 4 or 8
+  const int m = ng <= kMaxNT ? nw : ng <= 2 * kMaxNT ? nw / 2 : nw / 4;  // block-uniform
+  const int nteam = nw / m, team = warp / m, k = warp % m;
   const int ga = team * ng / nteam, ntl = (team + 1) * ng / nteam - ga;  // at most 4 groups: li.y <= 128
   Tgt<REF> tg[kMaxNT];
   double tn[kMaxNT][3], P[kMaxNT][4];
@@ -296,7 +302,7 @@ void launch_p2p_f64(int kernel, int nwork, const int2* work, const int2* leaf_i,
                     const Sem& s, double* pot, double* grad, int ni, cudaStream_t st) {
   if (nwork <= 0) return;
   auto go = [&](auto k) {
-    k<<<nwork, kThreads, 0, st>>>(work, leaf_i, leaf_j, list, tpos, tnrm, spos, snrm, qs, s.eps2, s.coef, pot, grad,
+    k<<<nwork, nwork <= kFewItems ? 256 : 128, 0, st>>>(work, leaf_i, leaf_j, list, tpos, tnrm, spos, snrm, qs, s.eps2, s.coef, pot, grad,
                                   ni);
   };
   auto pick = [&](auto ker) {  // reference semantics: self pairs included
