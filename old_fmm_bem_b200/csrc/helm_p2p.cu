@@ -17,13 +17,14 @@
 // Bounds.  Mixed: the special-function pipe (rsqrt, sine and cosine: 3 of 16
 // lanes a clock per pair, 3.57 G pairs in 2.3 ms), with the FP32 work next to it
 // in the two-lane instructions (15 lane operations a pair).  FP64 form: the FP64
-// pipe (the library's sincos is about half of some 50 operations a pair), the
-// inverse root a hardware estimate and one third-order step.
+// pipe (50 operations a pair, 30 of them sine and cosine), the inverse root a
+// hardware estimate and one third-order step.
 //
 // Measured against one or two targets a thread and scalar FP32 (or the library's
 // square root and divisions), this phase alone on one B200: mixed, 1,048,576
 // sphere points, k = 5, depth 5 (3.57 G pairs) 4.65 -> 2.73 ms; FP64, 30,011
-// points, depth 3 (46.8 M pairs, 272 leaves) 1.41 -> 0.38 ms.
+// points, depth 3 (46.8 M pairs, 272 leaves) 1.41 -> 0.27 ms (0.38 with the
+// library's sincos, whose branch keeps a lane's targets one after another).
 #include <cuda_runtime.h>
 
 #include <cmath>
@@ -35,8 +36,12 @@
 namespace fmmb {
 namespace {
 
-constexpr int kThreads = 128;
-constexpr int kWarps = kThreads / 32;
+constexpr int kItem = 128;  // targets of a work item
+// Warps of a block: 4; in the FP64 form 8 where all items are resident at once with
+// 4 (as p2p_f64.cu).  30,011 points (272 leaves): this kernel 0.309 ms with 4,
+// 0.269 with 8, the pass 0.368 / 0.341.
+constexpr int kFewItems = 4 * 148;
+constexpr int max_warps(bool f32) { return f32 ? 4 : 8; }
 constexpr int kG = 8;        // targets of a group (lanes g = lane % 8)
 constexpr int kS = 32 / kG;  // source streams of a warp (s = lane / 8)
 constexpr int kMaxNT = 4;    // groups of a tile
@@ -58,14 +63,14 @@ template <>
 struct Smem<true> {
   float4 A[kCap / 2], B[kCap / 2];
   float2 Q[kCap / 2];
-  double red[kWarps - 1][kMaxNT][2][kG];
+  double red[max_warps(true) - 1][kMaxNT][2][kG];
   SrcList src;
 };
 template <>
 struct Smem<false> {
   double2 A[kCap], B[kCap];
   double Q[kCap];
-  double red[kWarps - 1][kMaxNT][2][kG];
+  double red[max_warps(false) - 1][kMaxNT][2][kG];
   SrcList src;
 };
 
@@ -124,6 +129,40 @@ __device__ __forceinline__ double inv_sqrt(double a) {
   return fma(y * e, fma(0.375, e, 0.5), y);
 }
 
+// sin and cos of x >= 0 in 30 FP64 operations (the library's general routine takes
+// several times as many).  Cody and Waite's reduction by multiples of pi/2 in two
+// parts (W. J. Cody, W. Waite, Software Manual for the Elementary Functions,
+// 1980), then the Taylor series on [-pi/4, pi/4] up to x^17 and x^16: the next
+// terms are below 2^-63 and 2^-58.  The reduced argument carries x's own
+// rounding, as any reduction does.  For x <= kPhaseMax, where two parts of pi/2 do.
+constexpr double kPhaseMax = 1e5;
+__device__ __forceinline__ void sincos_phase(double x, double& sn, double& cs) {
+  constexpr double kMagic = 6755399441055744.0;  // 1.5 * 2^52: rounds to an integer in the low word
+  const double t = fma(x, M_2_PI, kMagic), n = t - kMagic;
+  const int q = __double2loint(t);
+  const double h = fma(-n, M_PI_2, x), lo = 6.123233995736766e-17;  // pi/2 - M_PI_2
+  const double r = fma(-n, lo, h), e = fma(-n, lo, h - r), z = r * r;  // r + e: the reduced argument
+  double a = fma(z, 1.0 / 355687428096000.0, -1.0 / 1307674368000.0);  // 1/17!, 1/15!
+  a = fma(z, a, 1.0 / 6227020800.0);
+  a = fma(z, a, -1.0 / 39916800.0);
+  a = fma(z, a, 1.0 / 362880.0);
+  a = fma(z, a, -1.0 / 5040.0);
+  a = fma(z, a, 1.0 / 120.0);
+  a = fma(z, a, -1.0 / 6.0);
+  const double s = r + fma(r * z, a, e);
+  double b = fma(z, 1.0 / 20922789888000.0, -1.0 / 87178291200.0);  // 1/16!, 1/14!
+  b = fma(z, b, 1.0 / 479001600.0);
+  b = fma(z, b, -1.0 / 3628800.0);
+  b = fma(z, b, 1.0 / 40320.0);
+  b = fma(z, b, -1.0 / 720.0);
+  b = fma(z, b, 1.0 / 24.0);
+  const double w = fma(z, -0.5, 1.0);  // 1 - z / 2, and what its rounding lost
+  const double c = w + fma(z * z, b, fma(-r, e, fma(z, -0.5, 1.0 - w)));
+  const double u = q & 1 ? c : s, v = q & 1 ? s : c;
+  sn = q & 2 ? -u : u;
+  cs = (q + 1) & 2 ? -v : v;
+}
+
 // the lane's 8 sources of a run of 32 (j0, j0 + 4, ...) against its NT targets
 template <bool YUK, bool ZERO, int NT>
 __device__ __forceinline__ void run32(const Smem<false>& S, int j0, double k, double eps2, bool excl,
@@ -132,27 +171,45 @@ __device__ __forceinline__ void run32(const Smem<false>& S, int j0, double k, do
   for (int u = 0; u < 32 / kS; u++) {
     const double2 a = S.A[j0 + kS * u], b = S.B[j0 + kS * u];
     const double qi = S.Q[j0 + kS * u];
+    // in steps over all targets, without branches, so that their serial chains
+    // (estimate, step, reduction, series) overlap: few warps run in this form
+    double ri[NT], ph[NT];
+    bool on[NT], big = false;
 #pragma unroll
     for (int t = 0; t < NT; t++) {
       const double dx = tg[t][0] - a.x, dy = tg[t][1] - a.y, dz = tg[t][2] - b.x;
       const double d2 = fma(dx, dx, fma(dy, dy, dz * dz)), r2 = d2 + eps2;
-      double ri = inv_sqrt(r2);
+      ri[t] = inv_sqrt(r2);
+      on[t] = true;
       if (ZERO) {  // below the estimate's range: the library's, and no term at zero
-        if (r2 < 0x1p-1000) ri = 1.0 / sqrt(r2);
-        if ((excl && d2 == 0.0) || r2 == 0.0) continue;
+        if (r2 < 0x1p-1000) ri[t] = 1.0 / sqrt(r2);
+        on[t] = !((excl && d2 == 0.0) || r2 == 0.0);
       }
-      const double ph = k * (r2 * ri);
+      ph[t] = on[t] ? k * (r2 * ri[t]) : 0.0;
+      big |= !(ph[t] <= kPhaseMax);
+    }
+    double sn[NT], cs[NT];
+    if (YUK) {
+#pragma unroll
+      for (int t = 0; t < NT; t++) cs[t] = exp(-ph[t]);
+    } else if (big) {
+#pragma unroll
+      for (int t = 0; t < NT; t++) sincos(ph[t], &sn[t], &cs[t]);
+    } else {
+#pragma unroll
+      for (int t = 0; t < NT; t++) sincos_phase(ph[t], sn[t], cs[t]);
+    }
+#pragma unroll
+    for (int t = 0; t < NT; t++) {
+      if (ZERO && !on[t]) continue;
+      cs[t] *= ri[t];
       if (YUK) {
-        const double e = exp(-ph) * ri;
-        acc[t][0] = fma(b.y, e, acc[t][0]);
-        acc[t][1] = fma(qi, e, acc[t][1]);
+        acc[t][0] = fma(b.y, cs[t], acc[t][0]);
+        acc[t][1] = fma(qi, cs[t], acc[t][1]);
       } else {
-        double sn, cs;
-        sincos(ph, &sn, &cs);
-        sn *= ri;
-        cs *= ri;
-        acc[t][0] = fma(b.y, cs, fma(-qi, sn, acc[t][0]));
-        acc[t][1] = fma(b.y, sn, fma(qi, cs, acc[t][1]));
+        sn[t] *= ri[t];
+        acc[t][0] = fma(b.y, cs[t], fma(-qi, sn[t], acc[t][0]));
+        acc[t][1] = fma(b.y, sn[t], fma(qi, cs[t], acc[t][1]));
       }
     }
   }
@@ -162,7 +219,7 @@ __device__ __forceinline__ void run32(const Smem<false>& S, int j0, double k, do
 __device__ __forceinline__ void stage(Smem<true>& S, int c0, int c1, float4 pad, const float4* __restrict__ spos,
                                       const float2* __restrict__ q) {
   __syncthreads();  // the previous chunk's readers are done
-  for (int u = threadIdx.x; u < (c1 - c0) / 2; u += kThreads) {
+  for (int u = threadIdx.x; u < (c1 - c0) / 2; u += 32 * max_warps(true)) {
     float4 x[2];
     float2 qq[2];
 #pragma unroll
@@ -185,7 +242,7 @@ __device__ __forceinline__ void stage(Smem<true>& S, int c0, int c1, float4 pad,
 __device__ __forceinline__ void stage(Smem<false>& S, int c0, int c1, float4 pad, const float4* __restrict__ spos,
                                       const float2* __restrict__ q) {
   __syncthreads();
-  for (int u = threadIdx.x; u < c1 - c0; u += kThreads) {
+  for (int u = threadIdx.x; u < c1 - c0; u += blockDim.x) {
     const int j = S.src.locate(c0 + u, c1);
     float4 x = pad;
     float2 qq = make_float2(0.f, 0.f);
@@ -247,7 +304,7 @@ struct Num<false> {
 };
 
 template <bool F32, bool YUK, bool REDUCE>
-__global__ void __launch_bounds__(kThreads) helm_p2p(float k, float eps2, int excl, float far, const int2* __restrict__ work,
+__global__ void __launch_bounds__(32 * max_warps(F32)) helm_p2p(float k, float eps2, int excl, float far, const int2* __restrict__ work,
                                                      const int2* __restrict__ leaf_i, const int2* __restrict__ leaf_j,
                                                      const int* __restrict__ list, const float4* __restrict__ tpos,
                                                      const float4* __restrict__ spos, const float2* __restrict__ q,
@@ -260,7 +317,7 @@ __global__ void __launch_bounds__(kThreads) helm_p2p(float k, float eps2, int ex
   float4 pad = tpos[li.x];
   pad.x += far;
   li.x += wk.y;
-  li.y = min(kThreads, li.y - wk.y);
+  li.y = min(kItem, li.y - wk.y);
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, g = lane & (kG - 1), s = lane / kG;
   if (warp == 0) S.src.build(b, list, leaf_j, lane);
   __syncthreads();
@@ -268,8 +325,9 @@ __global__ void __launch_bounds__(kThreads) helm_p2p(float k, float eps2, int ex
   const int nchunk = (vlen + kCap - 1) / kCap;
   // teams of m warps share a tile of up to 4 groups of targets and split its runs
   const int ng = (li.y + kG - 1) / kG;
-  const int m = ng <= kMaxNT ? 4 : ng <= 2 * kMaxNT ? 2 : 1;  // block-uniform
-  const int nteam = kWarps / m, team = warp / m, w = warp % m;
+  const int NW = F32 ? 4 : blockDim.x >> 5;
+  const int m = ng <= kMaxNT ? NW : ng <= 2 * kMaxNT ? NW / 2 : NW / 4;  // block-uniform
+  const int nteam = NW / m, team = warp / m, w = warp % m;
   const int ga = team * ng / nteam, ntl = (team + 1) * ng / nteam - ga;  // at most 4 groups: li.y <= 128
   typename Num<F32>::V tg[kMaxNT][3];
   double P[kMaxNT][2];
@@ -338,7 +396,7 @@ void launch_helm_p2p(bool f32, bool yuk, float k, float eps2, bool excl, float l
   const double rmax = std::sqrt(12.0 * (double)leaf_side * leaf_side + (double)eps2);
   const bool reduce = !((double)k * rmax < 0.999 * M_PI);
   auto go = [&](auto kern) {
-    kern<<<nwork, kThreads, 0, st>>>(k, eps2, excl ? 1 : 0, 16.f * leaf_side, work, leaf_i, leaf_j, list, tpos, spos, (const float2*)qs,
+    kern<<<nwork, !f32 && nwork <= kFewItems ? 256 : 128, 0, st>>>(k, eps2, excl ? 1 : 0, 16.f * leaf_side, work, leaf_i, leaf_j, list, tpos, spos, (const float2*)qs,
                                      (double2*)pot);
   };
   if (f32 && !yuk && reduce) go(helm_p2p<true, false, true>);
