@@ -701,8 +701,10 @@ void launch_helm_l2p(int nwork, int p, double k, bool yuk, const int2* work, con
   FMMB_CHECK_LAUNCH();
 }
 
-void prepare_helm(int p) {
-  FMMB_CUDA(cudaFuncSetAttribute(helm_p2m, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)helm_p2m_smem(p)));
+// The limit belongs to the function, not to a plan: one for every order, or a plan of
+// a lower order would take it back under the others' launches.
+void prepare_helm() {
+  FMMB_CUDA(cudaFuncSetAttribute(helm_p2m, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)helm_p2m_smem(kMaxP)));
 }
 
 void launch_helm_direct(int i0, int i1, const int* inv_i, const float4* tpos, int nj, const float4* spos,
@@ -734,7 +736,8 @@ void build_ops(int p, double k, bool yuk, int nops, const HelmOp* ops, const dou
   if (nops <= 0) return;
   const int K = (p + 1) * (p + 1), NQ = 2 * p + 8, NP = 2 * NQ;
   const size_t smem = helm_build_smem(p);
-  FMMB_CUDA(cudaFuncSetAttribute(helm_build_ops<PAR>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+  FMMB_CUDA(cudaFuncSetAttribute(helm_build_ops<PAR>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                 (int)helm_build_smem(kMaxP)));
   for (int o0 = 0; o0 < nops; o0 += 65535) {
     dim3 grid(PAR ? (p + 1) * (p + 2) / 2 : K, std::min(65535, nops - o0));
     helm_build_ops<PAR><<<grid, 256, smem, st>>>(p, K, k, yuk ? 1 : 0, ops + o0, NQ, NP, gl_x, gl_w, ybar_q,

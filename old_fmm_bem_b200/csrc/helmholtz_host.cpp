@@ -170,7 +170,7 @@ void helm_setup(fmmb_plan* pl) {
       }
     }
   upload_vec(pl->d_ylm, ylm);
-  prepare_helm(p);
+  prepare_helm();
   const int nr = pl->cfg.nrhs;
   pl->qs.alloc((size_t)2 * pl->nj * nr);
   pl->M.alloc((size_t)pl->tot_j * 2 * K);

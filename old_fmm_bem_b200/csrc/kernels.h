@@ -196,7 +196,7 @@ void launch_helm_p2m(int nleaf, int p, double k, bool yuk, const int* keys, cons
 void launch_helm_l2p(int nwork, int p, double k, bool yuk, const int2* work, const int* keys, const int2* leaf,
                      const float4* tpos, const double* ylm, const float* bbox, double w, const double* L, double* pot,
                      cudaStream_t st);
-void prepare_helm(int p);  // shared-memory limits, outside stream capture
+void prepare_helm();  // shared-memory limits, outside stream capture
 void launch_helm_direct(int i0, int i1, const int* inv_i, const float4* tpos, int nj, const float4* spos,
                         const float* qs, double k, bool yuk, double eps2, bool excl, double* out, cudaStream_t st);
 template <typename T>

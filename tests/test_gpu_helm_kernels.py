@@ -71,3 +71,18 @@ def test_far_field_of_one_pair_of_leaves(kernel, p, ni, nj):
         pot = np.asarray(pl.evaluate(q, f64=True)[0])
     want, mag = _direct(kernel, xt, xs, q, 2.0)
     assert np.all(abs(pot - want) <= max(10 * 0.2 ** (p + 1), 1e-12) * mag)
+
+
+def test_a_plan_of_lower_order_in_between():
+    # the shared-memory limits of the kernels are process-wide: a plan of order 4 made after one of order 16 leaves the
+    # first one's evaluates (its first, launched directly, included) as they are
+    rng = np.random.default_rng(8)
+    x = rng.random((3, 700)).astype(np.float32)
+    q = (rng.standard_normal(700) + 1j * rng.standard_normal(700)).astype(np.complex64)
+    kw = dict(kernel=ob.HELMHOLTZ_G, lmax=2, precision=ob.FP64, semantics=ob.SEM_ACCURATE, exclude_self=True, wavenumber=2.0)
+    with ob.Plan(p=16, **kw) as a, ob.Plan(p=4, **kw) as b:
+        a.set_geometry(x, x, bbox=(0, 0, 0, 1))
+        b.set_geometry(x, x, bbox=(0, 0, 0, 1))
+        got = np.asarray(a.evaluate(q, f64=True)[0])
+        want = np.asarray(a.direct(q)[0])
+    assert np.linalg.norm(got - want) <= 1e-6 * np.linalg.norm(want)
