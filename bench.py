@@ -363,7 +363,9 @@ def phase_rooflines(plan, p, lmax, npts, phase, phase_alone, ms_step, mixed, tra
       * M2L (translate_h16 / translate_tc + its pair-row reduction): 2 K^2
         algorithmic flops per box pair on the tensor cores; peak = the
         measured dense bf16 for the FP16 kernel (p <= 12: FP16 and BF16 run at
-        the same rate), half of it (TF32) above;
+        the same rate), half of it (TF32) above; where the FP64 M2L runs (the
+        FP64 form, p > 15, few box pairs) the flops of its two blocks and the
+        nominal FP64 peak;
     and the whole matvec against the sum of its phases' roofline times
     (algorithmic work of each phase over the peak of the unit it runs on: P2P,
     P2M, L2P FP32; M2L FP16 or TF32; M2M, L2L FP64 at the nominal 37 TFLOP/s).
@@ -378,7 +380,13 @@ def phase_rooflines(plan, p, lmax, npts, phase, phase_alone, ms_step, mixed, tra
     fp32_peak = 148 * 128 * 2 * sm_max * 1e6 / 1e12
     p2p_ach = 20.0 * st["p2p_pairs"] / (phase_alone[0] * 1e-3) / 1e12
     tc_peak = peaks["bf16_tflops"] if p <= 12 else peaks["bf16_tflops"] / 2  # FP16 / TF32 dense
-    m2l_ach = 2.0 * K * K * st["m2l_pairs"] / (phase_alone[3] * 1e-3) / 1e12
+    fp64_peak = 37.0
+    # FP64 M2L: blocks of (p+1)(p+2)/2 and p(p+1)/2 rows
+    par = not mixed or K > 256 or (K <= 169 and st["m2l_pairs"] * K * K <= 7e8)
+    m2l_flops = 2.0 * (((p + 1) * (p + 2) // 2) ** 2 + (p * (p + 1) // 2) ** 2) if par else 2.0 * K * K
+    if par:
+        tc_peak = fp64_peak
+    m2l_ach = m2l_flops * st["m2l_pairs"] / (phase_alone[3] * 1e-3) / 1e12
     roof_p2p = {"kernel": "p2p_mixed" if mixed else "p2p_f64", "bound": "fp32", "achieved": p2p_ach,
                 "peak": fp32_peak, "unit": "TFLOP/s", "frac": p2p_ach / fp32_peak,
                 "traffic": traffic.get("p2p_mixed"), "ms": float(phase_alone[0]),
@@ -387,22 +395,23 @@ def phase_rooflines(plan, p, lmax, npts, phase, phase_alone, ms_step, mixed, tra
                         f"(near field not overlapped), summed per evaluate; peak = nominal FP32 at "
                         f"{sm_max:.0f} MHz (no FP32 figure in MEASURED_PEAKS.json); traffic per evaluate (two "
                         f"launches)"}
-    roof_m2l = {"kernel": ("translate_h16+reduce_pairs (M2L)" if p <= 12 else "translate_tc+reduce_pairs (M2L)")
-                if mixed else "translate_f64 (M2L)", "bound": "tensor",
-                "achieved": m2l_ach, "peak": tc_peak if mixed else None, "unit": "TFLOP/s",
-                "frac": (m2l_ach / tc_peak) if mixed else None,
+    roof_m2l = {"kernel": "m2l_parity (M2L)" if par else
+                "translate_h16+reduce_pairs (M2L)" if p <= 12 else "translate_tc+reduce_pairs (M2L)",
+                "bound": "fp64 tensor" if par else "tensor",
+                "achieved": m2l_ach, "peak": tc_peak, "unit": "TFLOP/s", "frac": m2l_ach / tc_peak,
                 "traffic": traffic.get("translate_tc"), "ms": float(phase_alone[3]),
                 "ms_in_overlapped_step": float(phase[3]),
-                "note": f"algorithmic 2*K^2 flops per box pair (K={K}, {st['m2l_pairs']} pairs); the tensor cores "
+                "note": f"{m2l_flops:.0f} flops of the even and odd blocks per box pair ({st['m2l_pairs']} pairs); "
+                        f"peak = nominal FP64 of a B200" if par else
+                        f"algorithmic 2*K^2 flops per box pair (K={K}, {st['m2l_pairs']} pairs); the tensor cores "
                         f"execute 3 FP16 MMAs per product (p <= 12; TF32 above) on operators padded to a multiple "
                         f"of 16 rows; peak = {peak_kind} dense bf16 (= FP16) for p <= 12, half of it (TF32) above; "
                         f"traffic per evaluate (translate + reduce_pairs)"}
     nb_i, nb_j = plan.tree(4), plan.tree(5)
-    fp64_peak = 37.0
     ideal = {"p2p": 20.0 * st["p2p_pairs"] / fp32_peak,
              "p2m": 2.0 * npts * K / fp32_peak,
              "m2m": 2.0 * K * K * float(nb_j[3:lmax + 1].sum()) / fp64_peak,
-             "m2l": 2.0 * K * K * st["m2l_pairs"] / tc_peak,
+             "m2l": m2l_flops * st["m2l_pairs"] / tc_peak,
              "l2l": 2.0 * K * K * float(nb_i[3:lmax + 1].sum()) / fp64_peak,
              "l2p": 2.0 * npts * K / fp32_peak}
     ideal = {k: v / 1e9 for k, v in ideal.items()}  # flops / (TFLOP/s) -> ms
@@ -1009,17 +1018,17 @@ def run_c5(args):
             v = pot.cpu().numpy()[sel]
             st = plan.stats()
             ph = plan.timings()
-            kr = 2 * (p + 1) ** 2  # real operator size
-            m2l_tf = 2.0 * kr * kr * st["m2l_pairs"] / (ph["m2l"] * 1e-3) / 1e12
+            fl = 6 * (((p + 1) * (p + 2) // 2) ** 2 + (p * (p + 1) // 2) ** 2)  # even and odd block, 3 real products
+            m2l_tf = fl * st["m2l_pairs"] / (ph["m2l"] * 1e-3) / 1e12
             res[name] = {"lmax": lmax, "autotune_ms": tune, "setup_s": setup_s, "matvec_ms": t_f,
                          "matvec_plus_adjoint_ms": t_fa, "phase_ms": ph, "stats": st,
-                         "m2l_roofline": {"kernel": "pairs_dmma_f64 (M2L)", "bound": "fp64 tensor",
+                         "m2l_roofline": {"kernel": "m2l_parity (M2L)", "bound": "fp64 tensor",
                                           "achieved": m2l_tf, "peak": 37.0, "unit": "TFLOP/s",
                                           "frac": m2l_tf / 37.0,
-                                          "note": f"algorithmic 2*{kr}^2 flops per box pair ({st['m2l_pairs']} "
-                                                  "pairs) over the M2L phase time of the last evaluate "
-                                                  "(P2P overlapped on the side stream); the kernel runs 128-row "
-                                                  "blocks (640 rows for 578); peak = nominal FP64 of a B200"},
+                                          "note": f"{fl} flops of the even and odd blocks, three real products "
+                                                  f"each, per box pair ({st['m2l_pairs']} pairs) over the M2L phase "
+                                                  "time (P2P overlapped on the side stream); peak = nominal FP64 of "
+                                                  "a B200"},
                          "rel_err_vs_fp64_direct": float(np.linalg.norm(v - vd) / np.linalg.norm(vd))}
             plan.close()
     m = res["mixed"]
