@@ -905,26 +905,39 @@ void run_graph(fmmb_plan* pl, bool want_grad, bool far_only = false) {
 }
 
 // The phase times of the last evaluate (its last right-hand side): its launches
-// run once more on the plan's own buffers, which hold its charges, with events
-// between the phases.  The evaluates themselves carry none: 26 event records took
-// 40 to 130 us of each (2,000 points, mixed: 117 us against 71 without).
+// run once more, with events between the phases, on its charges, which the plan
+// still holds (nothing but an evaluate writes qs), and on expansions of their own,
+// so that fmmb_get_expansions returns the evaluate's.  The evaluates themselves
+// carry none: 26 event records took 40 to 130 us of each (2,000 points, mixed: 117 us
+// against 71 without).
 void measure_phases(fmmb_plan* pl) {
   fmmb_plan::Phases& ph = pl->phases;
   if (ph.state != fmmb_plan::Phases::kPending) return;
   const int launches = pl->launches;
+  DevBuf<double> scratch[2];
+  const size_t w = helm_family(pl->cfg.kernel) ? 2 : 1;
+  scratch[0].alloc((size_t)pl->tot_j * w * pl->K);
+  scratch[1].alloc((size_t)pl->tot_i * w * pl->K);
   FMMB_CUDA(cudaEventSynchronize(pl->ev[1]));  // the stream may have been changed since
-  pl->timing = true;
+  auto enter = [&](bool on) {
+    pl->timing = on;
+    pl->far_only = on && ph.far_only;
+    std::swap(pl->M.ptr, scratch[0].ptr);
+    std::swap(pl->L.ptr, scratch[1].ptr);
+  };
   pl->ev_used = 0;
   pl->ev_phase.clear();
-  pl->far_only = ph.far_only;
+  enter(true);
   try {
     run_one(pl, (ph.far_only ? pl->qs_far.get() : pl->qs.get()) + ph.charges, ph.want_grad);
   } catch (...) {
-    pl->timing = pl->far_only = false;
+    enter(false);
     pl->launches = launches;
+    cudaStreamSynchronize(pl->st.main);  // the scratch goes
+    cudaStreamSynchronize(pl->st.side);
     throw;
   }
-  pl->timing = pl->far_only = false;
+  enter(false);
   pl->launches = launches;
   FMMB_CUDA(cudaStreamSynchronize(pl->st.main));
   FMMB_CUDA(cudaStreamSynchronize(pl->st.side));
@@ -1488,11 +1501,13 @@ int fmmb_direct_f64(fmmb_plan* pl, const float* q, int i0, int i1, double* pot, 
     FMMB_REQUIRE(0 <= i0 && i0 <= i1 && i1 <= pl->ni, FMMB_ERR_ARG, "target range out of bounds");
     cudaStream_t m = pl->st.main;
     const int nj = pl->nj, cnt = i1 - i0;
+    TmpBuf<float> qs(m);  // not the plan's: those are the last evaluate's
+    qs.alloc((size_t)(helm_family(pl->cfg.kernel) ? 2 : 1) * nj);
     if (helm_family(pl->cfg.kernel)) {  // Helmholtz: pot holds 2 cnt doubles (re, im); Yukawa: cnt
       const bool yuk = pl->cfg.kernel == FMMB_YUKAWA;
       const float* qd = to_device(q, (size_t)(yuk ? 1 : 2) * nj, pl->stage_f, m);
-      if (yuk) launch_helm_gather_real(nj, 1, pl->perm_j.get(), qd, pl->qs.get(), m);
-      else launch_helm_gather(nj, 1, pl->perm_j.get(), qd, pl->qs.get(), m);
+      if (yuk) launch_helm_gather_real(nj, 1, pl->perm_j.get(), qd, qs.get(), m);
+      else launch_helm_gather(nj, 1, pl->perm_j.get(), qd, qs.get(), m);
       DevBuf<double> out;
       out.alloc((size_t)2 * cnt + 2);
       const std::vector<int>&to = pl->prob_toff, &so = pl->prob_soff;
@@ -1500,7 +1515,7 @@ int fmmb_direct_f64(fmmb_plan* pl, const float* q, int i0, int i1, double* pot, 
         const int a0 = std::max(i0, to[b]), a1 = std::min(i1, to[b + 1]);
         if (a0 >= a1) continue;
         launch_helm_direct(a0, a1, pl->inv_i.get(), pl->tpos.get(), so[b + 1] - so[b], pl->spos.get() + so[b],
-                           pl->qs.get() + (size_t)2 * so[b], pl->cfg.wavenumber, yuk, pl->cfg.eps2,
+                           qs.get() + (size_t)2 * so[b], pl->cfg.wavenumber, yuk, pl->cfg.eps2,
                            pl->cfg.exclude_self != 0, out.get() + (size_t)2 * (a0 - i0), m);
       }
       if (yuk) {
@@ -1518,13 +1533,13 @@ int fmmb_direct_f64(fmmb_plan* pl, const float* q, int i0, int i1, double* pot, 
       return;
     }
     const float* qd = to_device(q, nj, pl->stage_f, m);
-    launch_gather_charges(nj, 1, pl->perm_j.get(), qd, pl->qs.get(), m);
+    launch_gather_charges(nj, 1, pl->perm_j.get(), qd, qs.get(), m);
     const bool want_grad = grad != nullptr;  // every Laplace kernel (w.r.t. the target position, normals fixed)
     DevBuf<double> out;
     out.alloc((size_t)cnt * 4 + 1);
     if (pl->nprob == 1) {
       launch_direct_f64(pl->cfg.kernel, i0, i1, pl->inv_i.get(), pl->tpos.get(), pl->tnrm.get(), nj, pl->spos.get(),
-                        pl->snrm.get(), pl->qs.get(), make_sem(pl), out.get(), want_grad ? out.get() + cnt : nullptr, m);
+                        pl->snrm.get(), qs.get(), make_sem(pl), out.get(), want_grad ? out.get() + cnt : nullptr, m);
     } else {
       // one launch per problem over its own sources (sorted source positions
       // of problem b are [soff[b], soff[b+1]) like the caller's), then the
@@ -1538,7 +1553,7 @@ int fmmb_direct_f64(fmmb_plan* pl, const float* q, int i0, int i1, double* pot, 
         const int mb = a1 - a0;
         double* tb = tmp.get() + (size_t)4 * (a0 - i0);
         launch_direct_f64(pl->cfg.kernel, a0, a1, pl->inv_i.get(), pl->tpos.get(), pl->tnrm.get(), so[b + 1] - so[b],
-                          pl->spos.get() + so[b], pl->snrm.get() + so[b], pl->qs.get() + so[b], make_sem(pl), tb,
+                          pl->spos.get() + so[b], pl->snrm.get() + so[b], qs.get() + so[b], make_sem(pl), tb,
                           want_grad ? tb + mb : nullptr, m);
         for (int c = 0; c < (want_grad ? 4 : 1); c++)
           FMMB_CUDA(cudaMemcpyAsync(out.get() + (size_t)c * cnt + (a0 - i0), tb + (size_t)c * mb, mb * sizeof(double),

@@ -1,0 +1,44 @@
+"""fmmb_get_timings runs the last evaluate's launches once more: with that evaluate's charges, and without a trace in what
+the plan holds."""
+import numpy as np
+import pytest
+
+import old_fmm_bem_b200 as ob
+
+pytestmark = pytest.mark.gpu
+N = 3001
+
+
+def _case(kernel, precision, nrhs):
+    rng = np.random.default_rng(5)
+    helm = kernel in (ob.HELMHOLTZ_G, ob.YUKAWA)
+    x = rng.random((3, N)).astype(np.float32)
+    q = [rng.standard_normal(N * k).astype(np.float32) for k in (nrhs, 1)]
+    if kernel == ob.HELMHOLTZ_G:
+        q = [v.astype(np.complex64) for v in q]
+    pl = ob.Plan(kernel=kernel, p=6, lmax=3, precision=precision, semantics=ob.SEM_ACCURATE, exclude_self=True, nrhs=nrhs,
+                 **(dict(wavenumber=2.0) if helm else {}))
+    pl.set_geometry(x, x, bbox=(0, 0, 0, 1))
+    return pl, x, q
+
+
+@pytest.mark.parametrize("kernel,precision,nrhs", [(ob.LAPLACE_G, ob.FP64, 1), (ob.LAPLACE_G, ob.FP64, 3),
+                                                   (ob.LAPLACE_G, ob.MIXED, 1), (ob.LAPLACE_G, ob.MIXED, 3),
+                                                   (ob.HELMHOLTZ_G, ob.MIXED, 1), (ob.YUKAWA, ob.FP64, 2)])
+@pytest.mark.parametrize("switch", [False, True])
+@pytest.mark.parametrize("evaluates", [1, 3])
+def test_expansions_stay_the_last_evaluates(kernel, precision, nrhs, switch, evaluates):
+    # not even their last bits (the atomics' order) change: nothing writes them
+    pl, x, q = _case(kernel, precision, nrhs)
+    with pl:
+        for _ in range(evaluates):
+            pl.evaluate(q[0], f64=True)
+        want = [pl.expansions(w) for w in (0, 1)]
+        pl.direct(q[1])  # other charges
+        if switch:
+            pl.set_overlap(False)
+        ph = pl.timings()
+        assert all(ph[k] > 0 for k in ph if k != "p2p") and (ph["p2p"] > 0) != (nrhs > 1 and precision == ob.MIXED)
+        assert pl.timings() == ph  # measured once
+        for w in (0, 1):
+            assert np.array_equal(pl.expansions(w), want[w])
