@@ -906,9 +906,9 @@ void run_graph(fmmb_plan* pl, bool want_grad, bool far_only = false) {
 
 // The phase times of the last evaluate (its last right-hand side): its launches
 // run once more, with events between the phases, on its charges, which the plan
-// still holds (nothing but an evaluate writes qs), and on expansions of their own,
-// so that fmmb_get_expansions returns the evaluate's.  The evaluates themselves
-// carry none: 26 event records took 40 to 130 us of each (2,000 points, mixed: 117 us
+// still holds (nothing but an evaluate writes qs), in its stream layout, and on
+// expansions of their own, so that fmmb_get_expansions returns the evaluate's.  The
+// evaluates themselves carry none: 26 event records took 40 to 130 us of each (2,000 points, mixed: 117 us
 // against 71 without).
 void measure_phases(fmmb_plan* pl) {
   fmmb_plan::Phases& ph = pl->phases;
@@ -922,6 +922,7 @@ void measure_phases(fmmb_plan* pl) {
   auto enter = [&](bool on) {
     pl->timing = on;
     pl->far_only = on && ph.far_only;
+    std::swap(pl->serial, ph.serial);
     std::swap(pl->M.ptr, scratch[0].ptr);
     std::swap(pl->L.ptr, scratch[1].ptr);
   };
@@ -995,7 +996,7 @@ int evaluate_impl(fmmb_plan* pl, const float* q, T* pot, T* grad) {
         } else {
           run_one(pl, pl->qs.get() + (size_t)2 * r * nj, false);
         }
-        pl->phases = {fmmb_plan::Phases::kPending, false, false, pl->use_graph ? 0 : (size_t)2 * r * nj, {}};
+        pl->phases = {fmmb_plan::Phases::kPending, false, false, pl->serial, pl->use_graph ? 0 : (size_t)2 * r * nj, {}};
         if (yuk)  // (pi/2) e^{-l r}/(l r) = (2 pi^2 / l) e^{-l r}/(4 pi r)
           launch_helm_finalize_real<T>(ni, pl->perm_i.get(), pl->pot_s.get(), pl->pot_s.get() + 2 * (size_t)ni,
                                        2.0 * M_PI * M_PI / pl->cfg.wavenumber, pd + (size_t)r * ni, m);
@@ -1065,7 +1066,7 @@ int evaluate_impl(fmmb_plan* pl, const float* q, T* pot, T* grad) {
       } else {
         run_one(pl, pl->qs.get() + (size_t)r * nj, want_grad);
       }
-      pl->phases = {fmmb_plan::Phases::kPending, want_grad, multi, multi || pl->use_graph ? 0 : (size_t)r * nj, {}};
+      pl->phases = {fmmb_plan::Phases::kPending, want_grad, multi, pl->serial, multi || pl->use_graph ? 0 : (size_t)r * nj, {}};
       // near and far parts of right-hand side r
       const double* pnear = multi ? pl->near_all.get() + (size_t)r * ni : pl->pot_s.get();
       const double* gnear = multi ? pl->near_all.get() + (size_t)nr * ni + (size_t)3 * r * ni : pl->grad_s.get();
@@ -1702,7 +1703,6 @@ int fmmb_set_overlap(fmmb_plan* pl, int on) {
   return guarded([&] {
     FMMB_REQUIRE(pl, FMMB_ERR_ARG, "null plan");
     if (pl->serial == (on == 0)) return;
-    measure_phases(pl);  // of the last evaluate, in the layout it ran in
     for (int w = 0; w < 4; w++) {  // captured with the other stream layout
       if (pl->gexec[w]) {
         FMMB_CUDA(cudaStreamSynchronize(pl->st.main));

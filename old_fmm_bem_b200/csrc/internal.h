@@ -173,7 +173,7 @@ struct fmmb_plan {
   bool timing = false;
   struct Phases {
     enum State { kNone, kPending, kMeasured } state = kNone;
-    bool want_grad = false, far_only = false;
+    bool want_grad = false, far_only = false, serial = false;
     size_t charges = 0;  // where the measured right-hand side's charges start
     float ms[6] = {};
   } phases;

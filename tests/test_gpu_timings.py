@@ -1,5 +1,5 @@
-"""fmmb_get_timings runs the last evaluate's launches once more: with that evaluate's charges, and without a trace in what
-the plan holds."""
+"""fmmb_get_timings runs the last evaluate's launches once more: with that evaluate's charges, in its stream layout, and
+without a trace in what the plan holds; fmmb_set_overlap runs nothing."""
 import numpy as np
 import pytest
 
@@ -42,3 +42,21 @@ def test_expansions_stay_the_last_evaluates(kernel, precision, nrhs, switch, eva
         assert pl.timings() == ph  # measured once
         for w in (0, 1):
             assert np.array_equal(pl.expansions(w), want[w])
+
+
+def test_set_overlap_runs_nothing():
+    # it changes the plan's state and returns while the plan's stream is busy (here for some 0.2 s)
+    torch = pytest.importorskip("torch")
+    pl, x, q = _case(ob.LAPLACE_G, ob.MIXED, 1)
+    s, e = torch.cuda.Stream(), torch.cuda.Event()
+    with pl:
+        pl.set_stream(s)
+        pl.evaluate(q[0])
+        s.synchronize()
+        with torch.cuda.stream(s):
+            torch.cuda._sleep(400_000_000)
+            e.record(s)
+            pl.set_overlap(False)
+            assert not e.query()
+        s.synchronize()
+        assert all(v > 0 for v in pl.timings().values())
