@@ -350,9 +350,14 @@ FMMB_API int fmmb_get_expansions(fmmb_plan* plan, int which, double* out);
 /* Device time in ms of the phases of the last evaluate (its last right-hand
  * side), summed over the launches of each phase: [0] P2P, [1] P2M, [2] M2M,
  * [3] M2L, [4] L2L, [5] L2P, [6] whole evaluate (P2P overlaps the far field).
- * The phases are measured here, by running that evaluate's launches once more
- * inside the plan (no output changes), so that the evaluates themselves carry no
- * timing events; they read 0 when fmmb_set_geometry came since. */
+ * Mixed plans with nrhs > 1 sum the near field of all right-hand sides in a pass
+ * of its own, which only [6] holds: [0] reads 0.
+ * [6] is measured with the evaluate.  The phases are measured by the first call
+ * after it, which runs that evaluate's launches once more, in its stream layout
+ * (fmmb_set_overlap), on expansions allocated for the time: the evaluates carry no
+ * timing events, nothing the plan returns changes, and the call costs an evaluate
+ * and two waits.  It needs the evaluate's geometry: phases not read before
+ * fmmb_set_geometry read 0 after it, those that were read stay. */
 FMMB_API int fmmb_get_timings(fmmb_plan* plan, float* ms7);
 
 /* Overlap of the near field with the far field (default on).  With on = 0

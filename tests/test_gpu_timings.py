@@ -60,3 +60,18 @@ def test_set_overlap_runs_nothing():
             assert not e.query()
         s.synchronize()
         assert all(v > 0 for v in pl.timings().values())
+
+
+@pytest.mark.parametrize("read", [False, True])
+def test_phases_after_a_new_geometry(read):
+    # the last evaluate's where they were read in time, else 0; never another geometry's
+    pl, x, q = _case(ob.LAPLACE_G, ob.MIXED, 1)
+    with pl:
+        pl.evaluate(q[0])
+        before = pl.timings() if read else None
+        pl.set_geometry(x, x, bbox=(0, 0, 0, 1))
+        ph = pl.timings()
+        assert ph == before if read else ph.pop("total") > 0 and not any(ph.values())
+        pl.evaluate(q[0])
+        now = pl.timings()
+        assert all(v > 0 for v in now.values()) and now != before
