@@ -17,6 +17,12 @@ constexpr int kSelfSlot = 13;  // offset (0, 0, 0) in the 27-slot list
 
 __device__ __forceinline__ int pad32(int n) { return (n + 31) & ~31; }
 
+// Two points, given their coordinates' differences, are not the same one.  (Their
+// squared distance does not tell: a softening is in it, and it can underflow.)
+__device__ __forceinline__ bool apart(float dx, float dy, float dz) {
+  return ((__float_as_int(dx) | __float_as_int(dy) | __float_as_int(dz)) & 0x7fffffff) != 0;
+}
+
 struct SrcList {
   int2 seg[32];  // (first source, count), own leaf first; slot 31: (0, sources of the others)
   int vst[32];   // virtual start of each segment, then INT_MAX

@@ -128,8 +128,8 @@ __device__ __forceinline__ void run16(const Smem<KER>& S, int pb, const Tgt (&tg
       const float2 r2 = __ffma2_rn(dx, dx, __ffma2_rn(dy, dy, __ffma2_rn(dz, dz, e2)));
       float2 ri = make_float2(rsqrt_ftz(r2.x), rsqrt_ftz(r2.y));
       if (EXCL) {
-        ri.x = r2.x > 0.f ? ri.x : 0.f;
-        ri.y = r2.y > 0.f ? ri.y : 0.f;
+        ri.x = r2.x > 0.f && apart(dx.x, dy.x, dz.x) ? ri.x : 0.f;
+        ri.y = r2.y > 0.f && apart(dx.y, dy.y, dz.y) ? ri.y : 0.f;
       }
       if (KER == FMMB_LAPLACE_G) {
         const float2 qr = __fmul2_rn(q2, ri);

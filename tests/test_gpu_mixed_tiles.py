@@ -71,3 +71,37 @@ def test_mixed_expansions_match_fp64(kernel, p, ni, nj):
     if kernel == ob.LAPLACE_G:
         gm = (q / (4 * np.pi * r ** 2)).sum(1)
         assert np.all(abs(out[0][1] - out[1][1]).reshape(3, -1) <= 2e-6 * gm)
+
+
+@pytest.mark.parametrize("kernel", [ob.LAPLACE_G, ob.LAPLACE_GNI, ob.LAPLACE_GNJ])
+@pytest.mark.parametrize("precision", [ob.FP64, ob.MIXED])
+@pytest.mark.parametrize("nrhs", [1, 2, 8])
+def test_excluded_pairs_with_softening(kernel, precision, nrhs):
+    # pairs at zero distance are left out whatever the softening; distinct points whose squared distance underflows in
+    # FP32 (1e-24 apart) are not.  All points in one leaf; bounds as above
+    rng = np.random.default_rng(nrhs)
+    n, eps2 = 203, 1e-3
+    x = (rng.random((3, n)) * 0.24).astype(np.float32)
+    x[:, 50:60] = x[:, 40:50]
+    x[:, 0], x[:, 1] = (0.1, 0, 0), (0.1, 1e-24, 0)
+    nrm = _unit(rng, n)
+    q = rng.standard_normal((nrhs, n)).astype(np.float32)
+    with ob.Plan(kernel=kernel, p=4, lmax=2, precision=precision, semantics=ob.SEM_ACCURATE, exclude_self=True, eps2=eps2,
+                 nrhs=nrhs) as pl:
+        pl.set_geometry(x, x, nrm if kernel == ob.LAPLACE_GNI else None, nrm if kernel == ob.LAPLACE_GNJ else None,
+                        bbox=(0, 0, 0, 1))
+        pot, grad = pl.evaluate(q.reshape(-1), np.zeros(n * nrhs), np.zeros(3 * n * nrhs), f64=True)
+    d = x.astype(np.float64)[:, :, None] - x.astype(np.float64)[:, None, :]
+    ri = np.where((d == 0).all(0), 0.0, 1.0 / np.sqrt((d ** 2).sum(0) + eps2))
+    if kernel == ob.LAPLACE_G:
+        t = [ri] + [-d[k] * ri ** 3 for k in range(3)]
+        mag = [abs(v) for v in t]
+    else:
+        v = (nrm[:, :, None] if kernel == ob.LAPLACE_GNI else nrm[:, None, :]).astype(np.float64)
+        dot, m = (d * v).sum(0), abs(d * v).sum(0)
+        t = [dot * ri ** 3] + [ri ** 3 * (v[k] - 3 * dot * ri ** 2 * d[k]) for k in range(3)]
+        mag = [m * ri ** 3] + [ri ** 3 * (abs(v[k]) + 3 * m * ri ** 2 * abs(d[k])) for k in range(3)]
+    qd, c, tol = q.astype(np.float64).T, 0.25 / np.pi, 80 * 2.0 ** -24
+    out = [pot.reshape(nrhs, n)] + list(np.moveaxis(grad.reshape(nrhs, 3, n), 1, 0))
+    for a, tt, mm in zip(out, t, mag):
+        assert np.all(abs(a.T - c * tt @ qd) <= tol * c * (mm @ abs(qd)))
