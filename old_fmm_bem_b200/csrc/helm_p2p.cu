@@ -12,7 +12,9 @@
 // (p2p_list.cuh); a warp is 8 target lanes x 4 source streams, a lane holding
 // NT <= 4 targets, so that a leaf of any size fills the lanes and a
 // shared-memory read of sources serves NT targets; only the own leaf's runs and
-// the last one, which can hold padding, test for zero distance.
+// the last one, which can hold padding, test for zero distance.  (Mixed form: a chunk
+// with a coordinate so close to zero that r^2 may be below FP32's normal range takes
+// a plainer loop, near_zero_runs.)
 //
 // Bounds.  Mixed: the special-function pipe (rsqrt, sine and cosine: 3 of 16
 // lanes a clock per pair, 3.57 G pairs in 2.3 ms), with the FP32 work next to it
@@ -163,6 +165,46 @@ __device__ __forceinline__ void sincos_phase(double x, double& sn, double& cs) {
   cs = (q + 1) & 2 ? -v : v;
 }
 
+// A coordinate this close to zero can differ by less than 2^-60 from another, so that a squared distance underflows
+// in FP32; other coordinates are equal or at least that far apart.
+__device__ __forceinline__ bool tiny(float c) { return c != 0.f && fabsf(c) < 0x1p-36f; }
+__device__ __forceinline__ bool tiny(const float4& x) { return tiny(x.x) || tiny(x.y) || tiny(x.z); }
+
+// The lane's sources of the chunk's runs w, w + m, ... of nrun against one target, for any r^2: the library's inverse
+// root takes subnormal ones.  Out of line, so that the loops above keep their registers.
+template <bool YUK>
+__device__ __noinline__ double2 near_zero_runs(const Smem<true>& S, int nrun, int s, int w, int m, float k, float eps2,
+                                               bool excl, float x, float y, float z) {
+  double2 sum = make_double2(0.0, 0.0);
+#pragma unroll 1
+  for (int r = w; r < nrun; r += m) {
+    float re = 0.f, im = 0.f;
+#pragma unroll 1
+    for (int u = 0; u < 8; u++) {
+      const int pb = 16 * r + s + 4 * (u >> 1), h = u & 1;
+      const float4 a = S.A[pb], b = S.B[pb];
+      const float2 q = S.Q[pb];
+      const float dx = x + (h ? a.y : a.x), dy = y + (h ? a.w : a.z), dz = z + (h ? b.y : b.x);
+      const float d2 = dx * dx + dy * dy + dz * dz, r2 = d2 + eps2;
+      if ((excl && d2 == 0.f) || r2 == 0.f) continue;
+      const float ri = rsqrtf(r2), ph = k * (r2 * ri), qr = h ? b.w : b.z, qi = h ? q.y : q.x;
+      if (YUK) {
+        const float e = __expf(-ph) * ri;
+        re = fmaf(qr, e, re);
+        im = fmaf(qi, e, im);
+      } else {
+        float sn, cs;
+        __sincosf(fmaf(-6.28318530717958647f, rintf(ph * 0.159154943091895336f), ph), &sn, &cs);
+        re += (qr * cs - qi * sn) * ri;
+        im += (qr * sn + qi * cs) * ri;
+      }
+    }
+    sum.x += (double)re;
+    sum.y += (double)im;
+  }
+  return sum;
+}
+
 // the lane's 8 sources of a run of 32 (j0, j0 + 4, ...) against its NT targets
 template <bool YUK, bool ZERO, int NT>
 __device__ __forceinline__ void run32(const Smem<false>& S, int j0, double k, double eps2, bool excl,
@@ -215,9 +257,10 @@ __device__ __forceinline__ void run32(const Smem<false>& S, int j0, double k, do
   }
 }
 
-// pad: where the list's padding lies, 16 leaf sides from the targets (the phase stays moderate), no charge
-__device__ __forceinline__ void stage(Smem<true>& S, int c0, int c1, float4 pad, const float4* __restrict__ spos,
-                                      const float2* __restrict__ q) {
+// pad: where the list's padding lies, 16 leaf sides from the targets (the phase stays moderate), no charge.
+// Returns whether any thread's near0 is set or a source has a coordinate close to zero.
+__device__ __forceinline__ bool stage(Smem<true>& S, int c0, int c1, bool near0, float4 pad,
+                                      const float4* __restrict__ spos, const float2* __restrict__ q) {
   __syncthreads();  // the previous chunk's readers are done
   for (int u = threadIdx.x; u < (c1 - c0) / 2; u += 32 * max_warps(true)) {
     float4 x[2];
@@ -230,16 +273,17 @@ __device__ __forceinline__ void stage(Smem<true>& S, int c0, int c1, float4 pad,
       if (j >= 0) {
         x[h] = spos[j];
         qq[h] = q[j];
+        near0 |= tiny(x[h]);
       }
     }
     S.A[u] = make_float4(-x[0].x, -x[1].x, -x[0].y, -x[1].y);
     S.B[u] = make_float4(-x[0].z, -x[1].z, qq[0].x, qq[1].x);
     S.Q[u] = make_float2(qq[0].y, qq[1].y);
   }
-  __syncthreads();
+  return __syncthreads_or(near0);
 }
 
-__device__ __forceinline__ void stage(Smem<false>& S, int c0, int c1, float4 pad, const float4* __restrict__ spos,
+__device__ __forceinline__ bool stage(Smem<false>& S, int c0, int c1, bool, float4 pad, const float4* __restrict__ spos,
                                       const float2* __restrict__ q) {
   __syncthreads();
   for (int u = threadIdx.x; u < c1 - c0; u += blockDim.x) {
@@ -255,6 +299,7 @@ __device__ __forceinline__ void stage(Smem<false>& S, int c0, int c1, float4 pad
     S.Q[u] = qq.y;
   }
   __syncthreads();
+  return false;  // squared differences of floats are normal in FP64
 }
 
 // The team tile's runs of the chunk [c0, c1): runs k, k + m, ..., the own
@@ -331,10 +376,12 @@ __global__ void __launch_bounds__(32 * max_warps(F32)) helm_p2p(float k, float e
   const int ga = team * ng / nteam, ntl = (team + 1) * ng / nteam - ga;  // at most 4 groups: li.y <= 128
   typename Num<F32>::V tg[kMaxNT][3];
   double P[kMaxNT][2];
+  bool near0 = F32 && eps2 > 0.f && eps2 < 0x1p-126f;
 #pragma unroll
   for (int t = 0; t < kMaxNT; t++) {
     const int it = (ga + t) * kG + g;
     const float4 x = t < ntl && it < li.y ? tpos[li.x + it] : make_float4(0.f, 0.f, 0.f, 0.f);
+    near0 |= F32 && tiny(x);
     tg[t][0] = Num<F32>::make(x.x);
     tg[t][1] = Num<F32>::make(x.y);
     tg[t][2] = Num<F32>::make(x.z);
@@ -342,7 +389,20 @@ __global__ void __launch_bounds__(32 * max_warps(F32)) helm_p2p(float k, float e
   }
   for (int ch = 0; ch < nchunk; ch++) {
     const int c0 = ch * kCap, c1 = min(vlen, c0 + kCap);
-    stage(S, c0, c1, pad, spos, q);
+    const bool sub = stage(S, c0, c1, near0, pad, spos, q);  // block-uniform
+    if constexpr (F32) {
+      if (sub) {
+#pragma unroll
+        for (int t = 0; t < kMaxNT; t++) {
+          if (t >= ntl) break;
+          const double2 v = near_zero_runs<YUK>(S, (c1 - c0) >> 5, s, w, m, k, eps2, excl, tg[t][0].x, tg[t][1].x,
+                                                tg[t][2].x);
+          P[t][0] += v.x;
+          P[t][1] += v.y;
+        }
+        continue;
+      }
+    }
     switch (ntl) {
       case 0: break;
       case 1: tile_runs<YUK, REDUCE, 1>(S, c0, c1, self_end, vlen - 32, s, w, m, (T)k, (T)eps2, excl, tg, P); break;

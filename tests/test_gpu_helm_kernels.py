@@ -86,3 +86,30 @@ def test_a_plan_of_lower_order_in_between():
         got = np.asarray(a.evaluate(q, f64=True)[0])
         want = np.asarray(a.direct(q)[0])
     assert np.linalg.norm(got - want) <= 1e-6 * np.linalg.norm(want)
+
+
+@pytest.mark.parametrize("kernel", [ob.HELMHOLTZ_G, ob.YUKAWA])
+@pytest.mark.parametrize("precision", [ob.FP64, ob.MIXED])
+@pytest.mark.parametrize("where", ["one leaf", "across leaves", "softened"])
+def test_squared_distances_below_the_normal_range(kernel, precision, where):
+    # r^2 is subnormal in FP32 (r of 5e-21 and more, so 2^-14 of r^2 and less is lost): two close points, a whole domain
+    # of that size, and a softening of that size
+    rng = np.random.default_rng(11)
+    eps2 = 0.0
+    if where == "across leaves":
+        cells = np.array(np.unravel_index(rng.permutation(512)[:300], (8, 8, 8)))
+        x = (1e-20 * (cells + 0.1 + 0.2 * rng.random((3, 300)))).astype(np.float32)
+        side = np.float32(16e-20)
+    else:
+        x, side = (rng.random((3, 40)) * 0.4).astype(np.float32), 1.0
+        x[:, 7], x[:, 8] = (0.3, 0, 0.1), (0.3, 2e-20, 0.1)
+        if where == "softened":
+            eps2 = 1e-40
+            x[:, 8] = x[:, 7]
+    q = _charges(rng, kernel, x.shape[1])
+    with ob.Plan(kernel=kernel, p=4, lmax=2, precision=precision, semantics=ob.SEM_ACCURATE, exclude_self=where != "softened",
+                 eps2=eps2, wavenumber=1.0) as pl:
+        pl.set_geometry(x, x, bbox=(0, 0, 0, side))
+        pot = np.asarray(pl.evaluate(q, f64=True)[0])
+        want = np.asarray(pl.direct(q)[0])
+    assert np.all(np.isfinite(pot)) and np.linalg.norm(pot - want) <= 2.0 ** -12 * np.linalg.norm(want)
