@@ -812,7 +812,9 @@ __global__ void __launch_bounds__(kL2PHThreads) l2p_hess_gni(int p, int K, const
 // complex s_m once per order; here in the monic form (c_monic, above), fully
 // unrolled to order P (runtime order p <= P).  Coefficients are formed in
 // FP64 and rounded; B, the powers of t and the sums of one order are FP32, the
-// sums over the orders and the constant term, the largest, FP64.
+// sums over the orders and the terms of degree 0 of the potential and of each
+// derivative, the largest, FP64 (in the FP32 sums those made the gradient's
+// rounding error 7e-8 of it, 1e-8 to 2.3e-8 now).
 // Bound: the FP32 pipe: 3 + 8 lane operations a term and two 16-byte
 // shared-memory reads.  (Complex recurrences and derivative sums per term, 16
 // operations and three reads: 1,048,576 targets at p = 12: 0.20 ms; 0.11 now.)
@@ -846,7 +848,7 @@ __global__ void __launch_bounds__(kL2PF32Threads) l2p_f32(int p, int K, const in
     const double g = c_monic.g[idx], wm = m ? 2.0 : 1.0;
     float2 cf = make_float2(0.f, 0.f), cx = cf, cy = cf, cz = cf;
     if (n > 0 && n <= p && POT) cf = f2(cscale(Lnm(n, m), g * wm * fac[ifull_d(n, m)]));
-    if (DER && n < p) {  // as l2p_cart
+    if (DER && n > 0 && n < p) {  // as l2p_cart
       cz = f2(cscale(Lnm(n + 1, m), g * wm * fac[ifull_d(n + 1, m)] * (n + 1 + m)));
       const cplx cp = m >= 1 ? cscale(Lnm(n + 1, m - 1), (m - 1 ? 2.0 : 1.0) * fac[ifull_d(n + 1, m - 1)]) : cplx{0.0, 0.0};
       const cplx cm = cscale(Lnm(n + 1, m + 1), -2.0 * fac[ifull_d(n + 1, m + 1)] * (double)(n + m + 2) * (double)(n + m + 1));
@@ -873,7 +875,14 @@ __global__ void __launch_bounds__(kL2PF32Threads) l2p_f32(int p, int K, const in
   const float x = (float)(((double)xt.x - xc) * inv_rb), y = (float)(((double)xt.y - yc) * inv_rb),
               z = (float)(((double)xt.z - zc) * inv_rb);
   const float mr2 = -(x * x + y * y + z * z);
-  double F = POT ? Lb[0] * fac[0] : 0.0, gx = 0, gy = 0, gz = 0;
+  double F = 0, gx = 0, gy = 0, gz = 0;
+  if (POT) F = Lb[0] * fac[0];
+  if (DER) {  // p >= 1: d/dz from (1, 0), d/dx and d/dy (twice) from (1, 1)
+    const double f11 = 4.0 * fac[ifull_d(1, 1)];
+    gx = -f11 * Lb[2];
+    gy = f11 * Lb[3];
+    gz = fac[ifull_d(1, 0)] * Lb[1];
+  }
   float tr = 1.f, ti = 0.f;  // t^m
 #pragma unroll
   for (int m = 0; m <= P; m++) {

@@ -105,3 +105,29 @@ def test_excluded_pairs_with_softening(kernel, precision, nrhs):
     out = [pot.reshape(nrhs, n)] + list(np.moveaxis(grad.reshape(nrhs, 3, n), 1, 0))
     for a, tt, mm in zip(out, t, mag):
         assert np.all(abs(a.T - c * tt @ qd) <= tol * c * (mm @ abs(qd)))
+
+
+@pytest.mark.parametrize("kernel", [ob.LAPLACE_G, ob.LAPLACE_GNI])
+@pytest.mark.parametrize("p", [4, 8, 11, 12, 16])
+def test_fp32_l2p_rounding(kernel, p):
+    # the L2P alone: point sources at leaf centres (their multipoles are exact), no near field, the FP64 M2L.  The terms
+    # of degree 0 are added in FP64; what is left, FP32 terms of relative size 1/3 and less, carries coordinates, tables
+    # and recurrences of 2^-24 each and p + 1 sums of up to p + 1 terms, at random: 2^-24 of the field in the 2-norm
+    rng = np.random.default_rng(p)
+    far = np.array([(a, b, c) for a in range(8) for b in range(8) for c in range(8) if max(a, b, c) >= 5])
+    pick = far[rng.permutation(len(far))[:80]]
+    xs = ((pick.T + 0.5) / 8).astype(np.float32)
+    xt = (rng.random((3, 4000)) * 0.374).astype(np.float32)
+    tn = _unit(rng, 4000)
+    q = rng.standard_normal(80).astype(np.float32)
+    out = []
+    for prec in (ob.MIXED, ob.FP64):
+        with ob.Plan(kernel=kernel, p=p, lmax=3, precision=prec, semantics=ob.SEM_ACCURATE, exclude_self=True) as pl:
+            pl.set_geometry(xt, xs, tn if kernel == ob.LAPLACE_GNI else None, bbox=(0, 0, 0, 1))
+            out.append(pl.evaluate(q, f64=True))
+            assert pl.stats()["p2p_pairs"] == 0
+    for a, b in zip(*out):
+        if a is not None:
+            err = np.linalg.norm(a - b) / np.linalg.norm(b)
+            print(kernel, p, err)
+            assert err <= 2.0 ** -24
