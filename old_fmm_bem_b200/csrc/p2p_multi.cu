@@ -85,11 +85,12 @@ __device__ __forceinline__ void run32(const Smem<KER, R>& S, int pb, const Tgt (
 #pragma unroll
     for (int t = 0; t < kNT; t++) {
       const float2 dx = __fadd2_rn(tg[t].x, sx), dy = __fadd2_rn(tg[t].y, sy), dz = __fadd2_rn(tg[t].z, sz);
-      const float2 r2 = __ffma2_rn(dx, dx, __ffma2_rn(dy, dy, __ffma2_rn(dz, dz, e2)));
+      const float2 d2 = __ffma2_rn(dx, dx, __ffma2_rn(dy, dy, EXCL ? __fmul2_rn(dz, dz) : __ffma2_rn(dz, dz, e2)));
+      const float2 r2 = EXCL ? __fadd2_rn(d2, e2) : d2;
       float2 ri = make_float2(rsqrt_ftz(r2.x), rsqrt_ftz(r2.y));
-      if (EXCL) {
-        ri.x = r2.x > 0.f && apart(dx.x, dy.x, dz.x) ? ri.x : 0.f;
-        ri.y = r2.y > 0.f && apart(dx.y, dy.y, dz.y) ? ri.y : 0.f;
+      if (EXCL && fminf(d2.x, d2.y) == 0.f) {  // the same point, or a square that underflows
+        if (d2.x == 0.f && !(r2.x > 0.f && apart(dx.x, dy.x, dz.x))) ri.x = 0.f;
+        if (d2.y == 0.f && !(r2.y > 0.f && apart(dx.y, dy.y, dz.y))) ri.y = 0.f;
       }
       float2 kv[NC];
       if (KER == FMMB_LAPLACE_G) {
