@@ -161,7 +161,7 @@ __device__ void stage(Smem<KER, REF>& S, int c0, int c1, const float4* __restric
   __syncthreads();  // the previous chunk's readers are done
   for (int u = threadIdx.x; u < c1 - c0; u += blockDim.x) {
     const int j = S.src.locate(c0 + u, c1);
-    float4 x = make_float4(1e18f, 1e18f, 1e18f, 0.f), n = make_float4(0.f, 0.f, 0.f, 0.f);  // padding: far, no charge
+    float4 x = make_float4(1e18f, 0.f, 0.f, 0.f), n = make_float4(0.f, 0.f, 0.f, 0.f);  // padding: no charge
     float q = 0.f;
     if (j >= 0) {
       x = spos[j];
@@ -173,7 +173,7 @@ __device__ void stage(Smem<KER, REF>& S, int c0, int c1, const float4* __restric
       S.X[u] = x;
       S.Q[u] = cq;
     } else {
-      S.A[u] = make_double2(x.x, x.y);
+      S.A[u] = make_double2(j >= 0 ? (double)x.x : 1e100, x.y);  // padding: farther off than any float
       S.B[u] = make_double2(x.z, cq);
     }
     if (KER == FMMB_LAPLACE_GNJ) {

@@ -62,3 +62,22 @@ def test_included_coincident_pair_is_infinite():
         pl.set_geometry(x, x, bbox=(0, 0, 0, 1))
         pot, _ = pl.evaluate(np.ones(2, np.float32), f64=True)
     assert np.all(np.isposinf(pot))
+
+
+@pytest.mark.parametrize("kernel", [ob.LAPLACE_G, ob.LAPLACE_GNI, ob.LAPLACE_GNJ])
+def test_any_coordinates(kernel):
+    # no coordinates a caller can give meet the padding of the source lists: targets around 1e18, which FP32 holds to
+    # 2^36.  Bounds as above
+    rng = np.random.default_rng(2)
+    x = (rng.random((3, 70)) * 1.9e18).astype(np.float32)
+    x[:, 5] = 1e18
+    s = x[:, 20:57].copy()
+    tn, sn = rng.standard_normal((3, 70)).astype(np.float32), rng.standard_normal((3, 37)).astype(np.float32)
+    q = rng.standard_normal(37).astype(np.float32)
+    with ob.Plan(kernel=kernel, p=4, lmax=2, precision=ob.FP64, semantics=ob.SEM_ACCURATE, exclude_self=True) as pl:
+        pl.set_geometry(x, s, tn if kernel == ob.LAPLACE_GNI else None, sn if kernel == ob.LAPLACE_GNJ else None,
+                        bbox=(0, 0, 0, 4e18))
+        pot, grad = pl.evaluate(q, np.zeros(70), np.zeros(210), f64=True)
+    want, mag = _direct(kernel, x, s, tn, sn, q, False, True)
+    tol = (37 + 8) * 2.0 ** -53 * mag
+    assert np.all(abs(pot - want[0]) <= tol[0]) and np.all(abs(grad.reshape(3, -1) - want[1:]) <= tol[1:])
