@@ -13,10 +13,16 @@
 // shared-memory read of a pair of sources and its charges serves 4 pairs of
 // points; the two-lane FP32 instructions take the two sources.  Teams of warps
 // share a tile of 16 targets where a leaf has fewer than 65.  A lane's two sums
-// of 64 sources and the 4 streams' are added in FP32 (67 roundings at most of
-// 512 terms) and promoted to FP64 every 16 runs, the components dealt to the
-// streams' lanes.  Zero-distance pairs, which only the own leaf's runs can hold,
-// are skipped (their inverse distance is taken as 0) when the plan excludes them.
+// are added in FP32 and promoted to FP64 after at most 8 runs (32 sources in each),
+// 4 where a leaf has 33 to 64 targets, so that a FP32 chain is no longer than such a
+// leaf; the components of the 4 streams are added in FP64 and dealt to the streams'
+// lanes.  Zero-distance pairs, which only the own leaf's runs can hold, are skipped
+// (their inverse distance is taken as 0) when the plan excludes them.
+//
+// Rounding error of the potential of 8, 33, 64, 100 positive charges a leaf: 0.9, 1.1,
+// 0.9, 1.2 e-8 (one target per thread, chains of one leaf and at most 128 sources: 1.2,
+// 1.9, 2.5, 3.1; 16 runs, the streams added in FP32: 1.6, 2.5, 1.8, 2.5, for 1 to 2 %
+// less time).
 //
 // Bound: the FP32 pipe: 12 + R lane operations a pair for the normal-derivative
 // kernels, 13 + 4 R for G with its gradient.  Measured against one target per
@@ -175,6 +181,7 @@ __global__ void __launch_bounds__(kThreads) p2p_multi(const int2* __restrict__ w
 #pragma unroll
   for (int i = 0; i < NPL; i++) P[i] = 0.0;
   const float2 e2 = dup(eps2);
+  const int nrun = m == 2 ? 4 : 8;  // runs between promotions (with m = 4 and 8 a chunk has 4 and 2)
   for (int c0 = 0; c0 < vlen; c0 += kCap) {
     const int c1 = min(vlen, c0 + kCap);
     stage<KER, R>(S, c0, c1, spos, snrm, qs, nj);
@@ -188,19 +195,34 @@ __global__ void __launch_bounds__(kThreads) p2p_multi(const int2* __restrict__ w
         for (int q = 0; q < R; q++)
 #pragma unroll
           for (int c = 0; c < NC; c++) acc[t][q][c] = make_float2(0.f, 0.f);
-      for (int i = 0; i < 16 && r < rend; i++, r += m) {  // 16 runs: 64 sources in each of a lane's two sums
+      for (int i = 0; i < nrun && r < rend; i++, r += m) {
         const int pb = ((r * 32 - c0) >> 1) + s;
         if (EXCL && r * 32 < self_end) run32<KER, R, NC, true>(S, pb, tg, e2, acc);
         else run32<KER, R, NC, false>(S, pb, tg, e2, acc);
       }
+      // component kk to stream kk & 3: first across streams s, s ^ 2, then s, s ^ 1
+      double half[NPL][2];
 #pragma unroll
-      for (int kk = 0; kk < NK; kk++) {
-        const float2 a = acc[kk / (R * NC)][(kk / NC) % R][kk % NC];
-        float v = a.x + a.y;
-        v += __shfl_xor_sync(0xffffffffu, v, 8);
-        v += __shfl_xor_sync(0xffffffffu, v, 16);
-        if ((kk & 3) == s) P[kk / 4] += (double)v;
-      }
+      for (int i = 0; i < NPL; i++)
+#pragma unroll
+        for (int b = 0; b < 2; b++) {
+          float v[2];
+#pragma unroll
+          for (int h = 0; h < 2; h++) {
+            const int kk = 4 * i + 2 * h + b;
+            if (kk < NK) {
+              const float2 a = acc[kk / (R * NC)][(kk / NC) % R][kk % NC];
+              v[h] = a.x + a.y;
+            } else {
+              v[h] = 0.f;
+            }
+          }
+          const float other = __shfl_xor_sync(0xffffffffu, s & 2 ? v[0] : v[1], 16);
+          half[i][b] = (double)(s & 2 ? v[1] : v[0]) + (double)other;
+        }
+#pragma unroll
+      for (int i = 0; i < NPL; i++)
+        P[i] += (s & 1 ? half[i][1] : half[i][0]) + __shfl_xor_sync(0xffffffffu, s & 1 ? half[i][0] : half[i][1], 8);
     }
   }
   if (m > 1) {  // block-uniform: the team's warps through shared memory

@@ -131,3 +131,27 @@ def test_fp32_l2p_rounding(kernel, p):
             err = np.linalg.norm(a - b) / np.linalg.norm(b)
             print(kernel, p, err)
             assert err <= 2.0 ** -24
+
+
+@pytest.mark.parametrize("n", [33, 40, 100])
+def test_many_rhs_near_field_rounding(n):
+    # potentials of equal charges of one sign, n in each of 27 leaves.  A FP32 chain of c terms is off by
+    # 0.4 2^-24 sqrt(c / 3) of its sum, M chains by that over sqrt(M) of the total: 0.7e-8 with c = 16 and n = 33, 0.6e-8
+    # with c = 32 and n = 100, and the terms' own roundings; chains of 64 terms and sums of several chains in FP32, 2e-8
+    err = []
+    for seed in range(8):
+        rng = np.random.default_rng(seed)
+        cells = np.array(np.unravel_index(np.arange(27), (3, 3, 3))).T
+        xs = np.concatenate([(c + rng.random((n, 3))) / 4 for c in cells]).T.astype(np.float32)
+        xt = ((1 + rng.random((n, 3))) / 4).T.astype(np.float32)
+        q = rng.random((4, 27 * n)).astype(np.float32)
+        with ob.Plan(kernel=ob.LAPLACE_G, p=4, lmax=2, precision=ob.MIXED, semantics=ob.SEM_ACCURATE, exclude_self=True,
+                     nrhs=4) as pl:
+            pl.set_geometry(xt, xs, bbox=(0, 0, 0, 1))
+            pot, _ = pl.evaluate(q.reshape(-1), f64=True)
+        r = np.linalg.norm(xt.astype(np.float64)[:, :, None] - xs[:, None, :], axis=0)
+        want = q.astype(np.float64) @ (0.25 / (np.pi * r)).T
+        err.append(np.linalg.norm(pot.reshape(4, n) - want) / np.linalg.norm(want))
+    err = np.exp(np.mean(np.log(err)))
+    print(n, err)
+    assert err <= 1.6e-8
