@@ -171,9 +171,10 @@ namespace {
 // ---- stable LSD radix sort of (key, index) ----
 constexpr int kRsWarps = 8;
 constexpr int kRsThreads = kRsWarps * 32;
-// Elements per thread (ROUNDS): 8, and 2 below 2^19 elements, where blocks of 2,048
-// do not fill the 148 SMs twice (131,071 points, 64 blocks instead of 256: a new
-// geometry and its evaluate 1.15 ms, with 2 1.08).
+// Elements per thread (ROUNDS): 8, and 2 below 2^18 elements, where blocks of 2,048
+// are fewer than the 148 SMs.  fmmb_set_geometry with 8 / 2: 65,536 points 0.631 /
+// 0.560 ms, 131,072 0.609 / 0.565; 262,144 1.026 / 1.037, 393,216 1.033 / 1.054,
+// 1,048,576 1.132 / 1.141.
 template <int ROUNDS>
 __global__ void rs_hist(const int* keys, int n, int shift, int nblocks, int* counts) {
   constexpr int kRsTile = kRsThreads * ROUNDS;
@@ -242,7 +243,7 @@ __global__ void rs_scatter(const int* kin, const int* vin, int* kout, int* vout,
 
 void radix_sort(int* keys, int* vals, int n, int bits, cudaStream_t s) {
   if (n <= 1 || bits <= 0) return;
-  const bool small = n < (1 << 19);
+  const bool small = n < (1 << 18);
   const int tile = kRsThreads * (small ? 2 : 8), nb = (n + tile - 1) / tile;
   TmpBuf<int> k2(s), v2(s), counts(s);
   k2.alloc(n);

@@ -68,9 +68,9 @@ def test_more_slots_than_one_level_of_tile_sums(precision):
     assert np.linalg.norm(pot[1000:2000] - want) <= 1e-3 * np.linalg.norm(want)
 
 
-@pytest.mark.parametrize("n", [1, 511, 512, 513, 2049, 524287, 524288, 600001])
+@pytest.mark.parametrize("n", [1, 511, 512, 513, 2049, 262143, 262144, 524287, 524288, 600001])
 def test_sort_is_stable_at_tile_edges(n):
-    # tiles of 512 keys below 2^19 points, of 2,048 from there on: the permutation is numpy's stable one
+    # tiles of 512 keys below 2^18 points, of 2,048 from there on: the permutation is numpy's stable one
     x = _points(n, n)
     with ob.Plan(kernel=ob.LAPLACE_G, p=2, lmax=4, precision=ob.MIXED, semantics=ob.SEM_ACCURATE, exclude_self=True) as pl:
         pl.set_geometry(x, x, bbox=(0, 0, 0, 1))
