@@ -502,13 +502,18 @@ void build_work_dev(fmmb_plan* pl, bool tc_m2l, cudaStream_t s) {
   }
   radix_sort(skey.get(), sval.get(), n, 30, s);  // stable: leaf order among equal costs
   // One launch of the near field, beside the far field from its start on; two
-  // halves, before and after the M2L, only where the tensor-core M2L, which takes
-  // whole SMs, would have to wait for a long first one.  One instead of two: 32,768
-  // points FP64 (512 items) 257 -> 173 us, 2,000 mixed 49 -> 42, 262,144 clustered
-  // FP64 2.60 -> 2.43 ms, 131,071 mixed (2,989 items) moved and evaluated 1.06 ->
-  // 1.04, 245,760 on a surface mixed (4,626) 0.348 / 0.347, but 1,048,576 clustered
-  // mixed (21,892), forward and backward, 9.70 -> 9.74.
-  const int n0 = tc_m2l && n > (1 << 13) ? (n + 1) / 2 : n;
+  // halves, before and after the M2L, where the tensor-core M2L, which takes whole
+  // SMs, would have to wait for a long first one.  Both sides measured, two against
+  // one (repeats differ by 0.2 %), at 2,744 to 3,375 items (p = 8 to 12, 24 or 64
+  // points a leaf) between 3 % less and 1.6 % more, 2,989 items launched directly
+  // (131,071 points moved and evaluated) 1,072 / 1,055 us; from 4,096 on never more
+  // than 0.5 % more: 4,096 items 493 / 511 us at p = 12, 595 / 593 at p = 10, 4,626
+  // (245,760 points on a surface) 350 / 356, 10,648 at p = 12 1,147 / 1,177, 21,892
+  // (1,048,576 clustered points, forward and backward) 9.69 / 9.74 ms, 32,768 and
+  // more between 1.4 % less and equal.  Without a tensor-core M2L one is better
+  // throughout (32,768 points FP64, 512 items, 257 -> 173 us; 262,144 clustered
+  // points 2.60 -> 2.43 ms).
+  const int n0 = tc_m2l && n >= (1 << 12) ? (n + 1) / 2 : n;
   pl->p2p_work.alloc(std::max(n, 1));
   if (n > 0) {
     deal_items<<<nblk(n, kT), kT, 0, s>>>(n, n0, sval.get(), pl->m_p2p_work.get(), pl->p2p_work.get());

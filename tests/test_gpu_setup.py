@@ -82,6 +82,7 @@ def test_sort_is_stable_at_tile_edges(n):
 
 @pytest.mark.parametrize("kernel,precision,n", [(ob.LAPLACE_G, ob.FP64, 592), (ob.LAPLACE_G, ob.FP64, 593),
                                                 (ob.HELMHOLTZ_G, ob.FP64, 592), (ob.HELMHOLTZ_G, ob.FP64, 593),
+                                                (ob.LAPLACE_G, ob.MIXED, 4095), (ob.LAPLACE_G, ob.MIXED, 4096),
                                                 (ob.LAPLACE_G, ob.MIXED, 8192), (ob.LAPLACE_G, ob.MIXED, 8193),
                                                 (ob.LAPLACE_G, ob.FP64, 8193)])
 def test_near_field_launches_take_every_item_once(kernel, precision, n):
