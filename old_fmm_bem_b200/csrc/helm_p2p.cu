@@ -39,9 +39,11 @@ namespace fmmb {
 namespace {
 
 constexpr int kItem = 128;  // targets of a work item
-// Warps of a block: 4; in the FP64 form 8 where all items are resident at once with
-// 4 (as p2p_f64.cu).  30,011 points (272 leaves): this kernel 0.309 ms with 4,
-// 0.269 with 8, the pass 0.368 / 0.341.
+// Warps of a block: 4; in the FP64 form 8 where all items are resident at once with 4
+// (as p2p_f64.cu).  Whole evaluate with 4 / 8, us, p = 8: 64 points a leaf, 216 items
+// 221 / 177, 512 385 / 360, 729 496 / 505, 1,331 899 / 899, 4,096 2,822 / 2,881; 110 a
+// leaf, 216 items 458 / 366, 512 897 / 703, 729 1,016 / 993, 1,000 1,355 / 1,373, 4,096
+// 5,824 / 5,972.
 constexpr int kFewItems = 4 * 148;
 constexpr int max_warps(bool f32) { return f32 ? 4 : 8; }
 constexpr int kG = 8;        // targets of a group (lanes g = lane % 8)

@@ -39,10 +39,13 @@ namespace {
 
 constexpr int kItem = 128;   // targets of a work item
 constexpr int kMaxWarps = 8;
-// Warps of a block: 4; 8 where all items are resident at once with 4 (4 blocks fit
-// an SM by their registers) and leave the FP64 pipe short of warps.  512 items
-// (32,768 points, depth 3): this kernel 0.115 ms with 4, 0.086 with 8; 262,144
-// clustered points (4,219 items): 2.52 ms a pass with 8, 2.43 with 4.
+// Warps of a block: 4; 8 where all items are resident at once with 4 (4 blocks fit an
+// SM by their registers) and leave the FP64 pipe short of warps.  Whole evaluate
+// with 4 / 8, us: G with gradient, p = 8, 64 points a leaf: 64 items 77 / 63, 343 129 /
+// 124, 512 161 / 166, 729 213 / 221; 128 a leaf: 64 items 169 / 123, 343 311 / 235, 512
+// 377 / 334, 729 455 / 466; Gnj, p = 10, 64 a leaf: 216 items 204 / 105, 512 235 / 194,
+// 729 258 / 258; 24 a leaf within 4 % throughout.  4,219 items (262,144 clustered
+// points) 2.43 / 2.52 ms.
 constexpr int kFewItems = 4 * 148;
 constexpr int kG = 8;        // targets of a group (lanes g = lane % 8)
 constexpr int kS = 32 / kG;  // source streams of a warp (s = lane / 8)
