@@ -354,8 +354,9 @@ def setup_line(plan, npts, ms_step):
 # ------------------------------------------------------------------ our arm
 def phase_rooflines(plan, p, lmax, npts, phase, phase_alone, ms_step, mixed, traffic=None):
     """Rooflines of the two dominant kernels, from their CUDA-event durations
-    in timed steps (phase timers on the launching streams; phase_alone = the
-    same steps with the near field run after the far field):
+    in a step's launches run once more after an L2 flush (phase timers on the
+    launching streams; phase_alone = with the near field run after the far
+    field):
       * p2p_mixed: 20 flops per algorithmic pair (Laplace G: differences 3,
         r^2 6, rsqrt 1, r^-3 2, q r^-1 and q r^-3 2, potential 1, gradient 6;
         Gni/Gnj: the normal dot in place of the gradient); bound by the FP32
@@ -381,7 +382,8 @@ def phase_rooflines(plan, p, lmax, npts, phase, phase_alone, ms_step, mixed, tra
     p2p_ach = 20.0 * st["p2p_pairs"] / (phase_alone[0] * 1e-3) / 1e12
     tc_peak = peaks["bf16_tflops"] if p <= 12 else peaks["bf16_tflops"] / 2  # FP16 / TF32 dense
     fp64_peak = 37.0
-    # FP64 M2L: blocks of (p+1)(p+2)/2 and p(p+1)/2 rows
+    # FP64 M2L: blocks of (p+1)(p+2)/2 and p(p+1)/2 rows; taken by the FP64 form, above p = 15 and, for K <= 169, by
+    # geometries of few box pairs (few_pairs in csrc/api.cpp, whose limit this restates)
     par = not mixed or K > 256 or (K <= 169 and st["m2l_pairs"] * K * K <= 7e8)
     m2l_flops = 2.0 * (((p + 1) * (p + 2) // 2) ** 2 + (p * (p + 1) // 2) ** 2) if par else 2.0 * K * K
     if par:
@@ -393,8 +395,7 @@ def phase_rooflines(plan, p, lmax, npts, phase, phase_alone, ms_step, mixed, tra
                 "ms_in_overlapped_step": float(phase[0]),
                 "note": f"20 flops per algorithmic pair ({st['p2p_pairs']} pairs); ms = the kernel's own launches "
                         f"(near field not overlapped), summed per evaluate; peak = nominal FP32 at "
-                        f"{sm_max:.0f} MHz (no FP32 figure in MEASURED_PEAKS.json); traffic per evaluate (two "
-                        f"launches)"}
+                        f"{sm_max:.0f} MHz (no FP32 figure in MEASURED_PEAKS.json); traffic per evaluate"}
     roof_m2l = {"kernel": "m2l_parity (M2L)" if par else
                 "translate_h16+reduce_pairs (M2L)" if p <= 12 else "translate_tc+reduce_pairs (M2L)",
                 "bound": "fp64 tensor" if par else "tensor",
@@ -471,7 +472,7 @@ def run_ours(args, rank, world, secondary=False):
                 step()
                 ev[k][1].record(stream)
                 stream.synchronize()
-                phase += np.array(list(plan.timings().values()))
+                phase += np.array(list(_phases(plan, stream, flush).values()))
         torch.cuda.synchronize()
     ms = [a.elapsed_time(b) for a, b in ev]
     ms_step = float(np.mean(ms))
@@ -489,7 +490,7 @@ def run_ours(args, rank, world, secondary=False):
             flush.fill_(float(k))
             step()
             stream.synchronize()
-            phase_alone += np.array(list(plan.timings().values()))
+            phase_alone += np.array(list(_phases(plan, stream, flush).values()))
     phase_alone /= args.steps
     plan.set_overlap(True)
     ms_step = max_over_ranks(ms_step, world)
@@ -584,6 +585,15 @@ def _timed(step, stream, steps, warmup, flush, out=None):
     return float(np.mean(ms))
 
 
+def _phases(plan, stream, flush):
+    """Phase times (ms) of the plan's last evaluate from a cold L2: timings()
+    runs its launches once more on the plan's stream, here after a flush."""
+    import torch
+    with torch.cuda.stream(stream):
+        flush.fill_(0.0)
+    return plan.timings()
+
+
 def uniform_cube(n, seed):
     rng = np.random.default_rng(seed)
     return rng.random((3, n), dtype=np.float32), rng.uniform(-1, 1, n).astype(np.float32)
@@ -622,7 +632,7 @@ def run_c1(args):
                       "ms_per_step": ms, "dtype": "f64", "data": "synthetic",
                       "config": {"workload": "Laplace G, 32,768 points U[0,1]^3, q U[-1,1], p=8, lmax=3, FP64, "
                                              "self pairs excluded"},
-                      "rel_err_vs_fp64_direct": err, "phase_ms": plan.timings(), "cpu_baseline": cpu,
+                      "rel_err_vs_fp64_direct": err, "phase_ms": _phases(plan, stream, flush), "cpu_baseline": cpu,
                       "clocks": clk.summary()}))
     plan.close()
 
@@ -675,7 +685,7 @@ def run_headline(args, rank, world):
         torch.cuda.nvtx.range_push("timed")  # the timed steps, for a profiler's launch list
         t_fb = _timed(fwd_bwd, stream, args.steps, max(3, args.warmup), flush, per_step)
         torch.cuda.nvtx.range_pop()
-        ph = np.array(list(op.plan.timings().values()))
+        ph = np.array(list(_phases(op.plan, stream, flush).values()))
         launches = op.plan.stats()["launches"]
     # each kernel's own duration: one evaluate with gradient, near field after
     # the far field (phase timers, CUDA events on the launching streams)
@@ -688,7 +698,7 @@ def run_headline(args, rank, world):
             flush.fill_(float(k))
             fwd()
             stream.synchronize()
-            ph_alone += np.array(list(op.plan.timings().values()))
+            ph_alone += np.array(list(_phases(op.plan, stream, flush).values()))
     ph_alone /= max(3, args.steps // 2)
     op.plan.set_overlap(True)
     t_fb_job = max_over_ranks(t_fb, world)
@@ -1017,7 +1027,7 @@ def run_c5(args):
             dp.close()
             v = pot.cpu().numpy()[sel]
             st = plan.stats()
-            ph = plan.timings()
+            ph = _phases(plan, stream, flush)
             fl = 6 * (((p + 1) * (p + 2) // 2) ** 2 + (p * (p + 1) // 2) ** 2)  # even and odd block, 3 real products
             m2l_tf = fl * st["m2l_pairs"] / (ph["m2l"] * 1e-3) / 1e12
             res[name] = {"lmax": lmax, "autotune_ms": tune, "setup_s": setup_s, "matvec_ms": t_f,
@@ -1093,7 +1103,7 @@ def run_c3_matvec(args):
         plan.evaluate(qd, pot, grad, f64=True)
 
     ms = _timed(step, stream, args.steps, args.warmup, flush)
-    ph = np.array(list(plan.timings().values()))
+    ph = np.array(list(_phases(plan, stream, flush).values()))
     st = plan.stats()
     plan.close()
     print(json.dumps({"metric": "FMM matvec Mpts/s (Laplace G with field, 1,048,576 clustered points, p=12, "
