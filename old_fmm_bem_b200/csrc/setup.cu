@@ -9,7 +9,8 @@
 // allocations wait for; the lists themselves are a few passes over the box slots.
 // Measured on one B200 against M2M / L2L tiles and tree checks on the host, a
 // second sort for the CSR, one atomic per pair or box and a second tree build for
-// a set that is both targets and sources, fmmb_set_geometry: 131,071 clustered
+// a set that is both targets and sources, fmmb_set_geometry called with the same
+// points again, so that no buffer of the plan grows: 131,071 clustered
 // points 2.34 -> 1.00 ms, 1,048,576 13.3 -> 8.8 ms, 100,000 points in reference
 // semantics from host arrays 2.68 -> 0.86 ms.
 //
@@ -289,7 +290,9 @@ bool build_m2l_tiles(fmmb_plan* pl, bool sets, int per, const int* rel_to_op, in
     T.srcoff[l] = pl->off_j[lev];
     T.set[l] = sets ? lev - 2 : 0;
     V += (long long)pl->nbox_i[lev] * kM2LSlots;
-    if (V >= (1LL << 31) - 1) return false;  // the host loops take such sizes
+    // the host loops take such sizes; the last blocks of the kernels and of the scan
+    // (tiles of 4,096) index past V, which must not wrap around
+    if (V >= (1LL << 31) - 8192) return false;
   }
   T.vstart[T.nlev] = (int)V;
   const int nv = (int)V;
