@@ -53,8 +53,9 @@ extern "C" {
                                FMMB_SEM_ACCURATE only. */
 
 /* Precision of the evaluation. */
-#define FMMB_FP64 0   /* every phase in FP64 on the CUDA cores */
-#define FMMB_MIXED 1  /* FP32 P2P with compensated sums, M2L as TF32x3 tensor-core GEMMs */
+#define FMMB_FP64 0   /* every phase in FP64 (translations and P2M by the FP64 tensor instruction) */
+#define FMMB_MIXED 1  /* FP32 P2P, P2M and L2P with FP64 sums; Laplace M2L as FP16x3 (p <= 12) or TF32x3 (p <= 15)
+                         tensor-core GEMMs, in FP64 above, for few box pairs and for the Helmholtz family */
 
 /* Arithmetic semantics. */
 #define FMMB_SEM_REFERENCE 0 /* the reference's conventions: eps=1e-6f added to r^2 and to
@@ -376,8 +377,8 @@ FMMB_API int fmmb_get_stats(fmmb_plan* plan, long long* out8);
 
 /* Wall times (ms) of the last fmmb_set_geometry: [0] the octree build on the
  * GPU (keys, radix sort, levels, lists; it synchronises between levels),
- * [1] the whole call (tree, interaction tiles and work lists built on the
- * host, operator images, buffers). */
+ * [1] the whole call (tree, interaction tiles and work lists, operator images,
+ * buffers). */
 FMMB_API int fmmb_get_setup_times(fmmb_plan* plan, double* ms2);
 
 FMMB_API const char* fmmb_last_error(void);

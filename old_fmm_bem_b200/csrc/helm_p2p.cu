@@ -24,7 +24,7 @@
 //
 // Measured against one or two targets a thread and scalar FP32 (or the library's
 // square root and divisions), this phase alone on one B200: mixed, 1,048,576
-// sphere points, k = 5, depth 5 (3.57 G pairs) 4.65 -> 2.73 ms; FP64, 30,011
+// sphere points, k = 5, depth 5 (3.57 G pairs) 4.65 -> 2.75 ms; FP64, 30,011
 // points, depth 3 (46.8 M pairs, 272 leaves) 1.41 -> 0.27 ms (0.38 with the
 // library's sincos, whose branch keeps a lane's targets one after another).
 #include <cuda_runtime.h>
