@@ -323,8 +323,6 @@ int geometry_impl(fmmb_plan* pl, int nprob, const int* toff, const int* soff, in
       FMMB_REQUIRE(to[0] == 0 && so[0] == 0 && to[nprob] == ni && so[nprob] == nj, FMMB_ERR_ARG,
                    "problem offsets must run from 0 to the point counts");
     }
-    if (pl->phases.state == fmmb_plan::Phases::kPending)  // its charges and work lists go
-      pl->phases.state = fmmb_plan::Phases::kNone;
     for (int w = 0; w < 4; w++) {  // captured evaluates refer to the old buffers
       pl->gused[w] = false;
       if (pl->gexec[w]) {
@@ -354,6 +352,8 @@ int geometry_impl(fmmb_plan* pl, int nprob, const int* toff, const int* soff, in
     cudaStream_t s = pl->st.main;
     pl->have_geometry = false;
     pl->have_expansions = false;
+    if (pl->phases.state == fmmb_plan::Phases::kPending)  // its charges and work lists go
+      pl->phases.state = fmmb_plan::Phases::kNone;
     pl->same_tree = ni == nj && tx == sx && ty == sy && tz == sz && to == so;
     std::vector<TmpBuf<float>> st;
     for (int k = 0; k < 12; k++) st.emplace_back(s);

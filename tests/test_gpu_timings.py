@@ -75,3 +75,12 @@ def test_phases_after_a_new_geometry(read):
         pl.evaluate(q[0])
         now = pl.timings()
         assert all(v > 0 for v in now.values()) and now != before
+
+
+def test_a_refused_geometry_keeps_the_phases():
+    pl, x, q = _case(ob.LAPLACE_G, ob.MIXED, 1)
+    with pl:
+        pl.evaluate(q[0])
+        with pytest.raises(ob.FMMError):
+            pl.set_geometry(x, x, bbox=(0, 0, 0, -1))
+        assert all(v > 0 for v in pl.timings().values())
